@@ -1,177 +1,603 @@
-// Grouped (ragged) matrix products in one persistent launch with a device-side tile
-// scheduler.  `PrimDescriptor::BatchedGemm` (tenferro-prims/src/lib.rs:156-168) covers
-// uniform batches; a table of problems with individual sizes carries the same
-// C = alpha * A * B + beta * C to ragged batches such as 4096 problems with dims drawn
-// from {16, 32, 64, 128}.
+// Grouped (ragged) matrix products in one persistent launch.  `PrimDescriptor::BatchedGemm`
+// (tenferro-prims/src/lib.rs:156-168) covers uniform batches; a table of problems with
+// individual sizes carries the same C = alpha * A * B + beta * C to ragged batches such as the
+// sector blocks of a block-sparse tensor pair.
 //
-// Scheduling: every problem is cut into 32 x 32 output tiles; tiles are numbered over the
-// whole table (a prefix sum per problem) and persistent CTAs draw tile numbers from one
-// atomic ticket.  Nothing waits on anything, so the loop needs no bound.
+// This file holds the kernel for every table the f32 tensor-core kernels decline - double
+// precision, complex, f32 of any size, alignment and strides - and the entry points.
+//
+// Such a table is bound by latency: a block of 40 x 40 x 40 doubles is 38 KB and 0.5 us of one SM's
+// FP64 pipe.  So the kernel is arranged to wait for memory once and not per problem:
+//   * a unit of work is one output tile (64 x 64 real, 32 x 32 complex); the host deals
+//     them out when the table is prepared, longest first, each to the CTA with the least work so
+//     far, so nothing is uploaded, sorted or drawn from a ticket per call;
+//   * a CTA walks its list in 16-deep k stages through a ring of cp.async stages that runs across
+//     units: while one unit is computed and stored the next ones' operands are on their way;
+//   * f64 and Complex64 run on the FP64 tensor pipe (m16n8k8; four real products per complex one, so
+//     that Re and Im each keep their own accuracy), f32 and Complex32 as FMAs (exact products);
+//   * the four warps tile a unit as 2 x 2, 4 x 1 or 1 x 4 fragment blocks, whichever leaves the
+//     least padding, and dead blocks are not issued.
+// Measured against one thread-per-output tile drawn from an atomic ticket, the table uploaded per call:
+// 1024 f64 blocks with sides 4 .. 160 (41 MB, 128 MFLOP, floor 6 us of HBM) 159 -> 30 us a run, 3000 of
+// them 440 -> 88 us, f32 with such sides 183 -> 64 us; one-shot calls 122 -> 119 us (1024), 67 -> 58 us
+// (64).  What is left is latency: a third of the CTAs' time waits for the longest blocks' stages.
 #include <algorithm>
 
 #include "common.h"
+#include "contract_common.cuh"
 #include "scalar_ops.cuh"
 
 namespace tfb {
 
+namespace {
+
+constexpr int kGroupThreads = 128;
+constexpr int kGroupK = 16;     // depth of a stage
+constexpr int kGroupRecs = 16;  // unit records a CTA holds in shared memory
+
+// One output tile of one problem: pointers already moved to the tile's corner.
+struct __align__(16) GroupUnit {
+    const char* a;
+    const char* b;
+    char* c;
+    int64_t a_rs, a_cs, b_rs, b_cs, c_rs, c_cs;  // elements
+    int64_t k;
+    uint16_t mt, nt;
+    // bits 0-1: log2(warp rows); 2-3: 16-row blocks per warp; 4-7: 8-column blocks per warp (the
+    // tensor-pipe forms); kAFast / kBFast: the shared tile is k-fast; kAVec / kBVec: 16-byte chunks
+    uint32_t shape;
+};
+constexpr uint32_t kAFast = 1u << 8, kBFast = 1u << 9, kAVec = 1u << 10, kBVec = 1u << 11;
+constexpr int kGroupRecChunks = (int)sizeof(GroupUnit) / 16;
+static_assert(sizeof(GroupUnit) % 16 == 0, "records travel as 16-byte chunks");
+
+// Shared tiles are [row][PK] (k fast) or [k][PM] (row fast), following the operand's unit stride.  The
+// pitches keep a fragment read (half a warp of 8-byte, a quarter of 16-byte accesses) on distinct
+// banks.  CTAS x STAGES x tile fill an SM's shared memory.
+template <typename T>
+struct GroupCfg;
+template <> struct GroupCfg<double>  { static constexpr int TILE = 64, PK = 20, PM = 68, STAGES = 3, CTAS = 3, NI = 2, NJ = 4; };
+template <> struct GroupCfg<double2> { static constexpr int TILE = 32, PK = 20, PM = 34, STAGES = 3, CTAS = 3, NI = 2, NJ = 2; };
+template <> struct GroupCfg<float>   { static constexpr int TILE = 64, PK = 20, PM = 68, STAGES = 4, CTAS = 4, NI = 4, NJ = 8; };
+template <> struct GroupCfg<float2>  { static constexpr int TILE = 32, PK = 20, PM = 36, STAGES = 4, CTAS = 4, NI = 2, NJ = 4; };
+template <typename T>
+struct GroupSmem {
+    using Cfg = GroupCfg<T>;
+    static constexpr int KFAST = Cfg::TILE * Cfg::PK, MFAST = kGroupK * Cfg::PM;
+    static constexpr int ELEMS = KFAST > MFAST ? KFAST : MFAST;  // of one operand
+    static constexpr int STAGE = 2 * ELEMS * (int)sizeof(T);
+    static constexpr int RECS = kGroupRecs * (int)sizeof(GroupUnit);
+    static constexpr int BYTES = RECS + Cfg::STAGES * STAGE;
+};
+
 struct GroupedArgs {
-    const tfb_gemm_problem* problems;  // device copy
-    const int64_t* tile_prefix;        // [n + 1] tiles before problem p
-    int64_t n_problems, total_tiles;
-    unsigned long long* ticket;
+    const GroupUnit* units;  // CTA c owns units[starts[c]] .. units[starts[c + 1])
+    const int* starts;
     double alpha_re, alpha_im, beta_re, beta_im;
 };
 
-constexpr int GT = 32, GK = 16;
+__device__ __forceinline__ void cp_async_part(uint32_t dst, const void* src, int bytes16) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes16));
+}
+template <int ES>
+__device__ __forceinline__ void cp_async_one(uint32_t dst, const void* src, int bytes) {
+    if constexpr (ES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
+    else if constexpr (ES == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
+}
 
+// One operand's part of a stage: `rows` rows (row stride rs), k from `src` on (stride ks), `kv` <= 16 of
+// them live.  What lies past a live k is filled with zeros up to the next multiple of 8, which is
+// as far as the arithmetic reads; rows past the live ones may hold anything, nothing stored
+// depends on them (V > 1: a chunk's dead part is zero-filled).
+template <typename T, int V>
+__device__ __forceinline__ void load_operand(uint32_t dst, const T* src, int64_t rs, int64_t ks, int rows, int kv, bool kfast,
+                                             int tid) {
+    using Cfg = GroupCfg<T>;
+    constexpr int ES = (int)sizeof(T);
+    const int kr = (kv + 7) & ~7;
+    if (kfast) {
+        constexpr int KC = kGroupK / V;
+        const int k = (tid % KC) * V;
+        if (k >= kr) return;
+        const int live = min(max(kv - k, 0), V) * ES;
+        const T* p = src + (live ? (int64_t)k * ks : 0) + (int64_t)(tid / KC) * rs;
+        uint32_t d = dst + ((tid / KC) * Cfg::PK + k) * ES;
+        for (int r = tid / KC; r < rows; r += kGroupThreads / KC) {
+            if constexpr (V == 1) cp_async_one<ES>(d, p, live);
+            else cp_async_part(d, p, live);
+            p += (kGroupThreads / KC) * rs;
+            d += (kGroupThreads / KC) * Cfg::PK * ES;
+        }
+    } else {
+        // a power-of-two group of threads along the rows
+        const int chunks = (rows + V - 1) / V;
+        int lg = 2;
+        while ((1 << lg) < chunks) ++lg;
+        const int x = tid & ((1 << lg) - 1), step = kGroupThreads >> lg;
+        if (x >= chunks) return;
+        const int live = min(rows - x * V, V) * ES;
+        int k = tid >> lg;
+        const T* p = src + (int64_t)x * V * rs + (int64_t)k * ks;
+        uint32_t d = dst + (k * Cfg::PM + x * V) * ES;
+        for (; k < kr; k += step) {
+            const bool ok = k < kv;
+            if constexpr (V == 1) cp_async_one<ES>(d, ok ? p : src, ok ? live : 0);
+            else cp_async_part(d, ok ? p : src, ok ? live : 0);
+            p += step * ks;
+            d += step * Cfg::PM * ES;
+        }
+    }
+}
+
+__device__ __forceinline__ void group_dmma(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+// Runs CALL(NI, NJ) with the live block counts as compile-time constants: a small unit then issues
+// only its own instructions.
+#define TFB_GROUP_CASE(I, J, CALL) \
+    if constexpr ((I) <= Cfg::NI && (J) <= Cfg::NJ) { if (ni == (I) && nj == (J)) { CALL(I, J); return; } }
+
+// The FP64 tensor pipe.  Fragment numbering of m16n8k8: A rows g and g + 8, k = t and t + 4; C columns 2t, 2t + 1.
 template <typename T>
-__global__ void __launch_bounds__(64) grouped_simt_kernel(GroupedArgs g) {
-    __shared__ T As[GK][GT + 1];
-    __shared__ T Bs[GK][GT + 1];
-    __shared__ long long s_tile;
-    const int tid = threadIdx.x;
-    const int tx = tid & 7, ty = tid >> 3;  // 8 x 8 threads, 4 x 4 outputs each
-    const T alpha = Ops<T>::from(Scalar{g.alpha_re, g.alpha_im});
-    const T beta = Ops<T>::from(Scalar{g.beta_re, g.beta_im});
-    const bool read_c = g.beta_re != 0 || g.beta_im != 0;
-    for (;;) {
-        if (tid == 0) s_tile = (long long)atomicAdd(g.ticket, 1ull);
-        __syncthreads();
-        const int64_t tile = s_tile;
-        __syncthreads();
-        if (tile >= g.total_tiles) break;
-        // Problem of this tile: last p with tile_prefix[p] <= tile.
-        int64_t lo = 0, hi = g.n_problems;
-        while (hi - lo > 1) {
-            int64_t mid = (lo + hi) >> 1;
-            if (g.tile_prefix[mid] <= tile) lo = mid; else hi = mid;
-        }
-        const tfb_gemm_problem pr = g.problems[lo];
-        const int64_t local = tile - g.tile_prefix[lo];
-        const int64_t tiles_m = (pr.m + GT - 1) / GT;
-        const int64_t m0 = (local % tiles_m) * GT, n0 = (local / tiles_m) * GT;
-        const T* A = (const T*)pr.a;
-        const T* B = (const T*)pr.b;
-        T* C = (T*)pr.c;
-        // Threads follow whichever direction of each operand has the smaller stride.
-        const bool a_kfast = llabs(pr.a_cs) < llabs(pr.a_rs), b_kfast = llabs(pr.b_rs) < llabs(pr.b_cs);
-        T acc[4][4];
+struct TensorPath {
+    using Cfg = GroupCfg<T>;
+    static constexpr bool CPLX = Ops<T>::is_complex;
+    static constexpr int W = CPLX ? 2 : 1;
+    double acc[Cfg::NI][Cfg::NJ][W][4];
+    int wm, wn, ni, nj;
+
+    __device__ __forceinline__ void begin(const GroupUnit& u, int tid) {
+        const int warp = tid >> 5;
+        const int lw = u.shape & 3, pi = (u.shape >> 2) & 3, pj = (u.shape >> 4) & 15;
+        wm = (warp & ((1 << lw) - 1)) * 16 * pi;
+        wn = (warp >> lw) * 8 * pj;
+        ni = max(0, min(pi, ((int)u.mt - wm + 15) / 16));
+        nj = max(0, min(pj, ((int)u.nt - wn + 7) / 8));
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < Cfg::NI; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = Ops<T>::zero();
-        for (int64_t k0 = 0; k0 < pr.k; k0 += GK) {
+            for (int j = 0; j < Cfg::NJ; ++j)
 #pragma unroll
-            for (int r = 0; r < GT * GK / 64; ++r) {
-                int c = tid + r * 64;
-                int mm, kk;
-                if (a_kfast) { kk = c % GK; mm = c / GK; } else { mm = c % GT; kk = c / GT; }
-                T v = Ops<T>::zero();
-                if (m0 + mm < pr.m && k0 + kk < pr.k) v = A[(m0 + mm) * pr.a_rs + (k0 + kk) * pr.a_cs];
-                As[kk][mm] = v;
-                int nn;
-                if (b_kfast) { kk = c % GK; nn = c / GK; } else { nn = c % GT; kk = c / GT; }
-                T w = Ops<T>::zero();
-                if (n0 + nn < pr.n && k0 + kk < pr.k) w = B[(k0 + kk) * pr.b_rs + (n0 + nn) * pr.b_cs];
-                Bs[kk][nn] = w;
+                for (int w = 0; w < W; ++w)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[i][j][w][e] = 0.0;
+    }
+    template <int NI, int NJ>
+    __device__ __forceinline__ void stage_t(const T* As, const T* Bs, int a_sm, int a_sk, int b_sn, int b_sk, int steps, int tid) {
+        const int g = (tid & 31) >> 2, t = tid & 3;
+        const T* pa = As + (wm + g) * a_sm + t * a_sk;
+        const T* pb = Bs + (wn + g) * b_sn + t * b_sk;
+        for (int s = 0; s < steps; ++s, pa += 8 * a_sk, pb += 8 * b_sk) {
+            T av[NI][4], bv[NJ][2];
+#pragma unroll
+            for (int i = 0; i < NI; ++i)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) av[i][e] = pa[(16 * i + 8 * (e & 1)) * a_sm + 4 * (e >> 1) * a_sk];
+#pragma unroll
+            for (int j = 0; j < NJ; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) bv[j][e] = pb[8 * j * b_sn + 4 * e * b_sk];
+            if constexpr (CPLX) {
+                double ar[NI][4], ai[NI][4], an[NI][4], br[NJ][2], bi[NJ][2];
+#pragma unroll
+                for (int i = 0; i < NI; ++i)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) { ar[i][e] = av[i][e].x; ai[i][e] = av[i][e].y; an[i][e] = -av[i][e].y; }
+#pragma unroll
+                for (int j = 0; j < NJ; ++j)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) { br[j][e] = bv[j][e].x; bi[j][e] = bv[j][e].y; }
+#pragma unroll
+                for (int i = 0; i < NI; ++i)
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j) { group_dmma(acc[i][j][0], ar[i], br[j]); group_dmma(acc[i][j][1], ar[i], bi[j]); }
+#pragma unroll
+                for (int i = 0; i < NI; ++i)
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j) { group_dmma(acc[i][j][0], an[i], bi[j]); group_dmma(acc[i][j][1], ai[i], br[j]); }
+            } else {
+#pragma unroll
+                for (int i = 0; i < NI; ++i)
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j) group_dmma(acc[i][j][0], av[i], bv[j]);
             }
-            __syncthreads();
-#pragma unroll
-            for (int kk = 0; kk < GK; ++kk) {
-                T av[4], bv[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) av[i] = As[kk][tx + 8 * i];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][ty + 8 * j];
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] = Ops<T>::fma_(av[i], bv[j], acc[i][j]);
-            }
-            __syncthreads();
         }
+    }
+    __device__ __forceinline__ void stage(const T* As, const T* Bs, int a_sm, int a_sk, int b_sn, int b_sk, int kv, int tid) {
+        const int steps = (kv + 7) >> 3;
+#define TFB_CALL(I, J) stage_t<I, J>(As, Bs, a_sm, a_sk, b_sn, b_sk, steps, tid)
+        TFB_GROUP_CASE(1, 1, TFB_CALL) TFB_GROUP_CASE(1, 2, TFB_CALL) TFB_GROUP_CASE(1, 3, TFB_CALL) TFB_GROUP_CASE(1, 4, TFB_CALL)
+        TFB_GROUP_CASE(2, 1, TFB_CALL) TFB_GROUP_CASE(2, 2, TFB_CALL) TFB_GROUP_CASE(2, 3, TFB_CALL) TFB_GROUP_CASE(2, 4, TFB_CALL)
+#undef TFB_CALL
+    }
+    __device__ __forceinline__ void store(const GroupUnit& u, T alpha, T beta, bool read_c, int tid) {
+        const int g = (tid & 31) >> 2, t = tid & 3;
+        T* C = reinterpret_cast<T*>(u.c);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int64_t n = n0 + ty + 8 * j;
-            if (n >= pr.n) continue;
+        for (int i = 0; i < Cfg::NI; ++i)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int64_t m = m0 + tx + 8 * i;
-                if (m >= pr.m) continue;
-                T* p = C + m * pr.c_rs + n * pr.c_cs;
+            for (int j = 0; j < Cfg::NJ; ++j) {
+                if (i >= ni || j >= nj) continue;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int m = wm + 16 * i + 8 * (e >> 1) + g, n = wn + 8 * j + 2 * t + (e & 1);
+                    if (m >= u.mt || n >= u.nt) continue;
+                    T* p = C + m * u.c_rs + n * u.c_cs;
+                    T x;
+                    if constexpr (CPLX) x = make_double2(acc[i][j][0][e], acc[i][j][1][e]);
+                    else x = acc[i][j][0][e];
+                    T v = Ops<T>::mul(alpha, x);
+                    if (read_c) v = Ops<T>::add(v, Ops<T>::mul(beta, *p));
+                    *p = v;
+                }
+            }
+    }
+};
+
+// FMAs: 16 x 8 threads, rows tx + 16 i, columns ty + 8 j.
+template <typename T>
+struct FmaPath {
+    using Cfg = GroupCfg<T>;
+    T acc[Cfg::NI][Cfg::NJ];
+    int ni, nj;
+
+    __device__ __forceinline__ void begin(const GroupUnit& u, int) {
+        // block counts rounded up to powers of two: nine forms instead of thirty-two
+        ni = u.mt <= 16 ? 1 : u.mt <= 32 ? 2 : 4;
+        nj = u.nt <= 8 ? 1 : u.nt <= 16 ? 2 : u.nt <= 32 ? 4 : 8;
+#pragma unroll
+        for (int i = 0; i < Cfg::NI; ++i)
+#pragma unroll
+            for (int j = 0; j < Cfg::NJ; ++j) acc[i][j] = Ops<T>::zero();
+    }
+    template <int NI, int NJ>
+    __device__ __forceinline__ void stage_t(const T* As, const T* Bs, int a_sm, int a_sk, int b_sn, int b_sk, int kr, int tid) {
+        const T* pa = As + (tid & 15) * a_sm;
+        const T* pb = Bs + (tid >> 4) * b_sn;
+#pragma unroll 4
+        for (int k = 0; k < kr; ++k, pa += a_sk, pb += b_sk) {
+            T av[NI], bv[NJ];
+#pragma unroll
+            for (int i = 0; i < NI; ++i) av[i] = pa[16 * i * a_sm];
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) bv[j] = pb[8 * j * b_sn];
+#pragma unroll
+            for (int i = 0; i < NI; ++i)
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) acc[i][j] = Ops<T>::fma_(av[i], bv[j], acc[i][j]);
+        }
+    }
+    __device__ __forceinline__ void stage(const T* As, const T* Bs, int a_sm, int a_sk, int b_sn, int b_sk, int kv, int tid) {
+        const int kr = (kv + 3) & ~3;
+#define TFB_CALL(I, J) stage_t<I, J>(As, Bs, a_sm, a_sk, b_sn, b_sk, kr, tid)
+        TFB_GROUP_CASE(1, 1, TFB_CALL) TFB_GROUP_CASE(1, 2, TFB_CALL) TFB_GROUP_CASE(1, 4, TFB_CALL) TFB_GROUP_CASE(1, 8, TFB_CALL)
+        TFB_GROUP_CASE(2, 1, TFB_CALL) TFB_GROUP_CASE(2, 2, TFB_CALL) TFB_GROUP_CASE(2, 4, TFB_CALL) TFB_GROUP_CASE(2, 8, TFB_CALL)
+        TFB_GROUP_CASE(4, 1, TFB_CALL) TFB_GROUP_CASE(4, 2, TFB_CALL) TFB_GROUP_CASE(4, 4, TFB_CALL) TFB_GROUP_CASE(4, 8, TFB_CALL)
+#undef TFB_CALL
+    }
+    __device__ __forceinline__ void store(const GroupUnit& u, T alpha, T beta, bool read_c, int tid) {
+        T* C = reinterpret_cast<T*>(u.c);
+        const int tx = tid & 15, ty = tid >> 4;
+#pragma unroll
+        for (int j = 0; j < Cfg::NJ; ++j) {
+            const int n = ty + 8 * j;
+            if (n >= u.nt) continue;
+#pragma unroll
+            for (int i = 0; i < Cfg::NI; ++i) {
+                const int m = tx + 16 * i;
+                if (m >= u.mt) continue;
+                T* p = C + m * u.c_rs + n * u.c_cs;
                 T v = Ops<T>::mul(alpha, acc[i][j]);
                 if (read_c) v = Ops<T>::add(v, Ops<T>::mul(beta, *p));
                 *p = v;
             }
         }
     }
+};
+#undef TFB_GROUP_CASE
+
+template <typename T, typename Path>
+__global__ void __launch_bounds__(kGroupThreads, GroupCfg<T>::CTAS) grouped_units_kernel(GroupedArgs g) {
+    using Cfg = GroupCfg<T>;
+    using Sm = GroupSmem<T>;
+    constexpr int S = Cfg::STAGES;
+    extern __shared__ __align__(16) char group_smem[];
+    const GroupUnit* recs = reinterpret_cast<const GroupUnit*>(group_smem);
+    const uint32_t rec_addr = (uint32_t)__cvta_generic_to_shared(group_smem), ring_addr = rec_addr + Sm::RECS;
+    const int tid = threadIdx.x;
+    const int first = g.starts[blockIdx.x], n_units = g.starts[blockIdx.x + 1] - first;
+    if (n_units <= 0) return;
+    const char* table = reinterpret_cast<const char*>(g.units + first);
+    for (int c = tid; c < min(n_units, kGroupRecs) * kGroupRecChunks; c += kGroupThreads)
+        cp_async_part(rec_addr + 16 * c, table + 16 * c, 16);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+
+    // The next stage to request: unit pu, from k = pk on.  At most S - 1 units ahead of the unit being
+    // computed, so its record is in the shared window of kGroupRecs.
+    int pu = 0;
+    int64_t pk = 0;
+    auto request = [&](int slot) {
+        if (pu < n_units) {
+            const GroupUnit& u = recs[pu % kGroupRecs];
+            const int kv = (int)min((int64_t)kGroupK, u.k - pk);
+            const uint32_t da = ring_addr + slot * Sm::STAGE, db = da + Sm::ELEMS * (int)sizeof(T);
+            const T* a = reinterpret_cast<const T*>(u.a) + pk * u.a_cs;
+            const T* b = reinterpret_cast<const T*>(u.b) + pk * u.b_rs;
+            constexpr int V = 16 / (int)sizeof(T);
+            if (V > 1 && (u.shape & kAVec)) load_operand<T, V>(da, a, u.a_rs, u.a_cs, u.mt, kv, u.shape & kAFast, tid);
+            else load_operand<T, 1>(da, a, u.a_rs, u.a_cs, u.mt, kv, u.shape & kAFast, tid);
+            if (V > 1 && (u.shape & kBVec)) load_operand<T, V>(db, b, u.b_cs, u.b_rs, u.nt, kv, u.shape & kBFast, tid);
+            else load_operand<T, 1>(db, b, u.b_cs, u.b_rs, u.nt, kv, u.shape & kBFast, tid);
+            pk += kGroupK;
+            if (pk >= u.k) {
+                pk = 0;
+                ++pu;
+            }
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < S - 1; ++s) request(s);
+
+    const T alpha = Ops<T>::from(Scalar{g.alpha_re, g.alpha_im}), beta = Ops<T>::from(Scalar{g.beta_re, g.beta_im});
+    const bool read_c = g.beta_re != 0 || g.beta_im != 0;
+    Path path;
+    int slot = 0, next_slot = S - 1;
+    for (int cu = 0; cu < n_units; ++cu) {
+        const GroupUnit& u = recs[cu % kGroupRecs];
+        const int64_t K = u.k;
+        const int a_sm = u.shape & kAFast ? Cfg::PK : 1, a_sk = u.shape & kAFast ? 1 : Cfg::PM;
+        const int b_sn = u.shape & kBFast ? Cfg::PK : 1, b_sk = u.shape & kBFast ? 1 : Cfg::PM;
+        path.begin(u, tid);
+        int64_t k0 = 0;
+        do {
+            cp_async_wait<S - 2>();
+            __syncthreads();
+            if (k0 == 0 && cu > 0 && cu - 1 + kGroupRecs < n_units && tid < kGroupRecChunks)
+                // every thread has left the unit before: its record makes room (lands with the stage below)
+                cp_async_part(rec_addr + ((cu - 1) % kGroupRecs) * (int)sizeof(GroupUnit) + 16 * tid,
+                              table + (int64_t)(cu - 1 + kGroupRecs) * sizeof(GroupUnit) + 16 * tid, 16);
+            request(next_slot);
+            __syncwarp();  // the requests' branches end here: the MMAs below need whole warps
+            const T* As = reinterpret_cast<const T*>(group_smem + Sm::RECS + slot * Sm::STAGE);
+            path.stage(As, As + Sm::ELEMS, a_sm, a_sk, b_sn, b_sk, (int)min((int64_t)kGroupK, K - k0), tid);
+            if (++slot == S) slot = 0;
+            if (++next_slot == S) next_slot = 0;
+            k0 += kGroupK;
+        } while (k0 < K);
+        path.store(u, alpha, beta, read_c, tid);
+    }
+    cp_async_wait<0>();
 }
 
-tfb_status grouped_simt(tfb_ctx* ctx, int dtype, size_t n, const tfb_gemm_problem* problems, Scalar alpha, Scalar beta) {
-    if (n == 0) return TFB_OK;
-    std::vector<int64_t> prefix(n + 1, 0);
+// The CTAs' unit lists of one table, on the device.
+struct GroupedUnits {
+    PoolBlock mem;
+    size_t starts_at = 0;
+    int grid = 0;
+};
+
+tfb_status check_table(size_t n, const tfb_gemm_problem* problems) {
     for (size_t p = 0; p < n; ++p) {
         const auto& q = problems[p];
         if (q.m < 0 || q.n < 0 || q.k < 0) return fail(TFB_ERR_INVALID_ARGUMENT, "problem %zu has a negative size", p);
         if (q.m > 0 && q.n > 0 && (!q.c || (q.k > 0 && (!q.a || !q.b))))
             return fail(TFB_ERR_INVALID_ARGUMENT, "problem %zu has a NULL pointer", p);
-        prefix[p + 1] = prefix[p] + ((q.m + GT - 1) / GT) * ((q.n + GT - 1) / GT);
     }
-    const int64_t total = prefix[n];
-    if (total == 0) return TFB_OK;
-    // One scratch block: problems | prefix | ticket.
-    const size_t bytes_p = n * sizeof(tfb_gemm_problem), bytes_x = (n + 1) * sizeof(int64_t);
-    PoolBlock ws;
-    TFB_TRY(ws.alloc(ctx, bytes_p + bytes_x + 16));
-    char* d = (char*)ws.ptr;
-    TFB_CUDA(cudaMemcpyAsync(d, problems, bytes_p, cudaMemcpyHostToDevice, ctx->stream));
-    TFB_CUDA(cudaMemcpyAsync(d + bytes_p, prefix.data(), bytes_x, cudaMemcpyHostToDevice, ctx->stream));
-    TFB_CUDA(cudaMemsetAsync(d + bytes_p + bytes_x, 0, 16, ctx->stream));
-    // The host vectors above are pageable: the copies have been staged by the time the calls return.
-    GroupedArgs g;
-    g.problems = (const tfb_gemm_problem*)d;
-    g.tile_prefix = (const int64_t*)(d + bytes_p);
-    g.ticket = (unsigned long long*)(d + bytes_p + bytes_x);
-    g.n_problems = (int64_t)n;
-    g.total_tiles = total;
-    g.alpha_re = alpha.re; g.alpha_im = alpha.im; g.beta_re = beta.re; g.beta_im = beta.im;
-    const int grid = (int)std::min<int64_t>(total, (int64_t)ctx->sm_count * 16);
-    LaunchScope ls(ctx, "grouped_simt");
-    switch (dtype) {
-        case TFB_F32: grouped_simt_kernel<float><<<grid, 64, 0, ctx->stream>>>(g); break;
-        case TFB_F64: grouped_simt_kernel<double><<<grid, 64, 0, ctx->stream>>>(g); break;
-        case TFB_C32: grouped_simt_kernel<float2><<<grid, 64, 0, ctx->stream>>>(g); break;
-        case TFB_C64: grouped_simt_kernel<double2><<<grid, 64, 0, ctx->stream>>>(g); break;
-        default: return fail(TFB_ERR_INVALID_ARGUMENT, "unknown dtype %d", dtype);
+    return TFB_OK;
+}
+
+// Host buffers of the layout below, kept per thread: a one-shot call would spend as long faulting fresh
+// pages in as on the layout itself.  Given back above kKeep bytes.
+struct LayoutScratch {
+    struct Key { uint32_t cost, problem, m_tile, n_tile; uint16_t mt, nt; uint32_t split; };
+    static constexpr size_t kKeep = (size_t)4 << 20;
+    std::vector<Key> keys;
+    std::vector<uint32_t> order, owner;
+    std::vector<char> table;
+    void trim() {
+        if (table.capacity() > kKeep) std::vector<char>().swap(table);
+        if (keys.capacity() * sizeof(Key) > kKeep) {
+            std::vector<Key>().swap(keys);
+            std::vector<uint32_t>().swap(order);
+            std::vector<uint32_t>().swap(owner);
+        }
     }
+};
+
+// How the four warps tile a unit of mt x nt: the split with the fewest MMAs for the slowest warp.
+template <typename Cfg>
+uint32_t warp_split(int mt, int nt, int* mmas) {
+    const int rows16 = (mt + 15) / 16, cols8 = (nt + 7) / 8;
+    int lw = 1, ni = (rows16 + 1) / 2, nj = (cols8 + 1) / 2;
+    for (int w = 0; w <= 2; w += 2) {  // 1 x 4 and 4 x 1 warps
+        const int i = (rows16 + (1 << w) - 1) >> w, j = (cols8 + (4 >> w) - 1) >> (2 - w);
+        if (i <= Cfg::NI && j <= Cfg::NJ && i * j < ni * nj) { lw = w; ni = i; nj = j; }
+    }
+    *mmas = ni * nj;
+    return (uint32_t)(lw | (ni << 2) | (nj << 4));
+}
+
+// `balance`: a plan that will run again is worth a closer balance (1024 f64 blocks: 29 us a run against 34
+// with the units dealt back and forth) and twice the time on the host.
+template <typename T>
+tfb_status lay_out_units(tfb_ctx* ctx, size_t n, const tfb_gemm_problem* problems, bool balance, GroupedUnits* out) {
+    using Cfg = GroupCfg<T>;
+    constexpr int64_t TILE = Cfg::TILE, ES = sizeof(T), V = 16 / ES;
+    static thread_local LayoutScratch scratch;
+    auto& keys = scratch.keys;
+    keys.clear();
+    // Costs, in units of half an m16n8k8 of the slowest warp: the arithmetic, a stage's requests and
+    // barrier, and what a unit costs whatever its size.  Bucketed with an eighth's resolution.
+    auto bucket = [](uint64_t c) -> uint32_t {
+        if (c < 8) return (uint32_t)c;
+        const int e = 63 - __builtin_clzll(c);
+        return std::min<uint32_t>(255, (uint32_t)(e - 2) * 8 + (uint32_t)(c >> (e - 3) & 7));
+    };
+    uint32_t count[256] = {0};
+    for (size_t p = 0; p < n; ++p) {
+        const auto& q = problems[p];
+        if (q.m <= 0 || q.n <= 0) continue;
+        const int64_t tm = (q.m + TILE - 1) / TILE, tn = (q.n + TILE - 1) / TILE, steps = (q.k + 7) / 8;
+        const int64_t stages = std::max<int64_t>(1, (q.k + kGroupK - 1) / kGroupK);
+        if (keys.size() + (size_t)tm * (size_t)tn >= (size_t)INT32_MAX || p > UINT32_MAX)
+            return fail(TFB_ERR_INVALID_ARGUMENT, "the table has too many output tiles");
+        for (int64_t tj = 0; tj < tn; ++tj)
+            for (int64_t ti = 0; ti < tm; ++ti) {
+                const int mt = (int)std::min(TILE, q.m - ti * TILE), nt = (int)std::min(TILE, q.n - tj * TILE);
+                int mmas;
+                const uint32_t split = warp_split<Cfg>(mt, nt, &mmas);
+                const uint64_t cost = (uint64_t)(steps * mmas * 2 + stages * (8 + (mt + nt) / 8) + 16 + mmas * 2);
+                ++count[bucket(cost)];
+                keys.push_back({(uint32_t)std::min<uint64_t>(cost, UINT32_MAX), (uint32_t)p, (uint32_t)ti, (uint32_t)tj, (uint16_t)mt,
+                                (uint16_t)nt, split});
+            }
+    }
+    out->grid = 0;
+    const size_t n_units = keys.size();
+    if (n_units == 0) return TFB_OK;
+    // longest first
+    uint32_t at[256], sum = 0;
+    for (int c = 255; c >= 0; --c) { at[c] = sum; sum += count[c]; }
+    auto& order = scratch.order;
+    auto& owner = scratch.owner;
+    order.resize(n_units);
+    owner.resize(n_units);
+    for (size_t i = 0; i < n_units; ++i) order[at[bucket(keys[i].cost)]++] = (uint32_t)i;
+    const size_t grid = std::min<size_t>(n_units, (size_t)ctx->sm_count * Cfg::CTAS);
+    std::vector<int> starts(grid + 1, 0);
+    if (balance) {
+        // each to the CTA with the least work so far: the top of a heap of work << 16 | CTA
+        std::vector<uint64_t> heap(grid);
+        for (size_t c = 0; c < grid; ++c) heap[c] = c;
+        for (size_t i = 0; i < n_units; ++i) {
+            owner[i] = (uint32_t)(heap[0] & 0xffff);
+            const uint64_t top = heap[0] + ((uint64_t)keys[order[i]].cost << 16);
+            size_t h = 0;
+            for (size_t child; (child = 2 * h + 1) < grid; h = child) {
+                child += child + 1 < grid && heap[child + 1] < heap[child];
+                if (heap[child] >= top) break;
+                heap[h] = heap[child];
+            }
+            heap[h] = top;
+        }
+    } else {
+        for (size_t i = 0, c = 0, band = 0; i < n_units; ++i) {
+            owner[i] = (uint32_t)(band & 1 ? grid - 1 - c : c);
+            if (++c == grid) { c = 0; ++band; }
+        }
+    }
+    for (size_t i = 0; i < n_units; ++i) ++starts[owner[i] + 1];
+    for (size_t c = 0; c < grid; ++c) starts[c + 1] += starts[c];
+    const size_t unit_bytes = n_units * sizeof(GroupUnit), bytes = unit_bytes + starts.size() * sizeof(int);
+    if (scratch.table.size() < bytes) scratch.table.resize(bytes);
+    char* table = scratch.table.data();
+    memcpy(table + unit_bytes, starts.data(), starts.size() * sizeof(int));
+    GroupUnit* dealt = reinterpret_cast<GroupUnit*>(table);
+    for (size_t i = 0; i < n_units; ++i) {
+        const auto& key = keys[order[i]];
+        const auto& q = problems[key.problem];
+        const int64_t m0 = key.m_tile * TILE, n0 = key.n_tile * TILE;
+        GroupUnit& u = dealt[starts[owner[i]]++];
+        u.a = (const char*)q.a + m0 * q.a_rs * ES;
+        u.b = (const char*)q.b + n0 * q.b_cs * ES;
+        u.c = (char*)q.c + (m0 * q.c_rs + n0 * q.c_cs) * ES;
+        u.a_rs = q.a_rs; u.a_cs = q.a_cs; u.b_rs = q.b_rs; u.b_cs = q.b_cs; u.c_rs = q.c_rs; u.c_cs = q.c_cs;
+        u.k = q.k;
+        u.mt = key.mt;
+        u.nt = key.nt;
+        auto vec = [&](const void* base, int64_t unit, int64_t other) {
+            return V > 1 && unit == 1 && other % V == 0 && (uintptr_t)base % 16 == 0;
+        };
+        u.shape = key.split;
+        // the shared tile follows whichever direction of the operand has the smaller stride
+        if (std::llabs(q.a_cs) < std::llabs(q.a_rs)) u.shape |= kAFast | (vec(q.a, q.a_cs, q.a_rs) ? kAVec : 0);
+        else u.shape |= vec(q.a, q.a_rs, q.a_cs) ? kAVec : 0;
+        if (std::llabs(q.b_rs) < std::llabs(q.b_cs)) u.shape |= kBFast | (vec(q.b, q.b_rs, q.b_cs) ? kBVec : 0);
+        else u.shape |= vec(q.b, q.b_cs, q.b_rs) ? kBVec : 0;
+    }
+    TFB_TRY(out->mem.alloc(ctx, bytes));
+    // Pageable source: the copy has been staged by the time the call returns.
+    TFB_CUDA(cudaMemcpyAsync(out->mem.ptr, table, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    scratch.trim();
+    out->starts_at = unit_bytes;
+    out->grid = (int)grid;
+    return TFB_OK;
+}
+
+template <typename T, typename Path>
+tfb_status launch_units(tfb_ctx* ctx, const GroupedUnits& f, Scalar alpha, Scalar beta, const char* name) {
+    static std::mutex mu;
+    static std::map<int, bool> configured;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!configured[ctx->device]) {
+            TFB_CUDA(cudaFuncSetAttribute(grouped_units_kernel<T, Path>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          GroupSmem<T>::BYTES));
+            configured[ctx->device] = true;
+        }
+    }
+    GroupedArgs g{(const GroupUnit*)f.mem.ptr, (const int*)((const char*)f.mem.ptr + f.starts_at), alpha.re, alpha.im, beta.re, beta.im};
+    LaunchScope ls(ctx, name);
+    grouped_units_kernel<T, Path><<<f.grid, kGroupThreads, GroupSmem<T>::BYTES, ctx->stream>>>(g);
     TFB_CUDA(cudaGetLastError());
     return TFB_OK;
 }
 
+tfb_status lay_out(tfb_ctx* ctx, int dtype, size_t n, const tfb_gemm_problem* problems, bool balance, GroupedUnits* out) {
+    switch (dtype) {
+        case TFB_F32: return lay_out_units<float>(ctx, n, problems, balance, out);
+        case TFB_F64: return lay_out_units<double>(ctx, n, problems, balance, out);
+        case TFB_C32: return lay_out_units<float2>(ctx, n, problems, balance, out);
+        case TFB_C64: return lay_out_units<double2>(ctx, n, problems, balance, out);
+    }
+    return fail(TFB_ERR_INVALID_ARGUMENT, "unknown dtype %d", dtype);
+}
+
+tfb_status run_units(tfb_ctx* ctx, int dtype, const GroupedUnits& f, Scalar alpha, Scalar beta) {
+    if (f.grid == 0) return TFB_OK;
+    switch (dtype) {
+        case TFB_F32: return launch_units<float, FmaPath<float>>(ctx, f, alpha, beta, "grouped_simt");
+        case TFB_F64: return launch_units<double, TensorPath<double>>(ctx, f, alpha, beta, "grouped_dmma");
+        case TFB_C32: return launch_units<float2, FmaPath<float2>>(ctx, f, alpha, beta, "grouped_simt");
+        case TFB_C64: return launch_units<double2, TensorPath<double2>>(ctx, f, alpha, beta, "grouped_dmma");
+    }
+    return fail(TFB_ERR_INVALID_ARGUMENT, "unknown dtype %d", dtype);
+}
+
+}  // namespace
+
 }  // namespace tfb
 
-// A problem table prepared once: the tensor-core schedule on the device when the table
-// qualifies, else the host copy of the table for the SIMT kernel.
+// A problem table prepared once: the f32 tensor-core schedule on the device when the table
+// qualifies, else the unit lists of the general kernel.
 struct tfb_grouped_plan {
     tfb_ctx* ctx = nullptr;
     int dtype = 0;
     bool fast = false;
     tfb::GroupedFast schedule;
-    std::vector<tfb_gemm_problem> problems;
+    tfb::GroupedUnits units;
+    tfb_status invalid = TFB_OK;  // what is wrong with the table: reported by every execute
+    std::string why;
 };
 
 namespace {
 
-tfb_status prepare(tfb_ctx* ctx, int dtype, size_t n, const tfb_gemm_problem* problems, tfb_grouped_plan* plan) {
+tfb_status prepare(tfb_ctx* ctx, int dtype, size_t n, const tfb_gemm_problem* problems, bool balance, tfb_grouped_plan* plan) {
     using namespace tfb;
     DeviceGuard g(ctx->device);
     plan->ctx = ctx;
     plan->dtype = dtype;
-    plan->problems.assign(problems, problems + n);
     if (dtype == TFB_F32) {
         // The mma.sync kernel is the faster one on the tables it takes (dims in multiples of 16, K up to
         // 128); the tcgen05 kernel takes any dims with 16-byte aligned columns and K up to 512; the
-        // SIMT kernel takes everything.
+        // general kernel takes everything.
         const bool tcgen05_first = env_int("TFB_GROUPED_PREFER_TCGEN05", 0) != 0;
         bool declined = true;
         if (tcgen05_first) TFB_TRY(grouped_tcgen05_prepare(ctx, n, problems, &plan->schedule, &declined));
@@ -179,21 +605,24 @@ tfb_status prepare(tfb_ctx* ctx, int dtype, size_t n, const tfb_gemm_problem* pr
         if (declined && !tcgen05_first) TFB_TRY(grouped_tcgen05_prepare(ctx, n, problems, &plan->schedule, &declined));
         plan->fast = !declined;
     }
-    return TFB_OK;
+    if (plan->fast) return TFB_OK;
+    plan->invalid = check_table(n, problems);
+    if (plan->invalid != TFB_OK) {
+        size_t len = tfb_last_error(nullptr, 0);
+        plan->why.resize(len + 1);
+        tfb_last_error(plan->why.data(), plan->why.size());
+        return TFB_OK;
+    }
+    return lay_out(ctx, dtype, n, problems, balance, &plan->units);
 }
 
 tfb_status run(tfb_grouped_plan* plan, tfb::Scalar alpha, tfb::Scalar beta) {
     using namespace tfb;
+    if (plan->invalid != TFB_OK) return fail(plan->invalid, "%s", plan->why.c_str());
     DeviceGuard g(plan->ctx->device);
-    if (plan->fast) {
-        bool declined = true;
-        if (plan->schedule.tcgen05)
-            TFB_TRY(grouped_tcgen05_run(plan->ctx, plan->schedule, alpha, beta, &declined));
-        else
-            TFB_TRY(grouped_tf32_run(plan->ctx, plan->schedule, alpha, beta, &declined));
-        if (!declined) return TFB_OK;
-    }
-    return grouped_simt(plan->ctx, plan->dtype, plan->problems.size(), plan->problems.data(), alpha, beta);
+    if (!plan->fast) return run_units(plan->ctx, plan->dtype, plan->units, alpha, beta);
+    if (plan->schedule.tcgen05) return grouped_tcgen05_run(plan->ctx, plan->schedule, alpha, beta);
+    return grouped_tf32_run(plan->ctx, plan->schedule, alpha, beta);
 }
 
 tfb_status check_args(const char* who, tfb_ctx* ctx, int32_t dtype, size_t n, const tfb_gemm_problem* problems) {
@@ -212,7 +641,7 @@ extern "C" tfb_status tfb_grouped_gemm(tfb_ctx* ctx, int32_t dtype, size_t n_pro
     TFB_TRY(check_args("tfb_grouped_gemm", ctx, dtype, n_problems, problems));
     if (!alpha || !beta) return fail(TFB_ERR_INVALID_ARGUMENT, "tfb_grouped_gemm: alpha/beta are NULL");
     tfb_grouped_plan plan;
-    TFB_TRY(prepare(ctx, dtype, n_problems, problems, &plan));
+    TFB_TRY(prepare(ctx, dtype, n_problems, problems, false, &plan));
     return run(&plan, load_scalar(dtype, alpha), load_scalar(dtype, beta));
 }
 
@@ -223,7 +652,7 @@ extern "C" tfb_status tfb_grouped_plan_create(tfb_ctx* ctx, int32_t dtype, size_
     if (!out) return fail(TFB_ERR_INVALID_ARGUMENT, "tfb_grouped_plan_create: out is NULL");
     auto* plan = new (std::nothrow) tfb_grouped_plan;
     if (!plan) return fail(TFB_ERR_DEVICE, "out of host memory");
-    const tfb_status st = prepare(ctx, dtype, n_problems, problems, plan);
+    const tfb_status st = prepare(ctx, dtype, n_problems, problems, true, plan);
     if (st != TFB_OK) {
         delete plan;
         return st;

@@ -1,7 +1,7 @@
 // Grouped f32 products on the tcgen05 tensor cores: the kernel of tfb_grouped_gemm for ragged
 // tables of column-major problems that the mma.sync kernel (grouped_tf32.cu) declines - any
-// m, n, k >= 1 with 16-byte aligned columns and K up to 512 - where it is about five times as
-// fast as the SIMT kernel (4096 problems with dims from {20, 36, 72, 136}: 174 us against 832).
+// m, n, k >= 1 with 16-byte aligned columns and K up to 512 - where it is faster than the
+// general kernel of grouped.cu (4096 problems with dims from {20, 36, 72, 136}: 181 us against 276).
 // On tables the mma.sync kernel takes (dims in multiples of 16, K <= 128) that kernel is the
 // faster one (54 us against 96 for 4096 problems with dims from {16, 32, 64, 128}); see the end of
 // this comment for why.  TFB_GROUPED_PREFER_TCGEN05=1 asks for this kernel first.
@@ -537,10 +537,7 @@ tfb_status grouped_tcgen05_prepare(tfb_ctx* ctx, size_t n, const tfb_gemm_proble
     return TFB_OK;
 }
 
-tfb_status grouped_tcgen05_run(tfb_ctx* ctx, const GroupedFast& f, Scalar alpha, Scalar beta, bool* declined) {
-    *declined = true;
-    if (alpha.im != 0 || beta.im != 0) return TFB_OK;
-    *declined = false;
+tfb_status grouped_tcgen05_run(tfb_ctx* ctx, const GroupedFast& f, Scalar alpha, Scalar beta) {
     GtArgs g;
     g.stages = (const TcStage*)f.mem.ptr;
     g.pitch = f.pitch;

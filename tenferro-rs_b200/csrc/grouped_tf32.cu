@@ -363,10 +363,7 @@ tfb_status grouped_tf32_prepare(tfb_ctx* ctx, size_t n, const tfb_gemm_problem* 
     return TFB_OK;
 }
 
-tfb_status grouped_tf32_run(tfb_ctx* ctx, const GroupedFast& f, Scalar alpha, Scalar beta, bool* declined) {
-    *declined = true;
-    if (alpha.im != 0 || beta.im != 0) return TFB_OK;
-    *declined = false;
+tfb_status grouped_tf32_run(tfb_ctx* ctx, const GroupedFast& f, Scalar alpha, Scalar beta) {
     FastArgs g;
     g.stages = (const Stage*)f.mem.ptr;
     g.alpha = (float)alpha.re;
