@@ -37,6 +37,7 @@ struct ContractArgs {
     const int64_t* d_n;
     int conj_mul;
     int a_kfast, b_kfast;  // 1: the unit-stride direction of the operand tile is K; 0: M (resp. N)
+    int a_runs, b_runs;    // TMA-fed DMMA kernel: 1: one load per run of the unit-stride index
     int a_vec, b_vec;      // elements per cp.async (1, or 2 for f64 when 16-byte chunks are legal)
     // Work decomposition: tiles x k-iterations, cut into equal contiguous ranges ("stream-K").
     int64_t tiles_m, tiles_n, n_tiles, k_iters, total_iters, iters_per_cta;

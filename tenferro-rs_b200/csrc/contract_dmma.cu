@@ -480,15 +480,32 @@ static tfb_status run_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractArgs a
 namespace tfb {
 
 using RealTma = DmmaTmaCfg<false, 128, 128, 16, 4, 4, 6>;
-using CplxTma = DmmaTmaCfg<true, 64, 64, 16, 4, 4, 6>;
-using RealTmaSmall = DmmaTmaCfg<false, 64, 64, 16, 2, 2, 8>;
-using CplxTmaSmall = DmmaTmaCfg<true, 32, 32, 16, 2, 2, 8>;
+// 32-deep k-iterations, three stages: half the barrier hand-offs of 16-deep ones with six (chi = 512 chain,
+// per product: 68.0 -> 66.6 us).  The real kernel gains 1 % at 4000^3 and loses 6 % at K = 300 by it.
+using CplxTma = DmmaTmaCfg<true, 64, 64, 32, 4, 4, 3>;
+// Sixteen warps on a 64 x 64 tile (four took 13.6 us at 200^3, sixteen 10.4; 400^3: 22.4, 17.7): more
+// fragment loads per MMA, but a warp alone on its scheduler leaves the pipe idle while it loads.
+using RealTmaSmall = DmmaTmaCfg<false, 64, 64, 16, 4, 4, 8>;
+using CplxTmaSmall = DmmaTmaCfg<true, 32, 32, 16, 2, 4, 8>;
+using CplxTma4 = DmmaTmaCfg<true, 64, 64, 32, 4, 4, 3, true>;
+using CplxTma4Small = DmmaTmaCfg<true, 32, 32, 16, 2, 4, 6, true>;
 using RealTmaTiny = DmmaTmaCfg<false, 32, 32, 16, 2, 2, 8>;
 using RealBig = DmmaCfg<false, 128, 128, 16, 4, 4, 3>;
 using RealBig8 = DmmaCfg<false, 128, 128, 16, 2, 4, 3>;
 using RealSmall = DmmaCfg<false, 64, 64, 16, 2, 2, 4>;
 using CplxMain = DmmaCfg<true, 64, 64, 16, 4, 4, 4>;
 using CplxSmall = DmmaCfg<true, 32, 32, 8, 2, 2, 4>;
+
+// The TMA-fed kernel on `p`, tile by output size; *declined where an operand has no tensor map.
+static tfb_status run_tma(tfb_ctx* ctx, const ContractProblem& p, const ContractArgs& a, bool small, bool four, bool* declined) {
+    if (p.dtype == TFB_F64) {
+        // few outputs, long K: many small ranges
+        if (a.M * a.N * a.B <= 64 * 64) return run_tma_cfg<RealTmaTiny>(ctx, p, a, declined);
+        return small ? run_tma_cfg<RealTmaSmall>(ctx, p, a, declined) : run_tma_cfg<RealTma>(ctx, p, a, declined);
+    }
+    if (four) return small ? run_tma_cfg<CplxTma4Small>(ctx, p, a, declined) : run_tma_cfg<CplxTma4>(ctx, p, a, declined);
+    return small ? run_tma_cfg<CplxTmaSmall>(ctx, p, a, declined) : run_tma_cfg<CplxTma>(ctx, p, a, declined);
+}
 
 tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined, bool four_products) {
     *declined = false;
@@ -503,38 +520,44 @@ tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined,
     const int shape = env_int("TFB_DMMA_TILE", 0);  // 0 auto, 1 small, 2 big
     const bool use_tma = !env_int("TFB_NO_DMMA_TMA", 0);
     if (p.dtype == TFB_F64) {
-        bool small = (a.M <= 64 || a.N <= 64 || a.M * a.N * a.B < (int64_t)128 * 128 * ctx->sm_count / 2);
-        if (shape == 1) small = true;
-        if (shape == 2) small = false;
+        // 64 x 64 tiles below a fourteenth of the SMs' worth of 128 x 128 ones: 400^3 17.7 against 23.7 us,
+        // 500^3 22.3 against 21.6, 900^3 88 against 75.
+        bool small = (a.M <= 64 || a.N <= 64 || a.M * a.N * a.B < (int64_t)128 * 128 * ctx->sm_count / 14);
+        // The gather kernel's 128 x 128 tiles, one chunk of eight bytes per copy, want far more outputs
+        // (401 x 405 x 403: 77 us, 36 on 64 x 64).
+        bool small_gather = (a.M <= 64 || a.N <= 64 || a.M * a.N * a.B < (int64_t)128 * 128 * ctx->sm_count / 2);
+        if (shape == 1) small = small_gather = true;
+        if (shape == 2) small = small_gather = false;
         if (shape == 3) return run_cfg<RealBig8>(ctx, p, a);
         if (use_tma) {
             bool d = true;
-            if (a.M * a.N * a.B <= 64 * 64)
-                TFB_TRY(run_tma_cfg<RealTmaTiny>(ctx, p, a, &d));  // few outputs, long K: many small ranges
-            else if (small)
-                TFB_TRY(run_tma_cfg<RealTmaSmall>(ctx, p, a, &d));
-            else
-                TFB_TRY(run_tma_cfg<RealTma>(ctx, p, a, &d));
+            TFB_TRY(run_tma(ctx, p, a, small, false, &d));
             if (!d) return TFB_OK;
         }
-        return small ? run_cfg<RealSmall>(ctx, p, a) : run_cfg<RealBig>(ctx, p, a);
+        return small_gather ? run_cfg<RealSmall>(ctx, p, a) : run_cfg<RealBig>(ctx, p, a);
     }
-    bool small = (a.M <= 32 || a.N <= 32);
-    if (shape == 1) small = true;
-    if (shape == 2) small = false;
-    // The TMA-fed kernel forms a complex product from three real ones, whose imaginary part is a
-    // difference of sums as large as the real part: norm-wise exact, but when |Im| << |Re| the
-    // imaginary part alone loses digits.  A caller that needs each part to its own accuracy asks
-    // for four products, which the gather kernel below computes.
+    // 32 x 32 tiles below an eighth of the SMs' worth of 64 x 64 ones (eight launches of a chain, chi = 64: 80
+    // against 124 us, 97: 91 against 159, 192: 128 against 157, 338: 368 against 278).
+    bool small = (a.M <= 32 || a.N <= 32 || a.M * a.N * a.B < (int64_t)64 * 64 * ctx->sm_count / 8);
+    bool small_gather = (a.M <= 32 || a.N <= 32);
+    if (shape == 1) small = small_gather = true;
+    if (shape == 2) small = small_gather = false;
+    // Three real products make a complex one with an imaginary part that is a difference of sums as
+    // large as the real part: norm-wise exact, but when |Im| << |Re| the imaginary part alone loses
+    // digits (and the whole result about half a bit).  A caller that needs each part to its own
+    // accuracy asks for four products.  Layouts that the three-product form has no tensor map for
+    // (K no multiple of four along a K-major operand, an odd extent along an MN-major one) have always
+    // had four, and keep that accuracy.
+    bool d = true;
     if (use_tma && !four_products) {
-        bool d = true;
-        if (small)
-            TFB_TRY(run_tma_cfg<CplxTmaSmall>(ctx, p, a, &d));
-        else
-            TFB_TRY(run_tma_cfg<CplxTma>(ctx, p, a, &d));
+        TFB_TRY(run_tma(ctx, p, a, small, false, &d));
         if (!d) return TFB_OK;
     }
-    return small ? run_cfg<CplxSmall>(ctx, p, a) : run_cfg<CplxMain>(ctx, p, a);
+    if (use_tma) {
+        TFB_TRY(run_tma(ctx, p, a, small, true, &d));
+        if (!d) return TFB_OK;
+    }
+    return small_gather ? run_cfg<CplxSmall>(ctx, p, a) : run_cfg<CplxMain>(ctx, p, a);
 }
 
 }  // namespace tfb

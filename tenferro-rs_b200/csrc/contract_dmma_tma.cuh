@@ -1,7 +1,7 @@
 // TMA-fed variant of the f64 / Complex64 DMMA contraction (included by contract_dmma.cu).
 //
 // When each of M, N, K is a single fused mode and one side of every operand has unit stride,
-// the operand tiles need no per-thread gather: one thread issues two cp.async.bulk.tensor
+// the operand tiles need no per-thread gather: one thread at a time issues two cp.async.bulk.tensor
 // loads per k-iteration, a few iterations ahead, and the sixteen warps do nothing but
 // fragment loads and DMMAs, synchronised by full/empty mbarriers (no CTA-wide barrier in
 // the main loop, and the ring keeps running across the tiles of a stream-K range).
@@ -13,26 +13,42 @@
 // (a quarter warp of 16-byte loads, or a half warp of 8-byte loads, then covers one
 // contiguous 128-byte line).  Both are ordinary rank-4 tensor maps over the strided operand:
 // dimension 0 is the short run, and a second dimension walks the same index in steps of the
-// run length.
+// run length, which therefore has to divide the extent.
+//
+// The four-product complex form takes any extent.  A complex element is 16 bytes, all that TMA asks of
+// an address, so dimension 0 can be the whole extent (zero-filled past its end) with one load per
+// run.  To keep those few, runs are 128-byte lines:
+//   K-major   [k-panel of 8][row][8 k]    2 loads per 16 k
+//   MN-major  [group of 8 rows][k][8 rows]    8 loads for 64 rows (one load where 8 divides the extent)
+// with TMA's 128-byte swizzle; lane (row r, slot c) reads k = 2c and 2c + 1 of an 8-deep step, so a
+// quarter warp (two rows, four k of one parity) finds its 16-byte units in chunks (r ^ k) mod 8 that take
+// every value once.  (Which k meets which slot of an MMA does not matter while both operands agree.)
+// The issue of ten loads is nothing next to the 8000 clocks of a k-iteration's MMAs.  Such extents - odd
+// bond dimensions - used to be left to the gather kernel: a chain with chi = 97 took 18.5 + 10.5 us
+// (kernel and fix-up launch) per product, 11 us here.
 #pragma once
 #include "ptx_sm100.cuh"
 
 namespace tfb {
 
-template <bool CPLX, int BM_, int BN_, int BK_, int WARPS_M_, int WARPS_N_, int STAGES_>
+// FOUR (complex only): four real products per complex one, each part accurate to its own size.
+template <bool CPLX, int BM_, int BN_, int BK_, int WARPS_M_, int WARPS_N_, int STAGES_, bool FOUR = false>
 struct DmmaTmaCfg {
     using Base = DmmaCfg<CPLX, BM_, BN_, BK_, WARPS_M_, WARPS_N_, STAGES_>;  // tile shape, fix-up kernel
-    static constexpr bool kCplx = CPLX;
+    static constexpr bool kCplx = CPLX, kFour = FOUR;
+    static constexpr int ACC = CPLX ? (FOUR ? 4 : 6) : 2;  // accumulators per fragment element pair
     static constexpr int BM = BM_, BN = BN_, BK = BK_, WARPS_M = WARPS_M_, WARPS_N = WARPS_N_, STAGES = STAGES_;
     static constexpr int CONSUMERS = WARPS_M * WARPS_N;
-    static constexpr int NT = CONSUMERS * 32;  // lane 0 of warp 0 doubles as the TMA producer
+    static constexpr int NT = CONSUMERS * 32;
     static constexpr int WM = BM / WARPS_M, WN = BN / WARPS_N;
     static constexpr int TM = WM / 8, TN = WN / 8;
     static constexpr int ES = CPLX ? 16 : 8;
-    static constexpr int G = CPLX ? 2 : 4;  // rows per 32-byte run of an MN-major tile
+    static constexpr bool kLines = FOUR;             // 128-byte runs, swizzled
+    static constexpr int KR = kLines ? 8 : 4;        // k per run of a K-major tile
+    static constexpr int G = kLines ? 8 : CPLX ? 2 : 4;  // rows per run of an MN-major tile
     static constexpr int A_BYTES = BM * BK * ES, B_BYTES = BN * BK * ES;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 16 * STAGES + 128;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 16 * STAGES + 1024;
 };
 
 // Element offset of (row, k) inside a dense tile.
@@ -42,14 +58,65 @@ __device__ __forceinline__ int tile_off(int row, int k) {
     return ((k >> 2) * ROWS + row) * 4 + (k & 3);
 }
 
+// A lane's 16-byte units of a complex tile: row w0 + 8 i + lr, k = kk + 2 lc + q (kk a multiple of 8).  What
+// depends on the lane is computed here, once; the rest of an address is a constant.
+template <typename Cfg, int ROWS, bool MN>
+struct LineReader {
+    const char* at[2];
+    __device__ __forceinline__ LineReader(const char* tile, int w0, int lr, int lc) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int k = 2 * lc + q;
+            at[q] = tile + (MN ? w0 * (Cfg::BK * 16) + k * 128 : (w0 + lr) * 128) + ((lr ^ k) << 4);
+        }
+    }
+    __device__ __forceinline__ double2 get(int i, int kk, int q) const {
+        return *reinterpret_cast<const double2*>(at[q] + (MN ? i * Cfg::BK * 128 + kk * 128 : kk * ROWS * 16 + i * 1024));
+    }
+};
+
 template <typename Cfg, bool A_MN, bool B_MN>
-__device__ __forceinline__ void dmma_tma_consume(const char* sa, const char* sb, double (&acc)[Cfg::TM][Cfg::TN][Cfg::kCplx ? 6 : 2],
+__device__ __forceinline__ void dmma_tma_consume(const char* sa, const char* sb, double (&acc)[Cfg::TM][Cfg::TN][Cfg::ACC],
                                                  int wm0, int wn0, int lr, int lc, bool conj_a, bool conj_b) {
     constexpr bool CPLX = Cfg::kCplx;
     constexpr int TM = Cfg::TM, TN = Cfg::TN;
 #pragma unroll
     for (int kk = 0; kk < Cfg::BK; kk += 8) {
-        if (CPLX) {
+        if constexpr (Cfg::kFour) {
+            // Re += Ar Br - Ai Bi, Im += Ar Bi + Ai Br; acc[..][0..1] = Re, [2..3] = Im.
+            const LineReader<Cfg, Cfg::BM, A_MN> ra(sa, wm0, lr, lc);
+            const LineReader<Cfg, Cfg::BN, B_MN> rb(sb, wn0, lr, lc);
+            double ar[TM][2], ai[TM][2], br[TN][2], bi[TN][2], nbi[TN][2];
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const double2 v = ra.get(i, kk, q);
+                    ar[i][q] = v.x;
+                    ai[i][q] = conj_a ? -v.y : v.y;
+                }
+#pragma unroll
+            for (int j = 0; j < TN; ++j)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const double2 v = rb.get(j, kk, q);
+                    br[j][q] = v.x;
+                    bi[j][q] = conj_b ? -v.y : v.y;
+                    nbi[j][q] = -bi[j][q];
+                }
+            auto pass = [&](const double (&x)[TM][2], const double (&y)[TN][2], int at) {
+#pragma unroll
+                for (int i = 0; i < TM; i += 2)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j)
+                        dmma16(acc[i][j][at], acc[i][j][at + 1], acc[i + 1][j][at], acc[i + 1][j][at + 1], x[i][0], x[i + 1][0],
+                               x[i][1], x[i + 1][1], y[j][0], y[j][1]);
+            };
+            pass(ar, br, 0);
+            pass(ar, bi, 2);
+            pass(ai, nbi, 0);
+            pass(ai, br, 2);
+        } else if constexpr (CPLX) {
             // Three real products per complex one instead of four:
             //   P1 = Ar Br,  P2 = Ai Bi,  P3 = (Ar + Ai)(Br + Bi);  Re = P1 - P2,  Im = P3 - P1 - P2.
             // The sums cost two adds per fragment element; the FP64 pipe, which is what this
@@ -126,7 +193,7 @@ contract_dmma_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, TM = Cfg::TM, TN = Cfg::TN, STAGES = Cfg::STAGES;
     constexpr int ES = Cfg::ES;
     extern __shared__ __align__(128) char smem_dyn[];
-    char* smem = (char*)(((uintptr_t)smem_dyn + 127) & ~(uintptr_t)127);
+    char* smem = (char*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);  // the swizzle follows address bits
     const uint32_t ring = smem_u32(smem);
     const uint32_t bars = ring + STAGES * Cfg::STAGE_BYTES;
     auto bar_full = [&](int s) { return bars + 8u * s; };
@@ -150,53 +217,41 @@ contract_dmma_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const int64_t it_end = min(g.total_iters, it_begin + g.iters_per_cta);
     const bool a_mn = !g.a_kfast, b_mn = !g.b_kfast;
 
-    // ---------------------------------------------------------------- producer (lane 0 of warp 0)
-    // It runs `kLead` k-iterations ahead of the consumers.  Issuing iteration j needs the slot
-    // that iteration j - STAGES used, i.e. every warp must have finished that one; with
-    // kLead = STAGES - 2 that is two iterations behind warp 0 itself, so the wait is short.
+    // ---------------------------------------------------------------- loads
+    // They run `kLead` k-iterations ahead.  Issuing iteration j needs the slot that iteration
+    // j - STAGES used, i.e. every warp must have finished that one; with kLead = STAGES - 2 that is
+    // two iterations behind the issuing warp itself, so the wait is short.  The warps take turns, one
+    // iteration each: a warp that issued them all was a third of an iteration behind the others
+    // each time, and the whole CTA ran at its pace (chi = 512 chain, per product: 70.4 -> 68.0 us; f64 4000^3 3.99 ->
+    // 3.90 ms; 300 x 300 x 4000 50 -> 39 us).
     constexpr int kLead = STAGES - 2;
-    const int64_t my_iters = it_end - it_begin;
-    int64_t issued = 0;
-    // Position of the next k-iteration to issue, advanced without divisions: the producer is also a
-    // computing thread, and whatever it spends here its whole warp waits for.  (32-bit: the host
-    // keeps total_iters below 2^31 for this kernel.)
-    uint32_t p_kit, p_tm, p_tn, p_bb;
-    {
+    const uint32_t my_iters = (uint32_t)(it_end - it_begin);  // the host keeps total_iters below 2^31
+    auto issue = [&](uint32_t j) {
         const uint32_t k_iters = (uint32_t)g.k_iters, tiles_m = (uint32_t)g.tiles_m, tiles_n = (uint32_t)g.tiles_n;
-        const uint32_t tile = (uint32_t)it_begin / k_iters, rest = tile / tiles_m;
-        p_kit = (uint32_t)it_begin - tile * k_iters;
-        p_tm = tile - rest * tiles_m;
-        p_bb = rest / tiles_n;
-        p_tn = rest - p_bb * tiles_n;
-    }
-    auto produce_until = [&](int64_t target) {
-        if (target > my_iters) target = my_iters;
-        for (; issued < target; ++issued) {
-            const int m0 = (int)(p_tm * BM), n0 = (int)(p_tn * BN), k0 = (int)(p_kit * BK);
-            const uint32_t bb = p_bb;
-            const uint32_t iu = (uint32_t)issued;
-            const int s = (int)(iu % STAGES);
-            mbar_wait(bar_empty(s), ((iu / STAGES) & 1) ^ 1, status, 0x301);
-            const uint32_t a_dst = ring + s * Cfg::STAGE_BYTES, b_dst = a_dst + Cfg::A_BYTES;
-            mbar_expect_tx(bar_full(s), Cfg::STAGE_BYTES);
-            if (a_mn) tma_load_4d(a_dst, &map_a, bar_full(s), 0, k0, m0 / Cfg::G, (int)bb);
-            else      tma_load_4d(a_dst, &map_a, bar_full(s), 0, m0, k0 / 4, (int)bb);
-            if (b_mn) tma_load_4d(b_dst, &map_b, bar_full(s), 0, k0, n0 / Cfg::G, (int)bb);
-            else      tma_load_4d(b_dst, &map_b, bar_full(s), 0, n0, k0 / 4, (int)bb);
-            if (++p_kit == (uint32_t)g.k_iters) {
-                p_kit = 0;
-                if (++p_tm == (uint32_t)g.tiles_m) {
-                    p_tm = 0;
-                    if (++p_tn == (uint32_t)g.tiles_n) {
-                        p_tn = 0;
-                        ++p_bb;
-                    }
-                }
+        const uint32_t at = (uint32_t)it_begin + j, tile = at / k_iters, rest = tile / tiles_m, bb = rest / tiles_n;
+        const int m0 = (int)((tile - rest * tiles_m) * BM), n0 = (int)((rest - bb * tiles_n) * BN);
+        const int k0 = (int)((at - tile * k_iters) * BK);
+        const int s = (int)(j % STAGES);
+        mbar_wait(bar_empty(s), ((j / STAGES) & 1) ^ 1, status, 0x301);
+        const uint32_t a_dst = ring + s * Cfg::STAGE_BYTES, b_dst = a_dst + Cfg::A_BYTES;
+        mbar_expect_tx(bar_full(s), Cfg::STAGE_BYTES);
+        auto load = [&](const CUtensorMap* map, uint32_t dst, bool mn, bool runs, int r0, int rows) {
+            if (!Cfg::kLines || !runs) {
+                if (mn) tma_load_4d(dst, map, bar_full(s), 0, k0, r0 / Cfg::G, (int)bb);
+                else    tma_load_4d(dst, map, bar_full(s), 0, r0, k0 / Cfg::KR, (int)bb);
+            } else if (mn) {
+                for (int r = 0; r < rows; r += Cfg::G)
+                    tma_load_4d(dst + r * BK * ES, map, bar_full(s), 2 * (r0 + r), k0, 0, (int)bb);
+            } else {
+                for (int k = 0; k < BK; k += Cfg::KR)
+                    tma_load_4d(dst + k * rows * ES, map, bar_full(s), 2 * (k0 + k), r0, 0, (int)bb);
             }
-        }
+        };
+        load(&map_a, a_dst, a_mn, g.a_runs, m0, BM);
+        load(&map_b, b_dst, b_mn, g.b_runs, n0, BN);
     };
-    const bool is_producer = (tid == 0);
-    if (is_producer) produce_until(kLead);
+    // the first kLead iterations: one each, too
+    for (uint32_t j = warp; lane == 0 && j < kLead && j < my_iters; j += Cfg::CONSUMERS) issue(j);
 
     // -------------------------------------------------------------------- consumers
     const int wm0 = (warp % Cfg::WARPS_M) * Cfg::WM, wn0 = (warp / Cfg::WARPS_M) * Cfg::WN;
@@ -210,17 +265,17 @@ contract_dmma_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         const int64_t ke = min(g.k_iters, kb + (it_end - it));
         const int64_t tm = tile % g.tiles_m, rest = tile / g.tiles_m, tn = rest % g.tiles_n, bb = rest / g.tiles_n;
         const int64_t m0 = tm * BM, n0 = tn * BN;
-        double acc[TM][TN][CPLX ? 6 : 2];
+        double acc[TM][TN][Cfg::ACC];
 #pragma unroll
         for (int i = 0; i < TM; ++i)
 #pragma unroll
             for (int j = 0; j < TN; ++j)
 #pragma unroll
-                for (int e = 0; e < (CPLX ? 6 : 2); ++e) acc[i][j][e] = 0.0;
+                for (int e = 0; e < Cfg::ACC; ++e) acc[i][j][e] = 0.0;
 
         for (int64_t kit = kb; kit < ke; ++kit, ++n) {
             const int s = n % STAGES;
-            if (is_producer) produce_until((int64_t)n + kLead + 1);
+            if (lane == 0 && n % Cfg::CONSUMERS == (uint32_t)warp && n + kLead < my_iters) issue(n + kLead);
             if (lane == 0) mbar_wait(bar_full(s), (n / STAGES) & 1, status, 0x302);
             __syncwarp();
             const char* sa = smem + (size_t)s * Cfg::STAGE_BYTES;
@@ -236,7 +291,7 @@ contract_dmma_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             if (lane == 0) mbar_arrive(bar_empty(s));
         }
 
-        if constexpr (CPLX) {
+        if constexpr (CPLX && !Cfg::kFour) {
             // fold the three products of this k range into Re (slots 0-1) and Im (slots 2-3)
 #pragma unroll
             for (int i = 0; i < TM; ++i)
@@ -423,9 +478,10 @@ static EncodeTiledF64 encode_tiled_f64() {
 }
 
 // Tensor map of one operand (free group `fr`, tensor index tns); false when TMA cannot describe it.
+// *runs: one load per run (see the top of this file).
 template <typename Cfg>
 static bool make_f64_map(const ContractProblem& p, const std::vector<Mode>& fr, int tns, const void* base, int rows,
-                         bool* mn_major, CUtensorMap* map) {
+                         bool* mn_major, bool* runs, CUtensorMap* map) {
     EncodeTiledF64 enc = encode_tiled_f64();
     if (!enc || fr.size() > 1 || p.k.size() != 1 || p.batch.size() > 1) return false;
     constexpr int W = Cfg::kCplx ? 2 : 1;  // doubles per element
@@ -438,30 +494,39 @@ static bool make_f64_map(const ContractProblem& p, const std::vector<Mode>& fr, 
     cuuint64_t dims[4], strides[3];
     cuuint32_t box[4], estr[4] = {1, 1, 1, 1};
     const cuuint64_t bstride = (cuuint64_t)((B > 1 ? bs * W * 8 : 16));
-    if (ks == 1 && K % 4 == 0 && (R == 1 || ok16(rs))) {
+    // The unit-stride index (extent `fast`, runs of `run` elements, `step` of them per k-iteration) and the other one.
+    int64_t fast, slow, slow_stride;
+    int run, step, slow_box;
+    if (ks == 1 && (Cfg::kLines || K % Cfg::KR == 0) && (R == 1 || ok16(rs))) {
         *mn_major = false;
-        dims[0] = 4 * W; dims[1] = (cuuint64_t)R; dims[2] = (cuuint64_t)(K / 4); dims[3] = (cuuint64_t)B;
-        strides[0] = (cuuint64_t)((R == 1 ? K : rs) * W * 8);
-        strides[1] = 4 * W * 8;
-        strides[2] = bstride;
-        box[0] = 4 * W; box[1] = (cuuint32_t)rows; box[2] = Cfg::BK / 4; box[3] = 1;
-    } else if (rs == 1 && R % Cfg::G == 0 && R > 1 && (K == 1 || ok16(ks))) {
+        fast = K; run = Cfg::KR; step = Cfg::BK;
+        slow = R; slow_stride = R == 1 ? K : rs; slow_box = rows;
+    } else if (rs == 1 && (Cfg::kLines || R % Cfg::G == 0) && R > 1 && (K == 1 || ok16(ks))) {
         *mn_major = true;
-        dims[0] = Cfg::G * W; dims[1] = (cuuint64_t)K; dims[2] = (cuuint64_t)(R / Cfg::G); dims[3] = (cuuint64_t)B;
-        strides[0] = (cuuint64_t)((K == 1 ? R : ks) * W * 8);
-        strides[1] = Cfg::G * W * 8;
-        strides[2] = bstride;
-        box[0] = Cfg::G * W; box[1] = Cfg::BK; box[2] = (cuuint32_t)(rows / Cfg::G); box[3] = 1;
+        fast = R; run = Cfg::G; step = rows;
+        slow = K; slow_stride = K == 1 ? R : ks; slow_box = Cfg::BK;
     } else {
         return false;
     }
+    *runs = fast % run != 0;
+    dims[0] = (cuuint64_t)((*runs ? fast : run) * W);
+    dims[1] = (cuuint64_t)slow;
+    dims[2] = (cuuint64_t)(*runs ? 1 : fast / run);
+    dims[3] = (cuuint64_t)B;
+    strides[0] = (cuuint64_t)(slow_stride * W * 8);
+    strides[1] = (cuuint64_t)(run * W * 8);
+    strides[2] = bstride;
+    box[0] = (cuuint32_t)(run * W);
+    box[1] = (cuuint32_t)slow_box;
+    box[2] = (cuuint32_t)(*runs ? 1 : step / run);
+    box[3] = 1;
     for (int i = 0; i < 3; ++i)
         if (strides[i] % 16 != 0 || strides[i] >= (1ull << 40)) return false;
     for (int i = 0; i < 4; ++i)
         if (dims[i] == 0 || dims[i] > 0xffffffffull) return false;
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<void*>(base), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+               CU_TENSOR_MAP_INTERLEAVE_NONE, Cfg::kLines ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // Runs the TMA-fed kernel when both operands qualify; otherwise *declined = true.
@@ -471,11 +536,13 @@ static tfb_status run_tma_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractAr
     *declined = true;
     if (a.M > INT32_MAX - 512 || a.N > INT32_MAX - 512 || a.K > INT32_MAX - 64) return TFB_OK;
     CUtensorMap map_a, map_b;
-    bool a_mn = false, b_mn = false;
-    if (!make_f64_map<Cfg>(p, p.m, 0, p.a, Cfg::BM, &a_mn, &map_a)) return TFB_OK;
-    if (!make_f64_map<Cfg>(p, p.n, 1, p.b, Cfg::BN, &b_mn, &map_b)) return TFB_OK;
+    bool a_mn = false, b_mn = false, a_runs = false, b_runs = false;
+    if (!make_f64_map<Cfg>(p, p.m, 0, p.a, Cfg::BM, &a_mn, &a_runs, &map_a)) return TFB_OK;
+    if (!make_f64_map<Cfg>(p, p.n, 1, p.b, Cfg::BN, &b_mn, &b_runs, &map_b)) return TFB_OK;
     a.a_kfast = !a_mn;
     a.b_kfast = !b_mn;
+    a.a_runs = a_runs;
+    a.b_runs = b_runs;
     static std::mutex mu;
     static std::map<int, bool> configured;
     {
@@ -499,8 +566,8 @@ static tfb_status run_tma_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractAr
     // owner of a tile reads all its pieces itself - eight dependent round trips to L2 for 32
     // pieces - and 'abc,bcd->ad' at 64^4 took 16.4 us; here every load of the sum is independent.)
     int pieces = 0;
-    if (a.n_tiles * 4 <= slots && a.k_iters >= 16 && env_int("TFB_SK_TWO_PHASE", 1)) {
-        const int64_t want = std::min<int64_t>(std::min<int64_t>(32, slots / a.n_tiles), a.k_iters / 4);
+    if (a.n_tiles * 4 <= slots && a.k_iters * Cfg::BK >= 256 && env_int("TFB_SK_TWO_PHASE", 1)) {
+        const int64_t want = std::min<int64_t>(std::min<int64_t>(32, slots / a.n_tiles), a.k_iters * Cfg::BK / 64);
         a.iters_per_cta = (a.k_iters + want - 1) / want;
         pieces = (int)((a.k_iters + a.iters_per_cta - 1) / a.iters_per_cta);
     }
@@ -518,7 +585,9 @@ static tfb_status run_tma_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractAr
         grid = std::min(a.n_tiles, slots);
         a.iters_per_cta = ((a.n_tiles + grid - 1) / grid) * a.k_iters;
     } else {
-        grid = std::min<int64_t>(slots, std::max<int64_t>(1, a.total_iters / 4));
+        // At least two k-iterations per CTA (eight launches of a chain, chi = 64: 98 -> 84 us against
+        // at least four).
+        grid = std::min<int64_t>(slots, std::max<int64_t>(1, a.total_iters / 2));
         a.iters_per_cta = (a.total_iters + grid - 1) / grid;
         // One thread of the owner polls each contributor's flag and every contribution costs the
         // owner one pass over a slot: keep a tile in at most 32 pieces.
