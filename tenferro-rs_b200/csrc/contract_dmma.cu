@@ -507,6 +507,73 @@ static tfb_status run_tma(tfb_ctx* ctx, const ContractProblem& p, const Contract
     return small ? run_tma_cfg<CplxTmaSmall>(ctx, p, a, declined) : run_tma_cfg<CplxTma>(ctx, p, a, declined);
 }
 
+// Operands without a tensor map (odd leading extents of f64, groups of several modes that do not
+// fuse, the batch index innermost) are copied once into [batch][k][rows] blocks and the TMA-fed
+// kernel runs on those.  The copy moves 2 es (M K + K N) bytes, the product does 2 M N K operations, and
+// the gather kernel is a half to a tenth of the TMA-fed one's speed (one 8-byte cp.async per element,
+// uncoalesced where neither side of a tile has unit stride), so from about 2e8 operations with at
+// least 64 rows on the other side the copy is the cheaper way (f64, us by gather and with copies:
+// 301 x 305 x 303 30.7, 28.8; 903 x 907 x 905 114, 91; 1203^3 226, 158; 2505 x 3048 x 3261 2250, 1650;
+// 308 batches innermost of 118 x 113 x 327 930, 375).  q receives the product on the copies.
+static tfb_status repack_for_tma(tfb_ctx* ctx, const ContractProblem& p, const ContractArgs& a, PoolBlock* blk_a,
+                                 PoolBlock* blk_b, ContractProblem* q, bool* ready) {
+    *ready = false;
+    const double flops = 2.0 * (double)a.M * (double)a.N * (double)a.K * (double)a.B;
+    if (flops < 2e8 || a.M < 64 || a.N < 64 || a.K < 16) return TFB_OK;
+    bool mn = false, runs = false;
+    CUtensorMap map;
+    bool need[2];
+    if (p.dtype == TFB_F64) {
+        need[0] = !make_f64_map<RealTma>(p, p.m, 0, p.a, RealTma::BM, &mn, &runs, &map);
+        need[1] = !make_f64_map<RealTma>(p, p.n, 1, p.b, RealTma::BN, &mn, &runs, &map);
+    } else {
+        need[0] = !make_f64_map<CplxTma4>(p, p.m, 0, p.a, CplxTma4::BM, &mn, &runs, &map);
+        need[1] = !make_f64_map<CplxTma4>(p, p.n, 1, p.b, CplxTma4::BN, &mn, &runs, &map);
+    }
+    // A copy of at most an eighth of the device's memory each: a larger one could take the room that the
+    // caller's next tensors need.  Without room the gather kernel runs.
+    int64_t ld[2];
+    for (int t = 0; t < 2; ++t) {
+        ld[t] = ((t == 0 ? a.M : a.N) + 7) / 8 * 8;  // rows past the last only reach sums that are not stored
+        const double bytes = (double)dtype_size(p.dtype) * (double)ld[t] * (double)a.K * (double)a.B;
+        if (!need[t]) continue;
+        if (bytes > (double)ctx->total_mem / 8) return TFB_OK;
+        if ((t == 0 ? blk_a : blk_b)->alloc(ctx, (size_t)bytes) != TFB_OK) return TFB_OK;
+    }
+    *q = p;
+    if (need[0] && need[1]) {
+        q->k.assign(1, Mode{a.K, {0, 0, 0, 0}});
+        q->batch.assign(1, Mode{a.B, {0, 0, 0, 0}});
+    }
+    for (int t = 0; t < 2; ++t) {
+        if (!need[t]) continue;
+        void* dst = (t == 0 ? blk_a : blk_b)->ptr;
+        std::vector<Mode> modes;
+        auto put = [&](const std::vector<Mode>& g, int64_t stride) {
+            for (const Mode& m : g) {
+                modes.push_back(Mode{m.extent, {m.s[t], stride, 0, 0}});
+                stride *= m.extent;
+            }
+        };
+        put(t == 0 ? p.m : p.n, 1);
+        put(p.k, ld[t]);
+        put(p.batch, ld[t] * a.K);
+        sort_and_fuse(modes, 1, 2);
+        if ((int)modes.size() > kMaxRank) return TFB_OK;
+        LoopNest nest;
+        TFB_TRY(make_nest(modes, &nest));
+        TFB_TRY(launch_permute(ctx, p.dtype, nest, t == 0 ? p.a : p.b, dst, Scalar{1.0, 0.0}, Scalar{0.0, 0.0}, false));
+        std::vector<Mode>& free_q = t == 0 ? q->m : q->n;
+        free_q.assign(1, Mode{ld[t], {0, 0, 0, 0}});
+        free_q[0].s[t] = 1;
+        if (t == 0) q->a = dst; else q->b = dst;
+        q->k[0].s[t] = ld[t];
+        if (!q->batch.empty()) q->batch[0].s[t] = ld[t] * a.K;
+    }
+    *ready = true;
+    return TFB_OK;
+}
+
 tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined, bool four_products) {
     *declined = false;
     if (p.dtype != TFB_F64 && p.dtype != TFB_C64) {
@@ -519,6 +586,13 @@ tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined,
     fill_args(p, *t, &a);
     const int shape = env_int("TFB_DMMA_TILE", 0);  // 0 auto, 1 small, 2 big
     const bool use_tma = !env_int("TFB_NO_DMMA_TMA", 0);
+    auto on_copies = [&](bool small, bool* d) -> tfb_status {
+        PoolBlock blk_a, blk_b;
+        ContractProblem q;
+        bool ready = false;
+        TFB_TRY(repack_for_tma(ctx, p, a, &blk_a, &blk_b, &q, &ready));
+        return ready ? run_tma(ctx, q, a, small, true, d) : TFB_OK;
+    };
     if (p.dtype == TFB_F64) {
         // 64 x 64 tiles below a fourteenth of the SMs' worth of 128 x 128 ones: 400^3 17.7 against 23.7 us,
         // 500^3 22.3 against 21.6, 900^3 88 against 75.
@@ -532,6 +606,8 @@ tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined,
         if (use_tma) {
             bool d = true;
             TFB_TRY(run_tma(ctx, p, a, small, false, &d));
+            if (!d) return TFB_OK;
+            TFB_TRY(on_copies(small, &d));
             if (!d) return TFB_OK;
         }
         return small_gather ? run_cfg<RealSmall>(ctx, p, a) : run_cfg<RealBig>(ctx, p, a);
@@ -555,6 +631,8 @@ tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined,
     }
     if (use_tma) {
         TFB_TRY(run_tma(ctx, p, a, small, true, &d));
+        if (!d) return TFB_OK;
+        TFB_TRY(on_copies(small, &d));
         if (!d) return TFB_OK;
     }
     return small_gather ? run_cfg<CplxSmall>(ctx, p, a) : run_cfg<CplxMain>(ctx, p, a);

@@ -1,5 +1,5 @@
 """Double-precision contractions whose extents no short run divides: the four-product complex form on
-one load per run.  Sizes lie around
+one load per run, and products on copies of operands that no tensor map can describe.  Sizes lie around
 the edges of the tiles (32, 64, 128), of a k-iteration (16) and of a run (8, 4).
 
 The bound is that of a dot product, part by part: K + 4 roundings of |A| |B| (twice the terms in each
@@ -43,3 +43,17 @@ def test_complex_extents(tb, oracle, notation, mnk, conj):
     size = {"i": m, "k": n, "j": k, "b": 3}
     shapes = [tuple(size[c] for c in t) for t in notation.split("->")[0].split(",")]
     run(tb, oracle, notation, shapes, np.complex128, conj, 0.5)
+
+
+@pytest.mark.parametrize("notation,sizes", [
+    ("ij,jk->ik", dict(i=331, j=1021, k=333)),  # odd leading extents
+    ("ji,jk->ik", dict(i=129, j=6001, k=131)),
+    ("ijk,kjl->il", dict(i=131, j=57, k=103, l=137)),  # contracted modes in different orders
+    ("bij,bjk->bik", dict(b=21, i=67, j=1025, k=71)),  # the batch index innermost
+    ("ijab,abk->kij", dict(i=9, j=31, a=65, b=17, k=331)),
+])
+@pytest.mark.parametrize("dtype", [np.float64, np.complex128])
+def test_operands_without_a_map(tb, oracle, notation, sizes, dtype):
+    assert 2 * np.prod([float(v) for v in sizes.values()]) >= 2e8  # from here on operands are copied
+    shapes = [tuple(sizes[c] for c in t) for t in notation.split("->")[0].split(",")]
+    run(tb, oracle, notation, shapes, dtype, False, 0.5)
