@@ -1,0 +1,89 @@
+"""Reductions and element-wise products around the edges of their thread layouts: a handful of kept elements
+under a long range and the other way round, short inner runs, unit stride on either side, several
+slices, misaligned and odd rows.
+
+Sums: any order of n terms is off by at most n - 1 roundings of the sum of magnitudes (one more for
+alpha).  Max and Min are exact, products take one rounding (four of |x||y| for a complex one)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def eps(dtype):
+    return np.finfo(np.dtype(dtype)).eps / 2
+
+
+@pytest.mark.parametrize("shape,kept", [
+    ((1,), []), ((257,), []), ((100003,), []), ((5, 70001), [0]), ((70001, 5), [0]), ((3, 4099, 7), [0, 2]),
+    ((25, 8, 513), [1, 2]), ((27, 38, 1191), [1]), ((12, 56, 881, 17), [0, 3]), ((9, 40, 33), [0, 2]),
+    ((63, 300), [1]), ((64, 2049), [1]), ((2048, 65), [1]), ((129, 2, 130), [0, 2]), ((600, 700), [0]),
+])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.complex64, np.complex128])
+@pytest.mark.parametrize("turned", [False, True])
+def test_reduce_layouts(tb, oracle, shape, kept, dtype, turned):
+    x = oracle.normal(3, shape, dtype)
+    t = tb.Tensor.from_numpy(x)
+    if turned:  # reversed index order: the unit stride changes sides
+        order = list(range(len(shape)))[::-1]
+        t, x = t.permute(order), x.transpose(order)
+        kept = [len(shape) - 1 - k for k in kept][::-1]
+    axes = tuple(i for i in range(x.ndim) if i not in kept)
+    out_shape = tuple(x.shape[i] for i in kept)
+    ops = ["Sum"] if np.dtype(dtype).kind == "c" else ["Sum", "Max", "Min"]
+    if not axes:
+        return
+    for op in ops:
+        c = oracle.normal(4, out_shape or (1,), dtype).reshape(out_shape)
+        out = tb.Tensor.from_numpy(c)
+        plan = tb.CudaBackend.plan(tb.PrimDescriptor.Reduce(list(range(x.ndim)), kept, tb.ReduceOp[op]), [x.shape, out_shape], dtype)
+        beta = 0.5 if op == "Sum" else 0.0
+        tb.CudaBackend.execute(plan, 1.0, [t], beta, out)
+        got = out.to_numpy()
+        if op == "Sum":
+            wide = np.complex128 if np.dtype(dtype).kind == "c" else np.float64
+            n = x.size // max(1, got.size)
+            bound = 2 * (n + 2) * eps(dtype) * (abs(x).astype(np.float64).sum(axis=axes) + 0.5 * abs(c))
+            assert (abs(got - (x.astype(wide).sum(axis=axes) + 0.5 * c.astype(wide))) <= bound).all()
+        else:
+            assert np.array_equal(got, x.max(axis=axes) if op == "Max" else x.min(axis=axes))
+
+
+@pytest.mark.parametrize("special", [-np.inf, np.nan, np.finfo(np.float64).min])
+def test_max_of_special_values(tb, special):
+    x = np.full((300, 41), special)
+    x[7, 5] = np.finfo(np.float64).min if special == -np.inf else special
+    out = tb.Tensor.from_numpy(np.zeros(41))
+    plan = tb.CudaBackend.plan(tb.PrimDescriptor.Reduce([0, 1], [1], tb.ReduceOp.Max), [x.shape, (41,)], np.float64)
+    tb.CudaBackend.execute(plan, 1.0, [tb.Tensor.from_numpy(x)], 0.0, out)
+    assert np.array_equal(out.to_numpy(), x.max(axis=0), equal_nan=True)
+
+
+@pytest.mark.parametrize("notation", ["asb,b->asb", "a,asb->asb", "asb,asb->asb", "asb,a->asb", "asb,bsa->asb", "asb,s->asb"])
+@pytest.mark.parametrize("size", [(1, 1, 1), (4, 2, 8), (33, 3, 65), (64, 2, 130), (1025, 4, 31)])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.complex64, np.complex128])
+@pytest.mark.parametrize("beta,offset", [(0.0, 0), (0.5, 1)])
+def test_elementwise_layouts(tb, oracle, notation, size, dtype, beta, offset):
+    ext = dict(zip("asb", size))
+    ins, out_labels = notation.split("->")
+    arrays = [oracle.normal(5 + i, [ext[c] for c in t], dtype) for i, t in enumerate(ins.split(","))]
+    c = oracle.normal(8, [ext[l] for l in out_labels], dtype)
+
+    def put(x):  # `offset` elements into a buffer: rows lose their 16-byte alignment
+        flat = np.concatenate([np.zeros(offset, x.dtype), x.reshape(-1, order="F"), np.zeros(3, x.dtype)])
+        whole = tb.Tensor.from_numpy(flat)
+        strides, acc = [], 1
+        for d in x.shape:
+            strides.append(acc)
+            acc *= d
+        return tb.Tensor(whole._block, x.shape, strides, offset, x.dtype, whole.logical_memory_space())
+
+    ops = [put(x) for x in arrays]
+    out = put(c)
+    if np.dtype(dtype).kind == "c":
+        ops[1], arrays[1] = ops[1].into_conj(), arrays[1].conj()
+    tb.einsum_into(notation, ops, 1.0, beta, out)
+    wide = np.complex128 if np.dtype(dtype).kind == "c" else np.float64
+    prod = np.einsum(notation, *[x.astype(wide) for x in arrays])
+    bound = 8 * eps(dtype) * (np.einsum(notation, *[abs(x).astype(np.float64) for x in arrays]) + abs(beta) * abs(c))
+    assert (abs(out.to_numpy() - (prod + beta * c.astype(wide))) <= bound).all()
