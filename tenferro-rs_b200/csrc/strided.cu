@@ -495,14 +495,16 @@ tfb_status launch_elementwise_mul(tfb_ctx* ctx, int dtype, const LoopNest& nest,
 }
 
 // ------------------------------------------------------------------ reduce
-// Grid: x over groups of kept elements, y over `splits` slices of the reduced range.
-// Two thread layouts:
-//   LANES_ON_RED = true : a warp shares one kept element, lanes stride the reduced range
-//                         (input stride 1 lies in a reduced mode);
-//   LANES_ON_RED = false: each thread owns one kept element and walks its reduced slice
-//                         (input stride 1 lies in a kept mode: neighbouring threads coalesce).
-// With splits > 1 partial results go to `partial[split][kept]` and reduce_finish_kernel
-// combines them in a fixed order, so results do not depend on scheduling.
+// A block is TX kept elements x G threads each, the reduced range of an element dealt out to its G
+// threads in turns (times gridDim.y slices).  Neighbouring threads follow the input's unit stride:
+//   RED_FAST    the G threads of an element are neighbours (unit stride in a reduced mode)
+//   otherwise   neighbouring threads hold neighbouring kept elements
+// Each thread has eight loads in flight whatever the inner run's length.  With several slices the partial
+// results go to `partial[slice][kept]` and reduce_finish_kernel combines them.  All orders are fixed:
+// results do not depend on scheduling.  Bound by HBM from about 20 MB on.  Before, a warp took
+// one kept element (seven of eight warps idle when there was one only) and a thread of the finishing kernel
+// all slices of one: 700473 x 156 f32 to a scalar 446 -> 84 us, 12 x 56 x 8810 x 17 f64 keeping the outer ones
+// 307 -> 140, 27 x 38 x 11916 f64 keeping the middle 142 -> 24, 301 x 2003 x 203 keeping the outer 178 -> 158.
 template <typename T, int OP>
 struct Red {
     __device__ static T init() {
@@ -517,90 +519,237 @@ struct Red {
     }
 };
 
-template <typename T, int OP, bool LANES_ON_RED>
-__global__ void __launch_bounds__(256) reduce_kernel(LoopNest kept, LoopNest red, const T* __restrict__ in, T* out,
-                                                     T* partial, int splits, EpilogueArgs<T> ep) {
-    const int64_t n_red = red.total;
-    const int64_t chunk = (n_red + splits - 1) / splits;
-    const int64_t r0 = (int64_t)blockIdx.y * chunk;
-    const int64_t r1 = min(n_red, r0 + chunk);
-    if (LANES_ON_RED) {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const int64_t warps_total = (int64_t)gridDim.x * 8;
-        for (int64_t ko = (int64_t)blockIdx.x * 8 + warp; ko < kept.total; ko += warps_total) {
-            int64_t koff[2];
-            decompose<2>(kept, 0, ko, koff);
-            // Walk the reduced range in runs along its innermost mode (no division per
-            // element); eight independent partial results per lane keep loads in flight.
-            T part[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) part[u] = Red<T, OP>::init();
-            const int64_t e0 = red.extent[0], s0 = red.stride[0][0];
-            int64_t r = r0;
-            while (r < r1) {
-                int64_t q, i0;
-                divmod(r, e0, q, i0);
-                int64_t roff[1];
-                decompose<1>(red, 1, q, roff);
-                const int64_t run = min(e0 - i0, r1 - r);
-                const T* p = in + koff[0] + roff[0] + i0 * s0;
-                int64_t i = lane;
-                for (; i + 224 < run; i += 256) {
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) part[u] = Red<T, OP>::comb(part[u], p[(i + 32 * u) * s0]);
-                }
-                for (; i < run; i += 32) part[0] = Red<T, OP>::comb(part[0], p[i * s0]);
-                r += run;
-            }
-            T acc = Red<T, OP>::comb(Red<T, OP>::comb(Red<T, OP>::comb(part[0], part[1]), Red<T, OP>::comb(part[2], part[3])),
-                                     Red<T, OP>::comb(Red<T, OP>::comb(part[4], part[5]), Red<T, OP>::comb(part[6], part[7])));
-#pragma unroll
-            for (int s = 16; s > 0; s >>= 1) acc = Red<T, OP>::comb(acc, Ops<T>::shfl_down(acc, s));
-            if (lane == 0) {
-                if (splits == 1)
-                    out[koff[1]] = ep.apply(acc, out + koff[1]);
-                else
-                    partial[(int64_t)blockIdx.y * kept.total + ko] = acc;
-            }
+// Combines the values of the G threads of each kept element; the result is valid where g == 0.
+template <typename T, int OP>
+__device__ __forceinline__ T combine_group(T acc, T* sh, int g, int G, int step) {
+    if (G == 1) return acc;
+    __syncthreads();
+    sh[threadIdx.x] = acc;
+    for (int s = G >> 1; s > 0; s >>= 1) {
+        __syncthreads();
+        if (g < s) sh[threadIdx.x] = Red<T, OP>::comb(sh[threadIdx.x], sh[threadIdx.x + s * step]);
+    }
+    return sh[threadIdx.x];
+}
+
+// Walks a thread's elements r0 + g, r0 + g + G, ... of the reduced range without a division per element.
+// One mode: a pointer step.  Two: a step in both with a carry.  More: the linear index by multiplication.
+template <int RANK, typename N>
+struct RedWalk;
+template <typename N>
+struct RedWalk<1, N> {
+    int64_t off, step;
+    __device__ __forceinline__ RedWalk(const N& red, int64_t r, int G) : off(r * red.stride[0][0]), step(G * red.stride[0][0]) {}
+    __device__ __forceinline__ int64_t next(const N&, int64_t, int) {
+        const int64_t o = off;
+        off += step;
+        return o;
+    }
+};
+template <>
+struct RedWalk<2, Nest32> {
+    uint32_t i0, g0, e0;
+    int64_t off, step, wrap;
+    __device__ __forceinline__ RedWalk(const Nest32& red, int64_t r, int G) : e0(red.div[0].d) {
+        const uint32_t q = red.div[0].quotient((uint32_t)r), gq = red.div[0].quotient((uint32_t)G);
+        i0 = (uint32_t)r - q * e0;
+        g0 = (uint32_t)G - gq * e0;
+        off = i0 * red.stride[0][0] + q * red.stride[0][1];
+        step = g0 * red.stride[0][0] + gq * red.stride[0][1];
+        wrap = red.stride[0][1] - (int64_t)e0 * red.stride[0][0];
+    }
+    __device__ __forceinline__ int64_t next(const Nest32&, int64_t, int) {
+        const int64_t o = off;
+        i0 += g0;
+        off += step;
+        if (i0 >= e0) {
+            i0 -= e0;
+            off += wrap;
         }
-    } else {
-        const int64_t threads_total = (int64_t)gridDim.x * blockDim.x;
-        for (int64_t ko = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; ko < kept.total; ko += threads_total) {
-            int64_t koff[2];
+        return o;
+    }
+};
+template <typename N>
+struct RedWalk<0, N> {
+    __device__ __forceinline__ RedWalk(const N&, int64_t, int) {}
+    __device__ __forceinline__ int64_t next(const N& red, int64_t r, int) {
+        int64_t off[1];
+        decompose<1>(red, 0, r, off);
+        return off[0];
+    }
+};
+
+// Loads in flight per thread, and CTAs per SM that their registers leave: 48 to 64 KB per SM.
+template <typename T>
+constexpr int kRedLoads = sizeof(T) == 4 ? 16 : 8;
+template <typename T>
+constexpr int kRedCtas = sizeof(T) == 16 ? 2 : sizeof(T) == 4 ? 3 : 4;
+template <typename T, int OP, bool RED_FAST, int RANK, typename N>
+__global__ void __launch_bounds__(256, kRedCtas<T>) reduce_kernel(const __grid_constant__ N kept, const __grid_constant__ N red,
+                                                     const T* __restrict__ in, T* out, T* partial, int log_g, int64_t chunk,
+                                                     EpilogueArgs<T> ep) {
+    constexpr int U = kRedLoads<T>;
+    __shared__ T sh[256];
+    const int G = 1 << log_g, TX = 256 >> log_g;
+    const int g = RED_FAST ? threadIdx.x & (G - 1) : threadIdx.x / TX;
+    const int x = RED_FAST ? threadIdx.x >> log_g : threadIdx.x & (TX - 1);
+    const int64_t r0 = (int64_t)blockIdx.y * chunk, r1 = min(red.total, r0 + chunk);
+    const int64_t groups = (kept.total + TX - 1) / TX;
+    for (int64_t kb = blockIdx.x; kb < groups; kb += gridDim.x) {
+        const int64_t ko = kb * TX + x;
+        int64_t koff[2] = {0, 0};
+        T part[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) part[u] = Red<T, OP>::init();
+        if (ko < kept.total && r0 + g < r1) {
             decompose<2>(kept, 0, ko, koff);
-            T acc = Red<T, OP>::init();
-            // Walk the reduced range mode 0 innermost without re-dividing per element.
-            const int64_t e0 = red.extent[0], s0 = red.stride[0][0];
-            int64_t r = r0;
-            while (r < r1) {
-                int64_t q, i0;
-                divmod(r, e0, q, i0);
-                int64_t roff[1];
-                decompose<1>(red, 1, q, roff);
-                int64_t run = min(e0 - i0, r1 - r);
-                const T* p = in + koff[0] + roff[0] + i0 * s0;
-                for (int64_t i = 0; i < run; ++i) acc = Red<T, OP>::comb(acc, p[i * s0]);
-                r += run;
+            const T* p = in + koff[0];
+            RedWalk<RANK, N> walk(red, r0 + g, G);
+            int64_t r = r0 + g;
+            for (; r + (U - 1) * G < r1; r += U * G) {
+                T v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = p[walk.next(red, r + u * G, G)];
+#pragma unroll
+                for (int u = 0; u < U; ++u) part[u] = Red<T, OP>::comb(part[u], v[u]);
             }
-            if (splits == 1)
-                out[koff[1]] = ep.apply(acc, out + koff[1]);
-            else
-                partial[(int64_t)blockIdx.y * kept.total + ko] = acc;
+            T v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = r + u * G < r1 ? p[walk.next(red, r + u * G, G)] : Red<T, OP>::init();
+#pragma unroll
+            for (int u = 0; u < U; ++u) part[u] = Red<T, OP>::comb(part[u], v[u]);
+        }
+#pragma unroll
+        for (int s = U / 2; s > 0; s >>= 1)
+#pragma unroll
+            for (int u = 0; u < s; ++u) part[u] = Red<T, OP>::comb(part[u], part[u + s]);
+        const T acc = combine_group<T, OP>(part[0], sh, g, G, RED_FAST ? 1 : TX);
+        if (g == 0 && ko < kept.total) {
+            if (!partial) out[koff[1]] = ep.apply(acc, out + koff[1]);
+            else partial[(int64_t)blockIdx.y * kept.total + ko] = acc;
         }
     }
 }
 
-template <typename T, int OP>
-__global__ void __launch_bounds__(256) reduce_finish_kernel(LoopNest kept, const T* __restrict__ partial, T* out,
-                                                            int splits, EpilogueArgs<T> ep) {
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t ko = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; ko < kept.total; ko += stride) {
-        int64_t koff[2];
-        decompose<2>(kept, 0, ko, koff);
-        T acc = partial[ko];
-        for (int s = 1; s < splits; ++s) acc = Red<T, OP>::comb(acc, partial[(int64_t)s * kept.total + ko]);
-        out[koff[1]] = ep.apply(acc, out + koff[1]);
+// Combines the slices of each kept element: TX elements x G threads per block, as above.
+template <typename T, int OP, typename N>
+__global__ void __launch_bounds__(256) reduce_finish_kernel(N kept, const T* __restrict__ partial, T* out, int splits, int log_g,
+                                                            EpilogueArgs<T> ep) {
+    __shared__ T sh[256];
+    const int G = 1 << log_g, TX = 256 >> log_g, g = threadIdx.x / TX, x = threadIdx.x & (TX - 1);
+    const int64_t groups = (kept.total + TX - 1) / TX;
+    for (int64_t kb = blockIdx.x; kb < groups; kb += gridDim.x) {
+        const int64_t ko = kb * TX + x;
+        T acc = Red<T, OP>::init();
+        if (ko < kept.total) {
+#pragma unroll 8
+            for (int s = g; s < splits; s += G) acc = Red<T, OP>::comb(acc, partial[(int64_t)s * kept.total + ko]);
+        }
+        acc = combine_group<T, OP>(acc, sh, g, G, TX);
+        if (g == 0 && ko < kept.total) {
+            int64_t koff[2];
+            decompose<2>(kept, 0, ko, koff);
+            out[koff[1]] = ep.apply(acc, out + koff[1]);
+        }
     }
+}
+
+// How a reduction is laid out over the chip.
+struct ReduceShape {
+    bool red_fast;
+    int log_g = 0, splits = 1;
+    int64_t chunk = 0;
+    unsigned grid = 1;
+};
+static ReduceShape reduce_shape(const tfb_ctx* ctx, const LoopNest& kept, const LoopNest& red, int ctas, int64_t max_splits) {
+    // Smallest |input stride| among reduced and kept modes.
+    auto min_stride = [](const LoopNest& n) {
+        int64_t m = INT64_MAX;
+        for (int d = 0; d < n.rank; ++d) {
+            const int64_t s = n.stride[0][d] < 0 ? -n.stride[0][d] : n.stride[0][d];
+            if (n.extent[d] > 1 && s < m) m = s;
+        }
+        return m;
+    };
+    ReduceShape r;
+    r.red_fast = kept.rank == 0 || min_stride(red) < min_stride(kept);
+    const int64_t sms = ctx->sm_count;
+    int g = 1;
+    if (r.red_fast) {
+        // A block per element once the elements alone cannot fill the chip, a warp for long ranges, eight
+        // threads (64 bytes of f64) for short ones.
+        if (red.total >= 2048 && kept.total < sms * 64) g = 256;
+        else g = red.total >= 64 ? 32 : 8;
+    } else {
+        while (g < 32 && kept.total * g <= 128) g *= 2;  // few kept elements: the rest of the block shares them
+        while (g > 1 && g > red.total) g /= 2;
+    }
+    while ((1 << r.log_g) < g) ++r.log_g;
+    // Slices only where a thread keeps 32 elements (below that the finishing launch costs more): the fewest
+    // that leave no more than a fourteenth of the last wave's places empty, else the fullest.
+    const int64_t tx = 256 >> r.log_g, groups = (kept.total + tx - 1) / tx, slots = sms * ctas;
+    if (groups < 4 * slots) {
+        const int64_t most = std::min<int64_t>(std::min<int64_t>(red.total / ((int64_t)g * 32), max_splits),
+                                               std::max<int64_t>(1, 4 * slots / groups));
+        double best = 0;
+        for (int64_t s = 1; s <= most && best < 0.93; ++s) {
+            const int64_t blocks = groups * s;
+            const double full = (double)blocks / (double)((blocks + slots - 1) / slots * slots);
+            if (full > best) {
+                best = full;
+                r.splits = (int)s;
+            }
+        }
+    }
+    r.chunk = (red.total + r.splits - 1) / r.splits;
+    r.splits = (int)((red.total + r.chunk - 1) / r.chunk);
+    r.grid = (unsigned)std::min<int64_t>(groups, slots * 8);
+    return r;
+}
+
+template <typename T, int OP, typename N>
+static void reduce_launch(tfb_ctx* ctx, const N& kept, const N& red, const T* in, T* out, T* partial, const ReduceShape& r,
+                          const EpilogueArgs<T>& ep) {
+    const dim3 grid(r.grid, (unsigned)r.splits);
+    auto go = [&](auto rank) {
+        constexpr int RANK = decltype(rank)::value;
+        if (r.red_fast)
+            reduce_kernel<T, OP, true, RANK><<<grid, 256, 0, ctx->stream>>>(kept, red, in, out, partial, r.log_g, r.chunk, ep);
+        else
+            reduce_kernel<T, OP, false, RANK><<<grid, 256, 0, ctx->stream>>>(kept, red, in, out, partial, r.log_g, r.chunk, ep);
+    };
+    if (red.rank == 1) return go(std::integral_constant<int, 1>{});
+    if constexpr (std::is_same<N, Nest32>::value)
+        if (red.rank == 2) return go(std::integral_constant<int, 2>{});
+    go(std::integral_constant<int, 0>{});
+}
+template <typename T, int OP, typename N>
+static void reduce_finish_launch(tfb_ctx* ctx, const N& kept, T* out, const T* partial, const ReduceShape& r,
+                                 const EpilogueArgs<T>& ep) {
+    int log_g = 0;  // about eight slices per thread
+    while (log_g < 8 && (r.splits >> log_g) > 8) ++log_g;
+    const int64_t tx = 256 >> log_g;
+    const unsigned grid = (unsigned)std::min<int64_t>((kept.total + tx - 1) / tx, (int64_t)ctx->sm_count * 32);
+    reduce_finish_kernel<T, OP><<<grid, 256, 0, ctx->stream>>>(kept, partial, out, r.splits, log_g, ep);
+}
+// Both launches; `partial` holds r.splits slices when there are several.
+template <typename T, int OP>
+static tfb_status reduce_run(tfb_ctx* ctx, const LoopNest& kept, const LoopNest& red, const void* in, void* out, void* partial,
+                             const ReduceShape& r, const EpilogueArgs<T>& ep) {
+    const bool small = Nest32::fits(kept) && Nest32::fits(red);
+    {
+        LaunchScope ls(ctx, "reduce");
+        if (small) reduce_launch<T, OP>(ctx, Nest32(kept), Nest32(red), (const T*)in, (T*)out, (T*)partial, r, ep);
+        else reduce_launch<T, OP>(ctx, kept, red, (const T*)in, (T*)out, (T*)partial, r, ep);
+    }
+    TFB_CUDA(cudaGetLastError());
+    if (r.splits > 1) {
+        LaunchScope ls(ctx, "reduce_finish");
+        if (small) reduce_finish_launch<T, OP>(ctx, Nest32(kept), (T*)out, (const T*)partial, r, ep);
+        else reduce_finish_launch<T, OP>(ctx, kept, (T*)out, (const T*)partial, r, ep);
+    }
+    TFB_CUDA(cudaGetLastError());
+    return TFB_OK;
 }
 
 template <typename T, int OP>
@@ -621,54 +770,10 @@ static tfb_status reduce_typed(tfb_ctx* ctx, const LoopNest& kept, const LoopNes
                             }(),
                             out, beta);
     }
-    // Which layout?  Smallest |input stride| among reduced vs kept modes.
-    auto min_stride = [](const LoopNest& n) {
-        int64_t m = INT64_MAX;
-        for (int d = 0; d < n.rank; ++d) {
-            int64_t s = n.stride[0][d] < 0 ? -n.stride[0][d] : n.stride[0][d];
-            if (n.extent[d] > 1 && s < m) m = s;
-        }
-        return m;
-    };
-    const bool lanes_on_red = kept.rank == 0 || min_stride(red) < min_stride(kept);
-    const int sms = ctx->sm_count;
-    int64_t groups = lanes_on_red ? (kept.total + 7) / 8 : (kept.total + 255) / 256;
-    int64_t target = (int64_t)sms * 8;
-    int splits = 1;
-    if (groups < target) {
-        int64_t want = target / (groups > 0 ? groups : 1);
-        int64_t min_chunk = lanes_on_red ? 1024 : 64;
-        int64_t max_splits = (red.total + min_chunk - 1) / min_chunk;
-        splits = (int)(want < max_splits ? want : max_splits);
-        if (splits < 1) splits = 1;
-        if (splits > 1024) splits = 1024;
-    }
-    int64_t gx = groups < target * 4 ? groups : target * 4;
-    if (gx < 1) gx = 1;
-    dim3 grid((unsigned)gx, (unsigned)splits);
+    const ReduceShape r = reduce_shape(ctx, kept, red, kRedCtas<T>, INT64_MAX);
     PoolBlock ws;
-    T* partial = nullptr;
-    if (splits > 1) {
-        TFB_TRY(ws.alloc(ctx, sizeof(T) * (size_t)splits * (size_t)kept.total));
-        partial = (T*)ws.ptr;
-    }
-    {
-    LaunchScope ls(ctx, "reduce");
-    if (lanes_on_red)
-        reduce_kernel<T, OP, true><<<grid, 256, 0, ctx->stream>>>(kept, red, (const T*)in, (T*)out, partial, splits, ep);
-    else
-        reduce_kernel<T, OP, false><<<grid, 256, 0, ctx->stream>>>(kept, red, (const T*)in, (T*)out, partial, splits,
-                                                                   ep);
-    }
-    TFB_CUDA(cudaGetLastError());
-    if (splits > 1) {
-        int64_t blocks = (kept.total + 255) / 256;
-        int g2 = (int)(blocks < (int64_t)sms * 8 ? blocks : (int64_t)sms * 8);
-        LaunchScope ls(ctx, "reduce_finish");
-        reduce_finish_kernel<T, OP><<<g2, 256, 0, ctx->stream>>>(kept, partial, (T*)out, splits, ep);
-        TFB_CUDA(cudaGetLastError());
-    }
-    return TFB_OK;
+    if (r.splits > 1) TFB_TRY(ws.alloc(ctx, sizeof(T) * (size_t)r.splits * (size_t)kept.total));
+    return reduce_run<T, OP>(ctx, kept, red, in, out, ws.ptr, r, ep);
 }
 
 template <typename T>
@@ -733,49 +838,9 @@ template <typename T, int OP>
 static tfb_status reduce_static_typed(tfb_ctx* ctx, const LoopNest& kept, const LoopNest& red, const void* in, void* out,
                                       Scalar alpha, Scalar beta, bool conj, void* scratch) {
     EpilogueArgs<T> ep = EpilogueArgs<T>::make(alpha, beta, conj);
-    auto min_stride = [](const LoopNest& n) {
-        int64_t m = INT64_MAX;
-        for (int d = 0; d < n.rank; ++d) {
-            int64_t s = n.stride[0][d] < 0 ? -n.stride[0][d] : n.stride[0][d];
-            if (n.extent[d] > 1 && s < m) m = s;
-        }
-        return m;
-    };
-    const bool lanes_on_red = kept.rank == 0 || min_stride(red) < min_stride(kept);
-    const int sms = ctx->sm_count;
-    const int64_t groups = lanes_on_red ? (kept.total + 7) / 8 : (kept.total + 255) / 256;
-    const int64_t target = (int64_t)sms * 8;
-    int64_t splits = 1;
-    if (groups < target) {
-        const int64_t want = target / (groups > 0 ? groups : 1);
-        const int64_t min_chunk = lanes_on_red ? 1024 : 64;
-        const int64_t max_splits = (red.total + min_chunk - 1) / min_chunk;
-        splits = want < max_splits ? want : max_splits;
-        // The partials have to fit the fixed array.
-        const int64_t fit = (int64_t)(kStaticReduceBytes / (sizeof(T) * (size_t)kept.total));
-        if (splits > fit) splits = fit;
-        if (splits > 1024) splits = 1024;
-        if (splits < 1) splits = 1;
-    }
-    int64_t gx = groups < target * 4 ? groups : target * 4;
-    if (gx < 1) gx = 1;
-    dim3 grid((unsigned)gx, (unsigned)splits);
-    T* partial = splits > 1 ? (T*)scratch : nullptr;
-    count_launch(1);
-    if (lanes_on_red)
-        reduce_kernel<T, OP, true><<<grid, 256, 0, ctx->stream>>>(kept, red, (const T*)in, (T*)out, partial, (int)splits, ep);
-    else
-        reduce_kernel<T, OP, false><<<grid, 256, 0, ctx->stream>>>(kept, red, (const T*)in, (T*)out, partial, (int)splits,
-                                                                   ep);
-    TFB_CUDA(cudaGetLastError());
-    if (splits > 1) {
-        const int64_t blocks = (kept.total + 255) / 256;
-        const int g2 = (int)(blocks < (int64_t)sms * 8 ? blocks : (int64_t)sms * 8);
-        count_launch(1);
-        reduce_finish_kernel<T, OP><<<g2, 256, 0, ctx->stream>>>(kept, partial, (T*)out, (int)splits, ep);
-        TFB_CUDA(cudaGetLastError());
-    }
-    return TFB_OK;
+    // The partials have to fit the fixed array.
+    const ReduceShape r = reduce_shape(ctx, kept, red, kRedCtas<T>, (int64_t)(kStaticReduceBytes / (sizeof(T) * (size_t)kept.total)));
+    return reduce_run<T, OP>(ctx, kept, red, in, out, r.splits > 1 ? scratch : nullptr, r, ep);
 }
 
 template <typename T>
