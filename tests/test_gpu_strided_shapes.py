@@ -87,3 +87,40 @@ def test_elementwise_layouts(tb, oracle, notation, size, dtype, beta, offset):
     prod = np.einsum(notation, *[x.astype(wide) for x in arrays])
     bound = 8 * eps(dtype) * (np.einsum(notation, *[abs(x).astype(np.float64) for x in arrays]) + abs(beta) * abs(c))
     assert (abs(out.to_numpy() - (prod + beta * c.astype(wide))) <= bound).all()
+
+
+@pytest.mark.parametrize("shape,perm", [
+    ((5, 7), (1, 0)), ((3, 5, 7, 2, 9), (4, 3, 2, 1, 0)), ((14, 9, 15, 10, 11), (4, 2, 3, 1, 0)), ((33, 65, 7), (2, 0, 1)),
+    ((11, 13, 9, 7, 5), (0, 4, 1, 2, 3)), ((2, 300, 3, 70), (0, 3, 2, 1)), ((2, 129, 257), (0, 2, 1)), ((257, 2), (1, 0)),
+    ((1000, 3, 2), (2, 1, 0)), ((64, 64, 3), (1, 2, 0)), ((68, 132), (1, 0)), ((3, 6, 30, 33, 2, 3), (1, 2, 4, 3, 5, 0)),
+    ((1, 513, 1, 70), (3, 2, 1, 0)), ((70, 71, 72), (0, 2, 1)), ((600, 601), (1, 0)),
+])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.complex64, np.complex128])
+@pytest.mark.parametrize("padded", [False, True])
+def test_permute_orders(tb, oracle, shape, perm, dtype, padded):
+    x = oracle.normal(6, shape, dtype)
+    dims = [shape[i] for i in perm]
+    if padded:  # gaps between the columns on both sides, last index of the output reversed
+        big = np.zeros([d + 1 for d in shape], x.dtype)
+        big[tuple(slice(0, d) for d in shape)] = x
+        base = tb.Tensor.from_numpy(big)
+        t = tb.Tensor(base._block, shape, base.strides(), 0, x.dtype, base.logical_memory_space())
+        hold = tb.Tensor.from_numpy(np.full([d + 2 for d in dims], 7, x.dtype))
+        strides = list(hold.strides())
+        strides[-1] = -strides[-1]
+        out = tb.Tensor(hold._block, dims, strides, (dims[-1] - 1) * -strides[-1], x.dtype, hold.logical_memory_space())
+    else:
+        t, out = tb.Tensor.from_numpy(x), tb.Tensor.from_numpy(np.zeros(dims, x.dtype))
+    for alpha, beta in ((1.0, 0.0), (2.0, -1.0)):
+        plan = tb.CudaBackend.plan(tb.PrimDescriptor.Permute(list(range(len(shape))), list(perm)), [shape, dims], dtype)
+        tb.CudaBackend.execute(plan, alpha, [t], beta, out)
+    # 2 x - x is exact
+    want = x.transpose(perm)
+    if padded:
+        got = hold.to_numpy()
+        inside = tuple(slice(0, d) for d in dims)
+        assert np.array_equal(got[inside][..., ::-1], want)
+        got[inside] = 7
+        assert (got == 7).all()  # nothing between the columns was written
+    else:
+        assert np.array_equal(out.to_numpy(), want)
