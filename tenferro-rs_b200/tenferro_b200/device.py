@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import ctypes as C
 import enum
+import functools
 import threading
 from dataclasses import dataclass
 from typing import List, Optional
@@ -123,14 +124,19 @@ class OpKind(enum.IntEnum):
     ElementwiseMul = 5
 
 
-def preferred_compute_devices(space: LogicalMemorySpace, op_kind: OpKind) -> List[ComputeDevice]:
-    """tenferro-device/src/lib.rs:92-105."""
+@functools.lru_cache(maxsize=256)
+def _preferred(kind: int, space_id: int, op_kind: int) -> tuple:
+    # A pure function of its arguments, asked for by every einsum call.
     out = (_lib.TfbComputeDevice * 16)()
     n = C.c_size_t(0)
-    kind = 1 if space.is_gpu else 0
-    check(lib.tfb_preferred_compute_devices(kind, space.space_id or 0, int(op_kind), out, 16, C.byref(n)))
+    check(lib.tfb_preferred_compute_devices(kind, space_id, op_kind, out, 16, C.byref(n)))
     names = {0: "cpu", 1: "cuda", 2: "hip"}
-    return [ComputeDevice(names[out[i].kind], out[i].device_id) for i in range(min(n.value, 16))]
+    return tuple(ComputeDevice(names[out[i].kind], out[i].device_id) for i in range(min(n.value, 16)))
+
+
+def preferred_compute_devices(space: LogicalMemorySpace, op_kind: OpKind) -> List[ComputeDevice]:
+    """tenferro-device/src/lib.rs:92-105."""
+    return list(_preferred(1 if space.is_gpu else 0, space.space_id or 0, int(op_kind)))
 
 
 # ---------------------------------------------------------------- context

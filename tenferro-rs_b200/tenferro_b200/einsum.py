@@ -10,7 +10,7 @@ import numpy as np
 
 from . import _lib
 from ._lib import lib
-from .device import Context, InvalidArgument, NoCompatibleComputeDevice, OpKind, check
+from .device import Context, InvalidArgument, NoCompatibleComputeDevice, OpKind, check, preferred_compute_devices
 from .prims import scalar_arg
 from .tensor import MemoryOrder, Tensor, check_same_space, dtype_code
 
@@ -19,7 +19,7 @@ def _shape_args(shapes: Sequence[Sequence[int]]):
     n = len(shapes)
     ranks = (C.c_size_t * max(n, 1))(*[len(s) for s in shapes])
     rows = [(C.c_size_t * max(len(s), 1))(*[int(x) for x in s]) for s in shapes]
-    dims = (_lib.c_size_p * max(n, 1))(*[C.cast(r, _lib.c_size_p) for r in rows])
+    dims = (_lib.c_size_p * max(n, 1))(*rows)  # (holds the rows alive)
     return ranks, dims, rows
 
 
@@ -38,16 +38,31 @@ class Subscripts:
             check(lib.tfb_subscripts_new(n, ranks, ptrs, len(output), out, C.byref(h)))
             _handle = h
         self.handle = _handle
-        self.inputs: List[List[int]] = []
-        for i in range(lib.tfb_subscripts_n_inputs(self.handle)):
-            n = lib.tfb_subscripts_input(self.handle, i, None, 0)
-            buf = (C.c_uint32 * max(n, 1))()
-            lib.tfb_subscripts_input(self.handle, i, buf, n)
-            self.inputs.append([buf[j] for j in range(n)])
-        n = lib.tfb_subscripts_output(self.handle, None, 0)
-        buf = (C.c_uint32 * max(n, 1))()
-        lib.tfb_subscripts_output(self.handle, buf, n)
-        self.output: List[int] = [buf[j] for j in range(n)]
+        self._labels = None
+
+    # The labels as Python lists are read back when somebody asks for them: an einsum call does not.
+    def _lists(self):
+        if self._labels is None:
+            def read(count, *args):
+                n = count(self.handle, *args, None, 0)
+                buf = (C.c_uint32 * max(n, 1))()
+                count(self.handle, *args, buf, n)
+                return [buf[j] for j in range(n)]
+
+            self._labels = ([read(lib.tfb_subscripts_input, i) for i in range(self.n_inputs)], read(lib.tfb_subscripts_output))
+        return self._labels
+
+    @property
+    def n_inputs(self) -> int:
+        return lib.tfb_subscripts_n_inputs(self.handle)
+
+    @property
+    def inputs(self) -> List[List[int]]:
+        return self._lists()[0]
+
+    @property
+    def output(self) -> List[int]:
+        return self._lists()[1]
 
     @classmethod
     def new(cls, inputs, output) -> "Subscripts":
@@ -83,8 +98,8 @@ class ContractionTree:
     @classmethod
     def optimize(cls, subscripts: Subscripts, shapes: Sequence[Sequence[int]]) -> "ContractionTree":
         ranks, dims, _rows = _shape_args(shapes)
-        if len(shapes) != len(subscripts.inputs):
-            raise InvalidArgument(f"{len(subscripts.inputs)} operands in the subscripts, {len(shapes)} shapes")
+        if len(shapes) != subscripts.n_inputs:
+            raise InvalidArgument(f"{subscripts.n_inputs} operands in the subscripts, {len(shapes)} shapes")
         h = C.c_void_p()
         check(lib.tfb_tree_optimize(subscripts.handle, ranks, dims, C.byref(h)))
         return cls(h, subscripts)
@@ -92,8 +107,8 @@ class ContractionTree:
     @classmethod
     def from_pairs(cls, subscripts: Subscripts, shapes, pairs: Sequence[Tuple[int, int]]) -> "ContractionTree":
         ranks, dims, _rows = _shape_args(shapes)
-        if len(shapes) != len(subscripts.inputs):
-            raise InvalidArgument(f"{len(subscripts.inputs)} operands in the subscripts, {len(shapes)} shapes")
+        if len(shapes) != subscripts.n_inputs:
+            raise InvalidArgument(f"{subscripts.n_inputs} operands in the subscripts, {len(shapes)} shapes")
         flat = (C.c_size_t * max(2 * len(pairs), 1))(*[int(x) for p in pairs for x in p])
         h = C.c_void_p()
         check(lib.tfb_tree_from_pairs(subscripts.handle, ranks, dims, len(pairs), flat, C.byref(h)))
@@ -131,13 +146,13 @@ def _select_context(operands: Sequence[Tensor], output: Optional[Tensor] = None)
     (tenferro-einsum/src/lib.rs:16-20, 179-207)."""
     tensors = list(operands) + ([output] if output is not None else [])
     space = check_same_space(tensors)
-    choice = None
-    for t in tensors:
-        devs = t.effective_compute_devices(OpKind.Contract)
-        if choice is None:
-            choice = devs
-        else:
-            choice = [d for d in choice if d in devs]
+    # Tensors without a pin of their own all have the space's default devices: asked for once.
+    lists = [t.effective_compute_devices(OpKind.Contract) for t in tensors if t._preferred is not None]
+    if len(lists) < len(tensors):
+        lists.insert(0, preferred_compute_devices(space, OpKind.Contract))
+    choice = lists[0]
+    for devs in lists[1:]:
+        choice = [d for d in choice if d in devs]
     cuda = [d for d in (choice or []) if d.kind == "cuda"]
     if not cuda:
         raise NoCompatibleComputeDevice(f"no compatible compute device for Contract on {space!r}")

@@ -112,11 +112,14 @@ class _Borrowed:
 
 def make_view(ptr: int, dims, strides, offset: int, conj: bool, keep: list) -> _lib.TfbView:
     """Build a tfb_view; the ctypes arrays are appended to `keep` so they outlive the call."""
-    n = len(dims)
-    d = (C.c_size_t * max(n, 1))(*dims)
-    s = (C.c_ssize_t * max(n, 1))(*strides)
+    d, s = _view_arrays(dims, strides)
     keep += [d, s]
-    return _lib.TfbView(C.c_void_p(ptr), n, d, s, offset, 1 if conj else 0)
+    return _lib.TfbView(ptr, len(dims), d, s, offset, 1 if conj else 0)
+
+
+def _view_arrays(dims, strides):
+    n = max(len(dims), 1)
+    return (C.c_size_t * n)(*dims), (C.c_ssize_t * n)(*strides)
 
 
 class Tensor:
@@ -134,6 +137,7 @@ class Tensor:
         if event is not None:
             self.event = event
         self._conj = bool(conj) and self.dtype.kind == "c"
+        self._arrays = None
 
     @property
     def event(self) -> Optional[CompletionEvent]:
@@ -280,7 +284,12 @@ class Tensor:
         """Non-blocking operand view (tenferro-tensor/src/lib.rs:473-488): pending work is
         ordered by the stream, the host does not wait."""
         ptr = self._block.ptr if self._block is not None else 0
-        return make_view(ptr, self._dims, self._strides, self._offset, self._conj, keep)
+        # dims and strides of a tensor never change: their C arrays are made once per tensor
+        arrays = self._arrays
+        if arrays is None:
+            arrays = self._arrays = _view_arrays(self._dims, self._strides)
+        keep.append(arrays)
+        return _lib.TfbView(ptr, len(self._dims), arrays[0], arrays[1], self._offset, 1 if self._conj else 0)
 
     # ------------------------------------------------------------ view operations (zero-copy)
     def permute(self, perm: Sequence[int]) -> "Tensor":
@@ -471,7 +480,7 @@ def check_same_space(tensors: Sequence[Tensor]) -> LogicalMemorySpace:
     """Mixed spaces are an error (tenferro-device/src/lib.rs:144-150)."""
     space = tensors[0].logical_memory_space()
     for t in tensors[1:]:
-        if t.logical_memory_space() != space:
+        if t._space is not space and t.logical_memory_space() != space:
             raise CrossMemorySpaceOperation(
                 f"cross-memory-space operation between {space!r} and {t.logical_memory_space()!r}")
     return space
