@@ -218,95 +218,181 @@ void fill_args(const ContractProblem& p, const ContractTables& t, ContractArgs* 
 }
 
 // ------------------------------------------------------------------ SIMT kernel
-// 64 x 64 block tile, 16-deep k slices, 256 threads, 4 x 4 outputs per thread.  Exact in
-// the element type (FMA), any strides, any dtype.  It is the path of last resort: the
-// tensor-core kernels decline only layouts they cannot stage.
-// ALG selects the semiring (scalar_ops.cuh): the same loop nest computes
-// C = alpha (x) (+)_k A (x) B  (+)  beta (x) C for MaxPlus and MinPlus, which have no tensor-core form.
-template <typename T, int ALG = 0>
-__global__ void __launch_bounds__(256) contract_simt_kernel(ContractArgs g) {
+// Exact in the element type (FMA), any strides, any dtype: the path of what the tensor-core kernels
+// decline or would mostly pad - f32 and complex32 outputs with a short side, f32 layouts TMA cannot describe
+// below the size that repays a copy - and of the tropical semirings (ALG, scalar_ops.cuh: the same
+// loop nest computes C = alpha (x) (+)_k A (x) B  (+)  beta (x) C).
+//
+// 64 x 64 block tile, 16-deep k slices (8 for 16-byte elements), 256 threads, 4 x 4 outputs each.  The next
+// slice is in flight from global memory to registers while one is computed from shared memory, and a
+// fragment is four neighbours, one 16-byte access for f32.  Few tiles with a long K are cut into
+// gridDim.y ranges whose sums simt_finish_kernel adds in range order (no result depends on timing).
+// Small shapes are bound by latency, the rest by issue and shared memory (kernel and finish): 679 x 636 x 431 f32
+// 90 -> 33 us, 510 x 690 x 945 105 -> 48, 38 x 1209 x 31 complex32 240 -> 33 (one tile, so one CTA before),
+// 202 x 150 x 70 f32 27 -> 22.
+template <typename T>
+constexpr int kSimtK = sizeof(T) == 16 ? 8 : 16;
+template <typename T>
+constexpr int kSimtCtas = sizeof(T) == 4 ? 3 : 2;  // CTAs per SM, what their registers leave
+
+template <typename T, int ALG>
+__device__ __forceinline__ void simt_store(const ContractArgs& g, const T* D, int64_t m, int64_t n, T* Cb, T sum) {
     using S = Semi<T, ALG>;
-    constexpr int BM = 64, BN = 64, BK = 16;
-    __shared__ T As[BK][BM + 1];
-    __shared__ T Bs[BK][BN + 1];
-    const T* A = (const T*)g.a;
-    const T* Bp = (const T*)g.b;
-    T* C = (T*)g.c;
+    const T alpha = Ops<T>::from(Scalar{g.alpha_re, g.alpha_im});
+    const T beta = Ops<T>::from(Scalar{g.beta_re, g.beta_im});
+    // beta equal to the semiring's zero means "overwrite": the output is never read
+    const bool read_c = ALG == 0 ? (g.beta_re != 0 || g.beta_im != 0) : !(g.beta_re == (ALG == 1 ? -INFINITY : INFINITY));
+    T* p = Cb + g.c_m[m] + g.c_n[n];
+    if (D) {
+        const T d = D[g.d_m[m] + g.d_n[n]];
+        sum = Ops<T>::mul(sum, g.conj_mul ? Ops<T>::conj(d) : d);
+    }
+    T v = S::mul(alpha, sum);
+    if (read_c) v = S::add(v, S::mul(beta, *p));
+    *p = v;
+}
+
+template <typename T, int ALG = 0>
+__global__ void __launch_bounds__(256, kSimtCtas<T>) contract_simt_kernel(ContractArgs g) {
+    using S = Semi<T, ALG>;
+    constexpr int BM = 64, BN = 64, BK = kSimtK<T>, P = 68, L = BM * BK / 256;
+    __shared__ __align__(16) T As[2][BK][P];
+    __shared__ __align__(16) T Bs[2][BK][P];
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;  // 16 x 16 threads, each 4 x 4
+    // A thread's L elements of each operand slice: neighbouring threads follow the unit stride.
+    int am[L], ak[L], bn[L], bk[L];
+#pragma unroll
+    for (int r = 0; r < L; ++r) {
+        const int c = tid + r * 256;
+        if (g.a_kfast) { ak[r] = c % BK; am[r] = c / BK; } else { am[r] = c % BM; ak[r] = c / BM; }
+        if (g.b_kfast) { bk[r] = c % BK; bn[r] = c / BK; } else { bn[r] = c % BN; bk[r] = c / BN; }
+    }
+    const int64_t s0 = (int64_t)blockIdx.y * g.iters_per_cta, s1 = min(g.k_iters, s0 + g.iters_per_cta);
     for (int64_t tile = blockIdx.x; tile < g.n_tiles; tile += gridDim.x) {
-        int64_t tm = tile % g.tiles_m;
-        int64_t rest = tile / g.tiles_m;
-        int64_t tn = rest % g.tiles_n;
-        int64_t bb = rest / g.tiles_n;
+        const int64_t tm = tile % g.tiles_m, rest = tile / g.tiles_m, tn = rest % g.tiles_n, bb = rest / g.tiles_n;
         const int64_t m0 = tm * BM, n0 = tn * BN;
-        const T* Ab = A + g.a_b[bb];
-        const T* Bb = Bp + g.b_b[bb];
+        const T* Ab = (const T*)g.a + g.a_b[bb];
+        const T* Bb = (const T*)g.b + g.b_b[bb];
+        int64_t arow[L], brow[L];
+#pragma unroll
+        for (int r = 0; r < L; ++r) {
+            arow[r] = m0 + am[r] < g.M ? g.a_m[m0 + am[r]] : 0;
+            brow[r] = n0 + bn[r] < g.N ? g.b_n[n0 + bn[r]] : 0;
+        }
+        T va[L], vb[L];
+        auto fetch = [&](int64_t slice) {
+            const int64_t k0 = slice * BK;
+#pragma unroll
+            for (int r = 0; r < L; ++r) {
+                va[r] = vb[r] = S::zero();
+                if (m0 + am[r] < g.M && k0 + ak[r] < g.K) va[r] = Ab[arow[r] + g.a_k[k0 + ak[r]]];
+                if (n0 + bn[r] < g.N && k0 + bk[r] < g.K) vb[r] = Bb[brow[r] + g.b_k[k0 + bk[r]]];
+            }
+        };
+        auto put = [&](int buf) {
+#pragma unroll
+            for (int r = 0; r < L; ++r) {
+                As[buf][ak[r]][am[r]] = g.conj_a ? Ops<T>::conj(va[r]) : va[r];
+                Bs[buf][bk[r]][bn[r]] = g.conj_b ? Ops<T>::conj(vb[r]) : vb[r];
+            }
+        };
         T acc[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = S::zero();
-        for (int64_t k0 = 0; k0 < g.K; k0 += BK) {
-            // Gather the two operand slices; neighbouring threads follow the unit stride.
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                int c = tid + r * 256;
-                int mm, kk;
-                if (g.a_kfast) { kk = c % BK; mm = c / BK; } else { mm = c % BM; kk = c / BM; }
-                T v = S::zero();
-                if (m0 + mm < g.M && k0 + kk < g.K) v = Ab[g.a_m[m0 + mm] + g.a_k[k0 + kk]];
-                if (g.conj_a) v = Ops<T>::conj(v);
-                As[kk][mm] = v;
-                int nn;
-                if (g.b_kfast) { kk = c % BK; nn = c / BK; } else { nn = c % BN; kk = c / BN; }
-                T w = S::zero();
-                if (n0 + nn < g.N && k0 + kk < g.K) w = Bb[g.b_n[n0 + nn] + g.b_k[k0 + kk]];
-                if (g.conj_b) w = Ops<T>::conj(w);
-                Bs[kk][nn] = w;
-            }
-            __syncthreads();
-#pragma unroll
+        if (s0 < s1) {
+            fetch(s0);
+            put(0);
+        }
+        __syncthreads();
+        int buf = 0;
+        for (int64_t s = s0; s < s1; ++s, buf ^= 1) {
+            if (s + 1 < s1) fetch(s + 1);
+#pragma unroll 4
             for (int kk = 0; kk < BK; ++kk) {
                 T av[4], bv[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) av[i] = As[kk][tx + 16 * i];
+                for (int i = 0; i < 4; ++i) av[i] = As[buf][kk][4 * tx + i];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][ty + 16 * j];
+                for (int j = 0; j < 4; ++j) bv[j] = Bs[buf][kk][4 * ty + j];
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) acc[i][j] = S::fma_(av[i], bv[j], acc[i][j]);
             }
+            if (s + 1 < s1) put(buf ^ 1);
             __syncthreads();
         }
-        const T alpha = Ops<T>::from(Scalar{g.alpha_re, g.alpha_im});
-        const T beta = Ops<T>::from(Scalar{g.beta_re, g.beta_im});
-        // beta equal to the semiring's zero means "overwrite": the output is never read
-        const bool read_c = ALG == 0 ? (g.beta_re != 0 || g.beta_im != 0) : !(g.beta_re == (ALG == 1 ? -INFINITY : INFINITY));
-        T* Cb = C + g.c_b[bb];
+        if (g.partial) {
+            T* P0 = (T*)g.partial + ((int64_t)blockIdx.y * g.n_tiles + tile) * (BM * BN);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) P0[(4 * ty + j) * BM + 4 * tx + i] = acc[i][j];
+            continue;
+        }
+        T* Cb = (T*)g.c + g.c_b[bb];
         const T* D = g.mul ? reinterpret_cast<const T*>(g.mul) + g.d_b[bb] : nullptr;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            int64_t n = n0 + ty + 16 * j;
+            const int64_t n = n0 + 4 * ty + j;
             if (n >= g.N) continue;
-            int64_t cn = g.c_n[n];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                int64_t m = m0 + tx + 16 * i;
-                if (m >= g.M) continue;
-                T* p = Cb + g.c_m[m] + cn;
-                T sum = acc[i][j];
-                if (D) {
-                    const T d = D[g.d_m[m] + g.d_n[n]];
-                    sum = Ops<T>::mul(sum, g.conj_mul ? Ops<T>::conj(d) : d);
-                }
-                T v = S::mul(alpha, sum);
-                if (read_c) v = S::add(v, S::mul(beta, *p));
-                *p = v;
+                const int64_t m = m0 + 4 * tx + i;
+                if (m < g.M) simt_store<T, ALG>(g, D, m, n, Cb, acc[i][j]);
             }
         }
     }
+}
+
+// Adds the ranges of each output element in range order; one thread per element of a tile.
+template <typename T, int ALG = 0>
+__global__ void __launch_bounds__(256) simt_finish_kernel(ContractArgs g, int splits) {
+    constexpr int BM = 64, BN = 64;
+    const int64_t tile = blockIdx.x, tm = tile % g.tiles_m, rest = tile / g.tiles_m, tn = rest % g.tiles_n, bb = rest / g.tiles_n;
+    const int e = blockIdx.y * 256 + threadIdx.x;
+    const int64_t m = tm * BM + e % BM, n = tn * BN + e / BM;
+    if (m >= g.M || n >= g.N) return;
+    const T* P0 = (const T*)g.partial + tile * (BM * BN) + e;
+    T sum = P0[0];
+#pragma unroll 8
+    for (int s = 1; s < splits; ++s) sum = Semi<T, ALG>::add(sum, P0[(int64_t)s * g.n_tiles * (BM * BN)]);
+    simt_store<T, ALG>(g, g.mul ? reinterpret_cast<const T*>(g.mul) + g.d_b[bb] : nullptr, m, n, (T*)g.c + g.c_b[bb], sum);
+}
+
+template <typename T, int ALG>
+static tfb_status simt_launch(tfb_ctx* ctx, ContractArgs a, const char* name) {
+    constexpr int BK = kSimtK<T>;
+    a.tiles_m = (a.M + 63) / 64;
+    a.tiles_n = (a.N + 63) / 64;
+    a.n_tiles = a.tiles_m * a.tiles_n * a.B;
+    if (a.n_tiles == 0) return TFB_OK;
+    a.k_iters = (a.K + BK - 1) / BK;
+    // As many ranges as run at once; a range keeps at least eight slices, below which the finishing launch
+    // costs more than it saves.
+    int64_t splits = std::min<int64_t>((int64_t)ctx->sm_count * kSimtCtas<T> / a.n_tiles, a.k_iters / 8);
+    splits = std::max<int64_t>(1, std::min<int64_t>(splits, 64));
+    PoolBlock ws;
+    // Without room for the sums the ranges stay whole, as the call must not need memory to succeed.
+    if (splits > 1 && ws.alloc(ctx, (size_t)(splits * a.n_tiles) * 64 * 64 * sizeof(T)) != TFB_OK) splits = 1;
+    a.iters_per_cta = (a.k_iters + splits - 1) / splits;
+    if (splits > 1) splits = (a.k_iters + a.iters_per_cta - 1) / a.iters_per_cta;
+    a.partial = splits > 1 ? (char*)ws.ptr : nullptr;
+    const unsigned grid = (unsigned)std::min<int64_t>(a.n_tiles, (int64_t)ctx->sm_count * 8);
+    {
+        LaunchScope ls(ctx, name);
+        contract_simt_kernel<T, ALG><<<dim3(grid, (unsigned)splits), 256, 0, ctx->stream>>>(a);
+    }
+    TFB_CUDA(cudaGetLastError());
+    if (splits > 1) {
+        LaunchScope ls(ctx, "contract_simt_finish");
+        simt_finish_kernel<T, ALG><<<dim3((unsigned)a.n_tiles, 16), 256, 0, ctx->stream>>>(a, (int)splits);
+    }
+    TFB_CUDA(cudaGetLastError());
+    return TFB_OK;
 }
 
 tfb_status contract_simt(tfb_ctx* ctx, const ContractProblem& p) {
@@ -314,21 +400,13 @@ tfb_status contract_simt(tfb_ctx* ctx, const ContractProblem& p) {
     TFB_TRY(get_tables(ctx, p, &t));
     ContractArgs a;
     fill_args(p, *t, &a);
-    a.tiles_m = (a.M + 63) / 64;
-    a.tiles_n = (a.N + 63) / 64;
-    a.n_tiles = a.tiles_m * a.tiles_n * a.B;
-    if (a.n_tiles == 0) return TFB_OK;
-    int grid = (int)std::min<int64_t>(a.n_tiles, (int64_t)ctx->sm_count * 8);
-    LaunchScope ls(ctx, "contract_simt");
     switch (p.dtype) {
-        case TFB_F32: contract_simt_kernel<float><<<grid, 256, 0, ctx->stream>>>(a); break;
-        case TFB_F64: contract_simt_kernel<double><<<grid, 256, 0, ctx->stream>>>(a); break;
-        case TFB_C32: contract_simt_kernel<float2><<<grid, 256, 0, ctx->stream>>>(a); break;
-        case TFB_C64: contract_simt_kernel<double2><<<grid, 256, 0, ctx->stream>>>(a); break;
-        default: return fail(TFB_ERR_INVALID_ARGUMENT, "unknown dtype %d", p.dtype);
+        case TFB_F32: return simt_launch<float, 0>(ctx, a, "contract_simt");
+        case TFB_F64: return simt_launch<double, 0>(ctx, a, "contract_simt");
+        case TFB_C32: return simt_launch<float2, 0>(ctx, a, "contract_simt");
+        case TFB_C64: return simt_launch<double2, 0>(ctx, a, "contract_simt");
     }
-    TFB_CUDA(cudaGetLastError());
-    return TFB_OK;
+    return fail(TFB_ERR_INVALID_ARGUMENT, "unknown dtype %d", p.dtype);
 }
 
 // The same kernel over a non-Standard semiring (real types only): 1 MaxPlus, 2 MinPlus.
@@ -341,19 +419,12 @@ tfb_status contract_simt_semiring(tfb_ctx* ctx, const ContractProblem& p, int al
     TFB_TRY(get_tables(ctx, p, &t));
     ContractArgs a;
     fill_args(p, *t, &a);
-    a.tiles_m = (a.M + 63) / 64;
-    a.tiles_n = (a.N + 63) / 64;
-    a.n_tiles = a.tiles_m * a.tiles_n * a.B;
-    if (a.n_tiles == 0) return TFB_OK;
-    int grid = (int)std::min<int64_t>(a.n_tiles, (int64_t)ctx->sm_count * 8);
-    LaunchScope ls(ctx, "contract_simt_semiring");
-    if (p.dtype == TFB_F32 && algebra == 1) contract_simt_kernel<float, 1><<<grid, 256, 0, ctx->stream>>>(a);
-    else if (p.dtype == TFB_F32 && algebra == 2) contract_simt_kernel<float, 2><<<grid, 256, 0, ctx->stream>>>(a);
-    else if (p.dtype == TFB_F64 && algebra == 1) contract_simt_kernel<double, 1><<<grid, 256, 0, ctx->stream>>>(a);
-    else if (p.dtype == TFB_F64 && algebra == 2) contract_simt_kernel<double, 2><<<grid, 256, 0, ctx->stream>>>(a);
-    else return fail(TFB_ERR_INVALID_ARGUMENT, "unknown algebra %d", algebra);
-    TFB_CUDA(cudaGetLastError());
-    return TFB_OK;
+    const char* name = "contract_simt_semiring";
+    if (p.dtype == TFB_F32 && algebra == 1) return simt_launch<float, 1>(ctx, a, name);
+    if (p.dtype == TFB_F32 && algebra == 2) return simt_launch<float, 2>(ctx, a, name);
+    if (p.dtype == TFB_F64 && algebra == 1) return simt_launch<double, 1>(ctx, a, name);
+    if (p.dtype == TFB_F64 && algebra == 2) return simt_launch<double, 2>(ctx, a, name);
+    return fail(TFB_ERR_INVALID_ARGUMENT, "unknown algebra %d", algebra);
 }
 
 // ------------------------------------------------------------------ selection

@@ -598,7 +598,9 @@ static tfb_status run_tma_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractAr
     if (cuts) {
         // Scratch slots and flags live with the context (one slot per CTA, reused by every
         // launch; a flag is "raised" when it equals the launch's epoch, so nothing is reset).
-        const size_t need = (size_t)grid * Base::TILE_ELEMS * Base::ES;
+        // As large as any configuration asks for from the start (19 MB): a captured launch keeps the address.
+        static_assert((size_t)Base::TILE_ELEMS * Base::ES <= 128 * 128 * 8, "largest block tile");
+        const size_t need = std::max<size_t>((size_t)grid, (size_t)slots) * 128 * 128 * 8;
         if (ctx->sk_partial_bytes < need) {
             if (ctx->sk_partial) TFB_CUDA(cudaFree(ctx->sk_partial));
             ctx->sk_partial = nullptr;
