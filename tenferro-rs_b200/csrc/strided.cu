@@ -384,8 +384,8 @@ static bool plan_tiles(const LoopNest& n, TilePlan* p) {
         rest.total *= n.extent[d];
         ++rest.rank;
     }
-    p->strip = std::min<uint32_t>(8, p->I.tiles);
-    p->strips = (p->I.tiles + p->strip - 1) / p->strip;
+    p->strips = (p->I.tiles + 7) / 8;
+    p->strip = (p->I.tiles + p->strips - 1) / p->strips;
     p->n_tiles = (int64_t)p->strip * p->strips * p->J.tiles * rest.total;
     return true;
 }
@@ -483,7 +483,8 @@ static tfb_status permute_typed(tfb_ctx* ctx, const LoopNest& nest_out_order, co
     }
     // Two modes that fill square tiles well enough: a tile costs the same whatever is in it, but the tile path
     // above pays about three times as much per element (f64, 27 x 84 patches: 227 us square, 162 there; 87 x 22:
-    // 25, 28; 171 x 125: 271, 344).
+    // 25, 28; 171 x 125: 271, 344).  For 4-byte elements, where instructions are all that bounds it, nearer to
+    // four times (20 x 299: 20.6, 25.8).
     {
         int im = -1;
         for (int d = 1; d < nest.rank && nest.stride[1][0] == 1; ++d)
@@ -513,7 +514,7 @@ static tfb_status permute_typed(tfb_ctx* ctx, const LoopNest& nest_out_order, co
                 if (d != 1 && r.stride[1][d] % V != 0) vec = false;  // every output stride but the unit one
             }
             const double fill = (double)r.extent[0] * (double)r.extent[1] / ((double)kTile * kTile * (double)ti * (double)tj);
-            if (fill >= 0.3 || !plan_tiles<T>(nest, &tiles)) {
+            if (fill >= (sizeof(T) == 4 ? 0.2 : 0.3) || !plan_tiles<T>(nest, &tiles)) {
                 LaunchScope ls(ctx, "permute_tiled");
                 if constexpr (sizeof(T) <= 8) if (vec) {
                     // CTAs per SM: each holds 16 KB of loads in flight, and HBM wants about 90 KB per SM.
@@ -525,7 +526,8 @@ static tfb_status permute_typed(tfb_ctx* ctx, const LoopNest& nest_out_order, co
                     TFB_CUDA(cudaGetLastError());
                     return TFB_OK;
                 }
-                const int64_t strip = std::min<int64_t>(8, ti), strips = (ti + strip - 1) / strip, n_tiles = strips * strip * tj * rest;
+                // (4-byte elements gain nothing by strips: 27757 x 374 18.3 us without, 19.5 with)
+                const int64_t strips = sizeof(T) == 4 ? 1 : (ti + 7) / 8, strip = (ti + strips - 1) / strips, n_tiles = strips * strip * tj * rest;
                 const unsigned grid = (unsigned)std::min<int64_t>(n_tiles, (int64_t)sms * 32);
                 permute_tiled_kernel<T><<<grid, 256, 0, ctx->stream>>>(r, (const T*)in, (T*)out, ep, ti, tj, n_tiles, strip, strips);
                 TFB_CUDA(cudaGetLastError());
