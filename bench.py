@@ -928,7 +928,7 @@ def wl_permute(env: Env):
         "step": step, "work": bytes_step * env.world, "read_result": read_result, "e2e_step": e2e_step,
         "h2d": h2d * env.world, "d2h": d2h * env.world,
         "kernel": "permute_tiled", "kernel_label": "permute kernel (rows / tiled transpose / generic, whichever the layout selects)",
-        "kernels_any": ["permute_rows", "permute_tiled", "permute_generic"],
+        "kernels_any": ["permute_rows", "permute_tiled", "permute_tile", "permute_generic"],
         "per_launch": bytes_step, "bound": "hbm", "peak": (lambda: hbm) if hbm else ctx.probe_hbm_gbs,
         "peak_source": "MEASURED_PEAKS.json hbm_gbs" if hbm else "library copy probe (MEASURED_PEAKS.json absent)",
         "extra_kernels": [], "keep": (src_t, dst_t), "check": check, "check_tol": 0.0,
