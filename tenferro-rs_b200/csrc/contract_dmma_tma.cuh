@@ -27,6 +27,7 @@
 // bond dimensions - used to be left to the gather kernel: a chain with chi = 97 took 18.5 + 10.5 us
 // (kernel and fix-up launch) per product, 11 us here.
 #pragma once
+#include "f64_map.h"
 #include "ptx_sm100.cuh"
 
 namespace tfb {
@@ -483,48 +484,13 @@ template <typename Cfg>
 static bool make_f64_map(const ContractProblem& p, const std::vector<Mode>& fr, int tns, const void* base, int rows,
                          bool* mn_major, bool* runs, CUtensorMap* map) {
     EncodeTiledF64 enc = encode_tiled_f64();
-    if (!enc || fr.size() > 1 || p.k.size() != 1 || p.batch.size() > 1) return false;
-    constexpr int W = Cfg::kCplx ? 2 : 1;  // doubles per element
-    const int64_t R = fr.empty() ? 1 : fr[0].extent, rs = fr.empty() ? 0 : fr[0].s[tns];
-    const int64_t K = p.k[0].extent, ks = p.k[0].s[tns];
-    const int64_t B = p.batch.empty() ? 1 : p.batch[0].extent, bs = p.batch.empty() ? 0 : p.batch[0].s[tns];
-    if ((uintptr_t)base % 16 != 0) return false;
-    auto ok16 = [&](int64_t s) { return s > 0 && (s * W * 8) % 16 == 0; };
-    if (B > 1 && !ok16(bs)) return false;
-    cuuint64_t dims[4], strides[3];
-    cuuint32_t box[4], estr[4] = {1, 1, 1, 1};
-    const cuuint64_t bstride = (cuuint64_t)((B > 1 ? bs * W * 8 : 16));
-    // The unit-stride index (extent `fast`, runs of `run` elements, `step` of them per k-iteration) and the other one.
-    int64_t fast, slow, slow_stride;
-    int run, step, slow_box;
-    if (ks == 1 && (Cfg::kLines || K % Cfg::KR == 0) && (R == 1 || ok16(rs))) {
-        *mn_major = false;
-        fast = K; run = Cfg::KR; step = Cfg::BK;
-        slow = R; slow_stride = R == 1 ? K : rs; slow_box = rows;
-    } else if (rs == 1 && (Cfg::kLines || R % Cfg::G == 0) && R > 1 && (K == 1 || ok16(ks))) {
-        *mn_major = true;
-        fast = R; run = Cfg::G; step = rows;
-        slow = K; slow_stride = K == 1 ? R : ks; slow_box = Cfg::BK;
-    } else {
-        return false;
-    }
-    *runs = fast % run != 0;
-    dims[0] = (cuuint64_t)((*runs ? fast : run) * W);
-    dims[1] = (cuuint64_t)slow;
-    dims[2] = (cuuint64_t)(*runs ? 1 : fast / run);
-    dims[3] = (cuuint64_t)B;
-    strides[0] = (cuuint64_t)(slow_stride * W * 8);
-    strides[1] = (cuuint64_t)(run * W * 8);
-    strides[2] = bstride;
-    box[0] = (cuuint32_t)(run * W);
-    box[1] = (cuuint32_t)slow_box;
-    box[2] = (cuuint32_t)(*runs ? 1 : step / run);
-    box[3] = 1;
-    for (int i = 0; i < 3; ++i)
-        if (strides[i] % 16 != 0 || strides[i] >= (1ull << 40)) return false;
-    for (int i = 0; i < 4; ++i)
-        if (dims[i] == 0 || dims[i] > 0xffffffffull) return false;
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<void*>(base), dims, strides, box, estr,
+    F64MapShape d;
+    if (!enc || !f64_map_shape(p, fr, tns, base, rows, F64MapForm{Cfg::kCplx, Cfg::kLines, Cfg::KR, Cfg::G, Cfg::BK}, &d)) return false;
+    *mn_major = d.mn_major;
+    *runs = d.runs;
+    const cuuint64_t dims[4] = {d.dims[0], d.dims[1], d.dims[2], d.dims[3]}, strides[3] = {d.strides[0], d.strides[1], d.strides[2]};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<void*>(base), dims, strides, d.box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, Cfg::kLines ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }

@@ -1,0 +1,50 @@
+"""Decisions of the host side at sizes no test can allocate: which operands a tensor map describes.  The rules
+are plain host code (no CUDA call); tests/host_rules.cpp gives them C entry points."""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+CSRC = ROOT / "tenferro-rs_b200" / "csrc"
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    so = tmp_path_factory.mktemp("host_rules") / "host_rules.so"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-fsanitize=undefined", "-fno-sanitize-recover=undefined", "-shared", "-fPIC",
+                    f"-I{CSRC}", "-I/usr/local/cuda/include", str(ROOT / "tests" / "host_rules.cpp"), "-o", str(so)], check=True)
+    return C.CDLL(str(so))
+
+
+# ---------------------------------------------------------------- tensor maps of the f64 / Complex64 kernel
+# (complex, one load per run allowed, k per run, rows per run, k per iteration, rows per tile)
+FORMS = [(1, 1, 8, 8, 32, 64), (1, 1, 8, 8, 16, 32), (1, 0, 4, 2, 32, 64), (0, 0, 4, 4, 16, 128), (0, 0, 4, 4, 16, 64)]
+EDGE = 1 << 30
+
+
+def f64_map(rules, form, rows, k, mn_major, ld):
+    out = (C.c_uint64 * 9)()
+    ok = rules.f64_map(*form, C.c_int64(rows), C.c_int64(k), int(mn_major), C.c_int64(ld), out)
+    return list(out) if ok else None
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("mn_major", [False, True])
+@pytest.mark.parametrize("fast", [7, 97, 4096, EDGE - 64, EDGE - 63, EDGE - 31, EDGE - 1, EDGE, EDGE + 1, EDGE + 8, 1200000001, 2**31 - 577,
+                                  2**31 - 576])
+def test_load_coordinates_fit_32_bits(rules, form, mn_major, fast):
+    cplx, _, kr, g, bk, tile = form
+    width, run, step = 1 + cplx, g if mn_major else kr, tile if mn_major else bk
+    ld = fast + fast % 2  # (16-byte columns for the real forms too)
+    got = f64_map(rules, form, fast if mn_major else 2, 2 if mn_major else fast, mn_major, ld)
+    if got is None:
+        # no map: the extent is not a number of runs, and either the form wants one or the last step's coordinate
+        # would not fit
+        assert fast % run and (not form[1] or (fast + step) * width > 2**31 - 1)
+        return
+    last = -(-fast // step) * step - run  # element at which the last load of the last step begins
+    coordinate = width * last if got[0] else last // run
+    assert coordinate <= 2**31 - 1
+    assert bool(got[0]) == (fast % run != 0)
