@@ -48,3 +48,31 @@ def test_load_coordinates_fit_32_bits(rules, form, mn_major, fast):
     coordinate = width * last if got[0] else last // run
     assert coordinate <= 2**31 - 1
     assert bool(got[0]) == (fast % run != 0)
+
+
+# ---------------------------------------------------------------- units of a grouped table
+def deal(rules, dtype, table, balance):
+    """[(corner of C, rows, columns, k, CTA)] of the units that a table of (m, n, k) is cut into; C's are 1 << 32 apart."""
+    es, tile = {0: (4, 64), 1: (8, 64), 2: (8, 32), 3: (16, 32)}[dtype]
+    words = [w for p, (m, n, k) in enumerate(table) for w in (m, n, k, 1 << 20, 1, m, 1 << 20, 1, k, (p + 1) << 32, 1, m)]
+    flat = (C.c_int64 * max(1, len(words)))(*words)
+    want = [(((p + 1) << 32) + (i + j * m) * es, min(tile, m - i), min(tile, n - j), k)
+            for p, (m, n, k) in enumerate(table) for j in range(0, n, tile) for i in range(0, m, tile)]
+    out = (C.c_int64 * (5 * (len(want) + 1)))()
+    got = rules.group_units(dtype, C.c_size_t(len(table)), flat, 148, int(balance), C.c_size_t(len(want)), out)
+    assert got == len(want)
+    rows = [tuple(out[5 * i:5 * i + 5]) for i in range(got)]
+    assert sorted(r[:4] for r in rows) == sorted(want)  # each tile once
+    return rows
+
+
+@pytest.mark.parametrize("dtype", [0, 1, 2, 3])
+@pytest.mark.parametrize("balance", [False, True])
+def test_every_tile_is_dealt_once(rules, dtype, balance):
+    deal(rules, dtype, [(1 + 7 * p % 150, 1 + 11 * p % 130, 5 * p % 90) for p in range(1000)], balance)
+    deal(rules, dtype, [], balance)
+    deal(rules, dtype, [(0, 5, 3), (1, 1, 0), (5, 0, 3)], balance)
+    # costs beyond 32 bits, among ordinary ones and alone
+    for k in (2**32 - 1, 5_800_000_000, 2**34, 2**40):
+        deal(rules, dtype, [(1, 1, k), (1, 1, 8), (70, 64, 64), (33, 90, k), (16, 16, 16)], balance)
+        deal(rules, dtype, [(2, 3, k)], balance)
