@@ -251,7 +251,10 @@ tfb_status tfb_selftest_wait_expiry(tfb_ctx* ctx, unsigned polls);
  * scalars the captured calls were given.  The sequence must have run once before it is
  * captured (plans, offset tables and kernel attributes are set up on first use with calls that
  * capture does not allow); synchronize, profile_begin and set_stream are refused while capturing, and
- * events recorded then mark nothing (they read as complete). */
+ * events recorded then mark nothing (they read as complete).
+ * Tables of grouped products are no nodes: tfb_grouped_plan_create uploads its table at once also while
+ * capturing, the plan works inside and outside the graph and has to outlive the graph that runs it; the
+ * table of a captured tfb_grouped_gemm lives as long as the graph. */
 typedef struct tfb_graph tfb_graph;
 tfb_status tfb_ctx_capture_begin(tfb_ctx* ctx);
 tfb_status tfb_ctx_capture_end(tfb_ctx* ctx, tfb_graph** out);

@@ -87,6 +87,8 @@ struct tfb_ctx {
     };
     std::vector<ProfRec> prof;
     bool capturing = false;  // between tfb_ctx_capture_begin and _end: launches are recorded, not run
+    std::vector<void*> capture_keeps;  // pool memory that the recorded launches read: the graph's from capture_end on
+    std::vector<void*> free_later;     // pool memory given up while capturing: freed by capture_end
 };
 
 // A captured sequence of this library's launches, instantiated for replay (tfb_graph_*).
@@ -94,6 +96,7 @@ struct tfb_graph {
     tfb_ctx* ctx = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    std::vector<void*> keeps;  // pool memory that its launches read
 };
 
 struct tfb_event {
@@ -216,8 +219,13 @@ tfb_status contract_c32_embedded(tfb_ctx* ctx, const ContractProblem& p, bool* d
 struct PoolBlock {
     tfb_ctx* ctx = nullptr;
     void* ptr = nullptr;
+    bool in_graph = false;  // allocated by a node of the graph being captured
     ~PoolBlock();
     tfb_status alloc(tfb_ctx* c, size_t bytes);
+    // A table that later launches read, copied from host memory that the caller may drop on return.
+    tfb_status upload(tfb_ctx* c, const void* host, size_t bytes);
+    // While capturing: the memory lives as long as the graph from here on.
+    void keep_for_graph();
 };
 
 // Device-resident schedule of one problem table for the tensor-core grouped kernels.

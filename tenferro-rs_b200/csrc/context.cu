@@ -68,22 +68,59 @@ LaunchScope::~LaunchScope() {
     if (stop) cudaEventRecord(stop, ctx->stream);
 }
 
-PoolBlock::~PoolBlock() {
-    if (ptr && ctx) {
-        DeviceGuard g(ctx->device);
-        cudaFreeAsync(ptr, ctx->stream);
+// While the stream is capturing, a free is a node of the graph, which may name the graph's own memory only.
+static void pool_free(tfb_ctx* c, void* ptr, bool in_graph) {
+    if (c->capturing && !in_graph) {
+        c->free_later.push_back(ptr);
+        return;
     }
+    DeviceGuard g(c->device);
+    cudaFreeAsync(ptr, c->stream);
 }
-tfb_status PoolBlock::alloc(tfb_ctx* c, size_t bytes) {
-    ctx = c;
+static tfb_status pool_alloc(tfb_ctx* c, size_t bytes, cudaStream_t stream, void** ptr) {
     if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMallocFromPoolAsync(&ptr, bytes, c->pool, c->stream);
+    cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, c->pool, stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        ptr = nullptr;
+        *ptr = nullptr;
         return fail(TFB_ERR_DEVICE, "pool allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
     }
     return TFB_OK;
+}
+PoolBlock::~PoolBlock() {
+    if (ptr && ctx) pool_free(ctx, ptr, in_graph);
+}
+tfb_status PoolBlock::alloc(tfb_ctx* c, size_t bytes) {
+    ctx = c;
+    in_graph = c->capturing;
+    return pool_alloc(c, bytes, c->stream, &ptr);
+}
+tfb_status PoolBlock::upload(tfb_ctx* c, const void* host, size_t bytes) {
+    ctx = c;
+    in_graph = false;
+    if (!c->capturing) {
+        TFB_TRY(pool_alloc(c, bytes, c->stream, &ptr));
+        // Pageable source: the copy has been staged by the time the call returns.
+        TFB_CUDA(cudaMemcpyAsync(ptr, host, bytes, cudaMemcpyHostToDevice, c->stream));
+        return TFB_OK;
+    }
+    // On the capturing stream both would become nodes: memory that exists while the graph runs only, and a copy
+    // that reads `host` at each replay.  A stream of their own, waited for, makes them happen now.
+    cudaStream_t side;
+    TFB_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    tfb_status st = pool_alloc(c, bytes, side, &ptr);
+    if (st == TFB_OK) {
+        cudaError_t e = cudaMemcpyAsync(ptr, host, bytes, cudaMemcpyHostToDevice, side);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(side);
+        if (e != cudaSuccess) st = fail(TFB_ERR_DEVICE, "upload of a table while capturing: %s", cudaGetErrorString(e));
+    }
+    cudaStreamDestroy(side);
+    return st;
+}
+void PoolBlock::keep_for_graph() {
+    if (!ptr || !ctx->capturing) return;
+    ctx->capture_keeps.push_back(ptr);
+    ptr = nullptr;
 }
 
 }  // namespace tfb
@@ -298,7 +335,13 @@ tfb_status tfb_ctx_capture_end(tfb_ctx* ctx, tfb_graph** out) {
     ctx->capturing = false;
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
+    for (void* p : ctx->free_later) pool_free(ctx, p, false);
+    ctx->free_later.clear();
+    std::vector<void*> keeps;
+    keeps.swap(ctx->capture_keeps);
+    auto drop_keeps = [&] { for (void* p : keeps) pool_free(ctx, p, false); };
     if (e != cudaSuccess || !graph) {
+        drop_keeps();
         cudaGetLastError();  // a call that capture does not allow has ended it; the stream is usable again
         return fail(TFB_ERR_DEVICE, "the captured sequence contained a call that cannot be captured (%s): "
                                     "run the sequence once before capturing it", cudaGetErrorString(e));
@@ -307,12 +350,14 @@ tfb_status tfb_ctx_capture_end(tfb_ctx* ctx, tfb_graph** out) {
     e = cudaGraphInstantiate(&exec, graph, 0);
     if (e != cudaSuccess) {
         cudaGraphDestroy(graph);
+        drop_keeps();
         return fail(TFB_ERR_DEVICE, "cudaGraphInstantiate: %s", cudaGetErrorString(e));
     }
     tfb_graph* gr = new tfb_graph;
     gr->ctx = ctx;
     gr->graph = graph;
     gr->exec = exec;
+    gr->keeps.swap(keeps);
     *out = gr;
     return TFB_OK;
 }
@@ -331,6 +376,7 @@ void tfb_graph_destroy(tfb_graph* graph) {
     DeviceGuard g(graph->ctx->device);
     if (graph->exec) cudaGraphExecDestroy(graph->exec);
     if (graph->graph) cudaGraphDestroy(graph->graph);
+    for (void* p : graph->keeps) pool_free(graph->ctx, p, false);
     delete graph;
 }
 

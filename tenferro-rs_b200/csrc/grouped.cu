@@ -371,9 +371,7 @@ tfb_status lay_out_units(tfb_ctx* ctx, size_t n, const tfb_gemm_problem* problem
     size_t bytes = 0;
     TFB_TRY(deal_units<T>(n, problems, ctx->sm_count, balance, scratch, &bytes, &out->starts_at, &out->grid));
     if (out->grid == 0) return TFB_OK;
-    TFB_TRY(out->mem.alloc(ctx, bytes));
-    // Pageable source: the copy has been staged by the time the call returns.
-    TFB_CUDA(cudaMemcpyAsync(out->mem.ptr, scratch.table.data(), bytes, cudaMemcpyHostToDevice, ctx->stream));
+    TFB_TRY(out->mem.upload(ctx, scratch.table.data(), bytes));
     scratch.trim();
     return TFB_OK;
 }
@@ -489,7 +487,9 @@ extern "C" tfb_status tfb_grouped_gemm(tfb_ctx* ctx, int32_t dtype, size_t n_pro
     if (!alpha || !beta) return fail(TFB_ERR_INVALID_ARGUMENT, "tfb_grouped_gemm: alpha/beta are NULL");
     tfb_grouped_plan plan;
     TFB_TRY(prepare(ctx, dtype, n_problems, problems, false, &plan));
-    return run(&plan, load_scalar(dtype, alpha), load_scalar(dtype, beta));
+    TFB_TRY(run(&plan, load_scalar(dtype, alpha), load_scalar(dtype, beta)));
+    for (PoolBlock* b : {&plan.schedule.mem, &plan.units.mem}) b->keep_for_graph();  // a replay reads the table again
+    return TFB_OK;
 }
 
 extern "C" tfb_status tfb_grouped_plan_create(tfb_ctx* ctx, int32_t dtype, size_t n_problems,

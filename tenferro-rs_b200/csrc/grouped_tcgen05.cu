@@ -526,9 +526,7 @@ tfb_status grouped_tcgen05_prepare(tfb_ctx* ctx, size_t n, const tfb_gemm_proble
             ++unit_no;
         }
     }
-    TFB_TRY(out->mem.alloc(ctx, table.size() * sizeof(TcStage)));
-    // `table` is pageable: the copy has been staged by the time the call returns.
-    TFB_CUDA(cudaMemcpyAsync(out->mem.ptr, table.data(), table.size() * sizeof(TcStage), cudaMemcpyHostToDevice, ctx->stream));
+    TFB_TRY(out->mem.upload(ctx, table.data(), table.size() * sizeof(TcStage)));
     out->total_units = (int64_t)units.size();
     out->grid = grid;
     out->pitch = (int)pitch;

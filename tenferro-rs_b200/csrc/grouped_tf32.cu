@@ -354,9 +354,7 @@ tfb_status grouped_tf32_prepare(tfb_ctx* ctx, size_t n, const tfb_gemm_problem* 
     for (int c = 0; c < grid; ++c)
         for (size_t r = 0; r < per_cta[c].size(); ++r) table[r * grid + c] = per_cta[c][r];
     const size_t bytes = table.size() * sizeof(Stage);
-    TFB_TRY(out->mem.alloc(ctx, bytes));
-    // `table` is pageable: the copy has been staged by the time the call returns.
-    TFB_CUDA(cudaMemcpyAsync(out->mem.ptr, table.data(), bytes, cudaMemcpyHostToDevice, ctx->stream));
+    TFB_TRY(out->mem.upload(ctx, table.data(), bytes));
     out->total_units = (int64_t)units.size();
     out->grid = grid;
     *declined = false;
