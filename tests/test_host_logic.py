@@ -219,3 +219,34 @@ def test_device_preference(tb):
     t.set_preferred_compute_device(tb.ComputeDevice.Cuda(1))
     assert t.effective_compute_devices(tb.OpKind.Contract) == [tb.ComputeDevice.Cuda(1)]
     assert t.preferred_compute_device() == tb.ComputeDevice.Cuda(1)
+
+
+# ---------------------------------------------------------------- tables of grouped products
+def test_problem_table_forms(tb):
+    """Every row is one problem whatever the others hold: too many fields are an error, trailing ones left out are
+    zero, and pointers may be integers, None or ctypes pointers."""
+    import ctypes as C
+
+    from tenferro_b200.prims import _problem_table
+
+    def table(rows):
+        n, held, ptr = _problem_table(rows)
+        return [tuple(getattr(ptr[i], f) for f, _ in ptr[i]._fields_) for i in range(n)] if held is not None else None
+
+    row = (2, 3, 4, 4096, 1, 2, 8192, 1, 4, 12288, 1, 2)
+    other = (5, 6, 7, 4097, 8, 9, 8193, 10, 11, 12289, 12, 13)
+    assert table([row, other]) == [row, other]
+    assert table([list(row), iter(other)]) == [row, other]
+    assert table([]) == []
+    for bad in ([row + (1,), row[:11]], [row[:11], row + (1,)], [row + (1,)], [row, row + (0,)]):
+        with pytest.raises(TypeError):
+            table(bad)
+    with pytest.raises(TypeError):
+        table([(2.0,) + row[1:]])
+    assert table([row[:11], other]) == [row[:11] + (0,), other]
+    empty = (0, 3, 4, None, 1, 2, None, 1, 4, None, 1, 2)
+    assert table([empty, row]) == [empty, row]
+    ctypes_row = tuple(C.c_void_p(x) if i in (3, 6, 9) else x for i, x in enumerate(other))
+    assert table([ctypes_row, row]) == [other, row]
+    high = (1, 1, 1, 2**63 + 64, 1, 1, 64, 1, 1, 2**64 - 64, -1, -1)
+    assert table([high]) == [high]
