@@ -519,7 +519,11 @@ static tfb_status permute_typed(tfb_ctx* ctx, const LoopNest& nest_out_order, co
                 if (d != 1 && r.stride[1][d] % V != 0) vec = false;  // every output stride but the unit one
             }
             const double fill = (double)r.extent[0] * (double)r.extent[1] / ((double)kTile * kTile * (double)ti * (double)tj);
-            if (fill >= (sizeof(T) == 4 ? 0.2 : 0.3) || !plan_tiles<T>(nest, &tiles)) {
+            if (fill < (sizeof(T) == 4 ? 0.2 : 0.3) && plan_tiles<T>(nest, &tiles)) return run_tiles();
+            // What has no plan (2^31 elements, spans of a group above 1e9) and puts few elements into a tile is better off
+            // element by element (ms, that way and in tiles: f32 8 x 8 patches 16.6, 85.4; 12 x 12 19.4, 39.2; 15 x 15 25.1,
+            // 27.1; f64 8 x 8 22.7, 142; 14 x 14 40.4, 50.5; 15 x 15 42.6, 33.2; complex double 8 x 15 47.4, 64.7).
+            if (r.extent[0] * r.extent[1] >= (sizeof(T) == 4 ? 256 : 225) * ti * tj) {
                 LaunchScope ls(ctx, "permute_tiled");
                 if constexpr (sizeof(T) <= 8) if (vec) {
                     // CTAs per SM: each holds 16 KB of loads in flight, and HBM wants about 90 KB per SM.
@@ -537,7 +541,6 @@ static tfb_status permute_typed(tfb_ctx* ctx, const LoopNest& nest_out_order, co
                 TFB_CUDA(cudaGetLastError());
                 return TFB_OK;
             }
-            return run_tiles();
         }
     }
     if (plan_tiles<T>(nest, &tiles)) return run_tiles();

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 def broadcast_view(tb, rng, dims, strides, dtype):
-    """A buffer of small integers (f32: a few ones) under the given strides: (tensor, its part without the
+    """A buffer of small integers (f32: mostly zeros) under the given strides: (tensor, its part without the
     broadcast modes as an array, the number of times each of its elements is read)."""
     live = [d if s else 1 for d, s in zip(dims, strides)]
     first = sum((d - 1) * -s for d, s in zip(dims, strides) if s < 0)
@@ -54,3 +54,69 @@ def test_reduce(tb, dims, strides, kept, dtype):
         else:
             want = host.max(axis=axes) if op == "Max" else host.min(axis=axes)
         assert np.array_equal(out.to_numpy(), want)
+
+
+def same_as_rows(flat, want_block, times):
+    """Whether a flat device tensor is `times` repetitions of a host block."""
+    import torch
+
+    want = torch.from_numpy(want_block).cuda()
+    return bool((flat.view(times, want.numel()) == want).all())
+
+
+def device_output(tb, dims, dtype):
+    import torch
+
+    flat = torch.zeros(math.prod(dims), device="cuda", dtype={np.float32: torch.float32, np.float64: torch.float64}[dtype])
+    torch.cuda.synchronize()
+    return flat, tb.Tensor.from_device_pointer(flat.data_ptr(), flat.numel() * flat.element_size(), dims, dtype,
+                                               tb.LogicalMemorySpace.GpuMemory(0), flat)
+
+
+def kernels(ctx, fn, names):
+    ctx.profile_begin()
+    fn()
+    ctx.synchronize()
+    ran = [n for n in names if ctx.profile_read(n)[0]]
+    ctx.profile_end()
+    return ran
+
+
+# (dims and strides of the input, order of the output, kernel): a patch of the first and the last index, the middle
+# one broadcast
+@pytest.mark.parametrize("dims,strides,perm,kernel", [
+    ([8, 2**25 + 3, 8], [1, 0, 8], [2, 0, 1], "permute_generic"),
+    ([15, 9600003, 17], [1, 0, 15], [2, 0, 1], "permute_generic"),  # fewer than 256 elements in a tile
+    ([16, 8400003, 16], [1, 0, 16], [2, 0, 1], "permute_tiled"),  # 16-byte accesses
+    ([17, 7500003, 17], [1, 0, 17], [2, 0, 1], "permute_tiled"),
+    ([8, 1000003, 300], [1, 0, 9], [2, 0, 1], "permute_tiled"),
+    ([4099, 524003, 1], [1, 0, 1], [0, 2, 1], "permute_rows"),
+    ([4096, 524291, 1], [1, 0, 1], [0, 2, 1], "permute_rows"),  # 16-byte accesses
+])
+def test_permute(tb, dims, strides, perm, kernel):
+    assert math.prod(dims) >= 2**31
+    x, host, times = broadcast_view(tb, np.random.default_rng(6), dims, strides, np.float32)
+    assert host.any()
+    out_dims = [dims[i] for i in perm]
+    flat, out = device_output(tb, out_dims, np.float32)
+    plan = tb.CudaBackend.plan(tb.PrimDescriptor.Permute(list(range(3)), perm), [dims, out_dims], np.float32)
+    ran = kernels(plan.ctx, lambda: tb.CudaBackend.execute(plan, 1.0, [x], 0.0, out),
+                  ["permute_generic", "permute_tiled", "permute_rows", "permute_tile"])
+    assert ran == [kernel]
+    assert same_as_rows(flat, host.transpose(perm).reshape(-1, order="F"), times)
+
+
+@pytest.mark.parametrize("rows", [4099, 4100])  # element by element and in 16-byte accesses
+def test_elementwise(tb, rows):
+    cols = 2**31 // rows + 5
+    a = np.random.default_rng(7).integers(-9, 9, rows).astype(np.float32)
+    b = np.arange(rows, dtype=np.float32) % 7
+    views = []
+    for v in (a, b):
+        t = tb.Tensor.from_numpy(v)
+        views.append(tb.Tensor(t._block, [rows, cols], [1, 0], 0, np.float32, t.logical_memory_space()))
+    flat, out = device_output(tb, [rows, cols], np.float32)
+    plan = tb.CudaBackend.plan(tb.PrimDescriptor.ElementwiseMul(), [[rows, cols]] * 3, np.float32)
+    tb.CudaBackend.execute(plan, 1.0, views, 0.0, out)
+    plan.ctx.synchronize()
+    assert same_as_rows(flat, a * b, cols)
