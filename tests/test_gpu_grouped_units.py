@@ -72,3 +72,46 @@ def test_grouped_units(tb, oracle, dtype, layout, pad, beta):
         bound = 2 * terms * u * (abs(alpha) * (np.abs(a) @ np.abs(b)) + abs(beta) * np.abs(c0)) + 1e-300
         assert (np.abs(out[at] - want) <= bound).all(), (p, m, n, k)
     assert np.isnan(out[~live]).all()  # nothing outside the blocks was written
+
+
+# (m, n, k) and the strides of A, B and C: broadcast rows, columns or everything, reversed directions, both strides alike
+# (overlapping diagonals), a transposed and reversed C
+STRIDES = [((33, 20, 17), (0, 1), (1, 17), (1, 33)), ((33, 20, 17), (1, 0), (0, 1), (1, 33)), ((65, 9, 40), (0, 0), (1, 0), (1, 65)),
+           ((40, 66, 18), (-1, 40), (18, -1), (1, 40)), ((40, 66, 18), (18, 1), (-66, 1), (1, 40)),
+           ((31, 34, 19), (-1, -31), (1, 1), (1, 31)), ((17, 65, 16), (1, 1), (1, 16), (-65, 1)),
+           ((64, 64, 16), (2, 1), (1, 3), (-1, -64)), ((1, 1, 33), (5, 1), (1, 7), (3, 3)), ((70, 1, 9), (1, 70), (1, 1), (1, 1)),
+           ((1, 70, 9), (1, 1), (70, 1), (9, 1))]
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.complex64, np.complex128])
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+def test_strides(tb, oracle, dtype, beta):
+    dtype = np.dtype(dtype)
+    wide = np.complex128 if dtype.kind == "c" else np.float64
+    rows, mats = [], []
+    for p, ((m, n, k), *strides) in enumerate(STRIDES):
+        row, part = [m, n, k], []
+        for t, (shape, (rs, cs)) in enumerate(zip(((m, k), (k, n), (m, n)), strides)):
+            first = -min(0, (shape[0] - 1) * rs) - min(0, (shape[1] - 1) * cs)
+            size = first + max(0, (shape[0] - 1) * rs) + max(0, (shape[1] - 1) * cs) + 1
+            flat = oracle.normal(50 * p + t, (size + 3,), dtype)
+            dev = tb.Tensor.from_numpy(flat)
+            at = first + np.arange(shape[0])[:, None] * rs + np.arange(shape[1])[None, :] * cs
+            row += [dev._block.ptr + first * dtype.itemsize, rs, cs]
+            part.append((flat, at, dev))
+        rows.append(tuple(row))
+        mats.append(part)
+    plan = tb.PreparedGroupedGemm(rows, dtype, 1.0, beta)
+    plan.run()
+    plan.ctx.synchronize()
+    u = np.finfo(dtype).eps / 2
+    for ((m, n, k), *_), part in zip(STRIDES, mats):
+        (fa, ia, _), (fb, ib, _), (fc, ic, dev) = part
+        a, b, c0 = fa[ia].astype(wide), fb[ib].astype(wide), fc[ic].astype(wide)
+        out = dev.to_numpy()
+        terms = (2 if dtype.kind == "c" else 1) * k + 4
+        bound = 2 * terms * u * (np.abs(a) @ np.abs(b) + beta * np.abs(c0)) + 1e-300
+        assert (np.abs(out[ic] - (a @ b + beta * c0)) <= bound).all(), (m, n, k)
+        rest = np.ones(out.size, bool)
+        rest[ic] = False
+        assert np.array_equal(out[rest], fc[rest])

@@ -59,6 +59,27 @@ def test_max_of_special_values(tb, special):
     assert np.array_equal(out.to_numpy(), x.max(axis=0), equal_nan=True)
 
 
+@pytest.mark.parametrize("special", [-np.inf, np.inf, np.nan, np.finfo(np.float64).min])
+@pytest.mark.parametrize("shape,kept", [((300001, 3), 1), ((3, 300001), 0)])
+@pytest.mark.parametrize("op", ["Max", "Min"])
+def test_special_values_in_slices(tb, special, shape, kept, op):
+    """Few kept elements under a long range: several slices and the launch that combines them."""
+    x = np.full(shape, special)
+    rows = x if kept == 1 else x.T
+    rows[:, 1] = np.arange(300001.0)
+    rows[150000, 1] = special  # one special value among ordinary ones, somewhere in the middle
+    rows[299999, 2] = 1.0  # and the other way round, in the last slice
+    out = tb.Tensor.from_numpy(np.zeros(3))
+    plan = tb.CudaBackend.plan(tb.PrimDescriptor.Reduce([0, 1], [kept], tb.ReduceOp[op]), [x.shape, (3,)], np.float64)
+    plan.ctx.profile_begin()
+    tb.CudaBackend.execute(plan, 1.0, [tb.Tensor.from_numpy(x)], 0.0, out)
+    plan.ctx.synchronize()
+    assert plan.ctx.profile_read("reduce_finish")[0] == 1
+    plan.ctx.profile_end()
+    want = (np.max if op == "Max" else np.min)(rows, axis=0)
+    assert np.array_equal(out.to_numpy(), want, equal_nan=True)
+
+
 @pytest.mark.parametrize("notation", ["asb,b->asb", "a,asb->asb", "asb,asb->asb", "asb,a->asb", "asb,bsa->asb", "asb,s->asb"])
 @pytest.mark.parametrize("size", [(1, 1, 1), (4, 2, 8), (33, 3, 65), (64, 2, 130), (1025, 4, 31)])
 @pytest.mark.parametrize("dtype", [np.float32, np.float64, np.complex64, np.complex128])
