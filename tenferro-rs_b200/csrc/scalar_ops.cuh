@@ -24,7 +24,6 @@ struct Ops<float> {
     __device__ static float highest() { return INFINITY; }
     __device__ static float max_(float a, float b) { return a != a ? a : (b != b ? b : (a > b ? a : b)); }
     __device__ static float min_(float a, float b) { return a != a ? a : (b != b ? b : (a < b ? a : b)); }
-    __device__ static float shfl_down(float a, int s) { return __shfl_down_sync(0xffffffffu, a, s); }
 };
 
 template <>
@@ -41,7 +40,6 @@ struct Ops<double> {
     __device__ static double highest() { return INFINITY; }
     __device__ static double max_(double a, double b) { return a != a ? a : (b != b ? b : (a > b ? a : b)); }
     __device__ static double min_(double a, double b) { return a != a ? a : (b != b ? b : (a < b ? a : b)); }
-    __device__ static double shfl_down(double a, int s) { return __shfl_down_sync(0xffffffffu, a, s); }
 };
 
 template <>
@@ -66,9 +64,6 @@ struct Ops<float2> {
     __device__ static float2 highest() { return zero(); }
     __device__ static float2 max_(float2 a, float2) { return a; }
     __device__ static float2 min_(float2 a, float2) { return a; }
-    __device__ static float2 shfl_down(float2 a, int s) {
-        return make_float2(__shfl_down_sync(0xffffffffu, a.x, s), __shfl_down_sync(0xffffffffu, a.y, s));
-    }
 };
 
 template <>
@@ -93,9 +88,6 @@ struct Ops<double2> {
     __device__ static double2 highest() { return zero(); }
     __device__ static double2 max_(double2 a, double2) { return a; }
     __device__ static double2 min_(double2 a, double2) { return a; }
-    __device__ static double2 shfl_down(double2 a, int s) {
-        return make_double2(__shfl_down_sync(0xffffffffu, a.x, s), __shfl_down_sync(0xffffffffu, a.y, s));
-    }
 };
 
 // Semirings (tenferro-algebra/src/lib.rs:74-106: zero, one, add, mul).  ALG 0 is the Standard

@@ -110,13 +110,6 @@ class _Borrowed:
         self.event: Optional[CompletionEvent] = None
 
 
-def make_view(ptr: int, dims, strides, offset: int, conj: bool, keep: list) -> _lib.TfbView:
-    """Build a tfb_view; the ctypes arrays are appended to `keep` so they outlive the call."""
-    d, s = _view_arrays(dims, strides)
-    keep += [d, s]
-    return _lib.TfbView(ptr, len(dims), d, s, offset, 1 if conj else 0)
-
-
 def _view_arrays(dims, strides):
     n = max(len(dims), 1)
     return (C.c_size_t * n)(*dims), (C.c_ssize_t * n)(*strides)
