@@ -564,15 +564,21 @@ static tfb_status run_tma_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractAr
     if (cuts) {
         // Scratch slots and flags live with the context (one slot per CTA, reused by every
         // launch; a flag is "raised" when it equals the launch's epoch, so nothing is reset).
-        // As large as any configuration asks for from the start (19 MB): a captured launch keeps the address.
+        // As large as any configuration asks for from the start (19 MB): a captured launch keeps the address.  Where the
+        // device has no room for that, what this launch uses.
         static_assert((size_t)Base::TILE_ELEMS * Base::ES <= 128 * 128 * 8, "largest block tile");
-        const size_t need = std::max<size_t>((size_t)grid, (size_t)slots) * 128 * 128 * 8;
+        const size_t need = (size_t)grid * Base::TILE_ELEMS * Base::ES;
         if (ctx->sk_partial_bytes < need) {
             if (ctx->sk_partial) TFB_CUDA(cudaFree(ctx->sk_partial));
             ctx->sk_partial = nullptr;
             ctx->sk_partial_bytes = 0;
-            TFB_CUDA(cudaMalloc(&ctx->sk_partial, need));
-            ctx->sk_partial_bytes = need;
+            size_t take = std::max<size_t>((size_t)grid, (size_t)slots) * 128 * 128 * 8;
+            if (cudaMalloc(&ctx->sk_partial, take) != cudaSuccess) {
+                cudaGetLastError();
+                take = need;
+                TFB_CUDA(cudaMalloc(&ctx->sk_partial, take));
+            }
+            ctx->sk_partial_bytes = take;
         }
         if (ctx->sk_flags_n < (size_t)grid) {
             if (ctx->sk_flags) TFB_CUDA(cudaFree(ctx->sk_flags));
