@@ -530,16 +530,29 @@ static tfb_status repack_for_tma(tfb_ctx* ctx, const ContractProblem& p, const C
         need[0] = !make_f64_map<CplxTma4>(p, p.m, 0, p.a, CplxTma4::BM, &mn, &runs, &map);
         need[1] = !make_f64_map<CplxTma4>(p, p.n, 1, p.b, CplxTma4::BN, &mn, &runs, &map);
     }
-    // A copy of at most an eighth of the device's memory each: a larger one could take the room that the
-    // caller's next tensors need.  Without room the gather kernel runs.
+    // An operand that keeps its map and is K-major with its rows 2 MiB or more apart is read a page at a time, which
+    // costs the TMA-fed kernel a third of its rate (double, by gather and with the other operand copied: 161 x 161 x 578680
+    // 1766 us, 2621; 65 x 65 x 3550292 4757, 6366; 129 x 129 x 90136, rows 0.7 MiB apart, 347, 271).
+    for (int t = 0; t < 2; ++t) {
+        const std::vector<Mode>& free_p = t == 0 ? p.m : p.n;
+        if (!need[t] && need[1 - t] && p.k[0].s[t] == 1 && !free_p.empty() &&
+            free_p[0].s[t] * (int64_t)dtype_size(p.dtype) >= (2 << 20))
+            return TFB_OK;
+    }
+    // The copies come from the context's pool, which keeps what it has: a thirty-second of the device's memory (5.7 GB)
+    // for both together, so that the rest stays free for the caller's tensors.  Above that, and without room, the
+    // gather kernel runs (double, 2047 x 2049 x 300001, 9.8 GB of copies: 83 ms with them, 137 by gather).  Giving larger
+    // blocks back after each call costs 14 ms a GB to map them again, more than they save.
     int64_t ld[2];
+    double bytes[2], sum = 0;
     for (int t = 0; t < 2; ++t) {
         ld[t] = ((t == 0 ? a.M : a.N) + 7) / 8 * 8;  // rows past the last only reach sums that are not stored
-        const double bytes = (double)dtype_size(p.dtype) * (double)ld[t] * (double)a.K * (double)a.B;
-        if (!need[t]) continue;
-        if (bytes > (double)ctx->total_mem / 8) return TFB_OK;
-        if ((t == 0 ? blk_a : blk_b)->alloc(ctx, (size_t)bytes) != TFB_OK) return TFB_OK;
+        bytes[t] = need[t] ? (double)dtype_size(p.dtype) * (double)ld[t] * (double)a.K * (double)a.B : 0;
+        sum += bytes[t];
     }
+    if (sum > (double)ctx->total_mem / 32) return TFB_OK;
+    for (int t = 0; t < 2; ++t)
+        if (need[t] && (t == 0 ? blk_a : blk_b)->alloc(ctx, (size_t)bytes[t]) != TFB_OK) return TFB_OK;
     *q = p;
     if (need[0] && need[1]) {
         q->k.assign(1, Mode{a.K, {0, 0, 0, 0}});

@@ -4,6 +4,8 @@ the edges of the tiles (32, 64, 128), of a k-iteration (16) and of a run (8, 4).
 
 The bound is that of a dot product, part by part: K + 4 roundings of |A| |B| (twice the terms in each
 part of a complex product) at the unit roundoff, doubled for the split of K over several blocks."""
+import itertools
+
 import numpy as np
 import pytest
 
@@ -57,3 +59,100 @@ def test_operands_without_a_map(tb, oracle, notation, sizes, dtype):
     assert 2 * np.prod([float(v) for v in sizes.values()]) >= 2e8  # from here on operands are copied
     shapes = [tuple(sizes[c] for c in t) for t in notation.split("->")[0].split(",")]
     run(tb, oracle, notation, shapes, dtype, False, 0.5)
+
+
+COPIES = ("permute_rows", "permute_tiled", "permute_tile", "permute_generic")
+
+
+def launches(ctx, fn, names):
+    ctx.profile_begin()
+    fn()
+    ctx.synchronize()
+    got = [ctx.profile_read(name)[0] for name in names]
+    ctx.profile_end()
+    return got
+
+
+# (notation, sizes, pairs of the tree, operands copied): one operand keeps its map, two batch modes that do not fuse, a
+# multiplier fused into the product
+@pytest.mark.parametrize("notation,sizes,pairs,copies", [
+    ("ij,jk->ik", dict(i=331, j=1024, k=512), [(0, 1)], {"f": 1, "c": 0}),
+    ("ij,jk->ik", dict(i=332, j=1021, k=511), [(0, 1)], {"f": 1, "c": 0}),
+    ("ijl,jk->ilk", dict(i=33, j=640, l=17, k=514), [(0, 1)], {"f": 1, "c": 1}),
+    ("kj,ijl->kil", dict(i=33, j=640, l=17, k=516), [(0, 1)], {"f": 1, "c": 1}),
+    ("bijc,bjkc->bikc", dict(b=5, i=67, j=1201, c=4, k=70), [(0, 1)], {"f": 2, "c": 2}),
+    ("ijl,ljk,ik->ik", dict(i=255, j=51, l=33, k=257), [(0, 1), (2, 3)], {"f": 2, "c": 2}),
+])
+@pytest.mark.parametrize("dtype", [np.float64, np.complex128])
+@pytest.mark.parametrize("conj", [False, True])
+def test_copied_operands(tb, oracle, notation, sizes, pairs, copies, dtype, conj):
+    ins, out_labels = notation.split("->")
+    ins = ins.split(",")
+    assert 2 * np.prod([float(sizes[c]) for c in set(ins[0] + ins[1])]) >= 2e8
+    arrays = [oracle.normal(17 + t, [sizes[c] for c in term], dtype) for t, term in enumerate(ins)]
+    c0 = oracle.normal(29, [sizes[c] for c in out_labels], dtype)
+    ops, out = [tb.Tensor.from_numpy(x) for x in arrays], tb.Tensor.from_numpy(c0)
+    if conj:
+        ops, arrays = [x.into_conj() for x in ops], [x.conj() for x in arrays]
+    tree = tb.ContractionTree.from_pairs(tb.Subscripts.parse(notation), [x.shape for x in arrays], pairs)
+    ctx = tb.Context.get(0)
+    ran = launches(ctx, lambda: tb.einsum_with_plan_into(tree, ops, 1.0, 0.5, out), COPIES + ("contract_dmma", "contract_dmma_fixup"))
+    kind = np.dtype(dtype).kind
+    assert sum(ran[:4]) == copies[kind] and ran[4] == 1 and ran[5] == 0
+    parts = lambda x: (x.real, x.imag) if kind == "c" else (x,)
+    # products of magnitudes, part by part; the multiplier's parts on top
+    mag = sum(np.einsum(notation, *[abs(q) for q in pick], optimize=True)
+              for pick in itertools.product(*[parts(x) for x in arrays]))
+    want = np.einsum(notation, *arrays, optimize=True) + 0.5 * c0
+    k = np.prod([sizes[c] for c in set(ins[0] + ins[1]) - set(out_labels)]) + 8
+    bound = 2 * k * (2 if kind == "c" else 1) * U * (mag + 0.5 * abs(c0))
+    for x, y in zip(parts(out.to_numpy()), parts(want)):
+        assert (abs(x - y) <= bound).all()
+
+
+def device_product(tb, m, n, k):
+    """i j, j k -> i k on small integers (sums are exact in any order): (call, output, expected, whatever holds the operands)."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    a, b = (torch.randint(0, 4, s, device="cuda", generator=gen, dtype=torch.int8).double() for s in ((k, m), (n, k)))
+    out = torch.zeros((n, m), device="cuda", dtype=torch.float64)
+    want = b @ a
+    space = tb.LogicalMemorySpace.GpuMemory(0)
+    views = [tb.Tensor.from_device_pointer(t.data_ptr(), t.numel() * 8, dims, np.float64, space, t)
+             for t, dims in ((a, (m, k)), (b, (k, n)), (out, (m, n)))]
+    tree = tb.ContractionTree.optimize(tb.Subscripts.parse("ij,jk->ik"), [(m, k), (k, n)])
+    torch.cuda.synchronize()
+    return lambda: tb.einsum_with_plan_into(tree, views[:2], 1.0, 0.0, views[2]), out, want
+
+
+@pytest.mark.parametrize("m,n,k,copies", [
+    (65, 64, 262140, 1),  # B's rows just below 2 MiB apart
+    (65, 64, 262144, 0),
+    (65, 67, 6000001, 0),  # 6.9 GB of copies: more than the pool may keep
+])
+def test_when_operands_are_not_copied(tb, m, n, k, copies):
+    import torch
+
+    call, out, want = device_product(tb, m, n, k)
+    ctx = tb.Context.get(0)
+    kept = ctx.pool_stats()[0]
+    assert sum(launches(ctx, call, COPIES)) == copies
+    assert torch.equal(out, want)
+    if not copies:
+        assert ctx.pool_stats()[0] - kept < 1 << 30
+
+
+@pytest.mark.parametrize("notation,sizes", [
+    ("ibj,jbk->bik", dict(b=7, i=200, j=48, k=100)),  # K that 32-deep iterations would pad by a third
+    ("ij,jk->ik", dict(i=128, j=40000, k=128)),  # few outputs and a K that fills the chip: large tiles
+    ("ij,jk->ik", dict(i=97, j=20001, k=97)),  # ... in the four-product form
+    ("ij,jk->ik", dict(i=129, j=40000, k=65)),  # ... where they would be padding: small tiles
+    ("ij,ij->", dict(i=275, j=301)),  # one tile with a long K: by gather
+    ("ij,jk->ik", dict(i=20, j=70001, k=33)),
+    ("ji,kj->ki", dict(i=344, j=280, k=312)),  # tiles in equal ranges rather than three pieces each
+])
+@pytest.mark.parametrize("conj", [False, True])
+def test_complex_tiles(tb, oracle, notation, sizes, conj):
+    shapes = [tuple(sizes[c] for c in t) for t in notation.split("->")[0].split(",")]
+    run(tb, oracle, notation, shapes, np.complex128, conj, 0.5)
