@@ -482,7 +482,10 @@ namespace tfb {
 using RealTma = DmmaTmaCfg<false, 128, 128, 16, 4, 4, 6>;
 // 32-deep k-iterations, three stages: half the barrier hand-offs of 16-deep ones with six (chi = 512 chain,
 // per product: 68.0 -> 66.6 us).  The real kernel gains 1 % at 4000^3 and loses 6 % at K = 300 by it.
+// K = 48 would be a third padding (500 x 60 x 48, 76 batches: 59.9 us against 49.5), so K that 32 does not nearly divide
+// keeps 16-deep ones.
 using CplxTma = DmmaTmaCfg<true, 64, 64, 32, 4, 4, 3>;
+using CplxTma16 = DmmaTmaCfg<true, 64, 64, 16, 4, 4, 6>;
 // Sixteen warps on a 64 x 64 tile (four took 13.6 us at 200^3, sixteen 10.4; 400^3: 22.4, 17.7): more
 // fragment loads per MMA, but a warp alone on its scheduler leaves the pipe idle while it loads.
 using RealTmaSmall = DmmaTmaCfg<false, 64, 64, 16, 4, 4, 8>;
@@ -504,7 +507,9 @@ static tfb_status run_tma(tfb_ctx* ctx, const ContractProblem& p, const Contract
         return small ? run_tma_cfg<RealTmaSmall>(ctx, p, a, declined) : run_tma_cfg<RealTma>(ctx, p, a, declined);
     }
     if (four) return small ? run_tma_cfg<CplxTma4Small>(ctx, p, a, declined) : run_tma_cfg<CplxTma4>(ctx, p, a, declined);
-    return small ? run_tma_cfg<CplxTmaSmall>(ctx, p, a, declined) : run_tma_cfg<CplxTma>(ctx, p, a, declined);
+    if (small) return run_tma_cfg<CplxTmaSmall>(ctx, p, a, declined);
+    const int64_t k16 = (a.K + 15) / 16 * 16, k32 = (a.K + 31) / 32 * 32;
+    return k32 * 15 > k16 * 16 ? run_tma_cfg<CplxTma16>(ctx, p, a, declined) : run_tma_cfg<CplxTma>(ctx, p, a, declined);
 }
 
 // Operands without a tensor map (odd leading extents of f64, groups of several modes that do not
@@ -627,8 +632,17 @@ tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined,
     }
     // 32 x 32 tiles below an eighth of the SMs' worth of 64 x 64 ones (eight launches of a chain, chi = 64: 80
     // against 124 us, 97: 91 against 159, 192: 128 against 157, 338: 368 against 278).
-    bool small = (a.M <= 32 || a.N <= 32 || a.M * a.N * a.B < (int64_t)64 * 64 * ctx->sm_count / 8);
+    // But a long K fills the chip with ranges of 64 x 64 tiles as well, and those run at 1.3 (four products) to 1.5 times
+    // the rate of 32 x 32 ones, unless that is lost to padding.  A tile is cut into 32 ranges at most, and the
+    // fewer the tiles the more the pieces of each cost, so the K it takes grows with the square of their number going
+    // down (us on 32 x 32, on 64 x 64: 256 x 256 x 1000 31, 28; 192 x 192 x 1000 21, 26; x 2000 34.5, 33.4; x 30000 366, 254;
+    // 128 x 128 x 8000 53, 54; x 30000 169, 144; 160 x 160 x 30000 305, 255).
+    auto tiles = [&](int64_t t) { return ((a.M + t - 1) / t) * ((a.N + t - 1) / t); };
+    const int64_t tiles64 = tiles(64) * a.B;
+    const bool long_k = tiles64 * 40 >= ctx->sm_count && tiles64 * tiles64 * ((a.K + 31) / 32) >= (int64_t)ctx->sm_count * 32 &&
+                        tiles(64) * 4 * 20 <= tiles(32) * (a.K % 4 ? 25 : 29);
     bool small_gather = (a.M <= 32 || a.N <= 32);
+    bool small = small_gather || (a.M * a.N * a.B < (int64_t)64 * 64 * ctx->sm_count / 8 && !long_k);
     if (shape == 1) small = small_gather = true;
     if (shape == 2) small = small_gather = false;
     // Three real products make a complex one with an imaginary part that is a difference of sums as
@@ -642,7 +656,11 @@ tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined,
         TFB_TRY(run_tma(ctx, p, a, small, false, &d));
         if (!d) return TFB_OK;
     }
-    if (use_tma) {
+    // (A tile or two in 32 ranges each, the most that one tile is cut into, leave more than half the SMs idle: with a very
+    // long K the gather kernel, which cuts finer, is ahead.  "ij,ij->" of 80001 elements 131 us against 168, of 176551 277
+    // against 197.)
+    const bool idle = small && tiles(32) * a.B <= 2 && a.K >= 120000;
+    if (use_tma && !idle) {
         TFB_TRY(run_tma(ctx, p, a, small, true, &d));
         if (!d) return TFB_OK;
         TFB_TRY(on_copies(small, &d));

@@ -536,6 +536,9 @@ static tfb_status run_tma_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractAr
         const int64_t want = std::min<int64_t>(std::min<int64_t>(32, slots / a.n_tiles), a.k_iters * Cfg::BK / 64);
         a.iters_per_cta = (a.k_iters + want - 1) / want;
         pieces = (int)((a.k_iters + a.iters_per_cta - 1) / a.iters_per_cta);
+        // 32-deep iterations do not deal out as evenly: where fewer pieces than would fit leave a quarter of the SMs idle, the
+        // equal ranges below are ahead (344 x 312 x 280 complex double in 90 pieces of three iterations: 23.8 us, 19.9)
+        if (Cfg::BK > 16 && pieces < want && a.n_tiles * pieces * 4 < slots * 3) pieces = 0;
     }
     if (pieces > 1) {
         // ranges are per tile: CTA c takes piece c % pieces of tile c / pieces
