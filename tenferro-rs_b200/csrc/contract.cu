@@ -225,7 +225,7 @@ void fill_args(const ContractProblem& p, const ContractTables& t, ContractArgs* 
 //
 // 64 x 64 block tile, 16-deep k slices (8 for 16-byte elements), 256 threads, 4 x 4 outputs each.  The next
 // slice is in flight from global memory to registers while one is computed from shared memory, and a
-// fragment is four neighbours, one 16-byte access for f32.  Few tiles with a long K are cut into
+// f32 fragment is four neighbours, one 16-byte access.  Few tiles with a long K are cut into
 // gridDim.y ranges whose sums simt_finish_kernel adds in range order (no result depends on timing).
 // Small shapes are bound by latency, the rest by issue and shared memory (kernel and finish): 679 x 636 x 431 f32
 // 90 -> 33 us, 510 x 690 x 945 105 -> 48, 38 x 1209 x 31 complex32 240 -> 33 (one tile, so one CTA before),
@@ -233,29 +233,32 @@ void fill_args(const ContractProblem& p, const ContractTables& t, ContractArgs* 
 template <typename T>
 constexpr int kSimtK = sizeof(T) == 16 ? 8 : 16;
 template <typename T>
-constexpr int kSimtCtas = sizeof(T) == 4 ? 3 : 2;  // CTAs per SM, what their registers leave
+constexpr int kSimtCtas = sizeof(T) == 4 ? 3 : sizeof(T) == 16 ? 1 : 2;  // CTAs per SM, what their registers leave
 
+// beta equal to the semiring's zero means "overwrite": the output is never read.
+template <int ALG>
+__device__ __forceinline__ bool simt_reads_c(const ContractArgs& g) {
+    return ALG == 0 ? (g.beta_re != 0 || g.beta_im != 0) : !(g.beta_re == (ALG == 1 ? -INFINITY : INFINITY));
+}
+// `old`: what the output holds, where it is read.
 template <typename T, int ALG>
-__device__ __forceinline__ void simt_store(const ContractArgs& g, const T* D, int64_t m, int64_t n, T* Cb, T sum) {
+__device__ __forceinline__ T simt_result(const ContractArgs& g, const T* D, int64_t m, int64_t n, T old, T sum) {
     using S = Semi<T, ALG>;
-    const T alpha = Ops<T>::from(Scalar{g.alpha_re, g.alpha_im});
-    const T beta = Ops<T>::from(Scalar{g.beta_re, g.beta_im});
-    // beta equal to the semiring's zero means "overwrite": the output is never read
-    const bool read_c = ALG == 0 ? (g.beta_re != 0 || g.beta_im != 0) : !(g.beta_re == (ALG == 1 ? -INFINITY : INFINITY));
-    T* p = Cb + g.c_m[m] + g.c_n[n];
     if (D) {
         const T d = D[g.d_m[m] + g.d_n[n]];
         sum = Ops<T>::mul(sum, g.conj_mul ? Ops<T>::conj(d) : d);
     }
-    T v = S::mul(alpha, sum);
-    if (read_c) v = S::add(v, S::mul(beta, *p));
-    *p = v;
+    const T v = S::mul(Ops<T>::from(Scalar{g.alpha_re, g.alpha_im}), sum);
+    return simt_reads_c<ALG>(g) ? S::add(v, S::mul(Ops<T>::from(Scalar{g.beta_re, g.beta_im}), old)) : v;
 }
 
 template <typename T, int ALG = 0>
 __global__ void __launch_bounds__(256, kSimtCtas<T>) contract_simt_kernel(ContractArgs g) {
     using S = Semi<T, ALG>;
     constexpr int BM = 64, BN = 64, BK = kSimtK<T>, P = 68, L = BM * BK / 256;
+    // A thread's fragment: four neighbours for 4-byte elements, else four 16 apart, which meet no bank twice (988 x
+    // 1383 x 127 complex double 165 us with neighbours, 111 without) and leave a small output to more threads.
+    constexpr int E = sizeof(T) > 4 ? 1 : 4, J = sizeof(T) > 4 ? 16 : 1;
     __shared__ __align__(16) T As[2][BK][P];
     __shared__ __align__(16) T Bs[2][BK][P];
     const int tid = threadIdx.x;
@@ -314,9 +317,9 @@ __global__ void __launch_bounds__(256, kSimtCtas<T>) contract_simt_kernel(Contra
             for (int kk = 0; kk < BK; ++kk) {
                 T av[4], bv[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) av[i] = As[buf][kk][4 * tx + i];
+                for (int i = 0; i < 4; ++i) av[i] = As[buf][kk][E * tx + J * i];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) bv[j] = Bs[buf][kk][4 * ty + j];
+                for (int j = 0; j < 4; ++j) bv[j] = Bs[buf][kk][E * ty + J * j];
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -330,19 +333,29 @@ __global__ void __launch_bounds__(256, kSimtCtas<T>) contract_simt_kernel(Contra
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) P0[(4 * ty + j) * BM + 4 * tx + i] = acc[i][j];
+                for (int i = 0; i < 4; ++i) P0[(E * ty + J * j) * BM + E * tx + J * i] = acc[i][j];
             continue;
         }
         T* Cb = (T*)g.c + g.c_b[bb];
         const T* D = g.mul ? reinterpret_cast<const T*>(g.mul) + g.d_b[bb] : nullptr;
+        // A thread's outputs are read together, not one after the other's store.
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int64_t n = n0 + 4 * ty + j;
+            const int64_t n = n0 + E * ty + J * j;
             if (n >= g.N) continue;
+            T* col = Cb + g.c_n[n];
+            T old[4];
+            if (simt_reads_c<ALG>(g)) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int64_t m = m0 + E * tx + J * i;
+                    if (m < g.M) old[i] = col[g.c_m[m]];
+                }
+            }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int64_t m = m0 + 4 * tx + i;
-                if (m < g.M) simt_store<T, ALG>(g, D, m, n, Cb, acc[i][j]);
+                const int64_t m = m0 + E * tx + J * i;
+                if (m < g.M) col[g.c_m[m]] = simt_result<T, ALG>(g, D, m, n, old[i], acc[i][j]);
             }
         }
     }
@@ -360,7 +373,9 @@ __global__ void __launch_bounds__(256) simt_finish_kernel(ContractArgs g, int sp
     T sum = P0[0];
 #pragma unroll 8
     for (int s = 1; s < splits; ++s) sum = Semi<T, ALG>::add(sum, P0[(int64_t)s * g.n_tiles * (BM * BN)]);
-    simt_store<T, ALG>(g, g.mul ? reinterpret_cast<const T*>(g.mul) + g.d_b[bb] : nullptr, m, n, (T*)g.c + g.c_b[bb], sum);
+    T* at = (T*)g.c + g.c_b[bb] + g.c_m[m] + g.c_n[n];
+    const T old = simt_reads_c<ALG>(g) ? *at : sum;
+    *at = simt_result<T, ALG>(g, g.mul ? reinterpret_cast<const T*>(g.mul) + g.d_b[bb] : nullptr, m, n, old, sum);
 }
 
 template <typename T, int ALG>
