@@ -734,10 +734,23 @@ struct Red {
     }
 };
 
-// Combines the values of the G threads of each kept element; the result is valid where g == 0.
+template <typename T>
+__device__ __forceinline__ T shuffle_down(T v, int s) {
+    union { T t; uint32_t w[sizeof(T) / 4]; } u;
+    u.t = v;
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(T) / 4; ++i) u.w[i] = __shfl_down_sync(0xffffffffu, u.w[i], s);
+    return u.t;
+}
+// Combines the values of the G threads of each kept element; the result is valid where g == 0.  In the same order by
+// shuffles, where the threads are neighbours in a warp, and through shared memory.
 template <typename T, int OP>
 __device__ __forceinline__ T combine_group(T acc, T* sh, int g, int G, int step) {
     if (G == 1) return acc;
+    if (step == 1 && G <= 32) {
+        for (int s = G >> 1; s > 0; s >>= 1) acc = Red<T, OP>::comb(acc, shuffle_down(acc, s));
+        return acc;
+    }
     __syncthreads();
     sh[threadIdx.x] = acc;
     for (int s = G >> 1; s > 0; s >>= 1) {
@@ -847,11 +860,13 @@ constexpr int kRedCtas = sizeof(T) == 16 ? 2 : sizeof(T) == 4 ? 3 : 4;
 // (the walk in 64 bits holds too many values for more than two)
 template <typename T, int RANK, typename N>
 constexpr int kRedBound = RANK == 0 && std::is_same<N, LoopNest>::value ? 2 : kRedCtas<T>;
-template <typename T, int OP, bool RED_FAST, int RANK, typename N>
-__global__ void __launch_bounds__(256, (kRedBound<T, RANK, N>)) reduce_kernel(const __grid_constant__ N kept, const __grid_constant__ N red,
+// SHORT: a thread has no more than eight elements, and four loads in flight: with sixteen most of them would be
+// tests and neutral elements (496 x 1576 x 16 f32, the maximum over the last index: 30 us, 14 before).
+template <typename T, int OP, bool RED_FAST, int RANK, bool SHORT, typename N>
+__global__ void __launch_bounds__(256, (SHORT ? 4 : kRedBound<T, RANK, N>)) reduce_kernel(const __grid_constant__ N kept, const __grid_constant__ N red,
                                                      const T* __restrict__ in, T* out, T* partial, int log_g, int64_t chunk,
                                                      EpilogueArgs<T> ep) {
-    constexpr int U = kRedLoads<T>;
+    constexpr int U = SHORT ? 4 : kRedLoads<T>;
     __shared__ T sh[256];
     const int G = 1 << log_g, TX = 256 >> log_g;
     const int g = RED_FAST ? threadIdx.x & (G - 1) : threadIdx.x / TX;
@@ -876,11 +891,13 @@ __global__ void __launch_bounds__(256, (kRedBound<T, RANK, N>)) reduce_kernel(co
 #pragma unroll
                 for (int u = 0; u < U; ++u) part[u] = Red<T, OP>::comb(part[u], v[u]);
             }
-            T v[U];
+            if (r < r1) {
+                T v[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) v[u] = r + u * G < r1 ? p[walk.next(red, r + u * G, G)] : Red<T, OP>::init();
+                for (int u = 0; u < U; ++u) v[u] = r + u * G < r1 ? p[walk.next(red, r + u * G, G)] : Red<T, OP>::init();
 #pragma unroll
-            for (int u = 0; u < U; ++u) part[u] = Red<T, OP>::comb(part[u], v[u]);
+                for (int u = 0; u < U; ++u) part[u] = Red<T, OP>::comb(part[u], v[u]);
+            }
         }
 #pragma unroll
         for (int s = U / 2; s > 0; s >>= 1)
@@ -974,17 +991,24 @@ template <typename T, int OP, typename N>
 static void reduce_launch(tfb_ctx* ctx, const N& kept, const N& red, const T* in, T* out, T* partial, const ReduceShape& r,
                           const EpilogueArgs<T>& ep) {
     const dim3 grid(r.grid, (unsigned)r.splits);
-    auto go = [&](auto rank) {
+    auto go = [&](auto rank, auto few) {
         constexpr int RANK = decltype(rank)::value;
+        constexpr bool SHORT = decltype(few)::value;
         if (r.red_fast)
-            reduce_kernel<T, OP, true, RANK><<<grid, 256, 0, ctx->stream>>>(kept, red, in, out, partial, r.log_g, r.chunk, ep);
+            reduce_kernel<T, OP, true, RANK, SHORT><<<grid, 256, 0, ctx->stream>>>(kept, red, in, out, partial, r.log_g, r.chunk, ep);
         else
-            reduce_kernel<T, OP, false, RANK><<<grid, 256, 0, ctx->stream>>>(kept, red, in, out, partial, r.log_g, r.chunk, ep);
+            reduce_kernel<T, OP, false, RANK, SHORT><<<grid, 256, 0, ctx->stream>>>(kept, red, in, out, partial, r.log_g, r.chunk, ep);
     };
-    if (red.rank == 1) return go(std::integral_constant<int, 1>{});
     if constexpr (std::is_same<N, Nest32>::value)
-        if (red.rank == 2) return go(std::integral_constant<int, 2>{});
-    go(std::integral_constant<int, 0>{});
+        if (r.chunk <= (int64_t)8 << r.log_g) {
+            if (red.rank == 1) return go(std::integral_constant<int, 1>{}, std::true_type{});
+            if (red.rank == 2) return go(std::integral_constant<int, 2>{}, std::true_type{});
+            return go(std::integral_constant<int, 0>{}, std::true_type{});
+        }
+    if (red.rank == 1) return go(std::integral_constant<int, 1>{}, std::false_type{});
+    if constexpr (std::is_same<N, Nest32>::value)
+        if (red.rank == 2) return go(std::integral_constant<int, 2>{}, std::false_type{});
+    go(std::integral_constant<int, 0>{}, std::false_type{});
 }
 template <typename T, int OP, typename N>
 static void reduce_finish_launch(tfb_ctx* ctx, const N& kept, T* out, const T* partial, const ReduceShape& r,
