@@ -215,8 +215,8 @@ __global__ void __launch_bounds__(256) permute_tiled_kernel(LoopNest nest, const
 // All loads of a thread are issued before the first is used.  Neighbouring tiles in both directions run close in
 // time, since with odd extents they share sectors.
 // Bound by HBM for large tensors.  14 x 89 x 15 x 10 x 149 f64 in the order 4,2,3,1,0: 481 -> 110 us (generic
-// kernel), 27 x 9 x 68 x 24 x 84 f64 in 4,1,3,0,2: 227 -> 163 (square tiles of two modes), 11 x 130 x 9 x 75 x 9 f32
-// in 0,4,1,2,3: 59 -> 40 (rows of 44 bytes).  Some 35 instructions per element keep f32 at 2 TB/s.
+// kernel), 27 x 9 x 68 x 24 x 84 f64 in 4,1,3,0,2: 227 -> 163 (square tiles of two modes).  Some 35 instructions per
+// element keep f32 at 2 TB/s.
 constexpr int kSide = 256;  // longest side of a tile, (R, I) or (R, J)
 template <typename T>
 constexpr int kPatch = sizeof(T) >= 16 ? 2048 : 4096;  // elements of a tile
@@ -298,13 +298,22 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) permute_tile_kern
         for (int k = 0; k < L; ++k)
             if (tid + 256 * k < count) patch[at[k]] = v[k];
         __syncthreads();
+        if (ep.read_out) {
+            // all of a thread's outputs are on their way before the first store
+#pragma unroll
+            for (int k = 0; k < L; ++k) {
+                const uint32_t e = tid + 256 * k;
+                if (e >= count) continue;
+                const uint32_t i = dj.quotient(e), jr = e - i * dj.d;
+                v[k] = dst[(int64_t)out_j[jr] + out_i[i]];
+            }
+        }
 #pragma unroll
         for (int k = 0; k < L; ++k) {
             const uint32_t e = tid + 256 * k;
             if (e >= count) continue;
             const uint32_t i = dj.quotient(e), jr = e - i * dj.d;
-            T* o = dst + ((int64_t)out_j[jr] + out_i[i]);
-            *o = ep.apply(patch[i * pitch + jr], o);
+            dst[(int64_t)out_j[jr] + out_i[i]] = ep.apply(patch[i * pitch + jr], &v[k]);
         }
         __syncthreads();
     }
@@ -312,8 +321,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) permute_tile_kern
 
 // Fits the tile path to a nest in output order (mode 0 fastest); false where another path is the better one.
 template <typename T>
-static bool plan_tiles(const LoopNest& n, TilePlan* p) {
+static bool plan_tiles(const LoopNest& n, int sms, TilePlan* p) {
     if (n.rank < 2 || n.total >= ((int64_t)1 << 31) || n.stride[1][0] != 1) return false;
+    // Tiles for less than six tenths of the SMs: a tile's latency is longer than that of the one element a thread moves
+    // on the other paths (us there and in tiles: 54432 f64 4.8, 7.2; 349272 f32 6.3, 9.2; 599760 f32 10.3, 8.4; 425776
+    // complex double 8.8, 7.0).
+    if (n.total * 10 < (int64_t)sms * 6 * kPatch<T>) return false;
     auto mag = [](int64_t v) { return v < 0 ? -v : v; };
     int im = -1;
     for (int d = 0; d < n.rank; ++d)
@@ -461,14 +474,20 @@ static tfb_status permute_typed(tfb_ctx* ctx, const LoopNest& nest_out_order, co
         TFB_CUDA(cudaGetLastError());
         return TFB_OK;
     };
-    // Row path: both tensors walk mode 0.  Rows of less than 256 bytes whose neighbours lie apart in one of
-    // the tensors are the tile path's.
+    // Row path: both tensors walk mode 0.
     if (nest.rank >= 1 && nest.stride[0][0] == 1 && nest.stride[1][0] == 1) {
-        if (nest.extent[0] * (int64_t)sizeof(T) < 256 && plan_tiles<T>(nest, &tiles)) return run_tiles();
         constexpr int VMAX = 16 / sizeof(T) > 0 ? 16 / sizeof(T) : 1;
         bool vec = VMAX > 1 && nest.extent[0] % VMAX == 0 && ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0);
         for (int d = 1; d < nest.rank && vec; ++d)
             vec = nest.stride[0][d] % VMAX == 0 && nest.stride[1][d] % VMAX == 0;
+        // Short rows of 8- and 16-byte elements whose neighbours in the output lie a megabyte or more apart in the input
+        // reach HBM as single sectors: there the tile path, which gathers whole lines, is the better one (time by rows
+        // over time in tiles, 16 M elements, outer modes reversed: 24 bytes f64 1.42, 56 bytes 1.13; 32 and 96 bytes complex
+        // double 1.74, 1.35).  Not so with nearer neighbours (24 bytes f64 0.89, 56 bytes 0.5 to 0.9), from 72 bytes f64 on
+        // (0.62), where 8-byte elements move in 16-byte accesses (0.81) and for f32 (1.1 at most, mostly 0.3 to 0.9).
+        const int64_t row = nest.extent[0] * (int64_t)sizeof(T), most = sizeof(T) == 16 ? 128 : sizeof(T) == 8 && !vec ? 64 : 0;
+        if (row < most && nest.rank > 1 && std::llabs(nest.stride[0][1]) * (int64_t)sizeof(T) >= (1 << 20) && plan_tiles<T>(nest, sms, &tiles))
+            return run_tiles();
         const int64_t units = vec ? nest.total / VMAX : nest.total;
         const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((units + 1023) / 1024, (int64_t)sms * 16));
         LaunchScope ls(ctx, "permute_rows");
@@ -519,7 +538,7 @@ static tfb_status permute_typed(tfb_ctx* ctx, const LoopNest& nest_out_order, co
                 if (d != 1 && r.stride[1][d] % V != 0) vec = false;  // every output stride but the unit one
             }
             const double fill = (double)r.extent[0] * (double)r.extent[1] / ((double)kTile * kTile * (double)ti * (double)tj);
-            if (fill < (sizeof(T) == 4 ? 0.2 : 0.3) && plan_tiles<T>(nest, &tiles)) return run_tiles();
+            if (fill < (sizeof(T) == 4 ? 0.2 : 0.3) && plan_tiles<T>(nest, sms, &tiles)) return run_tiles();
             // What has no plan (2^31 elements, spans of a group above 1e9) and puts few elements into a tile is better off
             // element by element (ms, that way and in tiles: f32 8 x 8 patches 16.6, 85.4; 12 x 12 19.4, 39.2; 15 x 15 25.1,
             // 27.1; f64 8 x 8 22.7, 142; 14 x 14 40.4, 50.5; 15 x 15 42.6, 33.2; complex double 8 x 15 47.4, 64.7).
@@ -543,7 +562,7 @@ static tfb_status permute_typed(tfb_ctx* ctx, const LoopNest& nest_out_order, co
             }
         }
     }
-    if (plan_tiles<T>(nest, &tiles)) return run_tiles();
+    if (plan_tiles<T>(nest, sms, &tiles)) return run_tiles();
     int64_t blocks = (nest.total + 255) / 256;
     int64_t cap = (int64_t)sms * 16;
     int grid = (int)(blocks < cap ? blocks : cap);

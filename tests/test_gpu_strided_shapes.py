@@ -145,3 +145,24 @@ def test_permute_orders(tb, oracle, shape, perm, dtype, padded):
         assert (got == 7).all()  # nothing between the columns was written
     else:
         assert np.array_equal(out.to_numpy(), want)
+
+
+# Large enough for tiles of grouped modes, and what other paths take: (shape, order, types on tiles)
+EVERY = (np.float32, np.float64, np.complex64, np.complex128)
+
+
+@pytest.mark.parametrize("shape,perm,on_tiles", [
+    ((14, 89, 15, 10, 3), (4, 2, 3, 1, 0), EVERY), ((27, 9, 68, 24, 2), (4, 1, 3, 0, 2), EVERY), ((5, 70001, 2), (1, 2, 0), EVERY),
+    ((1000, 3, 6, 40), (2, 1, 3, 0), EVERY), ((3, 5, 7, 11, 13, 31), (5, 4, 3, 2, 1, 0), EVERY),
+    ((3, 40, 1200, 9), (0, 3, 2, 1), EVERY[1:]),  # short rows far apart
+    ((3, 9, 1200, 40), (0, 2, 1, 3), ()), ((701, 803), (1, 0), ()),
+])
+@pytest.mark.parametrize("dtype", EVERY)
+@pytest.mark.parametrize("padded", [False, True])
+def test_permute_tiles(tb, oracle, shape, perm, on_tiles, dtype, padded):
+    ctx = tb.Context.get(0)
+    ctx.profile_begin()
+    test_permute_orders(tb, oracle, shape, perm, dtype, padded)
+    ran = ctx.profile_read("permute_tile")[0]
+    ctx.profile_end()
+    assert ran == (2 if dtype in on_tiles else 0)
