@@ -151,6 +151,14 @@ __global__ void __launch_bounds__(256) permute_rows_kernel(N nest, const T* __re
     }
 }
 
+// CTAs of a kernel whose threads take up to four units each: one unit while the chip has room for all of them at
+// once (8 CTAs an SM), since a thread's four follow one another where there are few (57 x 128 complex double copied:
+// 5.8 us with four, 4.4 with one).
+static unsigned grid_of_four(int64_t units, int sms, int most) {
+    const int64_t one = (units + 255) / 256, room = (int64_t)sms * 8;
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(std::max<int64_t>(std::min(one, room), (units + 1023) / 1024), (int64_t)sms * most));
+}
+
 // Tiled transpose path: mode 0 is the input's stride-1 mode ("i"), mode 1 the output's
 // stride-1 mode ("j").  A TILE x TILE patch goes through shared memory so that both the
 // reads (along i) and the writes (along j) are full 128-byte lines.  Tiles run eight along i, then along j: with odd
@@ -489,7 +497,7 @@ static tfb_status permute_typed(tfb_ctx* ctx, const LoopNest& nest_out_order, co
         if (row < most && nest.rank > 1 && std::llabs(nest.stride[0][1]) * (int64_t)sizeof(T) >= (1 << 20) && plan_tiles<T>(nest, sms, &tiles))
             return run_tiles();
         const int64_t units = vec ? nest.total / VMAX : nest.total;
-        const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((units + 1023) / 1024, (int64_t)sms * 16));
+        const unsigned grid = grid_of_four(units, sms, 16);
         LaunchScope ls(ctx, "permute_rows");
         auto go = [&](const auto& n) {
             if (vec) permute_rows_kernel<T, VMAX><<<grid, 256, 0, ctx->stream>>>(n, (const T*)in, (T*)out, ep);
@@ -674,8 +682,7 @@ template <typename T, int V>
 static void launch_ewmul_rows(tfb_ctx* ctx, const LoopNest& nest, const T* a, const T* b, T* out, const EpilogueArgs<T>& ep, bool ca,
                               bool cb) {
     const bool run_a = nest.stride[0][0] != 0, run_b = nest.stride[1][0] != 0;
-    const int64_t blocks = (nest.total / V + 1023) / 1024, cap = (int64_t)ctx->sm_count * 8;
-    const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
+    const unsigned grid = grid_of_four(nest.total / V, ctx->sm_count, 8);
     if (Nest32::fits(nest)) {
         Nest32 n(nest);
         n.div[0] = FastDiv::of((uint32_t)(nest.extent[0] / V));
