@@ -233,7 +233,7 @@ void fill_args(const ContractProblem& p, const ContractTables& t, ContractArgs* 
 template <typename T>
 constexpr int kSimtK = sizeof(T) == 16 ? 8 : 16;
 template <typename T>
-constexpr int kSimtCtas = sizeof(T) == 4 ? 3 : sizeof(T) == 16 ? 1 : 2;  // CTAs per SM, what their registers leave
+constexpr int kSimtCtas = sizeof(T) == 4 ? 3 : sizeof(T) == 16 ? 1 : 2;  // CTAs per SM (f32 spills 84 bytes at three)
 
 // beta equal to the semiring's zero means "overwrite": the output is never read.
 template <int ALG>

@@ -480,6 +480,7 @@ static tfb_status run_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractArgs a
 namespace tfb {
 
 using RealTma = DmmaTmaCfg<false, 128, 128, 16, 4, 4, 6>;
+// (44 bytes of registers spilled at 128 a thread, 16 in the four-product form, 20 with 16-deep iterations.)
 // 32-deep k-iterations, three stages: half the barrier hand-offs of 16-deep ones with six (chi = 512 chain,
 // per product: 68.0 -> 66.6 us).  The real kernel gains 1 % at 4000^3 and loses 6 % at K = 300 by it.
 // K = 48 would be a third padding (500 x 60 x 48, 76 batches: 59.9 us against 49.5), so K that 32 does not nearly divide

@@ -2,8 +2,8 @@
 //
 // When each of M, N, K is a single fused mode and one side of every operand has unit stride,
 // the operand tiles need no per-thread gather: one thread at a time issues two cp.async.bulk.tensor
-// loads per k-iteration, a few iterations ahead, and the sixteen warps do nothing but
-// fragment loads and DMMAs, synchronised by full/empty mbarriers (no CTA-wide barrier in
+// loads per k-iteration, one to six iterations ahead, and the CTA's four to sixteen warps do nothing
+// else but fragment loads and DMMAs, synchronised by full/empty mbarriers (no CTA-wide barrier in
 // the main loop, and the ring keeps running across the tiles of a stream-K range).
 //
 // The tensor maps are built so that the box lands in the order the m16n8k8 fragments are
@@ -18,14 +18,14 @@
 // The four-product complex form takes any extent.  A complex element is 16 bytes, all that TMA asks of
 // an address, so dimension 0 can be the whole extent (zero-filled past its end) with one load per
 // run.  To keep those few, runs are 128-byte lines:
-//   K-major   [k-panel of 8][row][8 k]    2 loads per 16 k
+//   K-major   [k-panel of 8][row][8 k]    one load per 8 k
 //   MN-major  [group of 8 rows][k][8 rows]    8 loads for 64 rows (one load where 8 divides the extent)
 // with TMA's 128-byte swizzle; lane (row r, slot c) reads k = 2c and 2c + 1 of an 8-deep step, so a
 // quarter warp (two rows, four k of one parity) finds its 16-byte units in chunks (r ^ k) mod 8 that take
 // every value once.  (Which k meets which slot of an MMA does not matter while both operands agree.)
 // The issue of ten loads is nothing next to the 8000 clocks of a k-iteration's MMAs.  Such extents - odd
 // bond dimensions - used to be left to the gather kernel: a chain with chi = 97 took 18.5 + 10.5 us
-// (kernel and fix-up launch) per product, 11 us here.
+// (kernel and fix-up launch) per product, 9.8 us here.
 #pragma once
 #include "f64_map.h"
 #include "ptx_sm100.cuh"

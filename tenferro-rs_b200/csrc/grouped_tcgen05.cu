@@ -1,7 +1,7 @@
 // Grouped f32 products on the tcgen05 tensor cores: the kernel of tfb_grouped_gemm for ragged
 // tables of column-major problems that the mma.sync kernel (grouped_tf32.cu) declines - any
 // m, n, k >= 1 with 16-byte aligned columns and K up to 512 - where it is faster than the
-// general kernel of grouped.cu (4096 problems with dims from {20, 36, 72, 136}: 181 us against 276).
+// general kernel of grouped.cu (4096 problems with dims from {20, 36, 72, 136}: 171 us against 271).
 // On tables the mma.sync kernel takes (dims in multiples of 16, K <= 128) that kernel is the
 // faster one (54 us against 96 for 4096 problems with dims from {16, 32, 64, 128}); see the end of
 // this comment for why.  TFB_GROUPED_PREFER_TCGEN05=1 asks for this kernel first.
