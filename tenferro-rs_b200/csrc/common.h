@@ -72,12 +72,13 @@ struct tfb_ctx {
     size_t smem_optin = 0;
     // One-word device status used by kernels with bounded waits (0 = fine).
     int* dev_status = nullptr;
-    // Scratch of the in-kernel stream-K reduction: one accumulator slot and one flag per CTA.
+    // Scratch of the in-kernel stream-K reduction: two accumulator slots per CTA.
     void* sk_partial = nullptr;
     size_t sk_partial_bytes = 0;
-    unsigned* sk_flags = nullptr;
-    size_t sk_flags_n = 0;
-    unsigned sk_epoch = 0;
+    // Counters of kernels whose last CTA to arrive at an output finishes it: zero between launches (the last one to
+    // arrive puts its counter back), so one array serves every launch and replay of this in-order queue.
+    static constexpr size_t kArrived = 8192;
+    unsigned* arrived = nullptr;
     // Optional per-launch timing (tfb_ctx_profile_*): event pairs around named launches.
     bool profiling = false;
     float prof_pair_ms = 0;  // duration an empty event pair reports, subtracted from every launch
@@ -254,5 +255,33 @@ struct LaunchScope {
     LaunchScope(tfb_ctx* c, const char* name);
     ~LaunchScope();
 };
+
+// Launches a kernel that waits for the end of the one ahead of it by itself (launch_begin, before it touches
+// global memory), so that its CTAs may be placed and set themselves up meanwhile; `cluster` CTAs
+// (0, 1: none) form a cluster.  Not on the legacy default stream, which orders itself against other streams, and not while
+// capturing, where a plain edge is what a replay needs.
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(tfb_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (!ctx->capturing && ctx->stream != nullptr && ctx->stream != cudaStreamLegacy && ctx->stream != cudaStreamPerThread) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 }  // namespace tfb

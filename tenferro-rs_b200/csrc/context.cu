@@ -161,6 +161,7 @@ tfb_status tfb_ctx_create(int device_id, tfb_ctx** out) {
         void operator()(tfb_ctx* c) const {
             if (c->own_stream) cudaStreamDestroy(c->own_stream);
             if (c->dev_status) cudaFree(c->dev_status);
+            if (c->arrived) cudaFree(c->arrived);
             if (c->pool) cudaMemPoolDestroy(c->pool);
             delete c;
         }
@@ -199,6 +200,8 @@ tfb_status tfb_ctx_create(int device_id, tfb_ctx** out) {
     TFB_CUDA(cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &threshold));
     TFB_CUDA(cudaMalloc(&c->dev_status, sizeof(int)));
     TFB_CUDA(cudaMemset(c->dev_status, 0, sizeof(int)));
+    TFB_CUDA(cudaMalloc(&c->arrived, tfb_ctx::kArrived * sizeof(unsigned)));
+    TFB_CUDA(cudaMemsetAsync(c->arrived, 0, tfb_ctx::kArrived * sizeof(unsigned), c->stream));
     *out = c.release();
     return TFB_OK;
 }
@@ -273,7 +276,7 @@ tfb_status tfb_ctx_destroy(tfb_ctx* ctx) {
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     if (ctx->dev_status) cudaFree(ctx->dev_status);
     if (ctx->sk_partial) cudaFree(ctx->sk_partial);
-    if (ctx->sk_flags) cudaFree(ctx->sk_flags);
+    if (ctx->arrived) cudaFree(ctx->arrived);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     delete ctx;
     return TFB_OK;
@@ -390,6 +393,8 @@ tfb_status tfb_ctx_synchronize(tfb_ctx* ctx) {
     TFB_CUDA(cudaMemcpy(&st, ctx->dev_status, sizeof st, cudaMemcpyDeviceToHost));
     if (st != 0) {
         cudaMemset(ctx->dev_status, 0, sizeof(int));
+        // an output that was given up was not counted to its end
+        cudaMemsetAsync(ctx->arrived, 0, tfb_ctx::kArrived * sizeof(unsigned), ctx->stream);
         return fail(TFB_ERR_DEVICE, "a kernel gave up a bounded wait (status word 0x%x)", st);
     }
     return TFB_OK;

@@ -180,22 +180,28 @@ static bool all_even(const std::vector<Mode>& g, int t, size_t from) {
     return true;
 }
 
-void fill_args(const ContractProblem& p, const ContractTables& t, ContractArgs* a) {
+void fill_args(const ContractProblem& p, const ContractTables* tables, ContractArgs* a) {
     memset(a, 0, sizeof *a);
     a->a = (const char*)p.a;
     a->b = (const char*)p.b;
     a->c = (char*)p.c;
-    a->a_b = t.a_b; a->b_b = t.b_b; a->c_b = t.c_b;
-    a->a_m = t.a_m; a->c_m = t.c_m;
-    a->b_n = t.b_n; a->c_n = t.c_n;
-    a->a_k = t.a_k; a->b_k = t.b_k;
-    a->M = t.M; a->N = t.N; a->K = t.K; a->B = t.B;
+    if (tables) {
+        const ContractTables& t = *tables;
+        a->a_b = t.a_b; a->b_b = t.b_b; a->c_b = t.c_b;
+        a->a_m = t.a_m; a->c_m = t.c_m;
+        a->b_n = t.b_n; a->c_n = t.c_n;
+        a->a_k = t.a_k; a->b_k = t.b_k;
+        a->d_b = t.d_b; a->d_m = t.d_m; a->d_n = t.d_n;
+    }
+    a->M = p.M(); a->N = p.N(); a->K = p.K(); a->B = p.B();
+    auto step = [](const std::vector<Mode>& g, int slot) { return g.empty() ? (int64_t)0 : g[0].s[slot]; };
+    a->c_bs = step(p.batch, 2); a->c_ms = step(p.m, 2); a->c_ns = step(p.n, 2);
+    a->d_bs = step(p.batch, 3); a->d_ms = step(p.m, 3); a->d_ns = step(p.n, 3);
     a->alpha_re = p.alpha.re; a->alpha_im = p.alpha.im;
     a->beta_re = p.beta.re; a->beta_im = p.beta.im;
     a->conj_a = p.conj_a && dtype_is_complex(p.dtype);
     a->conj_b = p.conj_b && dtype_is_complex(p.dtype);
     a->mul = (const char*)p.mul;
-    a->d_b = t.d_b; a->d_m = t.d_m; a->d_n = t.d_n;
     a->conj_mul = p.conj_mul && dtype_is_complex(p.dtype);
     // Direction of the unit stride in each operand tile.  If neither group is unit-stride
     // the choice only affects which threads sit next to each other.
@@ -414,7 +420,7 @@ tfb_status contract_simt(tfb_ctx* ctx, const ContractProblem& p) {
     std::shared_ptr<ContractTables> t;
     TFB_TRY(get_tables(ctx, p, &t));
     ContractArgs a;
-    fill_args(p, *t, &a);
+    fill_args(p, t.get(), &a);
     switch (p.dtype) {
         case TFB_F32: return simt_launch<float, 0>(ctx, a, "contract_simt");
         case TFB_F64: return simt_launch<double, 0>(ctx, a, "contract_simt");
@@ -433,7 +439,7 @@ tfb_status contract_simt_semiring(tfb_ctx* ctx, const ContractProblem& p, int al
     std::shared_ptr<ContractTables> t;
     TFB_TRY(get_tables(ctx, p, &t));
     ContractArgs a;
-    fill_args(p, *t, &a);
+    fill_args(p, t.get(), &a);
     const char* name = "contract_simt_semiring";
     if (p.dtype == TFB_F32 && algebra == 1) return simt_launch<float, 1>(ctx, a, name);
     if (p.dtype == TFB_F32 && algebra == 2) return simt_launch<float, 2>(ctx, a, name);

@@ -126,7 +126,7 @@ static tfb_status embedded_product(tfb_ctx* ctx, const ContractProblem& p, bool*
     std::shared_ptr<ContractTables> t;
     TFB_TRY(get_tables(ctx, p, &t));
     ContractArgs ca;
-    fill_args(p, *t, &ca);
+    fill_args(p, t.get(), &ca);
 
     const bool b_in_place = b_is_real_view(p) && env_int("TFB_C32_B_IN_PLACE", 1);
     const size_t a_floats = (size_t)(2 * M * ld * B), b_floats = b_in_place ? 0 : (size_t)(N * ld * B);

@@ -25,6 +25,14 @@ struct ContractArgs {
     const int64_t* c_m;
     const int64_t* b_n;
     const int64_t* c_n;
+    // Steps of the output's (and the multiplier's) offsets where a group is one mode and has no table (null).
+    int64_t c_bs, c_ms, c_ns, d_bs, d_ms, d_ns;
+    __device__ __forceinline__ int64_t off_c_b(int64_t i) const { return c_b ? c_b[i] : i * c_bs; }
+    __device__ __forceinline__ int64_t off_c_m(int64_t i) const { return c_m ? c_m[i] : i * c_ms; }
+    __device__ __forceinline__ int64_t off_c_n(int64_t i) const { return c_n ? c_n[i] : i * c_ns; }
+    __device__ __forceinline__ int64_t off_d_b(int64_t i) const { return d_b ? d_b[i] : i * d_bs; }
+    __device__ __forceinline__ int64_t off_d_m(int64_t i) const { return d_m ? d_m[i] : i * d_ms; }
+    __device__ __forceinline__ int64_t off_d_n(int64_t i) const { return d_n ? d_n[i] : i * d_ns; }
     const int64_t* a_k;
     const int64_t* b_k;
     int64_t M, N, K, B;
@@ -41,10 +49,12 @@ struct ContractArgs {
     int a_vec, b_vec;      // elements per cp.async (1, or 2 for f64 when 16-byte chunks are legal)
     // Work decomposition: tiles x k-iterations, cut into equal contiguous ranges ("stream-K").
     int64_t tiles_m, tiles_n, n_tiles, k_iters, total_iters, iters_per_cta;
-    unsigned* sk_flags;  // per-CTA flags of the in-kernel stream-K reduction (TMA-fed DMMA kernel)
-    unsigned sk_epoch;   // a flag is raised when it equals this launch's epoch
+    // TMA-fed DMMA kernel: CTAs of a cluster that share a tile's K (0, 1: none), and the ranges of a cut tile that have
+    // parked their sums, counted at the CTA that starts the tile (zero between launches).
+    int cluster;
+    unsigned* sk_arrived;
     int sk_two_phase;    // 1: every range parks its sums in its slot; a finishing kernel adds the pieces of a tile
-    // Sums of ranges that cut a tile.  Gather DMMA kernel: two block tiles per CTA; TMA-fed kernel: one per CTA; exact-
+    // Sums of ranges that cut a tile.  Gather and TMA-fed DMMA kernels: two block tiles per CTA; exact-
     // arithmetic kernel: [range][tile].
     char* partial;
 };
@@ -61,6 +71,26 @@ __device__ __forceinline__ void apply_mul_c128(const ContractArgs& g, int64_t of
     xr = r;
 }
 
+// C = alpha * x + beta * C at one double-precision element.
+template <bool CPLX>
+__device__ __forceinline__ void dmma_store(const ContractArgs& g, char* p, bool read_c, double xr, double xi) {
+    if constexpr (CPLX) {
+        double2 o;
+        o.x = g.alpha_re * xr - g.alpha_im * xi;
+        o.y = g.alpha_re * xi + g.alpha_im * xr;
+        if (read_c) {
+            const double2 old = *reinterpret_cast<const double2*>(p);
+            o.x += g.beta_re * old.x - g.beta_im * old.y;
+            o.y += g.beta_re * old.y + g.beta_im * old.x;
+        }
+        *reinterpret_cast<double2*>(p) = o;
+    } else {
+        double o = g.alpha_re * xr;
+        if (read_c) o += g.beta_re * *reinterpret_cast<const double*>(p);
+        *reinterpret_cast<double*>(p) = o;
+    }
+}
+
 // Multiplies a thread's m16n8 accumulator fragments (TM x TN of them, element (i, j, e) at row
 // m_first + 8 i, column n_first + 8 j + e; complex sums keep the imaginary part at [2 + e]) by the
 // fused multiplier, before anything is stored: with no store in between, all the loads are in flight
@@ -68,20 +98,20 @@ __device__ __forceinline__ void apply_mul_c128(const ContractArgs& g, int64_t of
 template <bool CPLX, int TM, int TN, int W>
 __device__ __forceinline__ void apply_mul_fragments(const ContractArgs& g, int64_t bb, int64_t m_first, int64_t n_first,
                                                     double (&acc)[TM][TN][W]) {
-    const int64_t db = g.d_b[bb];
+    const int64_t db = g.off_d_b(bb);
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int64_t n = n_first + 8 * j + e;
             if (n >= g.N) continue;
-            const int64_t dn = db + g.d_n[n];
+            const int64_t dn = db + g.off_d_n(n);
 #pragma unroll
             for (int i = 0; i < TM; ++i) {
                 const int64_t m = m_first + 8 * i;
                 if (m >= g.M) continue;
-                if constexpr (CPLX) apply_mul_c128(g, dn + g.d_m[m], acc[i][j][e], acc[i][j][2 + e]);
-                else apply_mul_f64(g, dn + g.d_m[m], acc[i][j][e]);
+                if constexpr (CPLX) apply_mul_c128(g, dn + g.off_d_m(m), acc[i][j][e], acc[i][j][2 + e]);
+                else apply_mul_f64(g, dn + g.off_d_m(m), acc[i][j][e]);
             }
         }
     }

@@ -479,7 +479,9 @@ static tfb_status run_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractArgs a
 
 namespace tfb {
 
-using RealTma = DmmaTmaCfg<false, 128, 128, 16, 4, 4, 6>;
+// 128 x 64: a finer cut than 128 x 128 at the same rate (us on 128 x 64, on 128 x 128: 1531 x 1283 x 2013 278, 293; 900^3 69, 76;
+// 1024^3 79, 82; 4000 x 300 x 4000 330, 336; 4096^3 3966, 3969).
+using RealTma = DmmaTmaCfg<false, 128, 64, 16, 4, 4, 8>;
 // (44 bytes of registers spilled at 128 a thread, 16 in the four-product form, 20 with 16-deep iterations.)
 // 32-deep k-iterations, three stages: half the barrier hand-offs of 16-deep ones with six (chi = 512 chain,
 // per product: 68.0 -> 66.6 us).  The real kernel gains 1 % at 4000^3 and loses 6 % at K = 300 by it.
@@ -599,12 +601,20 @@ tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined,
         *declined = true;
         return TFB_OK;
     }
+    // Groups of one mode need no offset tables in the TMA-fed kernel; the gather kernel always reads them.
     std::shared_ptr<ContractTables> t;
-    TFB_TRY(get_tables(ctx, p, &t));
+    if (p.m.size() > 1 || p.n.size() > 1 || p.batch.size() > 1) TFB_TRY(get_tables(ctx, p, &t));
     ContractArgs a;
-    fill_args(p, *t, &a);
+    fill_args(p, t.get(), &a);
     const int shape = env_int("TFB_DMMA_TILE", 0);  // 0 auto, 1 small, 2 big
     const bool use_tma = !env_int("TFB_NO_DMMA_TMA", 0);
+    auto gather = [&](auto run) -> tfb_status {
+        if (!t) {
+            TFB_TRY(get_tables(ctx, p, &t));
+            fill_args(p, t.get(), &a);
+        }
+        return run(ctx, p, a);
+    };
     auto on_copies = [&](bool small, bool* d) -> tfb_status {
         PoolBlock blk_a, blk_b;
         ContractProblem q;
@@ -621,7 +631,7 @@ tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined,
         bool small_gather = (a.M <= 64 || a.N <= 64 || a.M * a.N * a.B < (int64_t)128 * 128 * ctx->sm_count / 2);
         if (shape == 1) small = small_gather = true;
         if (shape == 2) small = small_gather = false;
-        if (shape == 3) return run_cfg<RealBig8>(ctx, p, a);
+        if (shape == 3) return gather(run_cfg<RealBig8>);
         if (use_tma) {
             bool d = true;
             TFB_TRY(run_tma(ctx, p, a, small, false, &d));
@@ -629,7 +639,7 @@ tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined,
             TFB_TRY(on_copies(small, &d));
             if (!d) return TFB_OK;
         }
-        return small_gather ? run_cfg<RealSmall>(ctx, p, a) : run_cfg<RealBig>(ctx, p, a);
+        return small_gather ? gather(run_cfg<RealSmall>) : gather(run_cfg<RealBig>);
     }
     // 32 x 32 tiles below an eighth of the SMs' worth of 64 x 64 ones (eight launches of a chain, chi = 64: 80
     // against 124 us, 97: 91 against 159, 192: 128 against 157, 338: 368 against 278).
@@ -667,7 +677,7 @@ tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined,
         TFB_TRY(on_copies(small, &d));
         if (!d) return TFB_OK;
     }
-    return small_gather ? run_cfg<CplxSmall>(ctx, p, a) : run_cfg<CplxMain>(ctx, p, a);
+    return small_gather ? gather(run_cfg<CplxSmall>) : gather(run_cfg<CplxMain>);
 }
 
 }  // namespace tfb

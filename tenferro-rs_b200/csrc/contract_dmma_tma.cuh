@@ -49,7 +49,8 @@ struct DmmaTmaCfg {
     static constexpr int G = kLines ? 8 : CPLX ? 2 : 4;  // rows per run of an MN-major tile
     static constexpr int A_BYTES = BM * BK * ES, B_BYTES = BN * BK * ES;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 16 * STAGES + 1024;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 16 * STAGES + 16 + 1024;
+    static_assert(BM * BN * ES <= STAGES * STAGE_BYTES, "a tile's sums fit the ring");
 };
 
 // Element offset of (row, k) inside a dense tile.
@@ -76,9 +77,15 @@ struct LineReader {
     }
 };
 
+__device__ __forceinline__ double flip_sign(double x, unsigned mask) {
+    return __hiloint2double((int)((unsigned)__double2hiint(x) ^ mask), __double2loint(x));
+}
+
 template <typename Cfg, bool A_MN, bool B_MN>
 __device__ __forceinline__ void dmma_tma_consume(const char* sa, const char* sb, double (&acc)[Cfg::TM][Cfg::TN][Cfg::ACC],
                                                  int wm0, int wn0, int lr, int lc, bool conj_a, bool conj_b) {
+    [[maybe_unused]] const double sign_a = conj_a ? -1.0 : 1.0, sign_b = conj_b ? -1.0 : 1.0;
+    [[maybe_unused]] const unsigned flip_a = conj_a ? 0x80000000u : 0u, flip_b = conj_b ? 0x80000000u : 0u;
     constexpr bool CPLX = Cfg::kCplx;
     constexpr int TM = Cfg::TM, TN = Cfg::TN;
 #pragma unroll
@@ -94,7 +101,7 @@ __device__ __forceinline__ void dmma_tma_consume(const char* sa, const char* sb,
                 for (int q = 0; q < 2; ++q) {
                     const double2 v = ra.get(i, kk, q);
                     ar[i][q] = v.x;
-                    ai[i][q] = conj_a ? -v.y : v.y;
+                    ai[i][q] = flip_sign(v.y, flip_a);
                 }
 #pragma unroll
             for (int j = 0; j < TN; ++j)
@@ -102,8 +109,8 @@ __device__ __forceinline__ void dmma_tma_consume(const char* sa, const char* sb,
                 for (int q = 0; q < 2; ++q) {
                     const double2 v = rb.get(j, kk, q);
                     br[j][q] = v.x;
-                    bi[j][q] = conj_b ? -v.y : v.y;
-                    nbi[j][q] = -bi[j][q];
+                    bi[j][q] = flip_sign(v.y, flip_b);
+                    nbi[j][q] = flip_sign(v.y, flip_b ^ 0x80000000u);
                 }
             auto pass = [&](const double (&x)[TM][2], const double (&y)[TN][2], int at) {
 #pragma unroll
@@ -120,9 +127,10 @@ __device__ __forceinline__ void dmma_tma_consume(const char* sa, const char* sb,
         } else if constexpr (CPLX) {
             // Three real products per complex one instead of four:
             //   P1 = Ar Br,  P2 = Ai Bi,  P3 = (Ar + Ai)(Br + Bi);  Re = P1 - P2,  Im = P3 - P1 - P2.
-            // The sums cost two adds per fragment element; the FP64 pipe, which is what this
+            // The sums cost two FMAs per fragment element; the FP64 pipe, which is what this
             // kernel waits for, issues a quarter fewer MMAs.  acc[..][0..1] = P1, [2..3] = P2,
-            // [4..5] = P3; the caller folds them into Re / Im when a k range ends.
+            // [4..5] = P3; the caller folds them into Re / Im when a k range ends.  Conjugation is a sign in the sums
+            // and, for P2, the caller's: everything but MMAs in this loop is time that the pipe stands still.
             double ar[TM][2], ai[TM][2], as[TM][2], br[TN][2], bi[TN][2], bs[TN][2];
 #pragma unroll
             for (int i = 0; i < TM; ++i)
@@ -131,8 +139,8 @@ __device__ __forceinline__ void dmma_tma_consume(const char* sa, const char* sb,
                     const double2 v = *reinterpret_cast<const double2*>(
                         sa + (size_t)tile_off<Cfg, Cfg::BM, A_MN>(wm0 + 8 * i + lr, kk + 4 * q + lc) * 16);
                     ar[i][q] = v.x;
-                    ai[i][q] = conj_a ? -v.y : v.y;
-                    as[i][q] = ar[i][q] + ai[i][q];
+                    ai[i][q] = v.y;
+                    as[i][q] = fma(sign_a, v.y, v.x);
                 }
 #pragma unroll
             for (int j = 0; j < TN; ++j)
@@ -141,8 +149,8 @@ __device__ __forceinline__ void dmma_tma_consume(const char* sa, const char* sb,
                     const double2 v = *reinterpret_cast<const double2*>(
                         sb + (size_t)tile_off<Cfg, Cfg::BN, B_MN>(wn0 + 8 * j + lr, kk + 4 * q + lc) * 16);
                     br[j][q] = v.x;
-                    bi[j][q] = conj_b ? -v.y : v.y;
-                    bs[j][q] = br[j][q] + bi[j][q];
+                    bi[j][q] = v.y;
+                    bs[j][q] = fma(sign_b, v.y, v.x);
                 }
 #pragma unroll
             for (int i = 0; i < TM; i += 2)
@@ -186,6 +194,63 @@ __device__ __forceinline__ void dmma_tma_consume(const char* sa, const char* sb,
     }
 }
 
+// Element `t` (a thread of the main kernel) of fragment f = (i, j, e) of the tile at (m0, n0), finished and stored.
+template <typename Cfg>
+__device__ __forceinline__ void dmma_tma_store_one(const ContractArgs& g, int64_t bb, int64_t m0, int64_t n0, int f, int t, double xr,
+                                                   double xi) {
+    constexpr bool CPLX = Cfg::kCplx;
+    const int i = f / (2 * Cfg::TN), j = (f >> 1) % Cfg::TN, e = f & 1, lane = t & 31, warp = t >> 5;
+    const int64_t m = m0 + (warp % Cfg::WARPS_M) * Cfg::WM + 8 * i + (lane >> 2);
+    const int64_t n = n0 + (warp / Cfg::WARPS_M) * Cfg::WN + 8 * j + 2 * (lane & 3) + e;
+    if (m >= g.M || n >= g.N) return;
+    if (g.mul) {
+        const int64_t off = g.off_d_b(bb) + g.off_d_m(m) + g.off_d_n(n);
+        if (CPLX) apply_mul_c128(g, off, xr, xi);
+        else apply_mul_f64(g, off, xr);
+    }
+    dmma_store<CPLX>(g, g.c + (g.off_c_b(bb) + g.off_c_m(m) + g.off_c_n(n)) * (int64_t)Cfg::ES, g.beta_re != 0.0 || g.beta_im != 0.0, xr,
+                     xi);
+}
+
+// Scratch slot of CTA `c` for a range that starts inside its tile (kind 0) or starts its tile (kind 1).
+template <typename Cfg>
+__device__ __forceinline__ char* dmma_tma_slot(const ContractArgs& g, int kind, int64_t c) {
+    return g.partial + (size_t)(kind * (int64_t)gridDim.x + c) * (Cfg::BM * Cfg::BN) * Cfg::ES;
+}
+template <typename Cfg>
+__device__ __forceinline__ void dmma_tma_park(char* P, const double (&acc)[Cfg::TM][Cfg::TN][Cfg::ACC], int tid) {
+#pragma unroll
+    for (int i = 0; i < Cfg::TM; ++i)
+#pragma unroll
+        for (int j = 0; j < Cfg::TN; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                char* q = P + ((size_t)((i * Cfg::TN + j) * 2 + e) * Cfg::NT + tid) * Cfg::ES;
+                if constexpr (Cfg::kCplx) *reinterpret_cast<double2*>(q) = make_double2(acc[i][j][e], acc[i][j][2 + e]);
+                else *reinterpret_cast<double*>(q) = acc[i][j][e];
+            }
+}
+// A slot added to acc (ADD), or in its place.
+template <typename Cfg, bool ADD>
+__device__ __forceinline__ void dmma_tma_gather(const char* P, double (&acc)[Cfg::TM][Cfg::TN][Cfg::ACC], int tid) {
+#pragma unroll
+    for (int i = 0; i < Cfg::TM; ++i)
+#pragma unroll
+        for (int j = 0; j < Cfg::TN; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const char* q = P + ((size_t)((i * Cfg::TN + j) * 2 + e) * Cfg::NT + tid) * Cfg::ES;
+                if constexpr (Cfg::kCplx) {
+                    const double2 v = __ldcg(reinterpret_cast<const double2*>(q));
+                    acc[i][j][e] = ADD ? acc[i][j][e] + v.x : v.x;
+                    acc[i][j][2 + e] = ADD ? acc[i][j][2 + e] + v.y : v.y;
+                } else {
+                    const double v = __ldcg(reinterpret_cast<const double*>(q));
+                    acc[i][j][e] = ADD ? acc[i][j][e] + v : v;
+                }
+            }
+}
+
 template <typename Cfg>
 __global__ void __launch_bounds__(Cfg::NT, 1)
 contract_dmma_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -199,6 +264,7 @@ contract_dmma_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const uint32_t bars = ring + STAGES * Cfg::STAGE_BYTES;
     auto bar_full = [&](int s) { return bars + 8u * s; };
     auto bar_empty = [&](int s) { return bars + 8u * (STAGES + s); };
+    const uint32_t verdict = bars + 16u * STAGES;  // one word: who finishes a cut tile
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     if (tid == 0) {
@@ -213,9 +279,17 @@ contract_dmma_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
     }
     __syncthreads();
+    launch_begin();  // nothing above touches global memory
 
-    const int64_t it_begin = (int64_t)blockIdx.x * g.iters_per_cta;
-    const int64_t it_end = min(g.total_iters, it_begin + g.iters_per_cta);
+    int64_t it_begin = (int64_t)blockIdx.x * g.iters_per_cta;
+    int64_t it_end = min(g.total_iters, it_begin + g.iters_per_cta);
+    const int pieces = g.cluster, piece = pieces > 1 ? (int)(blockIdx.x % (unsigned)pieces) : 0;
+    if (pieces > 1) {
+        // the CTAs of a cluster share a tile's k-iterations evenly
+        const int64_t tile_first = (int64_t)(blockIdx.x / (unsigned)pieces) * g.k_iters;
+        it_begin = tile_first + g.k_iters * piece / pieces;
+        it_end = tile_first + g.k_iters * (piece + 1) / pieces;
+    }
     const bool a_mn = !g.a_kfast, b_mn = !g.b_kfast;
 
     // ---------------------------------------------------------------- loads
@@ -300,106 +374,112 @@ contract_dmma_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 for (int j = 0; j < TN; ++j)
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        const double p1 = acc[i][j][e], p2 = acc[i][j][2 + e], p3 = acc[i][j][4 + e];
+                        const double p1 = acc[i][j][e], p2 = conj_a != conj_b ? -acc[i][j][2 + e] : acc[i][j][2 + e], p3 = acc[i][j][4 + e];
                         acc[i][j][e] = p1 - p2;
                         acc[i][j][2 + e] = p3 - p1 - p2;
                     }
         }
-        // A range that starts inside a tile (kb > 0) only contributes: it parks its
-        // accumulators in this CTA's scratch slot and raises the CTA's flag.  The range that
-        // holds the tile's first k-iteration owns the tile: it collects the contributions of
-        // the CTAs after it, in CTA order, and writes C.  Contributions are the first thing a
-        // CTA does and collecting is the last, so owners rarely wait; the wait is bounded.
-        if (kb > 0 || g.sk_two_phase) {
-            char* P = g.partial + (size_t)blockIdx.x * (BM * BN) * ES;
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        char* q = P + ((size_t)((i * TN + j) * 2 + e) * Cfg::NT + tid) * ES;
-                        if (CPLX)
-                            *reinterpret_cast<double2*>(q) = make_double2(acc[i][j][e], acc[i][j][2 + e]);
-                        else
-                            *reinterpret_cast<double*>(q) = acc[i][j][e];
+        if (pieces > 1) {
+            // The tile's sums meet in the CTAs' shared memory: each parks its own (the ring is empty: every load
+            // that this CTA issued has been consumed), and adds a share of the tile over all of them, in the order
+            // of k.
+            __syncthreads();
+            dmma_tma_park<Cfg>(smem, acc, tid);
+            cluster_sync_all();
+            constexpr int TOTAL = BM * BN;
+            const int share = (TOTAL + pieces - 1) / pieces, at1 = min(TOTAL, (piece + 1) * share);
+            for (int at = piece * share + tid; at < at1; at += Cfg::NT) {
+                double xr = 0.0, xi = 0.0;
+                const uint32_t mine = ring + (uint32_t)at * ES;
+#pragma unroll 8
+                for (int c = 0; c < pieces; ++c) {
+                    const uint32_t q = map_to_cta(mine, (uint32_t)c);
+                    if constexpr (CPLX) {
+                        const double2 v = cluster_load_d2(q);
+                        xr += v.x;
+                        xi += v.y;
+                    } else {
+                        xr += cluster_load_d(q);
                     }
-            if (!g.sk_two_phase) {
+                }
+                dmma_tma_store_one<Cfg>(g, bb, m0, n0, at / Cfg::NT, at % Cfg::NT, xr, xi);
+            }
+            __syncwarp();
+            cluster_sync_all();  // no CTA leaves while another reads its sums
+            break;
+        }
+        // A range that cuts a tile without a cluster: every CTA but one parks its sums in a scratch slot and counts
+        // itself in; whoever comes last adds the slots in the order of k and writes C.  No CTA waits for another, so
+        // nothing depends on which of them run at the same time.  Contributions (kb > 0) are the first thing a
+        // CTA does and a tile's first range the last, so the range that starts the tile mostly finds the others
+        // there and keeps its own sums in registers.
+        bool finish = true;
+        if (g.sk_two_phase) {
+            dmma_tma_park<Cfg>(dmma_tma_slot<Cfg>(g, 0, blockIdx.x), acc, tid);
+            finish = false;
+        } else if (kb > 0 || ke < g.k_iters) {
+            const int64_t first = tile * g.k_iters / g.iters_per_cta, last = ((tile + 1) * g.k_iters - 1) / g.iters_per_cta;
+            const unsigned others = (unsigned)(last - first);
+            unsigned* arrived = g.sk_arrived + first;
+            auto told = [&]() -> bool {  // what thread 0 has put into the word
+                __syncthreads();
+                uint32_t v;
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(verdict) : "memory");
+                return v != 0;
+            };
+            auto count_in = [&]() -> bool {
                 __threadfence();
                 __syncthreads();
-                if (tid == 0)
-                    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(g.sk_flags + blockIdx.x), "r"(g.sk_epoch) : "memory");
-            }
-        } else {
-            if (ke < g.k_iters) {
-                const int64_t g_last = ((tile + 1) * g.k_iters - 1) / g.iters_per_cta;
-                // All contributors' flags first (thread c - first polls flag c, bounded), then one
-                // pass over their slots in CTA order: the loads of different slots overlap, the
-                // additions keep their order, so the sum does not depend on timing.
-                {
-                    const int64_t c = (int64_t)blockIdx.x + 1 + tid;
-                    if (c <= g_last) {
-                        uint32_t v = 0;
-                        for (uint32_t spin = 0; spin < (1u << 20); ++spin) {
-                            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(g.sk_flags + c) : "memory");
-                            if (v == g.sk_epoch) break;
-                            __nanosleep(64);
-                        }
-                        if (v != g.sk_epoch) atomicCAS(status, 0, 0x303);
-                    }
-                    __syncthreads();
+                if (tid == 0) {
+                    unsigned before;
+                    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(arrived) : "memory");
+                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(verdict), "r"((uint32_t)(before == others)) : "memory");
                 }
-#pragma unroll 4
-                for (int64_t c = (int64_t)blockIdx.x + 1; c <= g_last; ++c) {
-                    const char* P = g.partial + (size_t)c * (BM * BN) * ES;
-#pragma unroll
-                    for (int i = 0; i < TM; ++i)
-#pragma unroll
-                        for (int j = 0; j < TN; ++j)
-#pragma unroll
-                            for (int e = 0; e < 2; ++e) {
-                                const char* q = P + ((size_t)((i * TN + j) * 2 + e) * Cfg::NT + tid) * ES;
-                                if (CPLX) {
-                                    const double2 v = __ldcg(reinterpret_cast<const double2*>(q));
-                                    acc[i][j][e] += v.x;
-                                    acc[i][j][2 + e] += v.y;
-                                } else {
-                                    acc[i][j][e] += __ldcg(reinterpret_cast<const double*>(q));
-                                }
-                            }
+                return told();
+            };
+            if (kb > 0) {
+                dmma_tma_park<Cfg>(dmma_tma_slot<Cfg>(g, 0, blockIdx.x), acc, tid);
+                finish = count_in();
+                if (finish) {
+                    __threadfence();
+                    dmma_tma_gather<Cfg, false>(dmma_tma_slot<Cfg>(g, 1, first), acc, tid);
                 }
+            } else {
+                __syncthreads();  // (the word may still be being read for the tile before)
+                if (tid == 0) {
+                    unsigned now;
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(arrived) : "memory");
+                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(verdict), "r"((uint32_t)(now == others)) : "memory");
+                }
+                if (!told()) {
+                    dmma_tma_park<Cfg>(dmma_tma_slot<Cfg>(g, 1, blockIdx.x), acc, tid);
+                    finish = count_in();
+                }
+                __threadfence();
             }
-            if (g.mul) apply_mul_fragments<CPLX>(g, bb, m0 + wm0 + lr, n0 + wn0 + 2 * lc, acc);
-            char* Cb = g.c + g.c_b[bb] * (int64_t)ES;
+            if (finish) {
+                if (tid == 0) *arrived = 0;  // every range of the tile is in: the next launch counts from zero
+#pragma unroll 2
+                for (int64_t c = first + 1; c <= last; ++c) dmma_tma_gather<Cfg, true>(dmma_tma_slot<Cfg>(g, 0, c), acc, tid);
+            }
+        }
+        if (finish) {
+            const int64_t row0 = m0 + wm0 + lr, col0 = n0 + wn0 + 2 * lc;
+            if (g.mul) apply_mul_fragments<CPLX>(g, bb, row0, col0, acc);
+            char* Cb = g.c + g.off_c_b(bb) * (int64_t)ES;
             const bool read_c = g.beta_re != 0.0 || g.beta_im != 0.0;
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const int64_t nn = n0 + wn0 + 8 * j + 2 * lc + e;
+                    const int64_t nn = col0 + 8 * j + e;
                     if (nn >= g.N) continue;
-                    const int64_t cn = g.c_n[nn];
+                    const int64_t cn = g.off_c_n(nn);
 #pragma unroll
                     for (int i = 0; i < TM; ++i) {
-                        const int64_t m = m0 + wm0 + 8 * i + lr;
+                        const int64_t m = row0 + 8 * i;
                         if (m >= g.M) continue;
-                        char* p = Cb + (g.c_m[m] + cn) * (int64_t)ES;
-                        if (CPLX) {
-                            const double xr = acc[i][j][e], xi = acc[i][j][2 + e];
-                            double2 o;
-                            o.x = g.alpha_re * xr - g.alpha_im * xi;
-                            o.y = g.alpha_re * xi + g.alpha_im * xr;
-                            if (read_c) {
-                                const double2 old = *reinterpret_cast<const double2*>(p);
-                                o.x += g.beta_re * old.x - g.beta_im * old.y;
-                                o.y += g.beta_re * old.y + g.beta_im * old.x;
-                            }
-                            *reinterpret_cast<double2*>(p) = o;
-                        } else {
-                            double o = g.alpha_re * acc[i][j][e];
-                            if (read_c) o += g.beta_re * *reinterpret_cast<const double*>(p);
-                            *reinterpret_cast<double*>(p) = o;
-                        }
+                        dmma_store<CPLX>(g, Cb + (g.off_c_m(m) + cn) * (int64_t)ES, read_c, acc[i][j][e], acc[i][j][CPLX ? 2 + e : e]);
                     }
                 }
             }
@@ -417,13 +497,11 @@ contract_dmma_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 template <typename Cfg>
 __global__ void __launch_bounds__(Cfg::NT) dmma_tma_splitk_finish_kernel(ContractArgs g, int pieces) {
     constexpr bool CPLX = Cfg::kCplx;
-    constexpr int BM = Cfg::BM, BN = Cfg::BN, TN = Cfg::TN, ES = Cfg::ES;
+    constexpr int BM = Cfg::BM, BN = Cfg::BN, ES = Cfg::ES;
+    launch_begin();
     const int64_t tile = blockIdx.x;
-    const int f = blockIdx.y, i = f / (2 * TN), j = (f >> 1) % TN, e = f & 1;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int f = blockIdx.y, tid = threadIdx.x;
     const int64_t tm = tile % g.tiles_m, rest = tile / g.tiles_m, tn = rest % g.tiles_n, bb = rest / g.tiles_n;
-    const int64_t m = tm * BM + (warp % Cfg::WARPS_M) * Cfg::WM + 8 * i + (lane >> 2);
-    const int64_t n = tn * BN + (warp / Cfg::WARPS_M) * Cfg::WN + 8 * j + 2 * (lane & 3) + e;
     const char* P = g.partial + ((size_t)tile * pieces * (BM * BN) + (size_t)f * Cfg::NT + tid) * ES;
     double xr = 0.0, xi = 0.0;
 #pragma unroll 8
@@ -437,29 +515,7 @@ __global__ void __launch_bounds__(Cfg::NT) dmma_tma_splitk_finish_kernel(Contrac
             xr += __ldcg(reinterpret_cast<const double*>(q));
         }
     }
-    if (m >= g.M || n >= g.N) return;
-    if (g.mul) {
-        const int64_t off = g.d_b[bb] + g.d_m[m] + g.d_n[n];
-        if (CPLX) apply_mul_c128(g, off, xr, xi);
-        else apply_mul_f64(g, off, xr);
-    }
-    char* p = g.c + (g.c_b[bb] + g.c_m[m] + g.c_n[n]) * (int64_t)ES;
-    const bool read_c = g.beta_re != 0.0 || g.beta_im != 0.0;
-    if (CPLX) {
-        double2 o;
-        o.x = g.alpha_re * xr - g.alpha_im * xi;
-        o.y = g.alpha_re * xi + g.alpha_im * xr;
-        if (read_c) {
-            const double2 old = *reinterpret_cast<const double2*>(p);
-            o.x += g.beta_re * old.x - g.beta_im * old.y;
-            o.y += g.beta_re * old.y + g.beta_im * old.x;
-        }
-        *reinterpret_cast<double2*>(p) = o;
-    } else {
-        double o = g.alpha_re * xr;
-        if (read_c) o += g.beta_re * *reinterpret_cast<const double*>(p);
-        *reinterpret_cast<double*>(p) = o;
-    }
+    dmma_tma_store_one<Cfg>(g, bb, tm * BM, tn * BN, f, tid, xr, xi);
 }
 
 // ------------------------------------------------------------------ host side
@@ -495,6 +551,42 @@ static bool make_f64_map(const ContractProblem& p, const std::vector<Mode>& fr, 
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// CTAs of a cluster that share a tile's K, 0 for none: where all those clusters run at once, which what a
+// CTA takes of an SM decides (`fit`, by size: with 200 KB of shared memory 74 of two, 33 of four, 15 of eight), and no CTA
+// has more k-iterations than one of the ranges below would, or one more of the short iterations of the small tiles (half a
+// microsecond).  The sums then meet in shared memory, half a microsecond to two earlier than through scratch and counters
+// (us by cluster, by ranges: double, 56 tiles of 32 x 32 and K = 256 in two 9.8, 11.4, 18 and K = 1024 in eight 9.6, 11.6; complex,
+// 97 x 194 x 97 9.5, 10.7, 64 x 128 x 64 8.0, 9.8; in two turns, 36 tiles in four, 23.2, 13.8; 512 x 512 x 1024, 16 iterations
+// of 64 x 64 tiles against 14, 70.2, 67.5).
+template <typename Cfg>
+static int cluster_pieces(const ContractArgs& a, int64_t slots, const int (&fit)[3]) {
+    if (!env_int("TFB_DMMA_CLUSTER", 1)) return 0;
+    const int64_t ranges = std::min<int64_t>(slots, std::max<int64_t>(1, a.total_iters / 2));
+    const int64_t most = (a.total_iters + ranges - 1) / ranges + (Cfg::BM * Cfg::BN * Cfg::BK * (Cfg::kCplx ? 3 : 1) <= 65536);
+    for (int i = 2; i >= 0; --i) {
+        const int s = 2 << i;
+        if (a.k_iters >= s && a.n_tiles <= fit[i] && a.n_tiles * s <= slots && (a.k_iters + s - 1) / s <= most) return s;
+    }
+    return 0;
+}
+template <typename Cfg>
+static tfb_status clusters_that_fit(int (&fit)[3]) {
+    for (int i = 0; i < 3; ++i) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 2u << i;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(2u << i);
+        cfg.blockDim = dim3(Cfg::NT);
+        cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        TFB_CUDA(cudaOccupancyMaxActiveClusters(&fit[i], contract_dmma_tma_kernel<Cfg>, &cfg));
+    }
+    return TFB_OK;
+}
+
 // Runs the TMA-fed kernel when both operands qualify; otherwise *declined = true.
 template <typename Cfg>
 static tfb_status run_tma_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractArgs a, bool* declined) {
@@ -510,14 +602,19 @@ static tfb_status run_tma_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractAr
     a.a_runs = a_runs;
     a.b_runs = b_runs;
     static std::mutex mu;
-    static std::map<int, bool> configured;
+    struct Fit { int clusters[3]; };
+    static std::map<int, Fit> configured;
+    Fit fit;
     {
         std::lock_guard<std::mutex> lock(mu);
-        if (!configured[ctx->device]) {
+        auto it = configured.find(ctx->device);
+        if (it == configured.end()) {
             TFB_CUDA(cudaFuncSetAttribute(contract_dmma_tma_kernel<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           Cfg::SMEM_BYTES));
-            configured[ctx->device] = true;
+            TFB_TRY(clusters_that_fit<Cfg>(fit.clusters));
+            it = configured.emplace(ctx->device, fit).first;
         }
+        fit = it->second;
     }
     a.tiles_m = (a.M + Cfg::BM - 1) / Cfg::BM;
     a.tiles_n = (a.N + Cfg::BN - 1) / Cfg::BN;
@@ -526,56 +623,56 @@ static tfb_status run_tma_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractAr
     a.total_iters = a.n_tiles * a.k_iters;
     if (a.total_iters >= ((int64_t)1 << 31)) return TFB_OK;  // the producer indexes k-iterations with 32 bits
     const int64_t slots = ctx->sm_count;  // one CTA per SM
-    int64_t grid;
-    // A handful of tiles with a long K: cut every tile into the same number of k pieces, one CTA
-    // each, and add the pieces in a second, tiny launch.  (In the single-launch form below the
-    // owner of a tile reads all its pieces itself - eight dependent round trips to L2 for 32
-    // pieces - and 'abc,bcd->ad' at 64^4 took 16.4 us; here every load of the sum is independent.)
+    int64_t grid = 0;
     int pieces = 0;
-    if (a.n_tiles * 4 <= slots && a.k_iters * Cfg::BK >= 256 && env_int("TFB_SK_TWO_PHASE", 1)) {
+    a.cluster = cluster_pieces<Cfg>(a, slots, fit.clusters);
+    if (a.cluster > 1) grid = a.n_tiles * a.cluster;
+    // A handful of tiles with a long K: cut every tile into the same number of k pieces, one CTA
+    // each, and add the pieces in a second, tiny launch.  (In one launch the
+    // last range of a tile adds all its pieces - eight dependent round trips to L2 for 32
+    // pieces - and 'abc,bcd->ad' at 64^4 took 16.4 us; here every load of the sum is independent.)
+    if (!grid && a.n_tiles * 4 <= slots && a.k_iters * Cfg::BK >= 256 && env_int("TFB_SK_TWO_PHASE", 1)) {
         const int64_t want = std::min<int64_t>(std::min<int64_t>(32, slots / a.n_tiles), a.k_iters * Cfg::BK / 64);
         a.iters_per_cta = (a.k_iters + want - 1) / want;
         pieces = (int)((a.k_iters + a.iters_per_cta - 1) / a.iters_per_cta);
         // 32-deep iterations do not deal out as evenly: where fewer pieces than would fit leave a quarter of the SMs idle, the
         // equal ranges below are ahead (344 x 312 x 280 complex double in 90 pieces of three iterations: 23.8 us, 19.9)
         if (Cfg::BK > 16 && pieces < want && a.n_tiles * pieces * 4 < slots * 3) pieces = 0;
-    }
-    if (pieces > 1) {
-        // ranges are per tile: CTA c takes piece c % pieces of tile c / pieces
-        if (a.iters_per_cta * pieces != a.k_iters) {
-            // the kernel cuts the linear (tile, k) space into equal ranges: pieces must divide K's iterations
-            pieces = 0;
+        // ranges are per tile: CTA c takes piece c % pieces of tile c / pieces; the kernel cuts the linear (tile, k)
+        // space into equal ranges, so pieces must divide K's iterations
+        if (a.iters_per_cta * pieces != a.k_iters || pieces < 2) pieces = 0;
+        if (pieces) {
+            grid = a.n_tiles * pieces;
+            a.sk_two_phase = 1;
         }
     }
-    if (pieces > 1) {
-        grid = a.n_tiles * pieces;
-        a.sk_two_phase = 1;
-    } else if (a.n_tiles % slots == 0 || a.n_tiles >= 16 * slots) {
-        grid = std::min(a.n_tiles, slots);
-        a.iters_per_cta = ((a.n_tiles + grid - 1) / grid) * a.k_iters;
-    } else {
-        // At least two k-iterations per CTA (eight launches of a chain, chi = 64: 98 -> 84 us against
-        // at least four).
-        grid = std::min<int64_t>(slots, std::max<int64_t>(1, a.total_iters / 2));
-        a.iters_per_cta = (a.total_iters + grid - 1) / grid;
-        // One thread of the owner polls each contributor's flag and every contribution costs the
-        // owner one pass over a slot: keep a tile in at most 32 pieces.
-        a.iters_per_cta = std::max<int64_t>(a.iters_per_cta, (a.k_iters + 31) / 32);
+    if (!grid) {
+        if (a.n_tiles % slots == 0 || a.n_tiles >= 16 * slots) {
+            grid = std::min(a.n_tiles, slots);
+            a.iters_per_cta = ((a.n_tiles + grid - 1) / grid) * a.k_iters;
+        } else {
+            // At least two k-iterations per CTA (eight launches of a chain, chi = 64: 98 -> 84 us against
+            // at least four).
+            grid = std::min<int64_t>(slots, std::max<int64_t>(1, a.total_iters / 2));
+            a.iters_per_cta = (a.total_iters + grid - 1) / grid;
+            // Whoever finishes a tile passes over a slot per range of it: keep a tile in at most 32.
+            a.iters_per_cta = std::max<int64_t>(a.iters_per_cta, (a.k_iters + 31) / 32);
+        }
+        grid = (a.total_iters + a.iters_per_cta - 1) / a.iters_per_cta;
     }
-    if (!a.sk_two_phase) grid = (a.total_iters + a.iters_per_cta - 1) / a.iters_per_cta;
-    const bool cuts = a.iters_per_cta % a.k_iters != 0;
-    if (cuts) {
-        // Scratch slots and flags live with the context (one slot per CTA, reused by every
-        // launch; a flag is "raised" when it equals the launch's epoch, so nothing is reset).
-        // As large as any configuration asks for from the start (19 MB): a captured launch keeps the address.  Where the
+    if (a.cluster <= 1 && a.iters_per_cta % a.k_iters != 0) {
+        // Scratch slots and counters live with the context and are reused by every launch (a counter is back at zero
+        // when its tile is finished, so a replayed launch finds what a direct one does).
+        // As large as any configuration asks for from the start (38 MB): a captured launch keeps the address.  Where the
         // device has no room for that, what this launch uses.
         static_assert((size_t)Base::TILE_ELEMS * Base::ES <= 128 * 128 * 8, "largest block tile");
-        const size_t need = (size_t)grid * Base::TILE_ELEMS * Base::ES;
+        if ((size_t)grid > tfb_ctx::kArrived) return fail(TFB_ERR_DEVICE, "a device of more than %zu SMs", tfb_ctx::kArrived);
+        const size_t need = (a.sk_two_phase ? 1 : 2) * (size_t)grid * Base::TILE_ELEMS * Base::ES;
         if (ctx->sk_partial_bytes < need) {
             if (ctx->sk_partial) TFB_CUDA(cudaFree(ctx->sk_partial));
             ctx->sk_partial = nullptr;
             ctx->sk_partial_bytes = 0;
-            size_t take = std::max<size_t>((size_t)grid, (size_t)slots) * 128 * 128 * 8;
+            size_t take = 2 * std::max<size_t>((size_t)grid, (size_t)slots) * 128 * 128 * 8;
             if (cudaMalloc(&ctx->sk_partial, take) != cudaSuccess) {
                 cudaGetLastError();
                 take = need;
@@ -583,44 +680,19 @@ static tfb_status run_tma_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractAr
             }
             ctx->sk_partial_bytes = take;
         }
-        if (ctx->sk_flags_n < (size_t)grid) {
-            if (ctx->sk_flags) TFB_CUDA(cudaFree(ctx->sk_flags));
-            ctx->sk_flags = nullptr;
-            ctx->sk_flags_n = 0;
-            const size_t n = std::max<size_t>((size_t)grid, 1024);
-            TFB_CUDA(cudaMalloc(&ctx->sk_flags, n * sizeof(unsigned)));
-            TFB_CUDA(cudaMemset(ctx->sk_flags, 0, n * sizeof(unsigned)));
-            ctx->sk_flags_n = n;
-        }
         a.partial = (char*)ctx->sk_partial;
-        a.sk_flags = ctx->sk_flags;
-        if (ctx->capturing) {
-            // A replayed launch would meet the flags its last run raised: a captured launch clears
-            // them first and uses an epoch no live launch has.
-            TFB_CUDA(cudaMemsetAsync(ctx->sk_flags, 0, (size_t)grid * sizeof(unsigned), ctx->stream));
-            a.sk_epoch = 0xffffffffu;
-        } else {
-            a.sk_epoch = ++ctx->sk_epoch;
-            if (a.sk_epoch == 0xffffffffu) a.sk_epoch = ctx->sk_epoch = 1;
-        }
+        a.sk_arrived = ctx->arrived;
     }
     {
         LaunchScope ls(ctx, "contract_dmma");
         int* status = ctx->dev_status;
-        void* args[] = {(void*)&map_a, (void*)&map_b, (void*)&a, (void*)&status};
-        // Owners wait for contributors, so every CTA of the grid has to be resident: a
-        // cooperative launch makes the runtime check that (grid <= one CTA per SM).
-        if (cuts && !a.sk_two_phase && env_int("TFB_SK_COOP", 1))
-            TFB_CUDA(cudaLaunchCooperativeKernel((const void*)contract_dmma_tma_kernel<Cfg>, dim3((unsigned)grid),
-                                                 dim3(Cfg::NT), args, Cfg::SMEM_BYTES, ctx->stream));
-        else
-            contract_dmma_tma_kernel<Cfg><<<(unsigned)grid, Cfg::NT, Cfg::SMEM_BYTES, ctx->stream>>>(map_a, map_b, a, status);
+        TFB_CUDA(launch_overlapped(ctx, contract_dmma_tma_kernel<Cfg>, dim3((unsigned)grid), dim3(Cfg::NT), Cfg::SMEM_BYTES,
+                                   (unsigned)a.cluster, map_a, map_b, a, status));
     }
-    TFB_CUDA(cudaGetLastError());
     if (a.sk_two_phase) {
         LaunchScope ls(ctx, "contract_dmma_finish");
-        dmma_tma_splitk_finish_kernel<Cfg><<<dim3((unsigned)a.n_tiles, Cfg::TM * Cfg::TN * 2), Cfg::NT, 0, ctx->stream>>>(a, pieces);
-        TFB_CUDA(cudaGetLastError());
+        TFB_CUDA(launch_overlapped(ctx, dmma_tma_splitk_finish_kernel<Cfg>, dim3((unsigned)a.n_tiles, Cfg::TM * Cfg::TN * 2),
+                                   dim3(Cfg::NT), 0, 0u, a, pieces));
     }
     *declined = false;
     return TFB_OK;

@@ -22,6 +22,7 @@ struct ContractTables {
 };
 
 tfb_status get_tables(tfb_ctx* ctx, const ContractProblem& p, std::shared_ptr<ContractTables>* out);
-void fill_args(const ContractProblem& p, const ContractTables& t, ContractArgs* a);
+// `t` may be null for kernels that take groups of one mode by their strides.
+void fill_args(const ContractProblem& p, const ContractTables* t, ContractArgs* a);
 
 }  // namespace tfb

@@ -1893,7 +1893,7 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
         if (pack_a || pack_b) {
             TFB_TRY(get_tables(ctx, p, &t));
             ContractArgs ca;
-            fill_args(p, *t, &ca);
+            fill_args(p, t.get(), &ca);
             const int64_t Kp = (K + 3) / 4 * 4, Bn = p.B();
             auto repack = [&](int tns, PoolBlock* blk, OperandMap* out) -> tfb_status {
                 const int64_t rows = tns == 0 ? M : N;

@@ -42,6 +42,28 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, int* st
     atomicCAS(status, 0, code);
 }
 
+// Programmatic dependent launch.  A kernel that starts before the one ahead of it in the stream has finished waits
+// here for the end of it (all its writes visible); without such a launch both are no-ops.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// First statement of a kernel for launch_overlapped that reads or writes global memory after it only.
+__device__ __forceinline__ void launch_begin() {
+    grid_dependency_wait();
+    grid_launch_dependents();
+}
+
+// Reads of another CTA's shared memory (addresses from map_to_cta).
+__device__ __forceinline__ double cluster_load_d(uint32_t addr) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ double2 cluster_load_d2(uint32_t addr) {
+    double2 v;
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2,
                                             int c3) {
     asm volatile(

@@ -156,3 +156,25 @@ def test_when_operands_are_not_copied(tb, m, n, k, copies):
 def test_complex_tiles(tb, oracle, notation, sizes, conj):
     shapes = [tuple(sizes[c] for c in t) for t in notation.split("->")[0].split(",")]
     run(tb, oracle, notation, shapes, np.complex128, conj, 0.5)
+
+
+@pytest.mark.parametrize("cluster", ["0", "1"])
+@pytest.mark.parametrize("dtype,mnk", [
+    (np.float64, (64, 64, 4096)),  # pieces that meet in shared memory, or in a second launch
+    (np.float64, (32, 36, 128)),   # one iteration per CTA
+    (np.float64, (228, 252, 260)),
+    (np.float64, (448, 452, 1028)),  # ranges that cut tiles
+    (np.complex128, (64, 128, 64)),
+    (np.complex128, (98, 196, 100)),
+    (np.complex128, (258, 322, 324)),
+])
+@pytest.mark.parametrize("conj", [False, True])
+def test_split_of_k(tb, oracle, monkeypatch, dtype, mnk, cluster, conj):
+    monkeypatch.setenv("TFB_DMMA_CLUSTER", cluster)
+    m, n, k = mnk
+    run(tb, oracle, "ij,jk->ik", [(m, k), (k, n)], dtype, conj, 0.5)
+    # the order of the sums does not depend on which block comes last
+    x, y = (tb.Tensor.from_numpy(oracle.normal(3 + t, s, dtype)) for t, s in enumerate([(m, k), (k, n)]))
+    first = tb.einsum("ij,jk->ik", [x, y]).to_numpy()
+    for _ in range(3):
+        assert np.array_equal(tb.einsum("ij,jk->ik", [x, y]).to_numpy(), first)
