@@ -448,6 +448,102 @@ tfb_status contract_simt_semiring(tfb_ctx* ctx, const ContractProblem& p, int al
     return fail(TFB_ERR_INVALID_ARGUMENT, "unknown algebra %d", algebra);
 }
 
+// ------------------------------------------------------------------ batch index innermost
+// "bij,bjk->bik" in column-major order: neighbouring elements of the output belong to different products, so a kernel that
+// writes a tile of one of them touches a 32-byte sector per element, and reads its operands the same way.  From
+// the size on that repays copies at all, the operands that lie so are copied with the batch outermost, the
+// products go to a block of their own, and one pass over that applies alpha and beta and puts the batch back innermost: all
+// of it tiled permutations at the memory's rate.  Chunks of the batch keep the copies to about 1 GB.
+// (us before and now: f32, 484 of 736 x 824 x 1044 26100, 4650, 1000 of 100^3 383, 141, 8 of 600^3 259, 92; double, 484 of 736 x
+// 824 x 1044 199000, 23900, 220 of 580 x 408 x 308 2900, 1650, 16 of 600^3 353, 348, 8 of 600^3 186, 200; complex single, 1000 of
+// 100^3 337, 294, 8 of 600^3 167, 177.  Complex double elements are half a sector, and nothing is gained: 64 of 300^3 619, 628.)
+static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& p, const char** used, bool* done) {
+    *done = false;
+    if (p.batch.size() != 1 || p.batch[0].s[2] != 1 || p.batch[0].extent < (p.dtype == TFB_F32 ? 8 : 16) || p.mul || p.dtype == TFB_C64)
+        return TFB_OK;
+    if (p.dtype == TFB_F32 && p.k.size() > 2) return TFB_OK;  // the exact kernel's: not to be moved to 3xTF32 by a copy
+    const int64_t M = p.M(), N = p.N(), K = p.K(), B = p.B(), es = (int64_t)dtype_size(p.dtype);
+    const bool wide = p.dtype == TFB_F64;
+    const double flops = (dtype_is_complex(p.dtype) ? 8.0 : 2.0) * (double)M * (double)N * (double)K * (double)B;
+    if (M < 64 || N < 64 || K < 16 || flops < (wide ? 2e8 : 1e9)) return TFB_OK;
+    auto up = [](int64_t x, int64_t to) { return (x + to - 1) / to * to; };
+    // Copies as the kernels like them best: [batch][k][rows] for the FP64 pipe, [batch][rows][k] for tcgen05.
+    const bool copy[2] = {p.batch[0].s[0] == 1, p.batch[0].s[1] == 1};
+    const int64_t rows[2] = {M, N};
+    int64_t ld[3], per[3], bytes = 0;
+    for (int t = 0; t < 2; ++t) {
+        ld[t] = wide ? up(rows[t], 8) : up(K, 4);
+        per[t] = ld[t] * (wide ? K : rows[t]);
+        if (copy[t]) bytes += per[t] * es;
+    }
+    ld[2] = up(M, 8);
+    per[2] = ld[2] * up(N, 8);
+    bytes += per[2] * es;
+    const int64_t chunk = std::min(B, std::max<int64_t>(32, ((int64_t)1 << 30) / bytes / 32 * 32));
+    if ((double)bytes * (double)chunk > (double)ctx->total_mem / 16) return TFB_OK;
+    PoolBlock blk[3];
+    for (int t = 0; t < 3; ++t)
+        if ((t == 2 || copy[t]) && blk[t].alloc(ctx, (size_t)(per[t] * chunk * es)) != TFB_OK) return TFB_OK;
+    auto pass = [&](const std::vector<Mode>& modes, const void* in, void* out, Scalar alpha, Scalar beta) -> tfb_status {
+        std::vector<Mode> sorted = modes;
+        sort_and_fuse(sorted, 1, 2);
+        LoopNest nest;
+        TFB_TRY(make_nest(sorted, &nest));
+        return launch_permute(ctx, p.dtype, nest, in, out, alpha, beta, false);
+    };
+    auto dense = [](std::vector<Mode>& g, int t, int64_t step) {
+        for (Mode& m : g) {
+            m.s[t] = step;
+            step *= m.extent;
+        }
+    };
+    for (int64_t b0 = 0; b0 < B; b0 += chunk) {
+        const int64_t n = std::min(chunk, B - b0);
+        ContractProblem q = p;
+        q.batch[0].extent = n;
+        q.a = (const char*)p.a + b0 * p.batch[0].s[0] * es;
+        q.b = (const char*)p.b + b0 * p.batch[0].s[1] * es;
+        q.c = blk[2].ptr;
+        q.alpha = Scalar{1.0, 0.0};
+        q.beta = Scalar{0.0, 0.0};
+        for (int t = 0; t < 2; ++t) {
+            if (!copy[t]) continue;
+            std::vector<Mode>& free_q = t == 0 ? q.m : q.n;
+            dense(free_q, t, wide ? 1 : ld[t]);
+            dense(q.k, t, wide ? ld[t] : 1);
+            q.batch[0].s[t] = per[t];
+            std::vector<Mode> modes;
+            auto put = [&](const std::vector<Mode>& from, const std::vector<Mode>& to) {
+                for (size_t i = 0; i < from.size(); ++i) modes.push_back(Mode{to[i].extent, {from[i].s[t], to[i].s[t], 0, 0}});
+            };
+            put(t == 0 ? p.m : p.n, free_q);
+            put(p.k, q.k);
+            put(p.batch, q.batch);
+            TFB_TRY(pass(modes, t == 0 ? q.a : q.b, blk[t].ptr, Scalar{1.0, 0.0}, Scalar{0.0, 0.0}));
+            (t == 0 ? q.a : q.b) = blk[t].ptr;
+        }
+        dense(q.m, 2, 1);
+        dense(q.n, 2, ld[2]);
+        q.batch[0].s[2] = per[2];
+        std::vector<Mode> back;
+        auto put = [&](const std::vector<Mode>& from, const std::vector<Mode>& to) {
+            for (size_t i = 0; i < from.size(); ++i) back.push_back(Mode{from[i].extent, {from[i].s[2], to[i].s[2], 0, 0}});
+        };
+        put(q.m, p.m);
+        put(q.n, p.n);
+        put(q.batch, p.batch);
+        for (auto* g : {&q.m, &q.n, &q.k}) fuse_in_order(*g, 4);
+        // rows of a copy are a multiple of eight, which its tensor map asks for: those past the last are products of
+        // whatever lies there, and land between the block's columns
+        if (wide && copy[0]) q.m.assign(1, Mode{ld[0], {1, 0, 1, 0}});
+        if (wide && copy[1]) q.n.assign(1, Mode{ld[1], {0, 1, ld[2], 0}});
+        TFB_TRY(launch_contract(ctx, q, CK_AUTO, used));
+        TFB_TRY(pass(back, blk[2].ptr, (char*)p.c + b0 * es, p.alpha, p.beta));
+    }
+    *done = true;
+    return TFB_OK;
+}
+
 // ------------------------------------------------------------------ selection
 tfb_status launch_contract(tfb_ctx* ctx, const ContractProblem& p, int force_kernel, const char** used) {
     DeviceGuard g(ctx->device);
@@ -466,6 +562,11 @@ tfb_status launch_contract(tfb_ctx* ctx, const ContractProblem& p, int force_ker
     }
     int want = force_kernel != CK_AUTO ? force_kernel : env_int("TFB_FORCE_KERNEL", CK_AUTO);
     bool declined = false;
+    if (want == CK_AUTO && env_int("TFB_BATCH_OUTERMOST", 1)) {
+        bool done = false;
+        TFB_TRY(contract_batch_innermost(ctx, p, used, &done));
+        if (done) return TFB_OK;
+    }
     if (want == CK_AUTO || want == CK_TCGEN05) {
         if (p.dtype == TFB_F32 || p.dtype == TFB_C32) {
             if (p.dtype == TFB_C32)

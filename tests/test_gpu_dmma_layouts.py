@@ -178,3 +178,32 @@ def test_split_of_k(tb, oracle, monkeypatch, dtype, mnk, cluster, conj):
     first = tb.einsum("ij,jk->ik", [x, y]).to_numpy()
     for _ in range(3):
         assert np.array_equal(tb.einsum("ij,jk->ik", [x, y]).to_numpy(), first)
+
+
+@pytest.mark.parametrize("notation,sizes", [
+    ("bij,bjk->bik", dict(b=37, i=67, j=1025, k=71)),
+    ("bij,bjk->bik", dict(b=16, i=260, j=515, k=301)),
+    ("bij,bkj->bki", dict(b=33, i=129, j=517, k=131)),      # operands change places
+    ("bij,jkb->bik", dict(b=40, i=129, j=261, k=259)),      # one operand with the batch outermost
+    ("bijx,bjxk->bki", dict(b=32, i=128, j=33, k=129, x=31)),  # two contracted modes
+    ("bijx,bkj->bkix", dict(b=33, i=17, j=515, k=129, x=9)),   # two free modes
+])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.complex64, np.complex128])
+def test_batch_innermost(tb, oracle, monkeypatch, notation, sizes, dtype):
+    """On copies with the batch outermost and as the operands lie, both against the host product.  Frobenius: 1e-5 for a
+    3xTF32 product, 1e-13 for double (K + 4 roundings at 1.1e-16, K up to 1025); single elements ten times that of the largest."""
+    a, b = (oracle.normal(7 + t, tuple(sizes[c] for c in s), dtype) for t, s in enumerate(notation.split("->")[0].split(",")))
+    c = oracle.normal(9, tuple(sizes[x] for x in notation.split("->")[1]), dtype)
+    ta, tc = tb.Tensor.from_numpy(a), tb.Tensor.from_numpy(b).into_conj()
+    got = []
+    for on in "10":
+        monkeypatch.setenv("TFB_BATCH_OUTERMOST", on)
+        out = tb.Tensor.from_numpy(c)
+        tb.einsum_into(notation, [ta, tc], 0.75, 0.5, out)
+        got.append(out.to_numpy())
+    wide = np.complex128 if np.dtype(dtype).kind == "c" else np.float64
+    want = 0.75 * np.einsum(notation, a.astype(wide), np.conj(b).astype(wide), optimize=True) + 0.5 * c
+    tol = 1e-13 if dtype in (np.float64, np.complex128) else 1e-5
+    for x in got:
+        assert np.linalg.norm(x - want) <= tol * np.linalg.norm(want)
+    assert np.abs(got[0] - got[1]).max() <= 10 * tol * np.abs(want).max()
