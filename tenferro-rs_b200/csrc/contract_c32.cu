@@ -22,6 +22,8 @@
 //
 // Semantics: PrimDescriptor::{Contract, BatchedGemm} for Complex32,
 // tenferro-prims/src/lib.rs:156-168, 227-239.
+#include <algorithm>
+
 #include "contract_common.cuh"
 #include "contract_tables.h"
 
@@ -102,10 +104,15 @@ __global__ void __launch_bounds__(256) scale_output_kernel(float2* c, const int6
     }
 }
 
-// B can serve as B' in place when one contracted mode with unit stride carries all of K, nothing
+// B can serve as B' in place when its contracted modes follow one another from unit stride on, nothing
 // is conjugated, and every other stride keeps the doubled (float) strides 16-byte aligned.
 bool b_is_real_view(const ContractProblem& p) {
-    if (p.conj_b || p.k.size() != 1 || p.k[0].s[1] != 1) return false;
+    if (p.conj_b || p.k.empty()) return false;
+    int64_t run = 1;
+    for (const Mode& m : p.k) {
+        if (m.s[1] != run) return false;
+        run *= m.extent;
+    }
     if ((uintptr_t)p.b % 16 != 0 || p.n.size() > 2 || p.batch.size() > 1) return false;
     for (const Mode& m : p.n)
         if (m.extent > 1 && (m.s[1] <= 0 || (2 * m.s[1]) % 4 != 0)) return false;
@@ -115,6 +122,22 @@ bool b_is_real_view(const ContractProblem& p) {
 }
 
 }  // namespace
+
+// The first operand is gathered whatever its order, so rows follow the output - a tile whose rows follow the
+// operand instead stores every element to a sector of its own (the outer-product node of a network with extents
+// 79, 66, 94, 68, 86, 96, 72, 11352 x 6912 x 136 floats: 727 us by the operand's order, 183 by the output's) - and K follows
+// the second operand, which may then be read in place.
+static ContractProblem embedding_order(const ContractProblem& p) {
+    ContractProblem q = p;
+    auto by = [](std::vector<Mode>& g, int t) {
+        for (const Mode& m : g)
+            if (m.s[t] == 0) return;
+        std::stable_sort(g.begin(), g.end(), [t](const Mode& x, const Mode& y) { return std::llabs(x.s[t]) < std::llabs(y.s[t]); });
+    };
+    by(q.m, 2);
+    by(q.k, 1);
+    return q;
+}
 
 static tfb_status embedded_product(tfb_ctx* ctx, const ContractProblem& p, bool* declined) {
     *declined = true;
@@ -207,10 +230,10 @@ tfb_status contract_c32_embedded(tfb_ctx* ctx, const ContractProblem& p, bool* d
         // The embedded operand should be the small one: a tall first operand against a short second
         // one (M >> N) would spend more time being embedded than the product takes.
         if (env_int("TFB_C32_EXCHANGE", 1)) {
-            const ContractProblem q = exchange_roles(p);
-            if (setup_floats(q) < 0.6 * setup_floats(p)) return embedded_product(ctx, q, declined);
+            const ContractProblem q = embedding_order(exchange_roles(p));
+            if (setup_floats(q) < 0.6 * setup_floats(embedding_order(p))) return embedded_product(ctx, q, declined);
         }
-        return embedded_product(ctx, p, declined);
+        return embedded_product(ctx, embedding_order(p), declined);
     }
     // A fused multiplier is a complex product per element, and the real embedding holds the two
     // parts of an element in different rows: the product runs unfused and C is multiplied in
@@ -220,7 +243,7 @@ tfb_status contract_c32_embedded(tfb_ctx* ctx, const ContractProblem& p, bool* d
     ContractProblem q = p;
     q.mul = nullptr;
     q.conj_mul = false;
-    TFB_TRY(embedded_product(ctx, q, declined));
+    TFB_TRY(embedded_product(ctx, embedding_order(q), declined));
     if (*declined) return TFB_OK;
     std::vector<Mode> all;
     for (auto* g : {&p.m, &p.n, &p.batch})

@@ -471,8 +471,9 @@ tfb_status tfb_einsum_with_plan_into(tfb_ctx* ctx, const tfb_tree* tree, int32_t
     if (n == 1) {
         return run_unary(ctx, dtype, live[0].labels, live[0].view, out_labels, vout, a, b, TFB_REDUCE_SUM, &used);
     }
-    // Column-major intermediate with the given labels.
-    auto make_temp = [&](const std::vector<uint32_t>& labels, Live* l) -> tfb_status {
+    // Column-major intermediate with the given labels; whole 16-byte units from one value of what follows the first `run`
+    // labels to the next.
+    auto make_temp = [&](const std::vector<uint32_t>& labels, size_t run, Live* l) -> tfb_status {
         l->labels = labels;
         l->view.dims.clear();
         l->view.strides.clear();
@@ -482,6 +483,10 @@ tfb_status tfb_einsum_with_plan_into(tfb_ctx* ctx, const tfb_tree* tree, int32_t
             l->view.dims.push_back(e);
             l->view.strides.push_back(count);
             count *= e;
+            if (run != 0 && l->view.dims.size() == run) {
+                const int64_t unit = std::max<int64_t>(1, 16 / (int64_t)es);
+                count = (count + unit - 1) / unit * unit;
+            }
         }
         l->block = std::make_shared<PoolBlock>();
         TFB_TRY(l->block->alloc(ctx, (size_t)count * es));
@@ -505,7 +510,7 @@ tfb_status tfb_einsum_with_plan_into(tfb_ctx* ctx, const tfb_tree* tree, int32_t
         }
         if (!drop) return TFB_OK;
         Live t;
-        TFB_TRY(make_temp(keep, &t));
+        TFB_TRY(make_temp(keep, 0, &t));
         TFB_TRY(run_unary(ctx, dtype, l.labels, l.view, t.labels, t.view, one, zero, TFB_REDUCE_SUM, &used));
         live[id] = t;
         return TFB_OK;
@@ -516,8 +521,12 @@ tfb_status tfb_einsum_with_plan_into(tfb_ctx* ctx, const tfb_tree* tree, int32_t
     // operand: the consumer then finds the intermediate with unit stride along K and can feed it
     // to the tensor cores in place instead of copying it (contract_c32.cu).  Only when the
     // leading label is long enough for the producer's writes to stay coalesced.
-    auto temp_order = [&](size_t s) -> std::vector<uint32_t> {
+    // `run`: how many labels those are, 0 in the default order.  With an odd number of elements between them the consumer
+    // could not read the intermediate in place, so they are followed by padding (the pass over 5427 x 5760 elements that
+    // makes up for it: 130 us).
+    auto temp_order = [&](size_t s, size_t* run) -> std::vector<uint32_t> {
         const std::vector<uint32_t>& labs = tree->steps[s].labels;
+        *run = 0;
         if (dtype != TFB_C32) return labs;
         const size_t id = n + s;
         for (size_t c = s + 1; c < tree->steps.size(); ++c) {
@@ -539,6 +548,7 @@ tfb_status tfb_einsum_with_plan_into(tfb_ctx* ctx, const tfb_tree* tree, int32_t
             for (const auto& sl : by_stride)
                 if (has(labs, sl.second) && !has(kept, sl.second) && !has(order, sl.second)) order.push_back(sl.second);
             if (order.empty() || tree->extent.at(order[0]) < 32) return labs;
+            *run = order.size();
             for (auto lab : labs)
                 if (!has(order, lab)) order.push_back(lab);
             return order;
@@ -604,7 +614,9 @@ tfb_status tfb_einsum_with_plan_into(tfb_ctx* ctx, const tfb_tree* tree, int32_t
                                    &dmul.labels, &dmul.view));
             } else {
                 Live t;
-                TFB_TRY(make_temp(temp_order(c), &t));
+                size_t run = 0;
+                const std::vector<uint32_t> order = temp_order(c, &run);
+                TFB_TRY(make_temp(order, run, &t));
                 TFB_TRY(run_binary(ctx, dtype, x.labels, x.view, y.labels, y.view, t.labels, t.view, one, zero, 0, &used,
                                    &dmul.labels, &dmul.view));
                 live[n + c] = t;
@@ -613,7 +625,9 @@ tfb_status tfb_einsum_with_plan_into(tfb_ctx* ctx, const tfb_tree* tree, int32_t
             live.erase(partner);
         } else {
             Live t;
-            TFB_TRY(make_temp(temp_order(s), &t));
+            size_t run = 0;
+            const std::vector<uint32_t> order = temp_order(s, &run);
+            TFB_TRY(make_temp(order, run, &t));
             TFB_TRY(run_binary(ctx, dtype, x.labels, x.view, y.labels, y.view, t.labels, t.view, one, zero, 0, &used));
             live[n + s] = t;
         }

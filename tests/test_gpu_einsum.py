@@ -263,6 +263,19 @@ def test_config4_network_dim24(tb, oracle):
     assert oracle.rel_frobenius(got, oracle.np_einsum("ijk,jlm,kmn,lnp->ip", ops)) <= 1e-5
 
 
+@pytest.mark.parametrize("dims", [(33, 35, 37, 39, 41, 43, 45), (40, 33, 34, 36, 35, 32, 38), (34, 47, 33, 32, 49, 37, 36), (12, 70, 66, 9, 68, 64, 11)])
+@pytest.mark.parametrize("conj", [False, True])
+def test_network_of_unequal_extents(tb, oracle, dims, conj):
+    """Odd extents give intermediates whose rows and contracted runs fall on no 16-byte unit, in every order of the modes."""
+    size = dict(zip("ijklmnp", dims))
+    ops = [oracle.normal(4100 + i, tuple(size[c] for c in t), np.complex64) for i, t in enumerate(("ijk", "jlm", "kmn", "lnp"))]
+    held = [tb.Tensor.from_numpy(o) for o in ops]
+    if conj:
+        held[1], ops[1] = held[1].into_conj(), ops[1].conj()
+    got = tb.einsum("ijk,jlm,kmn,lnp->ip", held).to_numpy()
+    assert oracle.rel_frobenius(got, oracle.np_einsum("ijk,jlm,kmn,lnp->ip", ops)) <= 1e-5
+
+
 def test_config5_scaled(tb, oracle):
     """'ijkl,klmn->ijmn', f32, i=j=m=n=32, k=l=64 (128 / 256 in the benchmark), N(0,1)."""
     a, b = oracle.normal(5000, (32, 32, 64, 64), np.float32), oracle.normal(5001, (64, 64, 32, 32), np.float32)
