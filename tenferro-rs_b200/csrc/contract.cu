@@ -3,6 +3,7 @@
 // `PrimDescriptor::{Contract, BatchedGemm}` (tenferro-prims/src/lib.rs:156-168, 227-239).
 #include "contract_common.cuh"
 #include "contract_tables.h"
+#include "ptx_sm100.cuh"
 #include "scalar_ops.cuh"
 
 namespace tfb {
@@ -260,6 +261,7 @@ __device__ __forceinline__ T simt_result(const ContractArgs& g, const T* D, int6
 
 template <typename T, int ALG = 0>
 __global__ void __launch_bounds__(256, kSimtCtas<T>) contract_simt_kernel(ContractArgs g) {
+    launch_begin();
     using S = Semi<T, ALG>;
     constexpr int BM = 64, BN = 64, BK = kSimtK<T>, P = 68, L = BM * BK / 256;
     // A thread's fragment: four neighbours for 4-byte elements, else four 16 apart, which meet no bank twice (988 x
@@ -370,6 +372,7 @@ __global__ void __launch_bounds__(256, kSimtCtas<T>) contract_simt_kernel(Contra
 // Adds the ranges of each output element in range order; one thread per element of a tile.
 template <typename T, int ALG = 0>
 __global__ void __launch_bounds__(256) simt_finish_kernel(ContractArgs g, int splits) {
+    launch_begin();
     constexpr int BM = 64, BN = 64;
     const int64_t tile = blockIdx.x, tm = tile % g.tiles_m, rest = tile / g.tiles_m, tn = rest % g.tiles_n, bb = rest / g.tiles_n;
     const int e = blockIdx.y * 256 + threadIdx.x;
@@ -405,14 +408,12 @@ static tfb_status simt_launch(tfb_ctx* ctx, ContractArgs a, const char* name) {
     const unsigned grid = (unsigned)std::min<int64_t>(a.n_tiles, (int64_t)ctx->sm_count * 8);
     {
         LaunchScope ls(ctx, name);
-        contract_simt_kernel<T, ALG><<<dim3(grid, (unsigned)splits), 256, 0, ctx->stream>>>(a);
+        TFB_CUDA(launch_overlapped(ctx, contract_simt_kernel<T, ALG>, dim3(grid, (unsigned)splits), dim3(256), 0, 0u, a));
     }
-    TFB_CUDA(cudaGetLastError());
     if (splits > 1) {
         LaunchScope ls(ctx, "contract_simt_finish");
-        simt_finish_kernel<T, ALG><<<dim3((unsigned)a.n_tiles, 16), 256, 0, ctx->stream>>>(a, (int)splits);
+        TFB_CUDA(launch_overlapped(ctx, simt_finish_kernel<T, ALG>, dim3((unsigned)a.n_tiles, 16), dim3(256), 0, 0u, a, (int)splits));
     }
-    TFB_CUDA(cudaGetLastError());
     return TFB_OK;
 }
 

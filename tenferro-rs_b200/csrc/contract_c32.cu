@@ -26,6 +26,7 @@
 
 #include "contract_common.cuh"
 #include "contract_tables.h"
+#include "ptx_sm100.cuh"
 
 namespace tfb {
 
@@ -43,11 +44,33 @@ struct EmbedArgs {
     float* dst;              // embed: [B][2 rows][ld], else [B][rows][ld]
 };
 
+// Everything the real product needs, in one launch: the operands' jobs and the output's offset tables.
+struct SetupArgs {
+    EmbedArgs job[2];
+    int n_jobs;
+    // C seen as f32: row 2m + c -> 2 c_m[m] + c, column n -> 2 c_n[n], batch b -> 2 c_b[b]
+    const int64_t *c_m, *c_n, *c_b;
+    int64_t M, N, B;
+    int64_t *out_m, *out_n, *out_b;
+};
+
 // 32 x 32 (rows x k) patches through shared memory: reads follow the source's unit stride,
 // writes follow k.  embed = 1 writes the 2 x 2 real block of alpha * op(a) per element (two
-// output rows), embed = 0 the element itself.
-__global__ void __launch_bounds__(256) embed_operand_kernel(EmbedArgs g) {
+// output rows), embed = 0 the element itself.  blockIdx.y: the operands' jobs, then the tables.
+// A few MB each, bound by latency: one launch, and a thread's four loads in flight together.
+__global__ void __launch_bounds__(256) embed_setup_kernel(const __grid_constant__ SetupArgs args) {
     __shared__ float2 tile[32][33];
+    launch_begin();
+    if ((int)blockIdx.y == args.n_jobs) {
+        const int64_t n = max(2 * args.M, max(args.N, args.B));
+        for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+            if (i < 2 * args.M) args.out_m[i] = 2 * args.c_m[i >> 1] + (i & 1);
+            if (i < args.N) args.out_n[i] = 2 * args.c_n[i];
+            if (i < args.B) args.out_b[i] = 2 * args.c_b[i];
+        }
+        return;
+    }
+    const EmbedArgs g = args.job[blockIdx.y];
     const int64_t tiles_r = (g.rows + 31) / 32, tiles_k = (g.K + 31) / 32;
     const int64_t n_tiles = tiles_r * tiles_k * g.B;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
@@ -56,12 +79,19 @@ __global__ void __launch_bounds__(256) embed_operand_kernel(EmbedArgs g) {
         const int64_t tr = t % tiles_r, rest = t / tiles_r, tk = rest % tiles_k, b = rest / tiles_k;
         const int64_t r0 = tr * 32, k0 = tk * 32;
         const float2* src = g.src + g.b_tab[b];
-        for (int j = ty; j < 32; j += 8) {
+        float2 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
             // (r, k) of this thread's element: tx runs along the source's fast direction
+            const int j = ty + 8 * i;
             const int64_t r = r0 + (g.src_kfast ? j : tx), k = k0 + (g.src_kfast ? tx : j);
-            float2 v = make_float2(0.f, 0.f);
-            if (r < g.rows && k < g.K) v = src[g.row_tab[r] + g.k_tab[k]];
-            if (g.src_kfast) tile[j][tx] = v; else tile[tx][j] = v;  // tile[r][k]
+            v[i] = make_float2(0.f, 0.f);
+            if (r < g.rows && k < g.K) v[i] = src[g.row_tab[r] + g.k_tab[k]];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int j = ty + 8 * i;
+            if (g.src_kfast) tile[j][tx] = v[i]; else tile[tx][j] = v[i];  // tile[r][k]
         }
         __syncthreads();
         for (int j = ty; j < 32; j += 8) {
@@ -81,15 +111,6 @@ __global__ void __launch_bounds__(256) embed_operand_kernel(EmbedArgs g) {
         }
         __syncthreads();
     }
-}
-
-// Offset tables of C seen as f32: row 2m + c -> 2 c_m[m] + c, column n -> 2 c_n[n], batch b -> 2 c_b[b].
-__global__ void real_view_tables_kernel(const int64_t* c_m, const int64_t* c_n, const int64_t* c_b, int64_t M, int64_t N,
-                                        int64_t B, int64_t* out_m, int64_t* out_n, int64_t* out_b) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 2 * M) out_m[i] = 2 * c_m[i >> 1] + (i & 1);
-    if (i < N) out_n[i] = 2 * c_n[i];
-    if (i < B) out_b[i] = 2 * c_b[i];
 }
 
 // C *= beta (complex), through the tables.
@@ -162,26 +183,24 @@ static tfb_status embedded_product(tfb_ctx* ctx, const ContractProblem& p, bool*
     int64_t* tab_n = tab_m + 2 * M;
     int64_t* tab_b = tab_n + N;
 
-    auto embed = [&](const void* src, const int64_t* row_tab, const int64_t* k_tab, const int64_t* b_tab, int64_t rows,
-                     int kfast, bool conj, bool emb, float2 alpha, float* dst) -> tfb_status {
-        EmbedArgs g{(const float2*)src, row_tab, k_tab, b_tab, rows, K, B, ld, kfast, conj ? 1 : 0, emb ? 1 : 0, alpha, dst};
-        const int64_t n_tiles = ((rows + 31) / 32) * ((K + 31) / 32) * B;
-        const int grid = (int)std::min<int64_t>(n_tiles, (int64_t)ctx->sm_count * 16);
-        LaunchScope ls(ctx, "pack_planes");
-        embed_operand_kernel<<<grid, 256, 0, ctx->stream>>>(g);
-        TFB_CUDA(cudaGetLastError());
-        return TFB_OK;
+    SetupArgs setup = {};
+    int64_t most = (std::max<int64_t>(std::max<int64_t>(2 * M, N), B) + 255) / 256;
+    auto job = [&](const void* src, const int64_t* row_tab, const int64_t* k_tab, const int64_t* b_tab, int64_t rows,
+                   int kfast, bool conj, bool emb, float2 alpha, float* dst) {
+        setup.job[setup.n_jobs++] =
+            EmbedArgs{(const float2*)src, row_tab, k_tab, b_tab, rows, K, B, ld, kfast, conj ? 1 : 0, emb ? 1 : 0, alpha, dst};
+        most = std::max<int64_t>(most, ((rows + 31) / 32) * ((K + 31) / 32) * B);
     };
     const float2 alpha = make_float2((float)p.alpha.re, (float)p.alpha.im);
-    TFB_TRY(embed(p.a, t->a_m, t->a_k, t->a_b, M, ca.a_kfast, p.conj_a, true, alpha, a_real));
-    if (!b_in_place)
-        TFB_TRY(embed(p.b, t->b_n, t->b_k, t->b_b, N, ca.b_kfast, p.conj_b, false, make_float2(1.f, 0.f), b_real));
+    job(p.a, t->a_m, t->a_k, t->a_b, M, ca.a_kfast, p.conj_a, true, alpha, a_real);
+    if (!b_in_place) job(p.b, t->b_n, t->b_k, t->b_b, N, ca.b_kfast, p.conj_b, false, make_float2(1.f, 0.f), b_real);
+    setup.c_m = t->c_m; setup.c_n = t->c_n; setup.c_b = t->c_b;
+    setup.M = M; setup.N = N; setup.B = B;
+    setup.out_m = tab_m; setup.out_n = tab_n; setup.out_b = tab_b;
     {
-        const int64_t n = std::max<int64_t>(std::max<int64_t>(2 * M, N), B);
-        real_view_tables_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(t->c_m, t->c_n, t->c_b, M, N, B, tab_m,
-                                                                                    tab_n, tab_b);
-        count_launch();
-        TFB_CUDA(cudaGetLastError());
+        LaunchScope ls(ctx, "pack_planes");
+        const unsigned grid = (unsigned)std::min<int64_t>(most, (int64_t)ctx->sm_count * 16);
+        TFB_CUDA(launch_overlapped(ctx, embed_setup_kernel, dim3(grid, setup.n_jobs + 1), dim3(256), 0, 0u, setup));
     }
     double beta = p.beta.re;
     if (p.beta.im != 0) {

@@ -340,6 +340,7 @@ contract_tf32x3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     }
     tc_fence_before();
     __syncthreads();
+    launch_begin();  // nothing above touches global memory
     tc_fence_after();
     const uint32_t tmem_base = *tmem_word_ptr;
 
@@ -532,6 +533,7 @@ contract_tf32x3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 constexpr int kFinishCols = 8;  // columns of a tile per finishing CTA
 template <int BN>
 __global__ void __launch_bounds__(256) tf32x3_splitk_finish_kernel(TcArgs g) {
+    launch_begin();
     const int64_t tile_id = blockIdx.x;
     const TileCoord tc = decode_tile(tile_id, g.tiles_m, g.tiles_n, g.group_m);
     const int64_t bb = tc.batch, tm = tc.tm, tn = tc.tn;
@@ -790,6 +792,7 @@ contract_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     }
     tc_fence_before();
     cluster_sync_all();  // barriers of both CTAs exist before anyone arrives on the peer's
+    launch_begin();      // nothing above touches global memory
     tc_fence_after();
     const uint32_t tmem_base = *tmem_word_ptr;
 
@@ -1308,6 +1311,7 @@ contract_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __g
 
 // Split-K finish for the pair kernel: one CTA per (pair tile, rank), i.e. per 128 x 256 part.
 __global__ void __launch_bounds__(256) tf32x3_pair_splitk_finish_kernel(TcArgs g) {
+    launch_begin();
     constexpr int BN = PairCfg::BN;
     const int64_t part = blockIdx.x, pair_tile = part >> 1;
     const int rank = (int)(part & 1);
@@ -1354,11 +1358,13 @@ struct RepackArgs {
     int64_t rows, K, Kp, B;
     int src_kfast;
     float* dst;
+    bool beside;  // runs beside the other operand's copy (launch_begin)
 };
 constexpr int kRepackTile = 64;
 __global__ void __launch_bounds__(256) repack_kmajor_kernel(RepackArgs g) {
     constexpr int T = kRepackTile;
     __shared__ float tile[T][T + 1];
+    launch_begin(g.beside);
     const int64_t tiles_r = (g.rows + T - 1) / T, tiles_k = (g.Kp + T - 1) / T;
     const int64_t n_tiles = tiles_r * tiles_k * g.B;
     const int tx = threadIdx.x & (T - 1), ty = threadIdx.x / T;  // 64 x 4
@@ -1392,6 +1398,7 @@ __global__ void __launch_bounds__(256) repack_kmajor_kernel(RepackArgs g) {
         }
         __syncthreads();
     }
+    launch_end(g.beside);
 }
 
 // ------------------------------------------------------------------ host side
@@ -1599,13 +1606,12 @@ tfb_status launch_tc(tfb_ctx* ctx, const OperandMap& a, const OperandMap& b, TcA
     }
     {
         LaunchScope ls(ctx, "contract_tf32x3");
-        contract_tf32x3_kernel<BN><<<(unsigned)grid, 64 + kSplitThreads, Cfg::SMEM_BYTES, ctx->stream>>>(a.map, b.map, g);
-        TFB_CUDA(cudaGetLastError());
+        TFB_CUDA(launch_overlapped(ctx, contract_tf32x3_kernel<BN>, dim3((unsigned)grid), dim3(64 + kSplitThreads), Cfg::SMEM_BYTES, 0u,
+                                   a.map, b.map, g));
     }
     if (g.k_split > 1) {
         LaunchScope ls(ctx, "contract_tf32x3_finish");
-        tf32x3_splitk_finish_kernel<BN><<<dim3((unsigned)n_tiles, BN / kFinishCols), 256, 0, ctx->stream>>>(g);
-        TFB_CUDA(cudaGetLastError());
+        TFB_CUDA(launch_overlapped(ctx, tf32x3_splitk_finish_kernel<BN>, dim3((unsigned)n_tiles, BN / kFinishCols), dim3(256), 0, 0u, g));
     }
     return TFB_OK;
 }
@@ -1666,8 +1672,8 @@ tfb_status launch_tc_pair(tfb_ctx* ctx, const OperandMap& a, const OperandMap& b
         // than six k-blocks is dominated by its start and end and keeps the three TF32 MMAs
         const bool bf16c = env_int("TFB_TC_BF16_CORRECTIONS", 1) != 0 && (!short_k || g.num_kb >= 6);
 #define TFB_PAIR_LAUNCH(MUL_, SHORT_, C_)                                                                                   \
-    contract_tf32x3_pair_kernel<MUL_, SHORT_, C_><<<(unsigned)grid, pair_threads(SHORT_), Cfg::SMEM_BYTES, ctx->stream>>>(a.map, b.map, \
-                                                                                                                       mc, g)
+    TFB_CUDA(launch_overlapped(ctx, contract_tf32x3_pair_kernel<MUL_, SHORT_, C_>, dim3((unsigned)grid),                    \
+                               dim3(pair_threads(SHORT_)), Cfg::SMEM_BYTES, 0u, a.map, b.map, mc, g))
 #define TFB_PAIR_LAUNCH2(MUL_, SHORT_)                                                                                      \
     do {                                                                                                                    \
         if (bf16c) TFB_PAIR_LAUNCH(MUL_, SHORT_, true);                                                                     \
@@ -1683,8 +1689,8 @@ tfb_status launch_tc_pair(tfb_ctx* ctx, const OperandMap& a, const OperandMap& b
     }
     if (via_partials) {
         LaunchScope ls(ctx, "contract_tf32x3_finish");
-        tf32x3_pair_splitk_finish_kernel<<<dim3((unsigned)(2 * pair_tiles), Cfg::BN / kFinishCols), 256, 0, ctx->stream>>>(g);
-        TFB_CUDA(cudaGetLastError());
+        TFB_CUDA(launch_overlapped(ctx, tf32x3_pair_splitk_finish_kernel, dim3((unsigned)(2 * pair_tiles), Cfg::BN / kFinishCols),
+                                   dim3(256), 0, 0u, g));
     }
     return TFB_OK;
 }
@@ -1895,6 +1901,7 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
             ContractArgs ca;
             fill_args(p, t.get(), &ca);
             const int64_t Kp = (K + 3) / 4 * 4, Bn = p.B();
+            bool ahead = false;  // the other operand's copy is the launch ahead
             auto repack = [&](int tns, PoolBlock* blk, OperandMap* out) -> tfb_status {
                 const int64_t rows = tns == 0 ? M : N;
                 const tfb_status got = blk->alloc(ctx, (size_t)(rows * Kp * Bn) * sizeof(float));
@@ -1903,12 +1910,13 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
                     return got;
                 }
                 RepackArgs r{(const float*)(tns == 0 ? p.a : p.b), tns == 0 ? t->a_m : t->b_n, tns == 0 ? t->a_k : t->b_k,
-                             tns == 0 ? t->a_b : t->b_b, rows, K, Kp, Bn, tns == 0 ? ca.a_kfast : ca.b_kfast, (float*)blk->ptr};
+                             tns == 0 ? t->a_b : t->b_b, rows, K, Kp, Bn, tns == 0 ? ca.a_kfast : ca.b_kfast, (float*)blk->ptr, ahead};
                 const int64_t n_tiles = ((rows + kRepackTile - 1) / kRepackTile) * ((Kp + kRepackTile - 1) / kRepackTile) * Bn;
                 {
                     LaunchScope ls(ctx, "repack_operand");
-                    repack_kmajor_kernel<<<(unsigned)std::min<int64_t>(n_tiles, (int64_t)ctx->sm_count * 16), 256, 0, ctx->stream>>>(r);
-                    TFB_CUDA(cudaGetLastError());
+                    const unsigned grid = (unsigned)std::min<int64_t>(n_tiles, (int64_t)ctx->sm_count * 16);
+                    TFB_CUDA(launch_overlapped(ctx, repack_kmajor_kernel, dim3(grid), dim3(256), 0, 0u, r));
+                    ahead = true;
                 }
                 // the same product with this operand contiguous: one free mode, K split as in the other operand
                 ContractProblem q = p;
