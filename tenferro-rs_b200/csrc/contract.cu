@@ -485,12 +485,12 @@ static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& 
     PoolBlock blk[3];
     for (int t = 0; t < 3; ++t)
         if ((t == 2 || copy[t]) && blk[t].alloc(ctx, (size_t)(per[t] * chunk * es)) != TFB_OK) return TFB_OK;
-    auto pass = [&](const std::vector<Mode>& modes, const void* in, void* out, Scalar alpha, Scalar beta) -> tfb_status {
+    auto pass = [&](const std::vector<Mode>& modes, const void* in, void* out, Scalar alpha, Scalar beta, bool beside) -> tfb_status {
         std::vector<Mode> sorted = modes;
         sort_and_fuse(sorted, 1, 2);
         LoopNest nest;
         TFB_TRY(make_nest(sorted, &nest));
-        return launch_permute(ctx, p.dtype, nest, in, out, alpha, beta, false);
+        return launch_permute(ctx, p.dtype, nest, in, out, alpha, beta, false, beside);
     };
     auto dense = [](std::vector<Mode>& g, int t, int64_t step) {
         for (Mode& m : g) {
@@ -520,7 +520,7 @@ static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& 
             put(t == 0 ? p.m : p.n, free_q);
             put(p.k, q.k);
             put(p.batch, q.batch);
-            TFB_TRY(pass(modes, t == 0 ? q.a : q.b, blk[t].ptr, Scalar{1.0, 0.0}, Scalar{0.0, 0.0}));
+            TFB_TRY(pass(modes, t == 0 ? q.a : q.b, blk[t].ptr, Scalar{1.0, 0.0}, Scalar{0.0, 0.0}, t == 1 && copy[0]));
             (t == 0 ? q.a : q.b) = blk[t].ptr;
         }
         dense(q.m, 2, 1);
@@ -539,7 +539,7 @@ static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& 
         if (wide && copy[0]) q.m.assign(1, Mode{ld[0], {1, 0, 1, 0}});
         if (wide && copy[1]) q.n.assign(1, Mode{ld[1], {0, 1, ld[2], 0}});
         TFB_TRY(launch_contract(ctx, q, CK_AUTO, used));
-        TFB_TRY(pass(back, blk[2].ptr, (char*)p.c + b0 * es, p.alpha, p.beta));
+        TFB_TRY(pass(back, blk[2].ptr, (char*)p.c + b0 * es, p.alpha, p.beta, false));
     }
     *done = true;
     return TFB_OK;

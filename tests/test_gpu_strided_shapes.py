@@ -166,3 +166,19 @@ def test_permute_tiles(tb, oracle, shape, perm, on_tiles, dtype, padded):
     ran = ctx.profile_read("permute_tile")[0]
     ctx.profile_end()
     assert ran == (2 if dtype in on_tiles else 0)
+
+
+@pytest.mark.parametrize("shape,kept", [((20, 29, 13, 32), [0, 1]), ((119, 62, 465), [1]), ((31, 2003, 23), [0, 2]), ((5000, 40), [1]), ((200, 200), [])])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.complex128])
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+def test_slices_combined_by_the_last_block(tb, oracle, shape, kept, dtype, beta):
+    """Sums over whole numbers, exact in every type and order, three times over the same counters."""
+    x = oracle.normal(5, shape, np.float64).round().astype(dtype)
+    gone = tuple(i for i in range(len(shape)) if i not in kept)
+    c = np.arange(np.prod([shape[i] for i in kept], dtype=int), dtype=dtype).reshape([shape[i] for i in kept])
+    plan = tb.CudaBackend.plan(tb.PrimDescriptor.Reduce(list(range(len(shape))), kept, tb.ReduceOp.Sum), [shape, c.shape], dtype)
+    held = tb.Tensor.from_numpy(x)
+    for _ in range(3):
+        out = tb.Tensor.from_numpy(c)
+        tb.CudaBackend.execute(plan, 2.0, [held], beta, out)
+        assert np.array_equal(out.to_numpy(), 2 * x.sum(axis=gone) + dtype(beta) * c)
