@@ -154,6 +154,9 @@ class Context:
 
     @classmethod
     def get(cls, device_id: int = 0) -> "Context":
+        ctx = cls._by_device.get(device_id)
+        if ctx is not None:
+            return ctx
         with cls._lock:
             ctx = cls._by_device.get(device_id)
             if ctx is None:

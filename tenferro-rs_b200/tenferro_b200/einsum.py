@@ -4,13 +4,16 @@ tree walk all run in libtenferro_b200.so; intermediates never leave the device."
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
 
 from . import _lib
 from ._lib import lib
-from .device import Context, InvalidArgument, NoCompatibleComputeDevice, OpKind, check, preferred_compute_devices
+from .device import (
+    Context, InvalidArgument, LogicalMemorySpace, NoCompatibleComputeDevice, OpKind, check, preferred_compute_devices,
+)
 from .prims import scalar_arg
 from .tensor import MemoryOrder, Tensor, check_same_space, dtype_code
 
@@ -141,11 +144,23 @@ class ContractionTree:
             pass
 
 
+@functools.lru_cache(maxsize=64)
+def _computes_on_its_own(space_id: int) -> bool:
+    devices = [d for d in preferred_compute_devices(LogicalMemorySpace.GpuMemory(space_id), OpKind.Contract) if d.kind == "cuda"]
+    return bool(devices) and devices[0].device_id == space_id
+
+
 def _select_context(operands: Sequence[Tensor], output: Optional[Tensor] = None) -> Context:
     """Backend selection from the tensors' memory space and device pins
     (tenferro-einsum/src/lib.rs:16-20, 179-207)."""
-    tensors = list(operands) + ([output] if output is not None else [])
+    tensors = list(operands) if output is None else [*operands, output]
     space = check_same_space(tensors)
+    for t in tensors:
+        if t._preferred is not None:
+            break
+    else:  # nothing is pinned: the space's own device, where the space has one
+        if space.space_id is not None and _computes_on_its_own(space.space_id):
+            return Context.get(space.space_id)
     # Tensors without a pin of their own all have the space's default devices: asked for once.
     lists = [t.effective_compute_devices(OpKind.Contract) for t in tensors if t._preferred is not None]
     if len(lists) < len(tensors):
@@ -168,7 +183,7 @@ def einsum_with_plan_into(tree: ContractionTree, operands: Sequence[Tensor], alp
     ctx = _select_context(operands, output)
     dtype = output.dtype
     for t in operands:
-        if t.dtype != dtype:
+        if t.dtype is not dtype and t.dtype != dtype:
             raise InvalidArgument(f"operand dtype {t.dtype} differs from the output's {dtype}")
     keep: list = []
     views = (_lib.TfbView * max(len(operands), 1))(*[t.as_operand_view(keep) for t in operands])

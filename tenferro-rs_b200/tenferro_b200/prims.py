@@ -8,6 +8,7 @@ import array
 import ctypes as C
 import enum
 import itertools
+import math
 from dataclasses import dataclass, field
 from typing import List, Optional, Sequence, Tuple
 
@@ -162,8 +163,18 @@ _REAL_SCALAR = {
 }
 
 
+# The two scalars nearly every call passes, by element type (the library only reads them).
+_ONE, _ZERO = ({dt: C.byref(make(v)) for dt, make in _REAL_SCALAR.items()} for v in (1.0, 0.0))
+
+
 def scalar_arg(value, dtype):
     """One host scalar of `dtype` as a ctypes argument."""
+    if type(value) is float:
+        if value == 1.0:
+            if dtype in _ONE:
+                return _ONE[dtype]
+        elif value == 0.0 and math.copysign(1.0, value) > 0 and dtype in _ZERO:
+            return _ZERO[dtype]
     # Plain Python numbers convert without NumPy (0.4 us against 2), to the same bits.
     kind = type(value)
     if kind is float or kind is int:
@@ -202,18 +213,20 @@ class CudaBackend:
     def execute(plan: CudaPlan, alpha, inputs: Sequence[Tensor], beta, output: Tensor) -> None:
         """`execute(plan, alpha, inputs, beta, output)`: output = alpha * op(inputs) + beta * output.
         Returns once the work is enqueued; `output.event` marks its completion."""
-        tensors = list(inputs) + [output]
+        tensors = [*inputs, output]
+        dtype = plan.dtype
         for t in tensors:
-            if t.dtype != plan.dtype:
+            if t.dtype is not dtype and t.dtype != dtype:
                 raise InvalidArgument(f"plan was made for {plan.dtype}, got a {t.dtype} tensor")
         space = check_same_space(tensors)
         if not space.is_gpu:
             raise NoCompatibleComputeDevice(
                 "no compatible compute device on MainMemory: move the tensors with to_memory_space_async first")
         ctx = plan.ctx
-        for t in inputs:
-            if t.event is not None and t.ctx is not ctx:
-                ctx.wait_event(t.event)
+        if Context.get(space.space_id) is not ctx:
+            for t in inputs:
+                if t.event is not None:
+                    ctx.wait_event(t.event)
         keep: list = []
         views = (_lib.TfbView * max(len(inputs), 1))(*[t.as_operand_view(keep) for t in inputs])
         out_view = output.as_operand_view(keep)

@@ -130,7 +130,7 @@ class Tensor:
         if event is not None:
             self.event = event
         self._conj = bool(conj) and self.dtype.kind == "c"
-        self._arrays = None
+        self._view = None
 
     @property
     def event(self) -> Optional[CompletionEvent]:
@@ -276,13 +276,15 @@ class Tensor:
     def as_operand_view(self, keep: list) -> _lib.TfbView:
         """Non-blocking operand view (tenferro-tensor/src/lib.rs:473-488): pending work is
         ordered by the stream, the host does not wait."""
-        ptr = self._block.ptr if self._block is not None else 0
-        # dims and strides of a tensor never change: their C arrays are made once per tensor
-        arrays = self._arrays
-        if arrays is None:
-            arrays = self._arrays = _view_arrays(self._dims, self._strides)
-        keep.append(arrays)
-        return _lib.TfbView(ptr, len(self._dims), arrays[0], arrays[1], self._offset, 1 if self._conj else 0)
+        # neither the buffer nor the layout of a tensor ever changes: the view and its C arrays are made once per tensor
+        view = self._view
+        if view is None:
+            ptr = self._block.ptr if self._block is not None else 0
+            arrays = _view_arrays(self._dims, self._strides)
+            view = _lib.TfbView(ptr, len(self._dims), arrays[0], arrays[1], self._offset, 1 if self._conj else 0)
+            self._view = view
+        keep.append(view)  # (holds its arrays)
+        return view
 
     # ------------------------------------------------------------ view operations (zero-copy)
     def permute(self, perm: Sequence[int]) -> "Tensor":
