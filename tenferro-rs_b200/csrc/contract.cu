@@ -482,26 +482,59 @@ static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& 
     bytes += per[2] * es;
     const int64_t chunk = std::min(B, std::max<int64_t>(32, ((int64_t)1 << 30) / bytes / 32 * 32));
     if ((double)bytes * (double)chunk > (double)ctx->total_mem / 16) return TFB_OK;
-    PoolBlock blk[3];
-    for (int t = 0; t < 3; ++t)
-        if ((t == 2 || copy[t]) && blk[t].alloc(ctx, (size_t)(per[t] * chunk * es)) != TFB_OK) return TFB_OK;
-    auto pass = [&](const std::vector<Mode>& modes, const void* in, void* out, Scalar alpha, Scalar beta, bool beside) -> tfb_status {
-        std::vector<Mode> sorted = modes;
-        sort_and_fuse(sorted, 1, 2);
-        LoopNest nest;
-        TFB_TRY(make_nest(sorted, &nest));
-        return launch_permute(ctx, p.dtype, nest, in, out, alpha, beta, false, beside);
-    };
     auto dense = [](std::vector<Mode>& g, int t, int64_t step) {
         for (Mode& m : g) {
             m.s[t] = step;
             step *= m.extent;
         }
     };
+    // The product of n of the batch on the copies, and the nests of the passes that make them and put its output back;
+    // false where a pass has more modes than a nest takes, though each group of the product alone has not.
+    auto lay_out = [&](int64_t n, ContractProblem* q, LoopNest* nest) -> bool {
+        *q = p;
+        q->batch[0].extent = n;
+        for (int t = 0; t < 3; ++t) {
+            if (t < 2 && !copy[t]) continue;
+            std::vector<Mode> modes;
+            // from where the operand lies to its copy, from the block to where the output lies
+            auto put = [&](const std::vector<Mode>& outer, const std::vector<Mode>& block) {
+                for (size_t i = 0; i < block.size(); ++i)
+                    modes.push_back(t < 2 ? Mode{block[i].extent, {outer[i].s[t], block[i].s[t], 0, 0}}
+                                          : Mode{block[i].extent, {block[i].s[t], outer[i].s[t], 0, 0}});
+            };
+            if (t < 2) {
+                std::vector<Mode>& free_q = t == 0 ? q->m : q->n;
+                dense(free_q, t, wide ? 1 : ld[t]);
+                dense(q->k, t, wide ? ld[t] : 1);
+                put(t == 0 ? p.m : p.n, free_q);
+                put(p.k, q->k);
+            } else {
+                dense(q->m, 2, 1);
+                dense(q->n, 2, ld[2]);
+                put(p.m, q->m);
+                put(p.n, q->n);
+            }
+            q->batch[0].s[t] = per[t];
+            put(p.batch, q->batch);
+            sort_and_fuse(modes, 1, 2);
+            if ((int)modes.size() > kMaxRank || make_nest(modes, &nest[t]) != TFB_OK) return false;
+        }
+        for (auto* g : {&q->m, &q->n, &q->k}) fuse_in_order(*g, 4);
+        // rows of a copy are a multiple of eight, which its tensor map asks for: those past the last are products of
+        // whatever lies there, and land between the block's columns
+        if (wide && copy[0]) q->m.assign(1, Mode{ld[0], {1, 0, 1, 0}});
+        if (wide && copy[1]) q->n.assign(1, Mode{ld[1], {0, 1, ld[2], 0}});
+        return true;
+    };
+    ContractProblem q;
+    LoopNest nest[3];
+    for (int64_t n : {B % chunk, chunk})
+        if (n > 0 && !lay_out(n, &q, nest)) return TFB_OK;
+    PoolBlock blk[3];
+    for (int t = 0; t < 3; ++t)
+        if ((t == 2 || copy[t]) && blk[t].alloc(ctx, (size_t)(per[t] * chunk * es)) != TFB_OK) return TFB_OK;
     for (int64_t b0 = 0; b0 < B; b0 += chunk) {
-        const int64_t n = std::min(chunk, B - b0);
-        ContractProblem q = p;
-        q.batch[0].extent = n;
+        lay_out(std::min(chunk, B - b0), &q, nest);
         q.a = (const char*)p.a + b0 * p.batch[0].s[0] * es;
         q.b = (const char*)p.b + b0 * p.batch[0].s[1] * es;
         q.c = blk[2].ptr;
@@ -509,37 +542,12 @@ static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& 
         q.beta = Scalar{0.0, 0.0};
         for (int t = 0; t < 2; ++t) {
             if (!copy[t]) continue;
-            std::vector<Mode>& free_q = t == 0 ? q.m : q.n;
-            dense(free_q, t, wide ? 1 : ld[t]);
-            dense(q.k, t, wide ? ld[t] : 1);
-            q.batch[0].s[t] = per[t];
-            std::vector<Mode> modes;
-            auto put = [&](const std::vector<Mode>& from, const std::vector<Mode>& to) {
-                for (size_t i = 0; i < from.size(); ++i) modes.push_back(Mode{to[i].extent, {from[i].s[t], to[i].s[t], 0, 0}});
-            };
-            put(t == 0 ? p.m : p.n, free_q);
-            put(p.k, q.k);
-            put(p.batch, q.batch);
-            TFB_TRY(pass(modes, t == 0 ? q.a : q.b, blk[t].ptr, Scalar{1.0, 0.0}, Scalar{0.0, 0.0}, t == 1 && copy[0]));
-            (t == 0 ? q.a : q.b) = blk[t].ptr;
+            const void*& x = t == 0 ? q.a : q.b;
+            TFB_TRY(launch_permute(ctx, p.dtype, nest[t], x, blk[t].ptr, Scalar{1.0, 0.0}, Scalar{0.0, 0.0}, false, t == 1 && copy[0]));
+            x = blk[t].ptr;
         }
-        dense(q.m, 2, 1);
-        dense(q.n, 2, ld[2]);
-        q.batch[0].s[2] = per[2];
-        std::vector<Mode> back;
-        auto put = [&](const std::vector<Mode>& from, const std::vector<Mode>& to) {
-            for (size_t i = 0; i < from.size(); ++i) back.push_back(Mode{from[i].extent, {from[i].s[2], to[i].s[2], 0, 0}});
-        };
-        put(q.m, p.m);
-        put(q.n, p.n);
-        put(q.batch, p.batch);
-        for (auto* g : {&q.m, &q.n, &q.k}) fuse_in_order(*g, 4);
-        // rows of a copy are a multiple of eight, which its tensor map asks for: those past the last are products of
-        // whatever lies there, and land between the block's columns
-        if (wide && copy[0]) q.m.assign(1, Mode{ld[0], {1, 0, 1, 0}});
-        if (wide && copy[1]) q.n.assign(1, Mode{ld[1], {0, 1, ld[2], 0}});
         TFB_TRY(launch_contract(ctx, q, CK_AUTO, used));
-        TFB_TRY(pass(back, blk[2].ptr, (char*)p.c + b0 * es, p.alpha, p.beta, false));
+        TFB_TRY(launch_permute(ctx, p.dtype, nest[2], blk[2].ptr, (char*)p.c + b0 * es, p.alpha, p.beta, false));
     }
     *done = true;
     return TFB_OK;

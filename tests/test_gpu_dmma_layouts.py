@@ -207,3 +207,14 @@ def test_batch_innermost(tb, oracle, monkeypatch, notation, sizes, dtype):
     for x in got:
         assert np.linalg.norm(x - want) <= tol * np.linalg.norm(want)
     assert np.abs(got[0] - got[1]).max() <= 10 * tol * np.abs(want).max()
+
+
+@pytest.mark.parametrize("notation,sizes", [
+    # twelve free modes and the batch lie one by one in the output: no single pass puts it back
+    ("bacegikx,bxdfhjlm->badcfehgjilkm", dict(b=64, x=512)),
+    # ... and in an operand: no single pass copies it
+    ("bavcwexgyizks,bvwxyzsd->bacegikd", dict(b=64, d=400)),
+])
+def test_batch_innermost_in_more_modes_than_a_pass_takes(tb, oracle, notation, sizes):
+    shapes = [tuple(sizes.get(c, 2) for c in t) for t in notation.split("->")[0].split(",")]
+    run(tb, oracle, notation, shapes, np.float64, False, 0.5)
