@@ -206,6 +206,10 @@ enum ContractKernel { CK_AUTO = 0, CK_SIMT = 1, CK_DMMA = 2, CK_TCGEN05 = 3, CK_
 // Runs the problem on ctx's stream.  `used` receives the kernel family chosen.
 tfb_status launch_contract(tfb_ctx* ctx, const ContractProblem& p, int force_kernel, const char** used);
 
+// Operations of one product of the batch from which contract_tcgen05 copies operands that have no tensor map; below, such
+// products run on the exact kernel.
+constexpr double kTcCopyFlops = 1e9;
+
 // Family-specific launchers (each may decline with *declined = true and TFB_OK).
 tfb_status contract_simt(tfb_ctx* ctx, const ContractProblem& p);
 // Over a tropical semiring (tfb_algebra: 1 MaxPlus, 2 MinPlus); an empty K group is a single term.

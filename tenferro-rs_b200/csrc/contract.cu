@@ -455,14 +455,14 @@ tfb_status contract_simt_semiring(tfb_ctx* ctx, const ContractProblem& p, int al
 // the size on that repays copies at all, the operands that lie so are copied with the batch outermost, the
 // products go to a block of their own, and one pass over that applies alpha and beta and puts the batch back innermost: all
 // of it tiled permutations at the memory's rate.  Chunks of the batch keep the copies to about 1 GB.
-// (us before and now: f32, 484 of 736 x 824 x 1044 26100, 4650, 1000 of 100^3 383, 141, 8 of 600^3 259, 92; double, 484 of 736 x
+// (us before and now: f32, 484 of 736 x 824 x 1044 26100, 4650, the exact kernel 1000 of 100^3 380, 233, 8 of 600^3 255, 227; double, 484 of 736 x
 // 824 x 1044 199000, 23900, 220 of 580 x 408 x 308 2900, 1650, 16 of 600^3 353, 348, 8 of 600^3 186, 200; complex single, 1000 of
 // 100^3 337, 294, 8 of 600^3 167, 177.  Complex double elements are half a sector, and nothing is gained: 64 of 300^3 619, 628.)
 static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& p, const char** used, bool* done) {
     *done = false;
     if (p.batch.size() != 1 || p.batch[0].s[2] != 1 || p.batch[0].extent < (p.dtype == TFB_F32 ? 8 : 16) || p.mul || p.dtype == TFB_C64)
         return TFB_OK;
-    if (p.dtype == TFB_F32 && p.k.size() > 2) return TFB_OK;  // the exact kernel's: not to be moved to 3xTF32 by a copy
+    if (p.dtype == TFB_F32 && p.k.size() > 2) return TFB_OK;  // the exact kernel's, as are those below
     const int64_t M = p.M(), N = p.N(), K = p.K(), B = p.B(), es = (int64_t)dtype_size(p.dtype);
     const bool wide = p.dtype == TFB_F64;
     const double flops = (dtype_is_complex(p.dtype) ? 8.0 : 2.0) * (double)M * (double)N * (double)K * (double)B;
@@ -470,6 +470,9 @@ static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& 
     auto up = [](int64_t x, int64_t to) { return (x + to - 1) / to * to; };
     // Copies as the kernels like them best: [batch][k][rows] for the FP64 pipe, [batch][rows][k] for tcgen05.
     const bool copy[2] = {p.batch[0].s[0] == 1, p.batch[0].s[1] == 1};
+    // A batch index innermost leaves an operand without a tensor map, and contract_tcgen05 copies those of large products only:
+    // smaller ones run on the exact kernel, and do so on the copies (relative error of 1000 of 100^3 1.8e-7, as 3xTF32 8.7e-7).
+    const bool exact = p.dtype == TFB_F32 && (copy[0] || copy[1]) && 2.0 * (double)M * (double)N * (double)K < kTcCopyFlops;
     const int64_t rows[2] = {M, N};
     int64_t ld[3], per[3], bytes = 0;
     for (int t = 0; t < 2; ++t) {
@@ -546,7 +549,7 @@ static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& 
             TFB_TRY(launch_permute(ctx, p.dtype, nest[t], x, blk[t].ptr, Scalar{1.0, 0.0}, Scalar{0.0, 0.0}, false, t == 1 && copy[0]));
             x = blk[t].ptr;
         }
-        TFB_TRY(launch_contract(ctx, q, CK_AUTO, used));
+        TFB_TRY(launch_contract(ctx, q, exact ? CK_SIMT : CK_AUTO, used));
         TFB_TRY(launch_permute(ctx, p.dtype, nest[2], blk[2].ptr, (char*)p.c + b0 * es, p.alpha, p.beta, false));
     }
     *done = true;

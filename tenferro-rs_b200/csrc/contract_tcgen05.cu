@@ -1874,7 +1874,7 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
     PoolBlock packed_a, packed_b;
     // Large products only: repack an operand that has no tensor map, or whose tiles would be
     // more than a third padding.
-    if (!c_tables && 2.0 * M * N * K >= 1e9 && p.batch.size() <= 1 && p.k.size() <= 2) {
+    if (!c_tables && 2.0 * M * N * K >= kTcCopyFlops && p.batch.size() <= 1 && p.k.size() <= 2) {
         auto wasteful = [](const OperandMap& o, int64_t total, int rows) {
             if (!o.ok) return true;
             if (o.geom.pack) return false;

@@ -218,3 +218,22 @@ def test_batch_innermost(tb, oracle, monkeypatch, notation, sizes, dtype):
 def test_batch_innermost_in_more_modes_than_a_pass_takes(tb, oracle, notation, sizes):
     shapes = [tuple(sizes.get(c, 2) for c in t) for t in notation.split("->")[0].split(",")]
     run(tb, oracle, notation, shapes, np.float64, False, 0.5)
+
+
+@pytest.mark.parametrize("notation,sizes", [
+    ("bij,bjk->bik", dict(b=1000, i=100, j=100, k=100)),
+    ("bij,bkj->bki", dict(b=8, i=600, j=600, k=600)),
+    ("bij,jkb->bik", dict(b=33, i=257, j=700, k=120)),
+])
+def test_small_f32_products_stay_exact(tb, oracle, monkeypatch, notation, sizes):
+    """Products too small for their operands to be copied for 3xTF32 (1e9 operations each) keep the exact kernel's error,
+    which the cut of K moves by a few per cent at most; that of 3xTF32 is three to five times as large."""
+    assert 2 * np.prod([float(v) for v in sizes.values()]) >= 1e9 > 2.0 * sizes["i"] * sizes["j"] * sizes["k"]
+    a, b = (oracle.normal(7 + t, tuple(sizes[c] for c in s), np.float32) for t, s in enumerate(notation.split("->")[0].split(",")))
+    ta, tc = tb.Tensor.from_numpy(a), tb.Tensor.from_numpy(b)
+    want = np.einsum(notation, a.astype(np.float64), b.astype(np.float64), optimize=True)
+    err = []
+    for kernel in ("0", "1"):  # chosen by the library; the exact one
+        monkeypatch.setenv("TFB_FORCE_KERNEL", kernel)
+        err.append(oracle.rel_frobenius(tb.einsum(notation, [ta, tc]).to_numpy(), want))
+    assert err[0] <= 1.1 * err[1]
