@@ -155,10 +155,9 @@ struct HView {
 tfb_status to_hview(const tfb_view& v, int dtype, HView* out, const char* what);
 
 // ------------------------------------------------------------ kernel entry points (host launchers)
-// out[idx_out] = alpha * (conj?)in[idx_in] + beta * out[idx_out] over nest (tensor 0 = in, 1 = out).  `beside`: may run at
-// the same time as the launch just ahead of it, which was another permutation and shares no output with this one.
+// out[idx_out] = alpha * (conj?)in[idx_in] + beta * out[idx_out] over nest (tensor 0 = in, 1 = out).
 tfb_status launch_permute(tfb_ctx* ctx, int dtype, const LoopNest& nest, const void* in, void* out, Scalar alpha,
-                          Scalar beta, bool conj, bool beside = false);
+                          Scalar beta, bool conj);
 // out = alpha * a * b + beta * out (tensors 0,1 = a,b; 2 = out).
 tfb_status launch_elementwise_mul(tfb_ctx* ctx, int dtype, const LoopNest& nest, const void* a, const void* b,
                                   void* out, Scalar alpha, Scalar beta, bool conj_a, bool conj_b);

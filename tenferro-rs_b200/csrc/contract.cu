@@ -546,7 +546,7 @@ static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& 
         for (int t = 0; t < 2; ++t) {
             if (!copy[t]) continue;
             const void*& x = t == 0 ? q.a : q.b;
-            TFB_TRY(launch_permute(ctx, p.dtype, nest[t], x, blk[t].ptr, Scalar{1.0, 0.0}, Scalar{0.0, 0.0}, false, t == 1 && copy[0]));
+            TFB_TRY(launch_permute(ctx, p.dtype, nest[t], x, blk[t].ptr, Scalar{1.0, 0.0}, Scalar{0.0, 0.0}, false));
             x = blk[t].ptr;
         }
         TFB_TRY(launch_contract(ctx, q, exact ? CK_SIMT : CK_AUTO, used));

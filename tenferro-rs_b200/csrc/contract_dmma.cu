@@ -583,7 +583,7 @@ static tfb_status repack_for_tma(tfb_ctx* ctx, const ContractProblem& p, const C
         if ((int)modes.size() > kMaxRank) return TFB_OK;
         LoopNest nest;
         TFB_TRY(make_nest(modes, &nest));
-        TFB_TRY(launch_permute(ctx, p.dtype, nest, t == 0 ? p.a : p.b, dst, Scalar{1.0, 0.0}, Scalar{0.0, 0.0}, false, t == 1 && need[0]));
+        TFB_TRY(launch_permute(ctx, p.dtype, nest, t == 0 ? p.a : p.b, dst, Scalar{1.0, 0.0}, Scalar{0.0, 0.0}, false));
         std::vector<Mode>& free_q = t == 0 ? q->m : q->n;
         free_q.assign(1, Mode{ld[t], {0, 0, 0, 0}});
         free_q[0].s[t] = 1;

@@ -1358,13 +1358,10 @@ struct RepackArgs {
     int64_t rows, K, Kp, B;
     int src_kfast;
     float* dst;
-    bool beside;  // runs beside the other operand's copy (launch_begin)
 };
 constexpr int kRepackTile = 64;
-__global__ void __launch_bounds__(256) repack_kmajor_kernel(RepackArgs g) {
+__device__ __forceinline__ void repack_kmajor(const RepackArgs g, float (&tile)[kRepackTile][kRepackTile + 1]) {
     constexpr int T = kRepackTile;
-    __shared__ float tile[T][T + 1];
-    launch_begin(g.beside);
     const int64_t tiles_r = (g.rows + T - 1) / T, tiles_k = (g.Kp + T - 1) / T;
     const int64_t n_tiles = tiles_r * tiles_k * g.B;
     const int tx = threadIdx.x & (T - 1), ty = threadIdx.x / T;  // 64 x 4
@@ -1398,7 +1395,17 @@ __global__ void __launch_bounds__(256) repack_kmajor_kernel(RepackArgs g) {
         }
         __syncthreads();
     }
-    launch_end(g.beside);
+}
+__global__ void __launch_bounds__(256) repack_kmajor_kernel(RepackArgs g) {
+    __shared__ float tile[kRepackTile][kRepackTile + 1];
+    launch_begin();
+    repack_kmajor(g, tile);
+}
+__global__ void __launch_bounds__(256) repack_both_kernel(RepackArgs a, RepackArgs b) {
+    __shared__ float tile[kRepackTile][kRepackTile + 1];
+    launch_begin();
+    const RepackArgs g = blockIdx.y == 0 ? a : b;
+    repack_kmajor(g, tile);
 }
 
 // ------------------------------------------------------------------ host side
@@ -1901,7 +1908,9 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
             ContractArgs ca;
             fill_args(p, t.get(), &ca);
             const int64_t Kp = (K + 3) / 4 * 4, Bn = p.B();
-            bool ahead = false;  // the other operand's copy is the launch ahead
+            RepackArgs job[2];
+            int n_jobs = 0;
+            int64_t tiles[2] = {0, 0};
             auto repack = [&](int tns, PoolBlock* blk, OperandMap* out) -> tfb_status {
                 const int64_t rows = tns == 0 ? M : N;
                 const tfb_status got = blk->alloc(ctx, (size_t)(rows * Kp * Bn) * sizeof(float));
@@ -1909,15 +1918,10 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
                     if (tns == 0 ? opt_a : opt_b) return TFB_OK;  // no room for a copy that only saves time
                     return got;
                 }
-                RepackArgs r{(const float*)(tns == 0 ? p.a : p.b), tns == 0 ? t->a_m : t->b_n, tns == 0 ? t->a_k : t->b_k,
-                             tns == 0 ? t->a_b : t->b_b, rows, K, Kp, Bn, tns == 0 ? ca.a_kfast : ca.b_kfast, (float*)blk->ptr, ahead};
-                const int64_t n_tiles = ((rows + kRepackTile - 1) / kRepackTile) * ((Kp + kRepackTile - 1) / kRepackTile) * Bn;
-                {
-                    LaunchScope ls(ctx, "repack_operand");
-                    const unsigned grid = (unsigned)std::min<int64_t>(n_tiles, (int64_t)ctx->sm_count * 16);
-                    TFB_CUDA(launch_overlapped(ctx, repack_kmajor_kernel, dim3(grid), dim3(256), 0, 0u, r));
-                    ahead = true;
-                }
+                tiles[n_jobs] = ((rows + kRepackTile - 1) / kRepackTile) * ((Kp + kRepackTile - 1) / kRepackTile) * Bn;
+                job[n_jobs++] =
+                    RepackArgs{(const float*)(tns == 0 ? p.a : p.b), tns == 0 ? t->a_m : t->b_n, tns == 0 ? t->a_k : t->b_k,
+                               tns == 0 ? t->a_b : t->b_b, rows, K, Kp, Bn, tns == 0 ? ca.a_kfast : ca.b_kfast, (float*)blk->ptr};
                 // the same product with this operand contiguous: one free mode, K split as in the other operand
                 ContractProblem q = p;
                 std::vector<Mode> free_q{Mode{rows, {0, 0, 0}}};
@@ -1932,6 +1936,20 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
             if (pack_b) {
                 TFB_TRY(repack(1, &packed_b, &b));
                 narrow(&b);
+            }
+            // Small copies are bound by latency and run side by side in one launch; larger ones fill the chip one by one, in a
+            // kernel that keeps one operand's parameters (us in one launch, in two: 801 x 805 x 803, 338 tiles, 35.8, 38.2; 4001 x
+            // 4003 x 303, 630, 91.2, 93.7; 1401 x 1405 x 1403, 968, 60.2, 58.8; 4001 x 4003 x 2999, 5922, 456, 447).
+            auto blocks = [&](int64_t t) { return (unsigned)std::min<int64_t>(t, (int64_t)ctx->sm_count * 16); };
+            if (n_jobs == 2 && tiles[0] + tiles[1] <= (int64_t)ctx->sm_count * 5) {
+                LaunchScope ls(ctx, "repack_operand");
+                TFB_CUDA(launch_overlapped(ctx, repack_both_kernel, dim3(blocks(std::max(tiles[0], tiles[1])), 2), dim3(256), 0, 0u, job[0],
+                                           job[1]));
+            } else {
+                for (int j = 0; j < n_jobs; ++j) {
+                    LaunchScope ls(ctx, "repack_operand");
+                    TFB_CUDA(launch_overlapped(ctx, repack_kmajor_kernel, dim3(blocks(tiles[j])), dim3(256), 0, 0u, job[j]));
+                }
             }
         }
     }

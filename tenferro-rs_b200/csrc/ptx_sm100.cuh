@@ -46,16 +46,11 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, int* st
 // here for the end of it (all its writes visible); without such a launch both are no-ops.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// First statement of a kernel for launch_overlapped that reads or writes global memory after it only.  `beside`: it does
-// not wait for the kernel just ahead of it but runs at the same time; that one had waited for everything before
-// it when it let this one start, and with launch_end as its last statement whoever waits for the end of this kernel waits
-// for the end of both.
-__device__ __forceinline__ void launch_begin(bool beside = false) {
-    if (!beside) grid_dependency_wait();
+// Part of every kernel for launch_overlapped, ahead of its first access to global memory.  Writes of earlier launches are
+// visible after the wait only, so there is no kernel without it.
+__device__ __forceinline__ void launch_begin() {
+    grid_dependency_wait();
     grid_launch_dependents();
-}
-__device__ __forceinline__ void launch_end(bool beside) {
-    if (beside) grid_dependency_wait();
 }
 
 // Reads of another CTA's shared memory (addresses from map_to_cta).

@@ -128,7 +128,6 @@ template <typename T>
 struct EpilogueArgs {
     T alpha, beta;
     bool plain, read_out, conj, alpha_one;
-    bool beside = false;  // the launch runs beside the one ahead of it (launch_begin)
     static EpilogueArgs make(Scalar a, Scalar b, bool cj) {
         EpilogueArgs e;
         e.alpha = Ops<T>::from(a);

@@ -96,7 +96,7 @@ __device__ __forceinline__ void divide_inner(const Nest32& n, int64_t, int64_t u
 template <typename T, typename N>
 __global__ void __launch_bounds__(256) permute_generic_kernel(N nest, const T* __restrict__ in, T* out,
                                                               EpilogueArgs<T> ep) {
-    launch_begin(ep.beside);
+    launch_begin();
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < nest.total; idx += stride) {
         int64_t off[2];
@@ -104,7 +104,6 @@ __global__ void __launch_bounds__(256) permute_generic_kernel(N nest, const T* _
         T v = in[off[0]];
         out[off[1]] = ep.apply(v, out + off[1]);
     }
-    launch_end(ep.beside);
 }
 
 // Row path: mode 0 has stride 1 in both tensors.  V elements per thread move as one 16-byte
@@ -112,7 +111,7 @@ __global__ void __launch_bounds__(256) permute_generic_kernel(N nest, const T* _
 template <typename T, int V, typename N>
 __global__ void __launch_bounds__(256) permute_rows_kernel(N nest, const T* __restrict__ in, T* out,
                                                            EpilogueArgs<T> ep) {
-    launch_begin(ep.beside);
+    launch_begin();
     // One "unit" = V consecutive elements of mode 0.
     const int64_t units = nest.total / V;
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -153,7 +152,6 @@ __global__ void __launch_bounds__(256) permute_rows_kernel(N nest, const T* __re
             *reinterpret_cast<Pack<T, V>*>(dst) = o;
         }
     }
-    launch_end(ep.beside);
 }
 
 // CTAs of a kernel whose threads take up to four units each: one unit while the chip has room for all of them at
@@ -177,7 +175,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) permute_tiled_kernel(LoopNest nest, const T* __restrict__ in, T* out,
                                                             EpilogueArgs<T> ep, int64_t tiles_i, int64_t tiles_j,
                                                             int64_t n_tiles, int64_t strip, int64_t strips) {
-    launch_begin(ep.beside);
+    launch_begin();
     constexpr int kTile = TileOf<T>::value;
     constexpr int kStep = 256 / kTile;
     // Odd pitch: a column walk hits distinct banks.
@@ -218,7 +216,6 @@ __global__ void __launch_bounds__(256) permute_tiled_kernel(LoopNest nest, const
         }
         __syncthreads();
     }
-    launch_end(ep.beside);
 }
 
 // Tile path, for any order of any number of modes.  The modes are split into a run R that has unit stride in both
@@ -263,7 +260,7 @@ struct TilePlan {
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) permute_tile_kernel(const __grid_constant__ TilePlan p, const T* __restrict__ in, T* out,
                                                            EpilogueArgs<T> ep) {
-    launch_begin(ep.beside);
+    launch_begin();
     constexpr int L = kPatch<T> / 256;
     __shared__ T patch[kPatch<T> + kSide];
     __shared__ int32_t in_i[kSide], in_j[kSide], out_i[kSide], out_j[kSide];
@@ -333,7 +330,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) permute_tile_kern
         }
         __syncthreads();
     }
-    launch_end(ep.beside);
 }
 
 // Fits the tile path to a nest in output order (mode 0 fastest); false where another path is the better one.
@@ -432,7 +428,7 @@ template <typename T, int V, int MINB>
 __global__ void __launch_bounds__(256, MINB) permute_tiled_vec_kernel(LoopNest nest, const T* __restrict__ in, T* out,
                                                                 EpilogueArgs<T> ep, int64_t tiles_i, int64_t tiles_j,
                                                                 int64_t n_tiles) {
-    launch_begin(ep.beside);
+    launch_begin();
     constexpr int TILE = 64, VPR = TILE / V, LOADS = TILE * TILE / V / 256;
     __shared__ T tile[TILE][TILE + 1];  // tile[i][j]
     for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
@@ -475,14 +471,12 @@ __global__ void __launch_bounds__(256, MINB) permute_tiled_vec_kernel(LoopNest n
         }
         __syncthreads();
     }
-    launch_end(ep.beside);
 }
 
 template <typename T>
 static tfb_status permute_typed(tfb_ctx* ctx, const LoopNest& nest_out_order, const void* in, void* out, Scalar alpha,
-                                Scalar beta, bool conj, bool beside) {
+                                Scalar beta, bool conj) {
     EpilogueArgs<T> ep = EpilogueArgs<T>::make(alpha, beta, conj);
-    ep.beside = beside;
     LoopNest nest = nest_out_order;
     if (nest.total == 0) return TFB_OK;
     const int sms = ctx->sm_count;
@@ -594,13 +588,13 @@ static tfb_status permute_typed(tfb_ctx* ctx, const LoopNest& nest_out_order, co
 }
 
 tfb_status launch_permute(tfb_ctx* ctx, int dtype, const LoopNest& nest, const void* in, void* out, Scalar alpha,
-                          Scalar beta, bool conj, bool beside) {
+                          Scalar beta, bool conj) {
     DeviceGuard g(ctx->device);
     switch (dtype) {
-        case TFB_F32: return permute_typed<float>(ctx, nest, in, out, alpha, beta, conj, beside);
-        case TFB_F64: return permute_typed<double>(ctx, nest, in, out, alpha, beta, conj, beside);
-        case TFB_C32: return permute_typed<float2>(ctx, nest, in, out, alpha, beta, conj, beside);
-        case TFB_C64: return permute_typed<double2>(ctx, nest, in, out, alpha, beta, conj, beside);
+        case TFB_F32: return permute_typed<float>(ctx, nest, in, out, alpha, beta, conj);
+        case TFB_F64: return permute_typed<double>(ctx, nest, in, out, alpha, beta, conj);
+        case TFB_C32: return permute_typed<float2>(ctx, nest, in, out, alpha, beta, conj);
+        case TFB_C64: return permute_typed<double2>(ctx, nest, in, out, alpha, beta, conj);
     }
     return fail(TFB_ERR_INVALID_ARGUMENT, "unknown dtype %d", dtype);
 }

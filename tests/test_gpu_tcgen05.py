@@ -385,3 +385,28 @@ def test_complex64_narrow_rows_exchange_roles(tb, oracle, shape):
     tb.einsum_into("ik,kj->ij", [ta, tb_], 0.5 - 0.25j, 2.0, tc)
     want = (0.5 - 0.25j) * (a.astype(np.complex128) @ b.astype(np.complex128)) + 2.0 * c0.astype(np.complex128)
     assert oracle.rel_frobenius(tc.to_numpy(), want) <= 1e-5, shape
+
+
+@pytest.mark.parametrize("notation,sizes,launches", [
+    ("ij,jk->ik", dict(i=1001, j=1003, k=1005), 1),  # 512 tiles of 64 x 64: together
+    ("ijkl,klmn->ijmn", dict(i=45, j=43, k=37, l=31, m=47, n=41), 2),
+])
+def test_copies_of_both_operands(tb, oracle, notation, sizes, launches):
+    """Small copies run side by side in one launch, which waits for the writes of the launches ahead like any other: both
+    operands are written by the calls just before."""
+    ctx = tb.Context.get(0)
+    ops = [oracle.normal(60 + t, tuple(sizes[c] for c in s), np.float32) for t, s in enumerate(notation.split("->")[0].split(","))]
+    held = [tb.Tensor.from_numpy(x).permute(list(range(x.ndim))[::-1]) for x in ops]
+    want = oracle.np_einsum(notation, ops)
+    for _ in range(2):
+        ctx.profile_begin()
+        fresh = [h.contiguous().permute(list(range(h.ndim()))[::-1]) for h in held]
+        got = tb.einsum(notation, fresh)
+        ctx.synchronize()
+        count = ctx.profile_read("repack_operand")[0]
+        ctx.profile_end()
+        assert count == launches
+        # without the profile's events between the launches
+        fresh = [h.contiguous().permute(list(range(h.ndim()))[::-1]) for h in held]
+        for out in (got, tb.einsum(notation, fresh)):
+            assert oracle.rel_frobenius(out.to_numpy(), want) <= 1e-5

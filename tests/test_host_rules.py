@@ -1,6 +1,7 @@
 """Decisions of the host side at sizes no test can allocate: which operands a tensor map describes.  The rules
 are plain host code (no CUDA call); tests/host_rules.cpp gives them C entry points."""
 import ctypes as C
+import re
 import subprocess
 from pathlib import Path
 
@@ -76,3 +77,18 @@ def test_every_tile_is_dealt_once(rules, dtype, balance):
     for k in (2**32 - 1, 5_800_000_000, 2**34, 2**40):
         deal(rules, dtype, [(1, 1, k), (1, 1, 8), (70, 64, 64), (33, 90, k), (16, 16, 16)], balance)
         deal(rules, dtype, [(2, 3, k)], balance)
+
+
+# ---------------------------------------------------------------- kernels that start while the one ahead still runs
+def test_every_overlapped_kernel_waits(rules):
+    """Writes of the launches ahead are visible after griddepcontrol.wait: a kernel started by launch_overlapped has it,
+    unconditionally and in the body of the kernel itself."""
+    text = "\n".join(p.read_text() for p in sorted([*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")]))
+    started = set(re.findall(r"launch_overlapped\(\s*ctx,\s*(\w+)", text))
+    assert len(started) > 15
+    bodies = {}
+    for m in re.finditer(r"__global__[^;{]*?\b(\w+_kernel)\s*\(", text):
+        end = text.index("\n}", m.end())
+        bodies[m.group(1)] = text[m.start():end]
+    for kernel in started:
+        assert re.search(r"^    launch_begin\(\);", bodies[kernel], re.M), kernel
