@@ -45,13 +45,12 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, int* st
 // Programmatic dependent launch.  A kernel that starts before the one ahead of it in the stream has finished waits
 // here for the end of it (all its writes visible); without such a launch both are no-ops.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Part of every kernel for launch_overlapped, ahead of its first access to global memory.  Writes of earlier launches are
-// visible after the wait only, so there is no kernel without it.
-__device__ __forceinline__ void launch_begin() {
-    grid_dependency_wait();
-    grid_launch_dependents();
-}
+// visible after the wait only, so there is no kernel without it.  No kernel lets the next one start before its own blocks are
+// through: blocks that wait take shared memory and registers from those that compute (us a call, with such a start and
+// without: complex double 'efcab,efd->abcd' of 64 x 116 x 17136 100, 68; f32 'bagfc,dgef->ebcad' of 2520 x 1810 x 8272 with a batch
+// of five 695, 630; 97 x 194 x 97 complex double 13.4 both).
+__device__ __forceinline__ void launch_begin() { grid_dependency_wait(); }
 
 // Reads of another CTA's shared memory (addresses from map_to_cta).
 __device__ __forceinline__ double cluster_load_d(uint32_t addr) {
