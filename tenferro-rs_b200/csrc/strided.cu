@@ -94,7 +94,7 @@ __device__ __forceinline__ void divide_inner(const Nest32& n, int64_t, int64_t u
 // General path: linear over the nest in OUTPUT order (mode 0 = output's fastest), so writes
 // coalesce; reads are whatever the input strides give.
 template <typename T, typename N>
-__global__ void __launch_bounds__(256) permute_generic_kernel(N nest, const T* __restrict__ in, T* out,
+__global__ void __launch_bounds__(256) permute_generic_kernel(N nest, const T* in, T* out,
                                                               EpilogueArgs<T> ep) {
     launch_begin();
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(256) permute_generic_kernel(N nest, const T* _
 // Row path: mode 0 has stride 1 in both tensors.  V elements per thread move as one 16-byte
 // access when `vec` holds (alignment checked on the host).
 template <typename T, int V, typename N>
-__global__ void __launch_bounds__(256) permute_rows_kernel(N nest, const T* __restrict__ in, T* out,
+__global__ void __launch_bounds__(256) permute_rows_kernel(N nest, const T* in, T* out,
                                                            EpilogueArgs<T> ep) {
     launch_begin();
     // One "unit" = V consecutive elements of mode 0.
@@ -172,7 +172,7 @@ struct TileOf {
     static constexpr int value = sizeof(T) >= 16 ? 32 : 64;  // keeps the patch under 48 KB
 };
 template <typename T>
-__global__ void __launch_bounds__(256) permute_tiled_kernel(LoopNest nest, const T* __restrict__ in, T* out,
+__global__ void __launch_bounds__(256) permute_tiled_kernel(LoopNest nest, const T* in, T* out,
                                                             EpilogueArgs<T> ep, int64_t tiles_i, int64_t tiles_j,
                                                             int64_t n_tiles, int64_t strip, int64_t strips) {
     launch_begin();
@@ -258,7 +258,7 @@ struct TilePlan {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) permute_tile_kernel(const __grid_constant__ TilePlan p, const T* __restrict__ in, T* out,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) permute_tile_kernel(const __grid_constant__ TilePlan p, const T* in, T* out,
                                                            EpilogueArgs<T> ep) {
     launch_begin();
     constexpr int L = kPatch<T> / 256;
@@ -425,7 +425,7 @@ static bool plan_tiles(const LoopNest& n, int sms, TilePlan* p) {
 // input's unit stride, 16-byte stores along the output's, every load of a thread issued before
 // the first use (16 KB in flight per CTA; MINB CTAs per SM).  Needs both sides 16-byte aligned.
 template <typename T, int V, int MINB>
-__global__ void __launch_bounds__(256, MINB) permute_tiled_vec_kernel(LoopNest nest, const T* __restrict__ in, T* out,
+__global__ void __launch_bounds__(256, MINB) permute_tiled_vec_kernel(LoopNest nest, const T* in, T* out,
                                                                 EpilogueArgs<T> ep, int64_t tiles_i, int64_t tiles_j,
                                                                 int64_t n_tiles) {
     launch_begin();
@@ -634,7 +634,7 @@ tfb_status launch_scale(tfb_ctx* ctx, int dtype, const LoopNest& nest, void* out
 
 // ------------------------------------------------------------------ element-wise product
 template <typename T>
-__global__ void __launch_bounds__(256) ewmul_kernel(LoopNest nest, const T* __restrict__ a, const T* __restrict__ b,
+__global__ void __launch_bounds__(256) ewmul_kernel(LoopNest nest, const T* a, const T* b,
                                                     T* out, EpilogueArgs<T> ep, bool conj_a, bool conj_b) {
     launch_begin();
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -899,7 +899,7 @@ constexpr int kRedBound = RANK == 0 && std::is_same<N, LoopNest>::value ? 2 : kR
 // tests and neutral elements (496 x 1576 x 16 f32, the maximum over the last index: 30 us, 14 before).
 template <typename T, int OP, bool RED_FAST, int RANK, bool SHORT, typename N>
 __global__ void __launch_bounds__(256, (SHORT ? 4 : kRedBound<T, RANK, N>)) reduce_kernel(const __grid_constant__ N kept, const __grid_constant__ N red,
-                                                     const T* __restrict__ in, T* out, T* partial, unsigned* arrived, int log_g,
+                                                     const T* in, T* out, T* partial, unsigned* arrived, int log_g,
                                                      int64_t chunk, EpilogueArgs<T> ep) {
     launch_begin();
     constexpr int U = SHORT ? 4 : kRedLoads<T>;
@@ -970,7 +970,7 @@ __global__ void __launch_bounds__(256, (SHORT ? 4 : kRedBound<T, RANK, N>)) redu
 
 // Combines the slices of each kept element: TX elements x G threads per block, as above.
 template <typename T, int OP, typename N>
-__global__ void __launch_bounds__(256) reduce_finish_kernel(N kept, const T* __restrict__ partial, T* out, int splits, int log_g,
+__global__ void __launch_bounds__(256) reduce_finish_kernel(N kept, const T* partial, T* out, int splits, int log_g,
                                                             EpilogueArgs<T> ep) {
     launch_begin();
     __shared__ T sh[256];
