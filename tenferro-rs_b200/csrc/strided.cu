@@ -897,7 +897,8 @@ template <typename T, int RANK, typename N>
 constexpr int kRedBound = RANK == 0 && std::is_same<N, LoopNest>::value ? 2 : kRedCtas<T>;
 // SHORT: a thread has no more than eight elements, and four loads in flight: with sixteen most of them would be
 // tests and neutral elements (496 x 1576 x 16 f32, the maximum over the last index: 30 us, 14 before).
-template <typename T, int OP, bool RED_FAST, int RANK, bool SHORT, typename N>
+// ONE: the last block of a group combines its slices.
+template <typename T, int OP, bool RED_FAST, int RANK, bool SHORT, bool ONE, typename N>
 __global__ void __launch_bounds__(256, (SHORT ? 4 : kRedBound<T, RANK, N>)) reduce_kernel(const __grid_constant__ N kept, const __grid_constant__ N red,
                                                      const T* in, T* out, T* partial, unsigned* arrived, int log_g,
                                                      int64_t chunk, EpilogueArgs<T> ep) {
@@ -941,10 +942,10 @@ __global__ void __launch_bounds__(256, (SHORT ? 4 : kRedBound<T, RANK, N>)) redu
             for (int u = 0; u < s; ++u) part[u] = Red<T, OP>::comb(part[u], part[u + s]);
         const T acc = combine_group<T, OP>(part[0], sh, g, G, RED_FAST ? 1 : TX);
         if (g == 0 && ko < kept.total) {
-            if (!partial) out[koff[1]] = ep.apply(acc, out + koff[1]);
+            if (!ONE && !partial) out[koff[1]] = ep.apply(acc, out + koff[1]);
             else partial[(int64_t)blockIdx.y * kept.total + ko] = acc;
         }
-        if (partial && arrived) {
+        if constexpr (ONE) {
             // The block that completes a group's slices combines them, each thread its share in slice order.
             __shared__ bool last;
             __threadfence();
@@ -1054,25 +1055,25 @@ template <typename T, int OP, typename N>
 static void reduce_launch(tfb_ctx* ctx, const N& kept, const N& red, const T* in, T* out, T* partial, const ReduceShape& r,
                           const EpilogueArgs<T>& ep) {
     const dim3 grid(r.grid, (unsigned)r.splits);
-    unsigned* const arrived = r.one_launch ? ctx->arrived : nullptr;
-    auto go = [&](auto rank, auto few) {
+    auto go = [&](auto rank, auto few, auto one) {
         constexpr int RANK = decltype(rank)::value;
-        constexpr bool SHORT = decltype(few)::value;
+        constexpr bool SHORT = decltype(few)::value, ONE = decltype(one)::value;
         if (r.red_fast)
-            launch_overlapped(ctx, reduce_kernel<T, OP, true, RANK, SHORT, N>, grid, dim3(256), 0, 0u, kept, red, in, out, partial, arrived, r.log_g, r.chunk, ep);
+            launch_overlapped(ctx, reduce_kernel<T, OP, true, RANK, SHORT, ONE, N>, grid, dim3(256), 0, 0u, kept, red, in, out, partial, ctx->arrived, r.log_g, r.chunk, ep);
         else
-            launch_overlapped(ctx, reduce_kernel<T, OP, false, RANK, SHORT, N>, grid, dim3(256), 0, 0u, kept, red, in, out, partial, arrived, r.log_g, r.chunk, ep);
+            launch_overlapped(ctx, reduce_kernel<T, OP, false, RANK, SHORT, ONE, N>, grid, dim3(256), 0, 0u, kept, red, in, out, partial, ctx->arrived, r.log_g, r.chunk, ep);
     };
+    auto by_rank = [&](auto few, auto one) {
+        if (red.rank == 1) return go(std::integral_constant<int, 1>{}, few, one);
+        if constexpr (std::is_same<N, Nest32>::value)
+            if (red.rank == 2) return go(std::integral_constant<int, 2>{}, few, one);
+        go(std::integral_constant<int, 0>{}, few, one);
+    };
+    // (a slice has at least 32 elements a thread: none is short)
+    if (r.one_launch) return by_rank(std::false_type{}, std::true_type{});
     if constexpr (std::is_same<N, Nest32>::value)
-        if (r.chunk <= (int64_t)8 << r.log_g) {
-            if (red.rank == 1) return go(std::integral_constant<int, 1>{}, std::true_type{});
-            if (red.rank == 2) return go(std::integral_constant<int, 2>{}, std::true_type{});
-            return go(std::integral_constant<int, 0>{}, std::true_type{});
-        }
-    if (red.rank == 1) return go(std::integral_constant<int, 1>{}, std::false_type{});
-    if constexpr (std::is_same<N, Nest32>::value)
-        if (red.rank == 2) return go(std::integral_constant<int, 2>{}, std::false_type{});
-    go(std::integral_constant<int, 0>{}, std::false_type{});
+        if (r.chunk <= (int64_t)8 << r.log_g) return by_rank(std::true_type{}, std::false_type{});
+    by_rank(std::false_type{}, std::false_type{});
 }
 template <typename T, int OP, typename N>
 static void reduce_finish_launch(tfb_ctx* ctx, const N& kept, T* out, const T* partial, const ReduceShape& r,
