@@ -44,11 +44,8 @@ struct EmbedArgs {
     float* dst;              // embed: [B][2 rows][ld], else [B][rows][ld]
 };
 
-// Everything the real product needs, in one launch: the operands' jobs and the output's offset tables.
-struct SetupArgs {
-    EmbedArgs job[2];
-    int n_jobs;
-    // C seen as f32: row 2m + c -> 2 c_m[m] + c, column n -> 2 c_n[n], batch b -> 2 c_b[b]
+// The output's offset tables: C seen as f32, row 2m + c -> 2 c_m[m] + c, column n -> 2 c_n[n], batch b -> 2 c_b[b].
+struct RealTables {
     const int64_t *c_m, *c_n, *c_b;
     int64_t M, N, B;
     int64_t *out_m, *out_n, *out_b;
@@ -56,12 +53,18 @@ struct SetupArgs {
 
 // 32 x 32 (rows x k) patches through shared memory: reads follow the source's unit stride,
 // writes follow k.  embed = 1 writes the 2 x 2 real block of alpha * op(a) per element (two
-// output rows), embed = 0 the element itself.  blockIdx.y: the operands' jobs, then the tables.
-// A few MB each, bound by latency: one launch, and a thread's four loads in flight together.
-__global__ void __launch_bounds__(256) embed_setup_kernel(const __grid_constant__ SetupArgs args) {
+// output rows), embed = 0 the element itself.  blockIdx.y: the tables, the first operand, the second where it is copied.
+// A few MB each, bound by latency: one launch, and a thread's four loads in flight together.  Scattered sources of more than half of
+// L2 are bound by sectors that the next product of the batch, or the next patch, finds in L2 again if not too many are on their
+// way: one load at a time, and a launch for each operand (400 of 52 x 320 x 880, batch innermost: 2510 us as one launch with
+// four loads in flight, 1255 so; 30 of 60^3, which L2 holds, 21 us a call, 26 so).  (Two parameters and a choice rather than an indexed array of them, which is
+// read from memory at each use.)
+template <bool SCATTERED>
+__global__ void __launch_bounds__(256) embed_setup_kernel(EmbedArgs first, EmbedArgs second, RealTables args, int job0) {
     __shared__ float2 tile[32][33];
     launch_begin();
-    if ((int)blockIdx.y == args.n_jobs) {
+    const int job = job0 + (int)blockIdx.y;
+    if (job == 0) {
         const int64_t n = max(2 * args.M, max(args.N, args.B));
         for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
             if (i < 2 * args.M) args.out_m[i] = 2 * args.c_m[i >> 1] + (i & 1);
@@ -70,7 +73,7 @@ __global__ void __launch_bounds__(256) embed_setup_kernel(const __grid_constant_
         }
         return;
     }
-    const EmbedArgs g = args.job[blockIdx.y];
+    const EmbedArgs g = job == 1 ? first : second;
     const int64_t tiles_r = (g.rows + 31) / 32, tiles_k = (g.K + 31) / 32;
     const int64_t n_tiles = tiles_r * tiles_k * g.B;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
@@ -79,19 +82,23 @@ __global__ void __launch_bounds__(256) embed_setup_kernel(const __grid_constant_
         const int64_t tr = t % tiles_r, rest = t / tiles_r, tk = rest % tiles_k, b = rest / tiles_k;
         const int64_t r0 = tr * 32, k0 = tk * 32;
         const float2* src = g.src + g.b_tab[b];
-        float2 v[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        auto load = [&](int j) {
             // (r, k) of this thread's element: tx runs along the source's fast direction
-            const int j = ty + 8 * i;
             const int64_t r = r0 + (g.src_kfast ? j : tx), k = k0 + (g.src_kfast ? tx : j);
-            v[i] = make_float2(0.f, 0.f);
-            if (r < g.rows && k < g.K) v[i] = src[g.row_tab[r] + g.k_tab[k]];
-        }
+            return r < g.rows && k < g.K ? src[g.row_tab[r] + g.k_tab[k]] : make_float2(0.f, 0.f);
+        };
+        auto put = [&](int j, float2 v) {
+            if (g.src_kfast) tile[j][tx] = v; else tile[tx][j] = v;  // tile[r][k]
+        };
+        if constexpr (SCATTERED) {
+#pragma unroll 1
+            for (int j = ty; j < 32; j += 8) put(j, load(j));
+        } else {
+            float2 v[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int j = ty + 8 * i;
-            if (g.src_kfast) tile[j][tx] = v[i]; else tile[tx][j] = v[i];  // tile[r][k]
+            for (int i = 0; i < 4; ++i) v[i] = load(ty + 8 * i);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) put(ty + 8 * i, v[i]);
         }
         __syncthreads();
         for (int j = ty; j < 32; j += 8) {
@@ -144,20 +151,62 @@ bool b_is_real_view(const ContractProblem& p) {
 
 }  // namespace
 
-// The first operand is gathered whatever its order, so rows follow the output - a tile whose rows follow the
-// operand instead stores every element to a sector of its own (the outer-product node of a network with extents
-// 79, 66, 94, 68, 86, 96, 72, 11352 x 6912 x 136 floats: 727 us by the operand's order, 183 by the output's) - and K follows
-// the second operand, which may then be read in place.
+// Bytes that a patch or a tile moves per element of 8 where its lanes run along `g` in tensor t: a sector each unless neighbours
+// share one.
+static double lane_bytes(const std::vector<Mode>& g, int t) {
+    if (g.empty() || std::llabs(g[0].s[t]) != 1) return 32;
+    return std::max(8.0, 32.0 / (double)g[0].extent);
+}
+static double gather_bytes(const ContractProblem& p, const std::vector<Mode>& free, int t) {
+    return std::min(lane_bytes(free, t), lane_bytes(p.k, t));
+}
+
+// What tiles of 128 columns (the second operand's rows) compute over what they keep, where B serves in place with two modes.
+static double in_place_padding(const ContractProblem& p) {
+    if (p.n.size() != 2) return 1;
+    const int64_t e1 = p.n[0].extent;
+    return e1 < 128 && 128 % e1 == 0 ? 1 : (double)((e1 + 127) / 128 * 128) / (double)e1;
+}
+// In place, unless the tiles' padding costs more than the copy: some 8 operations at 100 TFLOP/s per padded element and row
+// against 24 bytes at 5 TB/s (162 rows, K = 16200, 20 of every 128 columns kept: 430 us in place, 95 and a copy of 35; 40 rows,
+// K = 32, 40 of 128 columns: 66 us a call in place, 49 copied).  One contracted mode is read in place as it always was:
+// short, and bound by the output.
+static bool second_in_place(const ContractProblem& p) {
+    if (!b_is_real_view(p) || !env_int("TFB_C32_B_IN_PLACE", 1)) return false;
+    return p.k.size() == 1 || (in_place_padding(p) - 1) * (double)p.M() < 64;
+}
+
+// Rows in the first operand's order or the output's, K in the first operand's or the second's: whatever moves the fewest bytes.
+// The first operand is gathered (and its 2 x 2 blocks written) in any order, so rows by the output cost nothing where the gather's
+// lanes keep a unit stride - a tile whose rows follow the operand instead stores every element to a sector of its own (the
+// outer-product node of a network with extents 79, 66, 94, 68, 86, 96, 72, 11352 x 6912 x 136 floats: 727 us by the operand's
+// order, 183 by the output's) - and K by the second operand spares the copy of that (130 us
+// for 5427 x 5760 elements) unless it scatters the gather of a larger first one ('efdab,fdce->abfc', 2016 x 4428 against 506 x 4428 in
+// eight products: set-up 1096 us by the second operand's order, 504 by the first's).
+static double embedding_bytes(const ContractProblem& p) {
+    const double M = (double)p.M(), N = (double)p.N(), K = (double)p.K();
+    const double second = second_in_place(p) ? 0.4 * (in_place_padding(p) - 1) * M : gather_bytes(p, p.n, 1) + 8;
+    return M * K * (gather_bytes(p, p.m, 0) + 16) + N * K * second + M * N * lane_bytes(p.m, 2);
+}
 static ContractProblem embedding_order(const ContractProblem& p) {
-    ContractProblem q = p;
     auto by = [](std::vector<Mode>& g, int t) {
         for (const Mode& m : g)
             if (m.s[t] == 0) return;
         std::stable_sort(g.begin(), g.end(), [t](const Mode& x, const Mode& y) { return std::llabs(x.s[t]) < std::llabs(y.s[t]); });
     };
-    by(q.m, 2);
-    by(q.k, 1);
-    return q;
+    ContractProblem best;
+    double least = 0;
+    for (int order = 0; order < 4; ++order) {
+        ContractProblem q = p;
+        by(q.m, order & 1 ? 0 : 2);
+        by(q.k, order & 2 ? 0 : 1);
+        const double bytes = embedding_bytes(q);
+        if (order == 0 || bytes < 0.95 * least) {
+            least = bytes;
+            best = q;
+        }
+    }
+    return best;
 }
 
 static tfb_status embedded_product(tfb_ctx* ctx, const ContractProblem& p, bool* declined) {
@@ -172,7 +221,7 @@ static tfb_status embedded_product(tfb_ctx* ctx, const ContractProblem& p, bool*
     ContractArgs ca;
     fill_args(p, t.get(), &ca);
 
-    const bool b_in_place = b_is_real_view(p) && env_int("TFB_C32_B_IN_PLACE", 1);
+    const bool b_in_place = second_in_place(p);
     const size_t a_floats = (size_t)(2 * M * ld * B), b_floats = b_in_place ? 0 : (size_t)(N * ld * B);
     const size_t tab_entries = (size_t)(2 * M + N + B);
     PoolBlock ws;
@@ -183,24 +232,28 @@ static tfb_status embedded_product(tfb_ctx* ctx, const ContractProblem& p, bool*
     int64_t* tab_n = tab_m + 2 * M;
     int64_t* tab_b = tab_n + N;
 
-    SetupArgs setup = {};
-    int64_t most = (std::max<int64_t>(std::max<int64_t>(2 * M, N), B) + 255) / 256;
-    auto job = [&](const void* src, const int64_t* row_tab, const int64_t* k_tab, const int64_t* b_tab, int64_t rows,
-                   int kfast, bool conj, bool emb, float2 alpha, float* dst) {
-        setup.job[setup.n_jobs++] =
-            EmbedArgs{(const float2*)src, row_tab, k_tab, b_tab, rows, K, B, ld, kfast, conj ? 1 : 0, emb ? 1 : 0, alpha, dst};
-        most = std::max<int64_t>(most, ((rows + 31) / 32) * ((K + 31) / 32) * B);
-    };
+    const int64_t for_tables = (std::max<int64_t>(std::max<int64_t>(2 * M, N), B) + 255) / 256;
+    auto patches = [&](int64_t rows) { return ((rows + 31) / 32) * ((K + 31) / 32) * B; };
     const float2 alpha = make_float2((float)p.alpha.re, (float)p.alpha.im);
-    job(p.a, t->a_m, t->a_k, t->a_b, M, ca.a_kfast, p.conj_a, true, alpha, a_real);
-    if (!b_in_place) job(p.b, t->b_n, t->b_k, t->b_b, N, ca.b_kfast, p.conj_b, false, make_float2(1.f, 0.f), b_real);
-    setup.c_m = t->c_m; setup.c_n = t->c_n; setup.c_b = t->c_b;
-    setup.M = M; setup.N = N; setup.B = B;
-    setup.out_m = tab_m; setup.out_n = tab_n; setup.out_b = tab_b;
-    {
+    const EmbedArgs first{(const float2*)p.a, t->a_m, t->a_k, t->a_b, M, K, B, ld, ca.a_kfast, p.conj_a, 1, alpha, a_real};
+    const EmbedArgs second{(const float2*)p.b, t->b_n, t->b_k, t->b_b, N, K, B, ld, ca.b_kfast, p.conj_b, 0, make_float2(1.f, 0.f), b_real};
+    const RealTables tables{t->c_m, t->c_n, t->c_b, M, N, B, tab_m, tab_n, tab_b};
+    auto scattered = [&](const std::vector<Mode>& g, int t, int64_t rows) {
+        return gather_bytes(p, g, t) > 16 && 8.0 * (double)rows * (double)K * (double)B > 64e6;
+    };
+    auto set_up = [&](bool scatters, int64_t blocks, int job0, unsigned jobs) -> tfb_status {
         LaunchScope ls(ctx, "pack_planes");
-        const unsigned grid = (unsigned)std::min<int64_t>(most, (int64_t)ctx->sm_count * 16);
-        TFB_CUDA(launch_overlapped(ctx, embed_setup_kernel, dim3(grid, setup.n_jobs + 1), dim3(256), 0, 0u, setup));
+        const dim3 grid((unsigned)std::min<int64_t>(blocks, (int64_t)ctx->sm_count * 16), jobs);
+        TFB_CUDA(scatters ? launch_overlapped(ctx, embed_setup_kernel<true>, grid, dim3(256), 0, 0u, first, second, tables, job0)
+                          : launch_overlapped(ctx, embed_setup_kernel<false>, grid, dim3(256), 0, 0u, first, second, tables, job0));
+        return TFB_OK;
+    };
+    const bool a_scatters = scattered(p.m, 0, M), b_scatters = !b_in_place && scattered(p.n, 1, N);
+    if (b_in_place || a_scatters || b_scatters) {
+        TFB_TRY(set_up(a_scatters, std::max(for_tables, patches(M)), 0, 2));
+        if (!b_in_place) TFB_TRY(set_up(b_scatters, patches(N), 2, 1));
+    } else {
+        TFB_TRY(set_up(false, std::max({for_tables, patches(M), patches(N)}), 0, 3));
     }
     double beta = p.beta.re;
     if (p.beta.im != 0) {
@@ -241,7 +294,7 @@ static tfb_status embedded_product(tfb_ctx* ctx, const ContractProblem& p, bool*
 // (2M x 2K), and a K-major copy of the second (N x 2K) unless it serves in place.
 static double setup_floats(const ContractProblem& p) {
     const double k2 = 2.0 * (double)p.K() * (double)p.B();
-    return 2.0 * (double)p.M() * k2 + ((b_is_real_view(p) && env_int("TFB_C32_B_IN_PLACE", 1)) ? 0.0 : (double)p.N() * k2);
+    return 2.0 * (double)p.M() * k2 + (second_in_place(p) ? 0.0 : (double)p.N() * k2);
 }
 
 tfb_status contract_c32_embedded(tfb_ctx* ctx, const ContractProblem& p, bool* declined) {

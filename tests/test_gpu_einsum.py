@@ -276,6 +276,32 @@ def test_network_of_unequal_extents(tb, oracle, dims, conj):
     assert oracle.rel_frobenius(got, oracle.np_einsum("ijk,jlm,kmn,lnp->ip", ops)) <= 1e-5
 
 
+@pytest.mark.parametrize("notation,sizes,launches", [
+    ("fade,defbc->acb", dict(a=162, b=20, c=32, d=9, e=11, f=15), 1),  # K in one run of the second operand: copied all the same
+    ("fade,defbc->acb", dict(a=34, b=32, c=9, d=4, e=5, f=3), 1),      # ... and read in place, its tiles are full
+    ("efdab,fdce->abfc", dict(a=24, b=14, c=106, d=7, e=64, f=8), 1),  # K by the second operand would scatter the first
+    ("bji,bjk->bik", dict(b=31, i=33, j=880, k=320), 2),               # a scattered operand of 70 MB
+    ("bji,kbj->ikb", dict(b=45, i=320, j=640, k=35), 2),
+])
+@pytest.mark.parametrize("conj", [False, True])
+def test_complex_single_orders(tb, oracle, notation, sizes, launches, conj):
+    """Whichever operand's order rows and K follow, and whether an operand is copied with the other or by itself."""
+    ops = [oracle.normal(70 + t, tuple(sizes[c] for c in s), np.complex64) for t, s in enumerate(notation.split("->")[0].split(","))]
+    held = [tb.Tensor.from_numpy(o) for o in ops]
+    if conj:
+        held[0], ops[0] = held[0].into_conj(), ops[0].conj()
+    want = 0.5 * oracle.normal(79, tuple(sizes[c] for c in notation.split("->")[1]), np.complex64)
+    out = tb.Tensor.from_numpy(want)
+    want = 0.5 * want + oracle.np_einsum(notation, ops)
+    ctx = tb.Context.get(0)
+    ctx.profile_begin()
+    tb.einsum_into(notation, held, 1.0, 0.5, out)
+    ctx.synchronize()
+    assert ctx.profile_read("pack_planes")[0] == launches
+    ctx.profile_end()
+    assert oracle.rel_frobenius(out.to_numpy(), want) <= 1e-5
+
+
 def test_config5_scaled(tb, oracle):
     """'ijkl,klmn->ijmn', f32, i=j=m=n=32, k=l=64 (128 / 256 in the benchmark), N(0,1)."""
     a, b = oracle.normal(5000, (32, 32, 64, 64), np.float32), oracle.normal(5001, (64, 64, 32, 32), np.float32)
