@@ -454,10 +454,11 @@ tfb_status contract_simt_semiring(tfb_ctx* ctx, const ContractProblem& p, int al
 // writes a tile of one of them touches a 32-byte sector per element, and reads its operands the same way.  From
 // the size on that repays copies at all, the operands that lie so are copied with the batch outermost, the
 // products go to a block of their own, and one pass over that applies alpha and beta and puts the batch back innermost: all
-// of it tiled permutations at the memory's rate.  Chunks of the batch keep the copies to about 1 GB.
-// (us before and now: f32, 484 of 736 x 824 x 1044 26100, 4650, the exact kernel 1000 of 100^3 380, 233, 8 of 600^3 255, 227; double, 484 of 736 x
-// 824 x 1044 199000, 23900, 220 of 580 x 408 x 308 2900, 1650, 16 of 600^3 353, 348, 8 of 600^3 186, 200; complex single, 1000 of
-// 100^3 337, 294, 8 of 600^3 167, 177.  Complex double elements are half a sector, and nothing is gained: 64 of 300^3 619, 628.)
+// of it tiled permutations at the memory's rate.
+// (us as they lie and on copies: f32, 100 of 900^3 4640, 1180, the exact kernel 1000 of 100^3 380, 233, 8 of 600^3 255, 227, 477 of 100
+// x 800 x 17 576, 386; double, 220 of 580 x 308 x 408 2340, 1540, 100 of 500 x 500 x 16 838, 167, 16 of 600^3 357, 334; complex
+// single, 1000 of 100^3 332, 260, 100 of 500 x 500 x 16 456, 186.  Complex double elements are half a sector, and nothing is gained:
+// 64 of 300^3 619, 628.)
 static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& p, const char** used, bool* done) {
     *done = false;
     if (p.batch.size() != 1 || p.batch[0].s[2] != 1 || p.batch[0].extent < (p.dtype == TFB_F32 ? 8 : 16) || p.mul || p.dtype == TFB_C64)
@@ -483,8 +484,11 @@ static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& 
     ld[2] = up(M, 8);
     per[2] = ld[2] * up(N, 8);
     bytes += per[2] * es;
-    const int64_t chunk = std::min(B, std::max<int64_t>(32, ((int64_t)1 << 30) / bytes / 32 * 32));
-    if ((double)bytes * (double)chunk > (double)ctx->total_mem / 16) return TFB_OK;
+    // Copies of as many products as a gigabyte holds, whole sectors of the batch (eight) at least: the pool keeps the memory, and more
+    // than a thirty-second of the device's (5.7 GB), as for the copies of a double precision product, is not asked for.
+    const int64_t most = env_int("TFB_BATCH_CHUNK", 0) > 0 ? env_int("TFB_BATCH_CHUNK", 0) : ((int64_t)1 << 30) / bytes;
+    const int64_t chunk = std::min(B, std::max<int64_t>(8, most >= 32 ? most / 32 * 32 : most / 8 * 8));
+    if ((double)bytes * (double)chunk > (double)ctx->total_mem / 32) return TFB_OK;
     auto dense = [](std::vector<Mode>& g, int t, int64_t step) {
         for (Mode& m : g) {
             m.s[t] = step;
@@ -549,7 +553,8 @@ static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& 
             TFB_TRY(launch_permute(ctx, p.dtype, nest[t], x, blk[t].ptr, Scalar{1.0, 0.0}, Scalar{0.0, 0.0}, false));
             x = blk[t].ptr;
         }
-        TFB_TRY(launch_contract(ctx, q, exact ? CK_SIMT : CK_AUTO, used));
+        const tfb_status st = launch_contract(ctx, q, exact ? CK_SIMT : CK_AUTO, used);
+        if (st != TFB_OK) return b0 == 0 ? TFB_OK : st;  // no room for its scratch beside the copies: as the operands lie
         TFB_TRY(launch_permute(ctx, p.dtype, nest[2], blk[2].ptr, (char*)p.c + b0 * es, p.alpha, p.beta, false));
     }
     *done = true;

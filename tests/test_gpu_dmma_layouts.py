@@ -237,3 +237,54 @@ def test_small_f32_products_stay_exact(tb, oracle, monkeypatch, notation, sizes)
         monkeypatch.setenv("TFB_FORCE_KERNEL", kernel)
         err.append(oracle.rel_frobenius(tb.einsum(notation, [ta, tc]).to_numpy(), want))
     assert err[0] <= 1.1 * err[1]
+
+
+# every type on its side of the route's thresholds; chunks of 32 and a last one of 1, 8 and 31 products
+@pytest.mark.parametrize("notation,sizes", [
+    ("bij,bjk->bik", dict(b=65, i=169, j=321, k=300)),
+    ("bij,bkj->bki", dict(b=72, i=331, j=260, k=129)),
+    ("bij,jkb->bik", dict(b=95, i=140, j=205, k=303)),  # the second operand is not copied
+    ("ijb,bjk->bik", dict(b=95, i=303, j=205, k=140)),
+    ("ijb,jkb->bik", dict(b=65, i=300, j=320, k=304)),  # ... nor the first
+    ("bijx,bjxk->bki", dict(b=65, i=301, j=13, k=300, x=16)),
+])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.complex64])
+@pytest.mark.parametrize("chunk", ["32", "0"])
+def test_batch_innermost_in_chunks(tb, oracle, monkeypatch, notation, sizes, dtype, chunk):
+    """The passes of each chunk are counted: both operands' copies where they lie so, and the output's.  Bounds as above."""
+    work = (8 if dtype is np.complex64 else 2) * np.prod([float(v) for v in sizes.values()])
+    assert work >= (2e8 if dtype is np.float64 else 1e9)
+    monkeypatch.setenv("TFB_BATCH_CHUNK", chunk)
+    terms = notation.split("->")[0].split(",")
+    a, b = (oracle.normal(7 + t, tuple(sizes[c] for c in s), dtype) for t, s in enumerate(terms))
+    c = oracle.normal(9, tuple(sizes[x] for x in notation.split("->")[1]), dtype)
+    ta, tc, out = tb.Tensor.from_numpy(a), tb.Tensor.from_numpy(b).into_conj(), tb.Tensor.from_numpy(c)
+    ctx = tb.Context.get(0)
+    ctx.profile_begin()
+    tb.einsum_into(notation, [ta, tc], 0.75, 0.5, out)
+    ctx.synchronize()
+    passes = sum(ctx.profile_read(k)[0] for k in ("permute_tile", "permute_tiled", "permute_rows", "permute_generic"))
+    ctx.profile_end()
+    chunks = -(-sizes["b"] // 32) if chunk == "32" else 1
+    if dtype is np.float64 and sum(t[0] == "b" for t in terms) < 2:  # one double precision operand in place may be copied besides
+        assert passes >= chunks * (1 + sum(t[0] == "b" for t in terms))
+    else:
+        assert passes == chunks * (1 + sum(t[0] == "b" for t in terms))
+    wide = np.complex128 if np.dtype(dtype).kind == "c" else np.float64
+    want = 0.75 * np.einsum(notation, a.astype(wide), np.conj(b).astype(wide), optimize=True) + 0.5 * c
+    tol = 1e-13 if dtype is np.float64 else 1e-5
+    got = out.to_numpy()
+    assert np.linalg.norm(got - want) <= tol * np.linalg.norm(want)
+    assert np.abs(got - want).max() <= 10 * tol * np.abs(want).max()
+
+
+@pytest.mark.parametrize("n,scratch", [(1000, 1.1e9), (2304, 1.1e9)])
+def test_batch_innermost_memory(tb, n, scratch):
+    """Copies of a gigabyte at most, or of eight products where those take more: the pool holds no more afterwards."""
+    ctx = tb.Context(0)
+    plan = tb.CudaBackend.plan(tb.PrimDescriptor.Contract([0, 1, 2], [0, 2, 3], [0, 1, 3]), [(40, n, n), (40, n, n), (40, n, n)], np.float64, ctx)
+    a, b, c = (tb.Tensor.zeros((40, n, n)) for _ in range(3))
+    tb.Context.get(0).synchronize()
+    tb.CudaBackend.execute(plan, 1.0, [a, b], 0.0, c)
+    ctx.synchronize()
+    assert ctx.pool_stats()[0] <= scratch
