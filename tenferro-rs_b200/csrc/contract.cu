@@ -461,24 +461,34 @@ tfb_status contract_simt_semiring(tfb_ctx* ctx, const ContractProblem& p, int al
 // 64 of 300^3 619, 628.)
 static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& p, const char** used, bool* done) {
     *done = false;
-    if (p.batch.size() != 1 || p.batch[0].s[2] != 1 || p.batch[0].extent < (p.dtype == TFB_F32 ? 8 : 16) || p.mul || p.dtype == TFB_C64)
-        return TFB_OK;
+    if (p.batch.size() != 1 || p.batch[0].s[2] != 1 || p.mul || p.dtype == TFB_C64) return TFB_OK;
+    if (p.batch[0].extent < (p.dtype == TFB_F32 ? 8 : p.dtype == TFB_F64 ? 16 : 32)) return TFB_OK;
     if (p.dtype == TFB_F32 && p.k.size() > 2) return TFB_OK;  // the exact kernel's, as are those below
     const int64_t M = p.M(), N = p.N(), K = p.K(), B = p.B(), es = (int64_t)dtype_size(p.dtype);
     const bool wide = p.dtype == TFB_F64;
     const double flops = (dtype_is_complex(p.dtype) ? 8.0 : 2.0) * (double)M * (double)N * (double)K * (double)B;
     if (M < 64 || N < 64 || K < 16 || flops < (wide ? 2e8 : 1e9)) return TFB_OK;
+    // Long and thin outputs of a short K are bound by their own passes (436 of 105 x 817 x 17 complex single: 874 us as they lie, 1069
+    // on copies; 100 of 500 x 500 x 16 444, 186).
+    if (p.dtype == TFB_C32 && K < 32 && std::max(M, N) > 5 * std::min(M, N)) return TFB_OK;
     auto up = [](int64_t x, int64_t to) { return (x + to - 1) / to * to; };
-    // Copies as the kernels like them best: [batch][k][rows] for the FP64 pipe, [batch][rows][k] for tcgen05.
+    // Copies as the kernels like them best: [batch][k][rows] for the FP64 pipe, [batch][rows][k] for tcgen05.  The first operand of
+    // a complex single product is embedded from either, and by rows it does not offer itself to be read in place with the
+    // roles exchanged, which would take rows across the block (488 of 260 x 80 x 16: 278 us exchanged, 131 so,
+    // 146 as they lie).
     const bool copy[2] = {p.batch[0].s[0] == 1, p.batch[0].s[1] == 1};
     // A batch index innermost leaves an operand without a tensor map, and contract_tcgen05 copies those of large products only:
     // smaller ones run on the exact kernel, and do so on the copies (relative error of 1000 of 100^3 1.8e-7, as 3xTF32 8.7e-7).
     const bool exact = p.dtype == TFB_F32 && (copy[0] || copy[1]) && 2.0 * (double)M * (double)N * (double)K < kTcCopyFlops;
+    // Double precision products whose output stays in L2 find the sectors of their stores there: nothing to gain where an operand is
+    // read in place besides (115 of 784 x 64 x 112, 46 MB: 85 us as they lie, 97 on copies; 533 of them 1105, 376).
+    if (wide && !(copy[0] && copy[1]) && (double)M * (double)N * (double)B * (double)es < 80e6) return TFB_OK;
+    const bool by_rows[2] = {p.dtype != TFB_F32, wide};
     const int64_t rows[2] = {M, N};
     int64_t ld[3], per[3], bytes = 0;
     for (int t = 0; t < 2; ++t) {
-        ld[t] = wide ? up(rows[t], 8) : up(K, 4);
-        per[t] = ld[t] * (wide ? K : rows[t]);
+        ld[t] = by_rows[t] ? up(rows[t], 8) : up(K, 4);
+        per[t] = ld[t] * (by_rows[t] ? K : rows[t]);
         if (copy[t]) bytes += per[t] * es;
     }
     ld[2] = up(M, 8);
@@ -511,8 +521,8 @@ static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& 
             };
             if (t < 2) {
                 std::vector<Mode>& free_q = t == 0 ? q->m : q->n;
-                dense(free_q, t, wide ? 1 : ld[t]);
-                dense(q->k, t, wide ? ld[t] : 1);
+                dense(free_q, t, by_rows[t] ? 1 : ld[t]);
+                dense(q->k, t, by_rows[t] ? ld[t] : 1);
                 put(t == 0 ? p.m : p.n, free_q);
                 put(p.k, q->k);
             } else {
