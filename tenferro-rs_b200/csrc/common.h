@@ -263,7 +263,13 @@ struct LaunchScope {
 // Launches a kernel that waits for the end of the one ahead of it by itself (launch_begin, before it touches
 // global memory), so that its CTAs may be placed and set themselves up meanwhile; `cluster` CTAs
 // (0, 1: none) form a cluster.  Not on the legacy default stream, which orders itself against other streams, and not while
-// capturing, where a plain edge is what a replay needs.
+// the stream is recorded, by this library or by the owner of the stream that it was given, where a plain edge is what a
+// replay needs.
+inline bool is_recorded(const tfb_ctx* ctx) {
+    if (ctx->capturing || ctx->stream == ctx->own_stream) return ctx->capturing;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(ctx->stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone;
+}
 template <typename... P, typename... A>
 cudaError_t launch_overlapped(tfb_ctx* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A&&... args) {
     cudaLaunchConfig_t cfg = {};
@@ -273,7 +279,7 @@ cudaError_t launch_overlapped(tfb_ctx* ctx, void (*kernel)(P...), dim3 grid, dim
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[2];
     unsigned n = 0;
-    if (!ctx->capturing && ctx->stream != nullptr && ctx->stream != cudaStreamLegacy && ctx->stream != cudaStreamPerThread) {
+    if (ctx->stream != nullptr && ctx->stream != cudaStreamLegacy && ctx->stream != cudaStreamPerThread && !is_recorded(ctx)) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n++].val.programmaticStreamSerializationAllowed = 1;
     }

@@ -298,3 +298,46 @@ def test_capture_and_replay_of_a_contraction_sequence(tb, oracle):
     assert oracle.rel_frobenius(out.to_numpy(), np.einsum("abc,bcd->ad", a2, b)) <= 1e-12
     with pytest.raises(tb.InvalidArgument):
         ctx.capture_end()  # not capturing
+
+
+def test_a_recorded_stream_gets_plain_edges(tb, oracle):
+    """The owner of a stream given to set_stream may record it: kernels that follow one another directly on it must end up
+    with full dependencies, as in the library's own capture, and the replay has to give what the direct calls do."""
+    import torch
+    from cuda.bindings import runtime as rt
+
+    def ok(r):
+        assert r[0] == rt.cudaError_t.cudaSuccess, r[0]
+        return r[1:] if len(r) > 2 else r[1] if len(r) == 2 else None
+
+    ctx = tb.Context.get(0)
+    a, b = (tb.Tensor.from_numpy(oracle.normal(1 + t, (128, 128), np.float64)) for t in range(2))
+    x, y = tb.Tensor.zeros((128, 128)), tb.Tensor.zeros((128, 128))
+    tree = tb.ContractionTree.optimize(tb.Subscripts.parse("ij,jk->ik"), [(128, 128), (128, 128)])
+
+    def calls():
+        tb.einsum_with_plan_into(tree, [a, b], 1.0, 0.0, x)
+        tb.einsum_with_plan_into(tree, [x, b], 1.0, 0.0, y)
+
+    calls()
+    want = y.to_numpy()
+    ctx.h2d(y._block.ptr, np.zeros_like(want).ctypes.data, want.nbytes)
+    ctx.synchronize()
+    stream = torch.cuda.Stream()
+    ctx.set_stream(stream.cuda_stream)
+    try:
+        ok(rt.cudaStreamBeginCapture(stream.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeRelaxed))
+        calls()
+        graph = ok(rt.cudaStreamEndCapture(stream.cuda_stream))
+        # this form of the query knows full dependencies only, and reports any other as an error
+        plain, *_, n = rt.cudaGraphGetEdges(graph, 64)
+        run = ok(rt.cudaGraphInstantiate(graph, 0))
+        ok(rt.cudaGraphLaunch(run, stream.cuda_stream))
+        stream.synchronize()
+        ok(rt.cudaGraphExecDestroy(run))
+        ok(rt.cudaGraphDestroy(graph))
+    finally:
+        ctx.set_stream(None)
+    assert plain == rt.cudaError_t.cudaSuccess and n >= 1, plain
+    x.event = y.event = None  # (recorded into the graph: neither to be waited for nor queried)
+    assert np.array_equal(y.to_numpy(), want)
