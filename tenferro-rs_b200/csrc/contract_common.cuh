@@ -52,6 +52,7 @@ struct ContractArgs {
     // TMA-fed DMMA kernel: CTAs of a cluster that share a tile's K (0, 1: none), and the ranges of a cut tile that have
     // parked their sums, counted at the CTA that starts the tile (zero between launches).
     int cluster;
+    int pieces;  // CTAs that share a tile's k-iterations evenly, a cluster or not (0, 1: ranges of iters_per_cta)
     unsigned* sk_arrived;
     int sk_two_phase;    // 1: every range parks its sums in its slot; a finishing kernel adds the pieces of a tile
     // Sums of ranges that cut a tile.  Gather and TMA-fed DMMA kernels: two block tiles per CTA; exact-

@@ -283,9 +283,9 @@ contract_dmma_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
     int64_t it_begin = (int64_t)blockIdx.x * g.iters_per_cta;
     int64_t it_end = min(g.total_iters, it_begin + g.iters_per_cta);
-    const int pieces = g.cluster, piece = pieces > 1 ? (int)(blockIdx.x % (unsigned)pieces) : 0;
+    const int pieces = g.pieces, piece = pieces > 1 ? (int)(blockIdx.x % (unsigned)pieces) : 0;
     if (pieces > 1) {
-        // the CTAs of a cluster share a tile's k-iterations evenly
+        // the CTAs of a tile share its k-iterations evenly
         const int64_t tile_first = (int64_t)(blockIdx.x / (unsigned)pieces) * g.k_iters;
         it_begin = tile_first + g.k_iters * piece / pieces;
         it_end = tile_first + g.k_iters * (piece + 1) / pieces;
@@ -379,7 +379,7 @@ contract_dmma_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                         acc[i][j][2 + e] = p3 - p1 - p2;
                     }
         }
-        if (pieces > 1) {
+        if (g.cluster > 1) {
             // The tile's sums meet in the CTAs' shared memory: each parks its own (the ring is empty: every load
             // that this CTA issued has been consumed), and adds a share of the tile over all of them, in the order
             // of k.
@@ -627,20 +627,16 @@ static tfb_status run_tma_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractAr
     int pieces = 0;
     a.cluster = cluster_pieces<Cfg>(a, slots, fit.clusters);
     if (a.cluster > 1) grid = a.n_tiles * a.cluster;
-    // A handful of tiles with a long K: cut every tile into the same number of k pieces, one CTA
+    // A handful of tiles with a long K: cut every tile into the same number of k pieces, as even as its iterations allow, one CTA
     // each, and add the pieces in a second, tiny launch.  (In one launch the
-    // last range of a tile adds all its pieces - eight dependent round trips to L2 for 32
-    // pieces - and 'abc,bcd->ad' at 64^4 took 16.4 us; here every load of the sum is independent.)
+    // last range of a tile adds all its pieces - dependent round trips to L2 - and 'abc,bcd->ad' at 64^4 took 16.4 us; here every
+    // load of the sum is independent.  us in one launch and so: double, 24 x 1044 x 992 20.5, 17.6, 128 x 128 x 5000 26.6, 19.6, 156 x
+    // 80 x 6752 31.3, 24.5; complex 16 x 12 x 5128 24.6, 20.5.)
     if (!grid && a.n_tiles * 4 <= slots && a.k_iters * Cfg::BK >= 256 && env_int("TFB_SK_TWO_PHASE", 1)) {
         const int64_t want = std::min<int64_t>(std::min<int64_t>(32, slots / a.n_tiles), a.k_iters * Cfg::BK / 64);
-        a.iters_per_cta = (a.k_iters + want - 1) / want;
-        pieces = (int)((a.k_iters + a.iters_per_cta - 1) / a.iters_per_cta);
-        // 32-deep iterations do not deal out as evenly: where fewer pieces than would fit leave a quarter of the SMs idle, the
-        // equal ranges below are ahead (344 x 312 x 280 complex double in 90 pieces of three iterations: 23.8 us, 19.9)
-        if (Cfg::BK > 16 && pieces < want && a.n_tiles * pieces * 4 < slots * 3) pieces = 0;
-        // ranges are per tile: CTA c takes piece c % pieces of tile c / pieces; the kernel cuts the linear (tile, k)
-        // space into equal ranges, so pieces must divide K's iterations
-        if (a.iters_per_cta * pieces != a.k_iters || pieces < 2) pieces = 0;
+        // (32-deep iterations do not deal out as evenly: where the longest piece is longer than the equal ranges below, those are
+        // ahead: 344 x 312 x 280 complex double in 90 pieces of three iterations 23.8 us, 19.9)
+        if (want >= 2 && (Cfg::BK <= 16 || (a.k_iters + want - 1) / want <= (a.total_iters + slots - 1) / slots)) pieces = (int)want;
         if (pieces) {
             grid = a.n_tiles * pieces;
             a.sk_two_phase = 1;
@@ -660,7 +656,8 @@ static tfb_status run_tma_cfg(tfb_ctx* ctx, const ContractProblem& p, ContractAr
         }
         grid = (a.total_iters + a.iters_per_cta - 1) / a.iters_per_cta;
     }
-    if (a.cluster <= 1 && a.iters_per_cta % a.k_iters != 0) {
+    a.pieces = a.cluster > 1 ? a.cluster : pieces;
+    if (a.sk_two_phase || (a.cluster <= 1 && a.iters_per_cta % a.k_iters != 0)) {
         // Scratch slots and counters live with the context and are reused by every launch (a counter is back at zero
         // when its tile is finished, so a replayed launch finds what a direct one does).
         // As large as any configuration asks for from the start (38 MB): a captured launch keeps the address.  Where the

@@ -164,6 +164,11 @@ def test_complex_tiles(tb, oracle, notation, sizes, conj):
     (np.float64, (32, 36, 128)),   # one iteration per CTA
     (np.float64, (228, 252, 260)),
     (np.float64, (448, 452, 1028)),  # ranges that cut tiles
+    (np.float64, (24, 1044, 992)),   # four pieces of 15 or 16 iterations
+    (np.float64, (128, 128, 5004)),
+    (np.float64, (60, 60, 260)),     # four pieces of 17 iterations
+    (np.complex128, (16, 12, 5128)),
+    (np.complex128, (30, 66, 1000)),
     (np.complex128, (64, 128, 64)),
     (np.complex128, (98, 196, 100)),
     (np.complex128, (258, 322, 324)),
