@@ -455,7 +455,7 @@ tfb_status contract_simt_semiring(tfb_ctx* ctx, const ContractProblem& p, int al
 // the size on that repays copies at all, the operands that lie so are copied with the batch outermost, the
 // products go to a block of their own, and one pass over that applies alpha and beta and puts the batch back innermost: all
 // of it tiled permutations at the memory's rate.
-// (us as they lie and on copies: f32, 100 of 900^3 4640, 1180, the exact kernel 1000 of 100^3 380, 233, 8 of 600^3 255, 227, 477 of 100
+// (us as they lie and on copies: f32, 100 of 900^3 4560, 1140, the exact kernel 1000 of 100^3 380, 233, 8 of 600^3 255, 227, 477 of 100
 // x 800 x 17 576, 386; double, 220 of 580 x 308 x 408 2340, 1540, 100 of 500 x 500 x 16 838, 167, 16 of 600^3 357, 334; complex
 // single, 1000 of 100^3 332, 260, 100 of 500 x 500 x 16 456, 186.  Complex double elements are half a sector, and nothing is gained:
 // 64 of 300^3 619, 628.)
@@ -474,8 +474,8 @@ static tfb_status contract_batch_innermost(tfb_ctx* ctx, const ContractProblem& 
     auto up = [](int64_t x, int64_t to) { return (x + to - 1) / to * to; };
     // Copies as the kernels like them best: [batch][k][rows] for the FP64 pipe, [batch][rows][k] for tcgen05.  The first operand of
     // a complex single product is embedded from either, and by rows it does not offer itself to be read in place with the
-    // roles exchanged, which would take rows across the block (488 of 260 x 80 x 16: 278 us exchanged, 131 so,
-    // 146 as they lie).
+    // roles exchanged, which would take rows across the block (488 of 260 x 80 x 16: 286 us exchanged, 133 so,
+    // 148 as they lie).
     const bool copy[2] = {p.batch[0].s[0] == 1, p.batch[0].s[1] == 1};
     // A batch index innermost leaves an operand without a tensor map, and contract_tcgen05 copies those of large products only:
     // smaller ones run on the exact kernel, and do so on the copies (relative error of 1000 of 100^3 1.8e-7, as 3xTF32 8.7e-7).

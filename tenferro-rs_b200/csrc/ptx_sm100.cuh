@@ -48,8 +48,7 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 // Part of every kernel for launch_overlapped, ahead of its first access to global memory.  Writes of earlier launches are
 // visible after the wait only, so there is no kernel without it.  No kernel lets the next one start before its own blocks are
 // through: blocks that wait take shared memory and registers from those that compute (us a call, with such a start and
-// without: complex double 'efcab,efd->abcd' of 64 x 116 x 17136 100, 68; f32 'bagfc,dgef->ebcad' of 2520 x 1810 x 8272 with a batch
-// of five 695, 630; 97 x 194 x 97 complex double 13.4 both).
+// without: complex double 'efcab,efd->abcd' of 64 x 116 x 17136 100, 68; f32 'bagfc,dgef->ebcad' 665, 607; 97 x 194 x 97 complex double 13.4 both).
 __device__ __forceinline__ void launch_begin() { grid_dependency_wait(); }
 
 // Reads of another CTA's shared memory (addresses from map_to_cta).

@@ -1209,7 +1209,7 @@ static tfb_status reduce_static_ops(tfb_ctx* ctx, int op, const LoopNest& kept, 
 }  // namespace tfb
 
 // See include/tenferro_b200.h.  The first call on a device looks up the scratch address
-// (cudaGetSymbolAddress); after that a call is two kernel launches and nothing else.
+// (cudaGetSymbolAddress); after that a call is one kernel launch, two where there are more slices than one block combines, and nothing else.
 extern "C" tfb_status tfb_reduce_static(tfb_ctx* ctx, int32_t dtype, int32_t reduce_op, const uint32_t* modes_a,
                                         size_t n_modes_a, const tfb_view* a, const uint32_t* modes_c, size_t n_modes_c,
                                         const tfb_view* c, const void* alpha, const void* beta) {
