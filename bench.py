@@ -321,7 +321,7 @@ def workload_identity(args):
     wl = args.workload
     if wl == "dense":
         ext, kext = dense_extents(args.scale)
-        return DENSE_METRIC, "GFLOP/s", "f32 (3xTF32)", "strong", dense_workload_name(ext, kext)
+        return DENSE_METRIC, "GFLOP/s", "f32 (products of fp16 pairs)", "strong", dense_workload_name(ext, kext)
     if wl == "chain":
         return (CHAIN_METRIC, "GFLOP/s", "c128 (f64 arithmetic)", "weak",
                 chain_workload_name(args.sites, args.chi, args.phys))
@@ -708,10 +708,10 @@ def wl_dense(env: Env):
         cfg["e2e_path"] = e2e_note
     return {
         "step": pm["step"], "work": flops, "read_result": read_result, "e2e_step": e2e_step, "h2d": h2d, "d2h": d2h,
-        "kernel": "contract_tf32x3",
-        "kernel_label": "contract_tf32x3_pair_kernel (tcgen05 cta_group::2, 256x256 tiles per CTA pair, 32-deep stages)",
-        "per_launch": flops / W, "bound": "tensor", "tf32_cold": tf32_cold, "tf32x3": True,
-        "extra_kernels": ["repack_operand"], "keep": (a_t, b_t, c_t, part_t, out_t),
+        "kernels_any": ["contract_f16x3", "contract_tf32x3"],
+        "kernel_label": "contract_f16x3_kernel (tcgen05 cta_group::2 on operands split into two fp16, 256x256 tiles per CTA pair)",
+        "per_step": flops / W, "bound": "tensor", "tf32_cold": tf32_cold, "tf32x3": True,
+        "extra_kernels": ["split_operands", "repack_operand"], "keep": (a_t, b_t, c_t, part_t, out_t),
         "check": pm["check"], "modes": modes, "primary": primary, "traffic": None,
         "config": cfg,
     }
@@ -833,14 +833,11 @@ def wl_network4(env: Env):
                                         [(out._block.ptr, out._block.nbytes)])
     return {
         "step": call.run, "work": flops * env.world, "read_result": read_result, "e2e_step": e2e_step,
-        "h2d": h2d * env.world, "d2h": d2h * env.world, "kernel": "contract_tf32x3",
-        "kernel_label": "contract_tf32x3 kernels (tcgen05; complex64 as one real product of doubled extents per tree node)",
-        "per_launch": flops / 3.0, "bound": "tensor", "tf32_cold": tf32_cold, "tf32x3": True,
-        "extra_kernels": ["pack_planes", "contract_tf32x3_finish"], "check": check,
-        # ncu, per launch averaged over the three product launches of a call: the two large nodes moved
-        # 667 MB and 703 MB; the third, whose operands (two 7 MB tensors) stay in L2, was not captured
-        # and is counted as zero
-        "traffic": (667.2e6 + 703.2e6) / 3.0 if dim == 96 else None,
+        "h2d": h2d * env.world, "d2h": d2h * env.world, "kernels_any": ["contract_f16x3", "contract_tf32x3"],
+        "kernel_label": "contract_f16x3 and contract_tf32x3 kernels (tcgen05; complex64 as one real product of doubled extents per tree node)",
+        "per_step": flops, "bound": "tensor", "tf32_cold": tf32_cold, "tf32x3": True,
+        "extra_kernels": ["split_operands", "pack_planes", "contract_tf32x3_finish"], "check": check,
+        "traffic": None,
         "config": {"tree": tree.pairs, "parallelism": f"{env.world} independent replica(s)",
                    "l2": f"intermediates of {dim ** 4 * 8 >> 20} MiB exceed L2" if dim >= 64 else "L2-resident (scaled down)",
                    "flop_total": flops},
@@ -1159,49 +1156,42 @@ def main():
     extras = {nm: ctx.profile_read(nm) for nm in wl["extra_kernels"]}
     ctx.profile_end()
     scale = 1e12 if wl["bound"] == "tensor" else 1e9
-    achieved = wl["per_launch"] / (ms_main / n_main * 1e-3) / scale if n_main else None
+    # the work of a step over its product launches (those behind a gate that stayed shut count a few microseconds), or of a launch
+    launch_ms = ms_main / args.steps if "per_step" in wl else ms_main / max(n_main, 1)
+    achieved = (wl["per_step"] if "per_step" in wl else wl["per_launch"]) / (launch_ms * 1e-3) / scale if n_main else None
     roofline = {"bound": wl["bound"], "achieved": achieved, "unit": "TFLOP/s" if wl["bound"] == "tensor" else "GB/s"}
     if wl.get("tf32x3"):
-        # f32 through 3xTF32: three MMAs per algorithmic MMA, so the relevant peak is a third of the
-        # dense TF32 rate, measured here by the library's tcgen05 probe (MEASURED_PEAKS.json holds no
-        # TF32 figure).  Two denominators: the burst rate of a cool GPU, and the rate the probe
-        # sustains when launched back to back for seconds under the board's power limit - the one
-        # that applies to a kernel timed inside a long step, as here.
-        #
-        # With the corrections as one bf16 MMA (the library's default, TFB_TC_BF16_CORRECTIONS) a k-step
-        # costs the tensor pipe TWO MMAs' time - a bf16 MMA of K = 16 takes what a TF32 MMA of K = 8
-        # takes - so the ceiling is HALF the TF32 rate and the fractions are quoted against that;
-        # `frac_of_three_mma_form` is the same figure against the third, for comparison with numbers
-        # taken before the bf16 form existed.
-        mmas = 2.0 if int(os.environ.get("TFB_TC_BF16_CORRECTIONS", "1") or 0) != 0 else 3.0
+        # f32 accuracy from three fp16 MMAs per algorithmic one, so the peak is a third of the 16-bit dense rate: MEASURED_PEAKS.json's
+        # burst figure for a cool GPU, its sustained one - seconds back to back under the board's power limit - for a kernel
+        # timed inside a long step, as here.  Without that file, and for the older forms, the library's TF32 probe: half its rate with
+        # the corrections as one bf16 MMA (two MMAs' time per k-step), a third with three TF32 MMAs
+        # (TFB_TC_BF16_CORRECTIONS=0), burst from the larger of a probe before and one after the run.
         burst_tf32 = max(wl["tf32_cold"], ctx.probe_tf32_tflops())
-        burst = burst_tf32 / mmas
-        sustained_tf32 = None
-        if args.sustained_seconds > 0 and rank == 0:
-            sustained_tf32 = ctx.probe_tf32_tflops_sustained(args.sustained_seconds)
-        sustained = sustained_tf32 / mmas if sustained_tf32 else None
+        sustained_tf32 = ctx.probe_tf32_tflops_sustained(args.sustained_seconds) if args.sustained_seconds > 0 and rank == 0 else None
+        mmas = 2.0 if int(os.environ.get("TFB_TC_BF16_CORRECTIONS", "1") or 0) != 0 else 3.0
+        split = mmas == 2.0 and int(os.environ.get("TFB_TC_SPLIT16", "1") or 0) != 0
+        peaks = env.peaks or {}
+        if split and peaks.get("bf16_tflops"):
+            burst, sustained = peaks["bf16_tflops"] / 3.0, (peaks.get("bf16_tflops_sustained") or 0) / 3.0 or None
+            source = "a third of MEASURED_PEAKS.json's 16-bit dense rate, sustained (`peak`) and burst (`peak_burst`)"
+        else:
+            burst, sustained = burst_tf32 / mmas, sustained_tf32 / mmas if sustained_tf32 else None
+            source = "the library's dense TF32 probe over the MMAs of a k-step, sustained (`peak`) and burst (`peak_burst`)"
         peak = sustained or burst
-        share = "half" if mmas == 2.0 else "one third"
         roofline.update({
             "peak": peak, "frac": (achieved / peak) if achieved else None,
             "peak_burst": burst, "frac_burst": (achieved / burst) if achieved else None,
             "peak_sustained": sustained, "frac_sustained": (achieved / sustained) if (achieved and sustained) else None,
-            "mma_per_k_step": int(mmas),
-            "frac_of_three_mma_form": (achieved / ((sustained_tf32 or burst_tf32) / 3.0)) if achieved else None,
-            "peak_source": (f"{share} of the dense TF32 rate of the library's tcgen05 probe on this GPU ({int(mmas)} MMAs' time per "
-                            "k-step): `peak` is the "
-                            f"sustained figure (probe launched back to back for {args.sustained_seconds:g} s, rate of "
-                            "the last quarter), `peak_burst` the larger of a single probe before and one after the run")
-            if sustained else
-            (f"{share} of the dense TF32 rate of the library's tcgen05 probe on this GPU ({int(mmas)} MMAs' time per k-step; "
-             "burst: the larger of a probe before and one after the run)")})
+            "mma_per_k_step": 3 if split else int(mmas), "peak_source": source,
+            # against a third of the TF32 rate, for comparison with numbers taken in the older forms
+            "frac_of_three_mma_form": (achieved / ((sustained_tf32 or burst_tf32) / 3.0)) if achieved else None})
     else:
         peak = wl["peak"]()
         roofline.update({"peak": peak, "frac": (achieved / peak) if (achieved and peak) else None,
                          "peak_source": wl["peak_source"]})
     roofline.update({
         "traffic": wl.get("traffic"), "kernel": wl["kernel_label"], "launches": n_main,
-        "avg_launch_us": ms_main / max(n_main, 1) * 1e3,
+        "avg_launch_us": launch_ms * 1e3,
         "other_kernels": {k: {"launches": v[0], "avg_us": v[1] / max(v[0], 1) * 1e3} for k, v in extras.items()}})
 
     # ---- end to end through the public API from pinned host memory

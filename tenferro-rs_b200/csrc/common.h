@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -209,6 +210,8 @@ tfb_status launch_contract(tfb_ctx* ctx, const ContractProblem& p, int force_ker
 // products run on the exact kernel.
 constexpr double kTcCopyFlops = 1e9;
 
+struct SplitProduct;  // contract_pair.cuh
+struct Gate;
 // Family-specific launchers (each may decline with *declined = true and TFB_OK).
 tfb_status contract_simt(tfb_ctx* ctx, const ContractProblem& p);
 // Over a tropical semiring (tfb_algebra: 1 MaxPlus, 2 MinPlus); an empty K group is a single term.
@@ -217,7 +220,8 @@ tfb_status contract_dmma(tfb_ctx* ctx, const ContractProblem& p, bool* declined,
 tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declined,
                             const int64_t* const* c_tables = nullptr, const std::vector<Mode>* c_n_modes = nullptr,
                             int c_scale = 1, const std::vector<Mode>* c_m_modes = nullptr,
-                            const std::vector<Mode>* c_batch_modes = nullptr);
+                            const std::vector<Mode>* c_batch_modes = nullptr, const SplitProduct* split = nullptr,
+                            const std::function<tfb_status(const Gate&)>* set_up = nullptr);
 tfb_status contract_c32_embedded(tfb_ctx* ctx, const ContractProblem& p, bool* declined);
 
 // Scratch from the context pool, released stream-ordered when the object dies.

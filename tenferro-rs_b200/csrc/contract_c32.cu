@@ -24,9 +24,8 @@
 // tenferro-prims/src/lib.rs:156-168, 227-239.
 #include <algorithm>
 
-#include "contract_common.cuh"
+#include "contract_pair.cuh"
 #include "contract_tables.h"
-#include "ptx_sm100.cuh"
 
 namespace tfb {
 
@@ -60,9 +59,10 @@ struct RealTables {
 // four loads in flight, 1255 so; 30 of 60^3, which L2 holds, 21 us a call, 26 so).  (Two parameters and a choice rather than an indexed array of them, which is
 // read from memory at each use.)
 template <bool SCATTERED>
-__global__ void __launch_bounds__(256) embed_setup_kernel(EmbedArgs first, EmbedArgs second, RealTables args, int job0) {
+__global__ void __launch_bounds__(256) embed_setup_kernel(EmbedArgs first, EmbedArgs second, RealTables args, int job0, Gate gate) {
     __shared__ float2 tile[32][33];
     launch_begin();
+    if (gate.closed()) return;
     const int job = job0 + (int)blockIdx.y;
     if (job == 0) {
         const int64_t n = max(2 * args.M, max(args.N, args.B));
@@ -241,20 +241,6 @@ static tfb_status embedded_product(tfb_ctx* ctx, const ContractProblem& p, bool*
     auto scattered = [&](const std::vector<Mode>& g, int t, int64_t rows) {
         return gather_bytes(p, g, t) > 16 && 8.0 * (double)rows * (double)K * (double)B > 64e6;
     };
-    auto set_up = [&](bool scatters, int64_t blocks, int job0, unsigned jobs) -> tfb_status {
-        LaunchScope ls(ctx, "pack_planes");
-        const dim3 grid((unsigned)std::min<int64_t>(blocks, (int64_t)ctx->sm_count * 16), jobs);
-        TFB_CUDA(scatters ? launch_overlapped(ctx, embed_setup_kernel<true>, grid, dim3(256), 0, 0u, first, second, tables, job0)
-                          : launch_overlapped(ctx, embed_setup_kernel<false>, grid, dim3(256), 0, 0u, first, second, tables, job0));
-        return TFB_OK;
-    };
-    const bool a_scatters = scattered(p.m, 0, M), b_scatters = !b_in_place && scattered(p.n, 1, N);
-    if (b_in_place || a_scatters || b_scatters) {
-        TFB_TRY(set_up(a_scatters, std::max(for_tables, patches(M)), 0, 2));
-        if (!b_in_place) TFB_TRY(set_up(b_scatters, patches(N), 2, 1));
-    } else {
-        TFB_TRY(set_up(false, std::max({for_tables, patches(M), patches(N)}), 0, 3));
-    }
     double beta = p.beta.re;
     if (p.beta.im != 0) {
         const int64_t blocks = (M * N * B + 255) / 256;
@@ -265,6 +251,24 @@ static tfb_status embedded_product(tfb_ctx* ctx, const ContractProblem& p, bool*
         beta = 1.0;
     }
 
+    // The set-up kernels, which contract_tcgen05 has run once it knows whether the product runs on split operands.
+    auto pass = [&](const Gate& gate, bool scatters, int64_t blocks, int job0, unsigned jobs) -> tfb_status {
+        LaunchScope ls(ctx, "pack_planes");
+        const dim3 grid((unsigned)std::min<int64_t>(blocks, (int64_t)ctx->sm_count * (gate.word ? 8 : 16)), jobs);
+        TFB_CUDA(scatters ? launch_overlapped(ctx, embed_setup_kernel<true>, grid, dim3(256), 0, 0u, first, second, tables, job0, gate)
+                          : launch_overlapped(ctx, embed_setup_kernel<false>, grid, dim3(256), 0, 0u, first, second, tables, job0, gate));
+        return TFB_OK;
+    };
+    const bool a_scatters = scattered(p.m, 0, M), b_scatters = !b_in_place && scattered(p.n, 1, N);
+    const std::function<tfb_status(const Gate&)> set_up = [&](const Gate& gate) -> tfb_status {
+        if (b_in_place || a_scatters || b_scatters) {
+            TFB_TRY(pass(gate, a_scatters, std::max(for_tables, patches(M)), 0, 2));
+            if (!b_in_place) TFB_TRY(pass(gate, b_scatters, patches(N), 2, 1));
+        } else {
+            TFB_TRY(pass(gate, false, std::max({for_tables, patches(M), patches(N)}), 0, 3));
+        }
+        return TFB_OK;
+    };
     // The real product: A' [B][2M][ld] K-major, B' [B][N][ld] K-major (or B itself), C through the tables.
     ContractProblem q;
     q.dtype = TFB_F32;
@@ -283,8 +287,36 @@ static tfb_status embedded_product(tfb_ctx* ctx, const ContractProblem& p, bool*
     q.m.push_back(Mode{2 * M, {ld, 0, 0}});
     q.k.push_back(Mode{2 * K, {1, 1, 0}});
     const int64_t* c_tables[3] = {tab_b, tab_m, tab_n};
+    // What the set-up kernels would write, split into 16-bit halves instead.  Scattered operands keep the kernels that are made
+    // for them.
+    SplitProduct split{};
+    split.a = SplitOperand{p.a, t->a_m, t->a_k, t->a_b, M, K, B, SplitOperand::Embedded, ca.a_kfast, p.conj_a, alpha,
+                           one_step(p.m, 0), one_step(p.k, 0), common_step(p.batch, 0)};
+    split.b = SplitOperand{p.b, t->b_n, t->b_k, t->b_b, N, K, B, SplitOperand::Parts, ca.b_kfast, p.conj_b, make_float2(1.f, 0.f),
+                           one_step(p.n, 1), one_step(p.k, 1), common_step(p.batch, 1)};
+    split.M = 2 * M;
+    split.N = N;
+    split.K = 2 * K;
+    split.B = B;
+    split.c = p.c;
+    split.complex_b = t->c_b;
+    split.complex_m = t->c_m;
+    split.complex_n = t->c_n;
+    split.complex_rows = true;
+    if (!p.n.empty() && p.n.size() <= 2 && p.n[0].extent < INT32_MAX) {
+        split.cn_e1 = p.n.size() == 2 ? (int)p.n[0].extent : INT32_MAX;
+        split.cn_s1 = 2 * p.n[0].s[2];
+        split.cn_s2 = p.n.size() == 2 ? 2 * p.n[1].s[2] : 0;
+    }
+    split.alpha = 1.f;
+    split.beta = (float)beta;
+    split.m_modes = &p.m;
+    split.n_modes = &p.n;
+    split.c_scale = 2;
+    split.cols_fast = !p.n.empty() && std::llabs(p.n[0].s[2]) == 1;
+    const bool pays = !a_scatters && !b_scatters && split_pays(2 * M, N, 2 * K, B, b_in_place ? 16.0 * (double)N * (double)K * (double)B : 0);
     bool d = false;
-    TFB_TRY(contract_tcgen05(ctx, q, &d, c_tables, &p.n, 2, &p.m, &p.batch));
+    TFB_TRY(contract_tcgen05(ctx, q, &d, c_tables, &p.n, 2, &p.m, &p.batch, pays ? &split : nullptr, &set_up));
     if (d) return fail(TFB_ERR_DEVICE, "internal: the embedded real product was declined by the tensor-core kernel");
     *declined = false;
     return TFB_OK;

@@ -1,0 +1,870 @@
+// Single precision products on operands split into two 16-bit floats each.
+//
+// An f32 element is x = 2^-s (hi + lo) with hi = fp16(2^s x) and lo = fp16(2^s x - hi): 22 bits of its mantissa.  The product
+// of two such sums is three MMAs of kind::f16 (hi hi + hi lo + lo hi; lo lo is 2^-22 of it and left out), K = 16 each: three
+// quarters of the tensor-pipe time of the TF32 + bf16 form in contract_tcgen05.cu - and, since a pass over the operands writes
+// them split, with nothing to convert inside the product: the loop is TMA and MMA alone.  What bounds it is the tensor pipe
+// (136 to 151 clocks per 256 x 256 x 16 MMA of a pair, 138 being what the TF32 form of the same bytes takes) and, in launches of a
+// millisecond, the board's power: 16384 x 16384 x 65536 97 ms, 122 in the TF32 form; 8192^3 2.4 ms, 3.5.  Errors against 64 bits are
+// half those of the TF32 form (9.3e-7, 1.8e-6 for N(0,1)): 48 truncating sums in tensor memory per 256 of K instead of 64.
+//
+// Scales.  s is chosen for every row and 256 of K (a promotion chunk) so that the largest element lies in [2^14, 2^15): products of
+// rows whose magnitudes differ lose nothing, and a chunk's sum is multiplied by 2^-(s_row + s_column) when it is promoted.  lo is
+// an fp16 number, so the pair's absolute error is at most 2^-40 of the chunk's largest element: 2^-19 relative (what the bf16
+// corrections leave) down to elements 2^-21 of it, and less than f32 keeps below.  The splitting pass counts the elements below that
+// line, and looks for infinities, NaN and magnitudes whose scale would leave f32: where a row has more than a sixteenth of such
+// elements in a chunk, or any of the others, it sets the product's gate word, this kernel returns at once and the TF32 form,
+// launched behind it, runs instead of returning at once.
+//
+// Layout of a split operand: [batch][row][k-block of 32][32 hi | 32 lo], 128 bytes a record, the size of the f32 it was made from
+// and one 128-byte swizzle row.
+//
+// Semantics: PrimDescriptor::{Contract, BatchedGemm}, tenferro-prims/src/lib.rs:156-168, 227-239.
+#include <cuda_fp16.h>
+
+#include <atomic>
+
+#include "contract_pair.cuh"
+
+namespace tfb {
+
+namespace {
+
+// ------------------------------------------------------------------ splitting pass
+constexpr int kSplitRows = 32;            // source rows of a block's patch
+constexpr int kSplitK = kChunk * kBK;     // floats of K: one chunk
+constexpr int kSplitPitch = kSplitK + 4;  // 16-byte rows whose first words lie in different banks
+constexpr int kMaxSmall = kSplitK / 16;   // elements below 2^-21 of their chunk's largest that a row may have
+constexpr float kMostMagnitude = 1.2676506e30f;  // 2^100: sums of scaled products then stay in f32 before and after each factor
+
+struct SplitJob {
+    SplitOperand s;
+    int num_kb;        // records per row
+    int64_t out_rows;  // rows of the split operand (twice the source's where it is embedded)
+    int64_t pad_rows;  // scales per chunk
+    uint32_t* dst;     // [B][out_rows][num_kb][32]
+    float* inv;        // [B][chunks][pad_rows]: 2^-s
+    int direct;        // rows are read as they lie, sixteen bytes at a time
+};
+struct TableJob {
+    const int64_t *b, *m, *n;  // of the complex output, null: nothing to do
+    int64_t *out_b, *out_m, *out_n;
+    int64_t M, N, B;  // complex extents
+};
+
+__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+// Eight elements of a row (k = 8 lane ..) into the row's records at `dst` (this lane's sixteen bytes of hi; null: past the last
+// record); the whole warp holds the row's part of a chunk.
+__device__ __forceinline__ void split_row(const float (&x)[8], uint4* dst, float* inv, const Gate& gate, int lane) {
+    uint32_t top = 0, least = 0xffffffffu;  // largest magnitude, and smallest but zero (less one) as bit patterns
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t u = __float_as_uint(x[i]) & 0x7fffffffu;
+        top = max(top, u);
+        least = min(least, u - 1);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    least = __reduce_min_sync(0xffffffffu, least);
+    // 2^s puts the largest element into [2^14, 2^15); tiny rows stop at 2^126, far below the last bit of any f32
+    const int s = top ? min(14 + 127 - (int)(top >> 23), 126) : 0;
+    const float scale = __uint_as_float((uint32_t)(127 + s) << 23);
+    const uint32_t line = __float_as_uint(__uint_as_float(top) * 4.76837158e-7f);  // 2^-21
+    int small = 0;
+    if (least < line && top != 0) {  // (the same in all lanes, and rare)
+        int mine = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mine += (__float_as_uint(x[i]) & 0x7fffffffu) - 1 < line;
+        small = __reduce_add_sync(0xffffffffu, mine);
+    }
+    if (lane == 0) {
+        *inv = __uint_as_float((uint32_t)(127 - s) << 23);
+        // (infinities and NaN have larger bit patterns than any number)
+        if (small > kMaxSmall || top > __float_as_uint(kMostMagnitude)) *(volatile unsigned long long*)gate.word = gate.value;
+    }
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float a = x[2 * i] * scale, c = x[2 * i + 1] * scale;
+        hi[i] = pack_half2(a, c);
+        const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi[i]));
+        lo[i] = pack_half2(a - h.x, c - h.y);
+    }
+    if (dst) {
+        dst[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        dst[4] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+}
+
+// A row's part of a chunk, this lane's eight floats of it, as the split operand has it: conjugated, or as the two rows of an embedding.
+template <bool COMPLEX>
+__device__ __forceinline__ void put_row(const SplitJob& j, float (&x)[8], uint4* dst, float* inv, const Gate& gate, int lane) {
+    if constexpr (!COMPLEX) {
+        split_row(x, dst, inv, gate, lane);
+        return;
+    }
+    if (j.s.conj) {
+#pragma unroll
+        for (int i = 1; i < 8; i += 2) x[i] = -x[i];
+    }
+    if (j.s.kind != SplitOperand::Embedded) {
+        split_row(x, dst, inv, gate, lane);
+        return;
+    }
+    float re[8], ri[8];
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+        const float wr = j.s.alpha.x * x[i] - j.s.alpha.y * x[i + 1], wi = j.s.alpha.x * x[i + 1] + j.s.alpha.y * x[i];
+        re[i] = wr;
+        re[i + 1] = -wi;
+        ri[i] = wi;
+        ri[i + 1] = wr;
+    }
+    split_row(re, dst, inv, gate, lane);
+    split_row(ri, dst ? dst + (int64_t)j.num_kb * 8 : nullptr, inv + 1, gate, lane);
+}
+
+// Offsets of a group: by its step, or by its table.
+template <bool STEP>
+struct GroupAt {
+    int64_t step;
+    const int64_t* tab;
+    __device__ __forceinline__ int64_t operator()(int64_t i) const { return STEP ? i * step : tab[i]; }
+};
+typedef float SplitTile[kSplitRows][kSplitPitch];
+// 32 rows of a chunk into shared memory, complex elements as their two parts; the reads follow the source's unit stride
+// (128 or 256 bytes of a warp across rows, 1 KB of a row along K), sixteen (eight complex) a thread in flight.
+template <typename T, bool KFAST, bool STEP>
+__device__ __forceinline__ void load_patch(const SplitJob& j, int64_t off_b, int64_t r0, int chunk, SplitTile& tile) {
+    constexpr int W = sizeof(T) / 4, PER = kSplitK / W, BATCH = 16 / W;  // floats of an element, elements of a row, loads in flight
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const GroupAt<STEP> at_k{j.s.k_step, j.s.k_tab}, at_row{j.s.row_step, j.s.row_tab};
+    const T* src = (const T*)j.s.src + off_b;
+    const int64_t k0 = (int64_t)chunk * PER;
+    T zero;
+    if constexpr (W == 1) zero = 0.f; else zero = make_float2(0.f, 0.f);
+    T v[BATCH];
+    if constexpr (KFAST) {
+        const int kc = t % PER, first = t / PER;  // a row is read by PER threads
+        const bool ok = k0 + kc < j.s.K;
+        if (ok) src += at_k(k0 + kc);
+        const int rows = (int)min((int64_t)kSplitRows, j.s.rows - r0);
+#pragma unroll
+        for (int i = 0; i < kSplitRows / W; i += BATCH) {
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u) {
+                const int r = first + W * (i + u);
+                v[u] = ok && r < rows ? src[at_row(r0 + r)] : zero;
+            }
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u) *reinterpret_cast<T*>(&tile[first + W * (i + u)][W * kc]) = v[u];
+        }
+    } else {
+        const bool ok = r0 + lane < j.s.rows;
+        if (ok) src += at_row(r0 + lane);
+        const int left = ok ? (int)min((int64_t)PER, j.s.K - k0) : 0;
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) {
+            // four floats of a row next to each other, so that they are stored as one; four such groups, 32 floats apart
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u) {
+                const int k = (warp + 8 * (i + u * W / 4)) * 4 / W + u % (4 / W);
+                v[u] = k < left ? src[at_k(k0 + k)] : zero;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                float4 f;
+                if constexpr (W == 1) f = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+                else f = make_float4(v[2 * u].x, v[2 * u].y, v[2 * u + 1].x, v[2 * u + 1].y);
+                *reinterpret_cast<float4*>(&tile[lane][(warp + 8 * (i + u)) * 4]) = f;
+            }
+        }
+    }
+}
+template <typename T>
+__device__ __forceinline__ void load_patch(const SplitJob& j, int64_t off_b, int64_t r0, int chunk, SplitTile& tile) {
+    const bool steps = j.s.k_step != 0 && j.s.row_step != 0;
+    if (j.s.kfast) {
+        if (steps) load_patch<T, true, true>(j, off_b, r0, chunk, tile);
+        else load_patch<T, true, false>(j, off_b, r0, chunk, tile);
+    } else {
+        if (steps) load_patch<T, false, true>(j, off_b, r0, chunk, tile);
+        else load_patch<T, false, false>(j, off_b, r0, chunk, tile);
+    }
+}
+
+// 32 rows x one chunk at a time: a warp takes four of the rows, finds the largest element of each and writes its records, 1 KB without
+// a gap.  Rows whose elements follow one another on 16-byte boundaries are read by the lanes that convert them; others go through
+// shared memory.  blockIdx.y: the first operand, the second, the offset tables of a complex output.
+template <bool COMPLEX>
+__global__ void __launch_bounds__(256, 4) split_operands_kernel(SplitJob ja, SplitJob jb, TableJob tables, Gate gate) {
+    __shared__ __align__(16) SplitTile tile;
+    launch_begin();
+    if (COMPLEX && blockIdx.y == 2) {
+        const int64_t n = max(2 * tables.M, max(tables.N, tables.B));
+        for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+            if (i < 2 * tables.M) tables.out_m[i] = 2 * tables.m[i >> 1] + (i & 1);
+            if (i < tables.N) tables.out_n[i] = 2 * tables.n[i];
+            if (i < tables.B) tables.out_b[i] = 2 * tables.b[i];
+        }
+        return;
+    }
+    const SplitJob j = blockIdx.y == 0 ? ja : jb;
+    const int chunks = (j.num_kb + kChunk - 1) / kChunk;
+    const int64_t tiles_r = (j.s.rows + kSplitRows - 1) / kSplitRows, n_tiles = tiles_r * chunks * j.s.B;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int per = COMPLEX && j.s.kind == SplitOperand::Embedded ? 2 : 1;
+    constexpr int w = COMPLEX ? 2 : 1;
+    const int64_t row_units = (int64_t)j.num_kb * 8;  // of sixteen bytes
+    for (int64_t i = blockIdx.x; i < n_tiles; i += gridDim.x) {
+        const int64_t rest = i / tiles_r, r0 = (i - rest * tiles_r) * kSplitRows, b = rest / chunks;
+        const int chunk = (int)(rest - b * chunks);
+        const int64_t off_b = j.s.b_tab[b];
+        const int kb = chunk * kChunk + (lane >> 2), rows = (int)min((int64_t)kSplitRows, j.s.rows - r0);
+        const int64_t row = per * (r0 + warp);
+        uint4* dst = reinterpret_cast<uint4*>(j.dst) + (b * j.out_rows + row) * row_units + kb * 8 + (lane & 3);
+        if (kb >= j.num_kb) dst = nullptr;
+        float* inv = j.inv + (b * chunks + chunk) * j.pad_rows + row;
+        if (j.direct) {
+            const int64_t k = (int64_t)chunk * kSplitK + 8 * lane;
+            const float* src = (const float*)j.s.src + w * (off_b + (r0 + warp) * j.s.row_step) + k;
+            const int left = (int)max((int64_t)0, min((int64_t)8, w * j.s.K - k));
+            // two rows in flight
+#pragma unroll 1
+            for (int u = 0; u < 4; u += 2) {
+                float x[2][8];
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    const float* s = src + 8 * (u + v) * w * j.s.row_step;
+                    const bool ok = warp + 8 * (u + v) < rows;
+                    if (ok && left == 8) {
+                        const float4 p = reinterpret_cast<const float4*>(s)[0], q = reinterpret_cast<const float4*>(s)[1];
+                        x[v][0] = p.x, x[v][1] = p.y, x[v][2] = p.z, x[v][3] = p.w, x[v][4] = q.x, x[v][5] = q.y, x[v][6] = q.z, x[v][7] = q.w;
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) x[v][e] = ok && e < left ? s[e] : 0.f;
+                    }
+                }
+#pragma unroll
+                for (int v = 0; v < 2; ++v)
+                    if (warp + 8 * (u + v) < rows)
+                        put_row<COMPLEX>(j, x[v], dst ? dst + 8 * (u + v) * per * row_units : nullptr, inv + 8 * (u + v) * per, gate, lane);
+            }
+            continue;
+        }
+        if constexpr (COMPLEX) load_patch<float2>(j, off_b, r0, chunk, tile);
+        else load_patch<float>(j, off_b, r0, chunk, tile);
+        __syncthreads();
+#pragma unroll 1
+        for (int u = 0; u < 4; ++u) {
+            const int r = warp + 8 * u;
+            if (r < rows) {
+                const float4 p = *reinterpret_cast<const float4*>(&tile[r][8 * lane]), q = *reinterpret_cast<const float4*>(&tile[r][8 * lane + 4]);
+                float x[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+                put_row<COMPLEX>(j, x, dst ? dst + 8 * u * per * row_units : nullptr, inv + 8 * u * per, gate, lane);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// ------------------------------------------------------------------ product
+struct F16Cfg {
+    static constexpr int BN = 256;                  // tile columns of the pair
+    static constexpr int A_BYTES = kBM * kBK * 4;   // this CTA's 128 rows of a k-block's records
+    static constexpr int B_BYTES = 128 * kBK * 4;   // this CTA's half of the columns
+    // Two k-blocks a stage: the MMA thread's wait and commit cost it some 700 clocks, the six MMAs of a k-block 820 (2048 x 2048 x 16384
+    // with a k-block a stage and a commit for each CTA 349 us, two k-blocks 280, and one commit that arrives in both CTAs 261).
+    static constexpr int KPS = 2;
+    static constexpr int KB_BYTES = A_BYTES + B_BYTES, STAGE_BYTES = KPS * KB_BYTES;
+    static constexpr int STAGES = 3;
+    static constexpr int BAR_BYTES = 256;
+    static constexpr int SCALE_BUFS = 4;            // chunks whose scales are on their way: the producer is a ring ahead of the workers
+    static constexpr int SCALE_BYTES = (kBM + BN) * 4;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + SCALE_BUFS * SCALE_BYTES + 1024;
+    static constexpr int LEAD = 128;                // threads of the first warpgroup: producer, MMA issuer, two warps without a role
+};
+static_assert(F16Cfg::SMEM_BYTES <= 232448, "a CTA's shared memory");
+// Worker warps promote and store.  What each does is a chain of latencies (tensor memory, then a store per column).  Where K is one
+// chunk they are what a tile waits for, and there are sixteen, of 64 columns each (8192 x 8192 x 192: 76 us, 94 with eight; the 18432 x 9216
+// x 192 product of a complex network 180, 210); longer ones have eight of 128 columns (2048 x 2048 x 2048 complex 145 us,
+// 147 with sixteen; 8191 x 8191 x 512 153, 161).  Registers: the block is launched with LAUNCH a thread, the first
+// warpgroup keeps LEAD_REGS and the workers, who hold the running sums, take WORKER_REGS.
+template <int WORKERS>
+struct F16Workers {
+    static constexpr int CPW = F16Cfg::BN * 4 / WORKERS, THREADS = F16Cfg::LEAD + 32 * WORKERS;
+    static constexpr int LAUNCH = WORKERS == 16 ? 96 : 168, LEAD_REGS = WORKERS == 16 ? 32 : 72, WORKER_REGS = WORKERS == 16 ? 112 : 216;
+    static_assert(THREADS * LAUNCH >= F16Cfg::LEAD * LEAD_REGS + 32 * WORKERS * WORKER_REGS && THREADS * LAUNCH <= 65536,
+                  "the registers that the workers take are given up before");
+};
+
+// Division by a number known at launch (Granlund and Montgomery): the compiler's own takes some 150 clocks, and a tile's place is five.
+struct FastDiv {
+    uint32_t d, mul, shift;
+    FastDiv() = default;
+    explicit FastDiv(uint32_t by) : d(by), shift(0) {
+        while ((1ull << shift) < by) ++shift;
+        mul = (uint32_t)(((1ull << 32) * ((1ull << shift) - by)) / by + 1);
+    }
+    __device__ __forceinline__ uint32_t operator()(uint32_t n) const { return (uint32_t)(((uint64_t)__umulhi(mul, n) + n) >> shift); }
+};
+
+struct F16Args {
+    float* c;
+    const int64_t *c_b, *c_m, *c_n;
+    int cn_e1;  // column offsets in closed form, (n % cn_e1) * cn_s1 + (n / cn_e1) * cn_s2; 0: the table
+    int64_t cn_s1, cn_s2;
+    int64_t M, N;
+    float alpha, beta;
+    const float *inv_a, *inv_b;  // [batch][chunks][pad_a], [pad_b]
+    int64_t pad_a, pad_b;
+    int num_kb, chunks;          // of the whole K
+    uint32_t tiles_m, tiles_n, group_m;  // pair tiles; m-tiles that are visited together share B panels through L2
+    FastDiv by_split, by_batch, by_group, by_rows, by_rows_last;  // work items of a tile, tiles of a product, of a group, m-tiles of a group, of the last
+    int k_split, chunks_per_split;
+    int n_work;
+    float* partial;  // [pair tile][rank][split][BN columns][128 rows]
+    int* status;
+    int half_w;
+    int cols_fast;
+    Gate gate;
+};
+struct F16Work {
+    int batch, row0, col0, tile;  // this CTA's first row, the pair tile's first column
+    int split, chunk0, kb0, num_kb, num_chunks;
+};
+__device__ __forceinline__ F16Work f16_work(const F16Args& g, uint32_t w, uint32_t rank) {
+    F16Work k;
+    const uint32_t pt = g.by_split(w), batch = g.by_batch(pt), tile = pt - batch * g.by_batch.d, grp = g.by_group(tile);
+    const uint32_t in = tile - grp * g.by_group.d, first = grp * g.group_m;
+    const bool last = first + g.group_m > g.tiles_m;
+    const uint32_t tn = last ? g.by_rows_last(in) : g.by_rows(in), tm = first + in - tn * (last ? g.by_rows_last.d : g.group_m);
+    k.tile = (int)pt;
+    k.split = (int)(w - pt * g.by_split.d);
+    k.batch = (int)batch;
+    k.row0 = (int)((2 * tm + rank) * kBM);
+    k.col0 = (int)(tn * 2 * g.half_w);
+    k.chunk0 = k.split * g.chunks_per_split;
+    k.num_chunks = min(g.chunks_per_split, g.chunks - k.chunk0);
+    k.kb0 = k.chunk0 * kChunk;
+    k.num_kb = min(k.num_chunks * kChunk, g.num_kb - k.kb0);
+    return k;
+}
+
+__device__ __forceinline__ void tma_load_pair_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
+    // into this CTA's shared memory; the bytes are counted at a barrier of the pair's leader
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
+}
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+                 "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+// a0 += (r0 s0) row, a1 += (r1 s1) row, as two-wide operations
+__device__ __forceinline__ void scaled_add(float& a0, float& a1, uint32_t r0, uint32_t r1, float s0, float s1, float row) {
+    asm("{\n\t.reg .b64 r, s, a, w;\n\t"
+        "mov.b64 r, {%2, %3};\n\tmov.b64 s, {%4, %5};\n\tmov.b64 a, {%0, %1};\n\tmov.b64 w, {%6, %6};\n\t"
+        "mul.rn.f32x2 r, r, s;\n\tfma.rn.f32x2 a, r, w, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "+f"(a0), "+f"(a1)
+        : "r"(r0), "r"(r1), "f"(s0), "f"(s1), "f"(row));
+}
+
+// CTA pairs on 256 x 2 half_w tiles, one pair per two SMs, walking the list of work.  Roles and barriers:
+//   full[s]      LEADER    both CTAs' loads of stage s have landed             -> MMA thread
+//   empty[s]     each CTA  the MMAs that read stage s have retired             -> own producer
+//   chunk[b]     each CTA  work accumulator b holds a chunk's sum              -> own workers
+//   promoted[b]  LEADER    both CTAs' workers have read accumulator b          -> MMA thread
+//   scales[i]    each CTA  the scales of a chunk have landed                   -> own workers
+//   free[i]      each CTA  and have been used                                  -> own producer
+// The workers only promote and store, so a finished tile leaves while the next one's first chunk is multiplied.
+template <int WORKERS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(F16Workers<WORKERS>::THREADS, 1)
+contract_f16x3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, F16Args g) {
+    using Cfg = F16Cfg;
+    constexpr int STAGES = Cfg::STAGES, BN = Cfg::BN, CPW = F16Workers<WORKERS>::CPW, SB = Cfg::SCALE_BUFS;
+    extern __shared__ char smem_raw[];
+    // both CTAs lay their rings out identically: descriptors and barrier offsets are interpreted in each one's own memory
+    char* smem = (char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const uint32_t ring = smem_u32(smem), bars = ring + STAGES * Cfg::STAGE_BYTES;
+    auto bar_full = [&](int s) { return bars + 8u * s; };
+    auto bar_empty = [&](int s) { return bars + 8u * (STAGES + s); };
+    auto bar_chunk = [&](int b) { return bars + 8u * (2 * STAGES + b); };
+    auto bar_promoted = [&](int b) { return bars + 8u * (2 * STAGES + 2 + b); };
+    auto bar_scales = [&](int i) { return bars + 8u * (2 * STAGES + 4 + i); };
+    auto bar_free = [&](int i) { return bars + 8u * (2 * STAGES + 4 + SB + i); };
+    constexpr int kTmemWord = 8 * (2 * STAGES + 4 + 2 * SB);
+    static_assert(kTmemWord + 4 <= Cfg::BAR_BYTES, "the barriers and the tensor-memory word");
+    const uint32_t scales = bars + Cfg::BAR_BYTES;
+    const float* scales_ptr = (const float*)(smem + STAGES * Cfg::STAGE_BYTES + Cfg::BAR_BYTES);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(bar_full(s), 1);
+            mbar_init(bar_empty(s), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(bar_chunk(b), 1);
+            mbar_init(bar_promoted(b), 2 * WORKERS);
+        }
+        for (int i = 0; i < SB; ++i) {
+            mbar_init(bar_scales(i), 1);
+            mbar_init(bar_free(i), WORKERS);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (threadIdx.x == 64) {
+        prefetch_map(&map_a);
+        prefetch_map(&map_b);
+    }
+    if (warp == 1) {
+        tmem_alloc_pair(bars + kTmemWord, 2 * BN);
+        tmem_relinquish_pair();
+    }
+    tc_fence_before();
+    cluster_sync_all();  // barriers of both CTAs exist before anyone arrives on the peer's
+    launch_begin();      // nothing above touches global memory
+    tc_fence_after();
+    const uint32_t tmem_base = *(volatile uint32_t*)(smem + STAGES * Cfg::STAGE_BYTES + kTmemWord);
+    // the same answer in every thread of the launch: the word was written, if at all, by the launch ahead
+    const uint32_t n_work = g.gate.set() ? 0 : (uint32_t)g.n_work;
+    const uint32_t w0 = blockIdx.x >> 1, wstep = gridDim.x >> 1;
+
+    if (warp < 4) {
+        reg_release<F16Workers<WORKERS>::LEAD_REGS>();
+        if (warp == 0 && lane == 0) {
+            // ------------------------------------------------------------ TMA producer (each CTA its own tiles)
+            const uint32_t b_bytes = (uint32_t)g.half_w * kBK * 4;
+            const uint32_t leader_full0 = map_to_cta(bar_full(0), 0);
+            int stage = 0, sbuf = 0;
+            uint32_t parity = 0, sparity = 0;
+            for (uint32_t w = w0; w < n_work; w += wstep) {
+                const F16Work k = f16_work(g, w, rank);
+                const int col = k.col0 + (int)rank * g.half_w;
+                for (int kb = 0; kb < k.num_kb; kb += Cfg::KPS) {
+                    const int n = min(Cfg::KPS, k.num_kb - kb);
+                    mbar_wait(bar_empty(stage), parity ^ 1, g.status, 0x301);
+                    // the leader expects both CTAs' bytes
+                    if (rank == 0) mbar_expect_tx(bar_full(stage), (uint32_t)(2 * n) * (Cfg::A_BYTES + b_bytes));
+                    const uint32_t full = leader_full0 + 8u * stage;
+#pragma unroll
+                    for (int i = 0; i < Cfg::KPS; ++i) {
+                        const uint32_t dst = ring + stage * Cfg::STAGE_BYTES + i * Cfg::KB_BYTES;
+                        if (i < n) {
+                            tma_load_pair_3d(dst, &map_a, full, (k.kb0 + kb + i) * kBK, k.row0, k.batch);
+                            tma_load_pair_3d(dst + Cfg::A_BYTES, &map_b, full, (k.kb0 + kb + i) * kBK, col, k.batch);
+                        }
+                    }
+                    if (++stage == STAGES) {
+                        stage = 0;
+                        parity ^= 1;
+                    }
+                    if (kb % kChunk == 0) {
+                        const int64_t at = (int64_t)k.batch * g.chunks + k.chunk0 + kb / kChunk;
+                        const uint32_t sdst = scales + sbuf * Cfg::SCALE_BYTES;
+                        mbar_wait(bar_free(sbuf), sparity ^ 1, g.status, 0x302);
+                        mbar_expect_tx(bar_scales(sbuf), (uint32_t)(kBM + 2 * g.half_w) * 4);
+                        bulk_load(sdst, g.inv_a + at * g.pad_a + k.row0, kBM * 4, bar_scales(sbuf));
+                        bulk_load(sdst + kBM * 4, g.inv_b + at * g.pad_b + k.col0, (uint32_t)(2 * g.half_w) * 4, bar_scales(sbuf));
+                        if (++sbuf == SB) {
+                            sbuf = 0;
+                            sparity ^= 1;
+                        }
+                    }
+                }
+            }
+        } else if (warp == 1 && lane == 0 && rank == 0) {
+            // ------------------------------------------------------------ MMA issuer (leader only)
+            // fp16 x fp16 -> f32, both K-major, M = 256, N = 2 half_w
+            const uint32_t idesc = (1u << 4) | ((uint32_t)((2 * g.half_w) >> 3) << 17) | ((uint32_t)((2 * kBM) >> 4) << 24);
+            // descriptors of a record's first sixteen hi; a k-step moves 32 bytes (2 units), lo lies 64 bytes (4 units) on
+            const uint64_t da0 = smem_desc(ring, 16u, 1024u, 2u), db0 = smem_desc(ring + Cfg::A_BYTES, 16u, 1024u, 2u);
+            int stage = 0;
+            uint32_t parity = 0, ch = 0;  // chunks issued before
+            for (uint32_t w = w0; w < n_work; w += wstep) {
+                const int split = (int)(w - g.by_split(w) * g.by_split.d), chunk0 = split * g.chunks_per_split;
+                const int num_kb = min(g.chunks_per_split * kChunk, g.num_kb - chunk0 * kChunk);
+                for (int kb = 0; kb < num_kb; kb += Cfg::KPS) {
+                    const bool first = kb % kChunk == 0, last = kb % kChunk == kChunk - Cfg::KPS || kb + Cfg::KPS >= num_kb;
+                    const int buf = ch & 1;
+                    const uint32_t d = tmem_base + (uint32_t)(buf * BN);
+                    const uint64_t off = (uint64_t)(stage * (Cfg::STAGE_BYTES >> 4));
+                    const uint64_t da = da0 + off, db = db0 + off;
+                    if (first && ch >= 2) {
+                        mbar_wait(bar_promoted(buf), ((ch >> 1) - 1) & 1, g.status, 0x303);
+                        tc_fence_after();
+                    }
+                    mbar_wait(bar_full(stage), parity, g.status, 0x304);
+                    tc_fence_after();
+#pragma unroll
+                    for (int i = 0; i < Cfg::KPS; ++i) {
+                        if (i == 0 || kb + i < num_kb) {
+#pragma unroll
+                            for (int ks = 0; ks < kBK / 16; ++ks) {
+                                const int u = i * (Cfg::KB_BYTES >> 4) + 2 * ks;
+                                tc_mma_f16_pair(d, da + u + 4, db + u, idesc, !(first && i == 0 && ks == 0));  // lo hi
+                                tc_mma_f16_pair(d, da + u, db + u + 4, idesc, 1);                              // hi lo
+                                tc_mma_f16_pair(d, da + u, db + u, idesc, 1);                                  // hi hi
+                            }
+                        }
+                    }
+                    tc_commit_both(bar_empty(stage));
+                    if (last) {
+                        tc_commit_both(bar_chunk(buf));
+                        ++ch;
+                    }
+                    if (++stage == STAGES) {
+                        stage = 0;
+                        parity ^= 1;
+                    }
+                }
+            }
+        }
+    } else {
+        // ---------------------------------------------------------------- workers: promote, then store
+        reg_acquire<F16Workers<WORKERS>::WORKER_REGS>();
+        const int lane_grp = warp & 3;
+        const int row_in = lane_grp * 32 + lane, col_in = ((warp - 4) >> 2) * CPW;  // this thread's row and first column of the tile
+        const bool mine = col_in < 2 * g.half_w;
+        const uint32_t tmem_mine = tmem_base + ((uint32_t)(lane_grp * 32) << 16) + (uint32_t)col_in;
+        const uint32_t leader_promoted0 = map_to_cta(bar_promoted(0), 0);
+        const bool read_c = g.beta != 0.f;
+        uint32_t ch = 0;
+        float acc[CPW];
+        for (uint32_t w = w0; w < n_work; w += wstep) {
+            const F16Work k = f16_work(g, w, rank);
+#pragma unroll
+            for (int j = 0; j < CPW; ++j) acc[j] = 0.f;
+            for (int c = 0; c < k.num_chunks; ++c, ++ch) {
+                const int buf = ch & 1, sbuf = (int)(ch % SB);
+                if (lane == 0) {
+                    mbar_wait(bar_scales(sbuf), (ch / SB) & 1, g.status, 0x305);
+                    mbar_wait(bar_chunk(buf), (ch >> 1) & 1, g.status, 0x306);
+                }
+                __syncwarp();
+                tc_fence_after();
+                const float* sc = scales_ptr + sbuf * (Cfg::SCALE_BYTES / 4);
+                const float row_scale = sc[row_in];
+                const float4* col_scale = reinterpret_cast<const float4*>(sc + kBM + col_in);
+                if (mine) {
+#pragma unroll
+                    for (int c0 = 0; c0 < CPW; c0 += 16) {
+                        uint32_t r[16];
+                        tc_ld16(tmem_mine + (uint32_t)(buf * BN + c0), r);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 16; j += 4) {
+                            const float4 s = col_scale[(c0 + j) / 4];
+                            scaled_add(acc[c0 + j], acc[c0 + j + 1], r[j], r[j + 1], s.x, s.y, row_scale);
+                            scaled_add(acc[c0 + j + 2], acc[c0 + j + 3], r[j + 2], r[j + 3], s.z, s.w, row_scale);
+                        }
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive_cluster(leader_promoted0 + 8u * buf);
+                    mbar_arrive(bar_free(sbuf));
+                }
+            }
+            const int col = k.col0 + col_in;
+            const int valid = mine ? (int)min((int64_t)CPW, g.N - col) : 0;  // columns of this warp (<= 0: none)
+            if (g.partial) {
+                float* P = g.partial + ((size_t)(k.tile * 2 + (int)rank) * g.k_split + k.split) * BN * kBM + (size_t)col_in * kBM + row_in;
+#pragma unroll
+                for (int j = 0; j < CPW; ++j)
+                    if (j < valid) P[(size_t)j * kBM] = acc[j];
+            } else if (k.row0 + row_in < g.M) {
+                float* C = g.c + g.c_b[k.batch] + g.c_m[k.row0 + row_in];
+                // Sixteen columns at a time: what they hold is read before the first of them is written.  Along a run of the inner
+                // column mode an address is one addition; sixteen that cross its end, or have no closed form, take theirs from the table.
+                const int e1 = g.cn_e1 ? g.cn_e1 : 1;
+                int outer = col / e1, inner = col - outer * e1;
+                char* p = reinterpret_cast<char*>(C + inner * g.cn_s1 + outer * g.cn_s2);
+                const int64_t step = 4 * g.cn_s1;
+#pragma unroll
+                for (int c0 = 0; c0 < CPW; c0 += 16) {
+                    if (c0 + 16 <= valid && inner + 16 <= e1) {
+                        float old[16];
+                        if (read_c) {
+                            const char* q = p;
+#pragma unroll
+                            for (int j = 0; j < 16; ++j, q += step) old[j] = *reinterpret_cast<const float*>(q);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 16; ++j, p += step) {
+                            const float v = g.alpha * acc[c0 + j];
+                            *reinterpret_cast<float*>(p) = read_c ? v + g.beta * old[j] : v;
+                        }
+                    } else if (c0 < valid) {
+                        const int64_t* tab = g.c_n + col + c0;
+#pragma unroll
+                        for (int h = 0; h < 16; h += 4) {
+                            float* at[4];
+                            float old[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) at[j] = C + (c0 + h + j < valid ? tab[h + j] : 0);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) old[j] = read_c && c0 + h + j < valid ? *at[j] : 0.f;
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const float v = g.alpha * acc[c0 + h + j];
+                                if (c0 + h + j < valid) *at[j] = read_c ? v + g.beta * old[j] : v;
+                            }
+                        }
+                    }
+                    inner += 16;
+                    if (inner >= e1 && g.cn_e1) {
+                        inner -= e1;
+                        ++outer;
+                        p = reinterpret_cast<char*>(C + inner * g.cn_s1 + outer * g.cn_s2);
+                    }
+                }
+            }
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    cluster_sync_all();  // neither CTA leaves (or frees tensor memory) while the other may still reach into it
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, 2 * BN);
+    }
+}
+
+// Split K: C = alpha * (the ranges' sums, in their order) + beta * C, 32 x 32 elements a block.  The sums lie with rows next to each
+// other; where the output's columns do, the patch is turned in shared memory.
+__global__ void __launch_bounds__(256) f16x3_finish_kernel(F16Args g) {
+    __shared__ float patch[32][33];
+    launch_begin();
+    if (g.gate.set()) return;
+    constexpr int BN = F16Cfg::BN;
+    const uint32_t part = blockIdx.x, rank = part & 1;
+    const F16Work k = f16_work(g, (part >> 1) * g.by_split.d, rank);
+    const int c0 = (int)(blockIdx.y >> 2) * 32, r0 = (int)(blockIdx.y & 3) * 32;
+    const int64_t row0 = k.row0 + r0, col0 = k.col0 + c0;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int cols = min(32, min(2 * g.half_w - c0, (int)min((int64_t)32, g.N - col0))), rows = (int)min((int64_t)32, g.M - row0);
+    const float* P = g.partial + ((size_t)part * g.k_split * BN + c0) * kBM + r0 + tx;
+    float sum[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[i] = 0.f;
+    for (int s = 0; s < g.k_split; ++s)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (tx < rows && ty + 8 * i < cols) sum[i] += P[((size_t)s * BN + ty + 8 * i) * kBM];
+    if (g.cols_fast) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) patch[ty + 8 * i][tx] = sum[i];
+        __syncthreads();
+    }
+    const bool read_c = g.beta != 0.f;
+    float* C = g.c + g.c_b[k.batch];
+    float* at[4];
+    float old[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = g.cols_fast ? ty + 8 * i : tx, c = g.cols_fast ? tx : ty + 8 * i;
+        at[i] = r < rows && c < cols ? C + g.c_m[row0 + r] + g.c_n[col0 + c] : nullptr;
+        if (g.cols_fast) sum[i] = patch[c][r];
+        old[i] = read_c && at[i] ? *at[i] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (at[i]) *at[i] = read_c ? g.alpha * sum[i] + g.beta * old[i] : g.alpha * sum[i];
+}
+
+// A split operand as rows of words; a box is a k-block's records of a tile's rows (zeros past the last row).
+bool split_operand_map(uint32_t* base, int num_kb, int64_t rows, int64_t B, int box_rows, CUtensorMap* map) {
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return false;
+    cuuint64_t dims[3] = {(cuuint64_t)num_kb * kBK, (cuuint64_t)rows, (cuuint64_t)B};
+    cuuint64_t strides[2] = {(cuuint64_t)num_kb * 128, (cuuint64_t)num_kb * 128 * (cuuint64_t)rows};
+    cuuint32_t box[3] = {kBK, (cuuint32_t)box_rows, 1}, estr[3] = {1, 1, 1};
+    if (dims[0] > 0xffffffffull || dims[1] > 0xffffffffull || dims[2] > 0xffffffffull || strides[1] >= (1ull << 40)) return false;
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+}  // namespace
+
+bool split_pays(int64_t M, int64_t N, int64_t K, int64_t B, double extra_bytes) {
+    // (the second switch asks for one form of the TF32 kernel)
+    const int split = env_int("TFB_TC_SPLIT16", 1);
+    if (!split || !env_int("TFB_TC_BF16_CORRECTIONS", 1)) return false;
+    const double flops = 2.0 * (double)M * (double)N * (double)K * (double)B;
+    // The pass runs at 5 TB/s and the launches behind the gate take 4 to 5 us (us in the TF32 form and so: 2048 x 2048 x 512 both K-major
+    // 31.4, 31.1; 2048^3 76, 63; 1536^3 52, 56; 1935 x 1927 x 1147, copied in either form, 63.5, 49; 3000^3 196, 148; 4096^3 505, 350).
+    return split == 2 || flops * (1 / 290e12 - 1 / 445e12) > 5e-6 + extra_bytes / 5e12;
+}
+
+// Columns per half of a pair tile: 128, or of a single tile with no columns to spare; 0: fewer rows than one CTA takes.
+static int half_width(int64_t M, int64_t N) { return M <= kBM || N < 32 ? 0 : N <= 256 ? (int)((N + 63) / 64) * 32 : 128; }
+
+// Which operand supplies rows and which columns is a matter of names.  The tiles' padding decides first, then the stores: a warp holds
+// 32 rows of a column, a line where the output's unit stride runs along the rows.
+static SplitProduct oriented(const SplitProduct& p) {
+    SplitProduct q = p;
+    std::swap(q.a, q.b);
+    std::swap(q.M, q.N);
+    std::swap(q.c_m, q.c_n);
+    q.complex_rows = !q.complex_rows;
+    q.cols_fast = !q.cols_fast;
+    std::swap(q.m_modes, q.n_modes);
+    // (columns that are parts of complex numbers have no closed form)
+    const std::vector<Mode>* n = q.n_modes;
+    q.cn_e1 = 0;
+    if (n && !n->empty() && n->size() <= 2 && (*n)[0].extent < INT32_MAX && (q.c_scale == 1 || q.complex_rows)) {
+        q.cn_e1 = n->size() == 2 ? (int)(*n)[0].extent : INT32_MAX;
+        q.cn_s1 = q.c_scale * (*n)[0].s[2];
+        q.cn_s2 = n->size() == 2 ? q.c_scale * (*n)[1].s[2] : 0;
+    }
+    auto padded = [](const SplitProduct& x) {
+        const int64_t w = 2 * half_width(x.M, x.N);
+        return w ? (double)((x.M + 255) / 256 * 256) * (double)((x.N + w - 1) / w * w) : 1e30;
+    };
+    const double here = padded(p), there = padded(q);
+    if (there < 0.9 * here) return q;
+    return here < 0.9 * there || !p.cols_fast ? p : q;
+}
+
+tfb_status contract_split(tfb_ctx* ctx, const SplitProduct& given, PoolBlock* mem, Gate* gate, bool* done) {
+    *done = false;
+    const SplitProduct p = oriented(given);
+    const int half_w = half_width(p.M, p.N);
+    if (!half_w || p.M > INT32_MAX - 512 || p.N > INT32_MAX - 512 || p.K > INT32_MAX - 512) return TFB_OK;
+    auto up = [](int64_t x, int64_t to) { return (x + to - 1) / to * to; };
+    F16Args g;
+    memset(&g, 0, sizeof g);
+    g.num_kb = (int)((p.K + kBK - 1) / kBK);
+    g.chunks = (g.num_kb + kChunk - 1) / kChunk;
+    g.pad_a = up(p.M, 2 * kBM);
+    g.pad_b = up(p.N, F16Cfg::BN);
+    const int64_t tiles_m = (p.M + 2 * kBM - 1) / (2 * kBM), tiles_n = (p.N + 2 * half_w - 1) / (2 * half_w);
+    const size_t words_a = (size_t)(p.B * p.M * g.num_kb * kBK), words_b = (size_t)(p.B * p.N * g.num_kb * kBK);
+    const size_t scales = (size_t)(p.B * g.chunks * (g.pad_a + g.pad_b));
+    const size_t tabs = p.complex_m ? (size_t)(p.M + p.N + p.B) : 0;
+    // at most an eighth of the device's memory: more could take the room that the caller's next tensors need
+    const size_t bytes = (words_a + words_b + scales) * 4 + tabs * 8 + 64;
+    if (bytes > ctx->total_mem / 8) return TFB_OK;
+    CUtensorMap ma, mb;
+    const int64_t pair_tiles = tiles_m * tiles_n * p.B, slots = std::max(1, ctx->sm_count / 2);
+    // K is cut where the tiles leave SMs idle, at chunks: rounds x (k-blocks + start and end), and the finishing launch
+    int splits = 1;
+    {
+        double best = 0;
+        for (int s = 1; s <= std::min(64, g.chunks); ++s) {
+            const int per = (g.chunks + s - 1) / s, real = (g.chunks + per - 1) / per;
+            const double cost = (double)((pair_tiles * real + slots - 1) / slots) * (per * kChunk + 8.0) + (real > 1 ? 8.0 : 0.0);
+            if (s == 1 || cost < 0.9 * best) {
+                best = cost;
+                splits = real;
+                g.chunks_per_split = per;
+            }
+        }
+    }
+    g.k_split = splits;
+    const int64_t n_work = pair_tiles * splits;
+    if (2 * n_work > 0x7fffffff) return TFB_OK;
+    if (mem->alloc(ctx, bytes) != TFB_OK) return TFB_OK;
+    uint32_t* split_a = (uint32_t*)mem->ptr;
+    uint32_t* split_b = split_a + words_a;
+    float* inv_a = (float*)(split_b + words_b);
+    float* inv_b = inv_a + (size_t)p.B * g.chunks * g.pad_a;
+    int64_t* tab = (int64_t*)(((uintptr_t)(inv_b + (size_t)p.B * g.chunks * g.pad_b) + 15) & ~(uintptr_t)15);
+    static std::atomic<unsigned long long> products{0x9e3779b97f4a7c15ull};
+    gate->value = ++products;
+    gate->word = (unsigned long long*)(tab + tabs);
+    if (!split_operand_map(split_a, g.num_kb, p.M, p.B, kBM, &ma) || !split_operand_map(split_b, g.num_kb, p.N, p.B, half_w, &mb)) {
+        *gate = Gate{};
+        return TFB_OK;
+    }
+    PoolBlock ws;
+    if (splits > 1) {
+        if (ws.alloc(ctx, (size_t)(2 * n_work) * F16Cfg::BN * kBM * sizeof(float)) != TFB_OK) {
+            *gate = Gate{};
+            return TFB_OK;
+        }
+        g.partial = (float*)ws.ptr;
+    }
+    static std::mutex mu;
+    static std::map<int, bool> configured;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!configured[ctx->device]) {
+            TFB_CUDA(cudaFuncSetAttribute(contract_f16x3_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, F16Cfg::SMEM_BYTES));
+            TFB_CUDA(cudaFuncSetAttribute(contract_f16x3_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, F16Cfg::SMEM_BYTES));
+            configured[ctx->device] = true;
+        }
+    }
+    auto direct = [](const SplitOperand& o) {
+        const int w = o.kind == SplitOperand::Real ? 1 : 2;
+        return o.k_step == 1 && o.row_step != 0 && w * o.row_step % 4 == 0 && w * o.b_step % 4 == 0 && (uintptr_t)o.src % 16 == 0;
+    };
+    SplitJob ja{p.a, g.num_kb, p.M, g.pad_a, split_a, inv_a, direct(p.a)}, jb{p.b, g.num_kb, p.N, g.pad_b, split_b, inv_b, direct(p.b)};
+    TableJob tables{};
+    g.c_b = p.c_b;
+    g.c_m = p.c_m;
+    g.c_n = p.c_n;
+    if (p.complex_m) {
+        // the doubled index and the other one, whichever of them is the rows'
+        const int64_t M2 = p.complex_rows ? p.M : p.N, N1 = p.complex_rows ? p.N : p.M;
+        tables = TableJob{p.complex_b, p.complex_m, p.complex_n, tab + M2 + N1, tab, tab + M2, M2 / 2, N1, p.B};
+        g.c_b = tables.out_b;
+        g.c_m = p.complex_rows ? tables.out_m : tables.out_n;
+        g.c_n = p.complex_rows ? tables.out_n : tables.out_m;
+    }
+    {
+        auto patches = [&](const SplitJob& j) { return (j.s.rows + kSplitRows - 1) / kSplitRows * g.chunks * j.s.B; };
+        const int64_t blocks = std::min<int64_t>(std::max(patches(ja), patches(jb)), (int64_t)ctx->sm_count * 24);
+        LaunchScope ls(ctx, "split_operands");
+        TFB_CUDA(p.complex_m ? launch_overlapped(ctx, split_operands_kernel<true>, dim3((unsigned)blocks, 3), dim3(256), 0, 0u, ja, jb, tables, *gate)
+                             : launch_overlapped(ctx, split_operands_kernel<false>, dim3((unsigned)blocks, 2), dim3(256), 0, 0u, ja, jb, tables, *gate));
+    }
+    g.c = (float*)p.c;
+    g.cn_e1 = p.cn_e1;
+    g.cn_s1 = p.cn_s1;
+    g.cn_s2 = p.cn_s2;
+    g.M = p.M;
+    g.N = p.N;
+    g.alpha = p.alpha;
+    g.beta = p.beta;
+    g.inv_a = inv_a;
+    g.inv_b = inv_b;
+    g.tiles_m = (uint32_t)tiles_m;
+    g.tiles_n = (uint32_t)tiles_n;
+    g.group_m = (uint32_t)env_int("TFB_TC_GROUP_M", 8);
+    g.by_split = FastDiv((uint32_t)splits);
+    g.by_batch = FastDiv(g.tiles_m * g.tiles_n);
+    g.by_group = FastDiv(g.group_m * g.tiles_n);
+    g.by_rows = FastDiv(g.group_m);
+    g.by_rows_last = FastDiv(std::max(1u, g.tiles_m % g.group_m));
+    g.n_work = (int)n_work;
+    g.status = ctx->dev_status;
+    g.half_w = half_w;
+    g.cols_fast = p.cols_fast;
+    g.gate = *gate;
+    {
+        LaunchScope ls(ctx, "contract_f16x3");
+        const dim3 grid((unsigned)(2 * std::min(n_work, slots)));
+        TFB_CUDA(g.chunks_per_split == 1
+                     ? launch_overlapped(ctx, contract_f16x3_kernel<16>, grid, dim3(F16Workers<16>::THREADS), F16Cfg::SMEM_BYTES, 0u, ma, mb, g)
+                     : launch_overlapped(ctx, contract_f16x3_kernel<8>, grid, dim3(F16Workers<8>::THREADS), F16Cfg::SMEM_BYTES, 0u, ma, mb, g));
+    }
+    if (splits > 1) {
+        LaunchScope ls(ctx, "contract_f16x3_finish");
+        TFB_CUDA(launch_overlapped(ctx, f16x3_finish_kernel, dim3((unsigned)(2 * pair_tiles), (unsigned)((2 * half_w + 31) / 32 * 4)), dim3(256), 0, 0u, g));
+    }
+    *done = true;
+    return TFB_OK;
+}
+
+}  // namespace tfb

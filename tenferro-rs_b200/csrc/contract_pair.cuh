@@ -1,0 +1,118 @@
+// What the CTA-pair kernels for single precision share: tile constants, matrix descriptors, the raster of output
+// tiles, tensor maps of outputs, and the gate that decides on the device which of two launched forms of a product runs.
+#pragma once
+#include <cuda.h>
+
+#include <numeric>
+
+#include "contract_common.cuh"
+#include "ptx_sm100.cuh"
+
+namespace tfb {
+
+constexpr int kBM = 128, kBK = 32;  // tile rows of a CTA, k per stage (32 f32 = one 128-byte swizzle row)
+constexpr int kChunk = 8;           // k-blocks accumulated inside TMEM before promotion (K = 256)
+
+// A word that a launch ahead sets to `value` when the product has to run in its general form.  The word is not
+// cleared beforehand: `value` is a number of its own for every product, so whatever else lies there reads as "not set", and
+// a replay of a recorded product that finds it set by an earlier replay runs the general form, which is always right.
+struct Gate {
+    unsigned long long* word = nullptr;
+    unsigned long long value = 0;
+    __device__ __forceinline__ bool set() const { return *(volatile unsigned long long*)word == value; }
+    // for the general form: nothing to do, since the special one has run
+    __device__ __forceinline__ bool closed() const { return word != nullptr && !set(); }
+};
+
+// Shared-memory matrix descriptor, sm_100 format: start address, leading and stride byte
+// offsets in 16-byte units, version 1 at bit 46, layout type at bits 61-63
+// (2: 128-byte swizzle of 16-byte units; 1: 128-byte swizzle of 32-byte units, the only
+// layout the tensor core accepts for MN-major 32-bit operands).
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint32_t layout) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo_bytes >> 4) << 16) | ((uint64_t)(sbo_bytes >> 4) << 32) |
+           (1ull << 46) | ((uint64_t)layout << 61);
+}
+
+// Raster of output tiles: m-tiles are visited in groups of `group_m` so that CTAs running
+// together share B panels (and the A panels of the group) through L2.
+struct TileCoord {
+    int64_t batch, tm, tn;
+};
+// In 32-bit arithmetic (the host keeps the number of work items below 2^31): a 64-bit
+// division costs several times a 32-bit one, and these run in the threads whose latency the
+// pipeline feels.
+__device__ __forceinline__ TileCoord decode_tile32(uint32_t tile, uint32_t tiles_m, uint32_t tiles_n, uint32_t group_m) {
+    TileCoord t;
+    const uint32_t tiles_per_batch = tiles_m * tiles_n;
+    const uint32_t batch = tile / tiles_per_batch;
+    tile -= batch * tiles_per_batch;
+    const uint32_t group_sz = group_m * tiles_n;
+    const uint32_t grp = tile / group_sz;
+    const uint32_t first_m = grp * group_m;
+    const uint32_t rows_in_group = min(group_m, tiles_m - first_m);
+    const uint32_t in_grp = tile - grp * group_sz;
+    const uint32_t tn = in_grp / rows_in_group;
+    t.batch = batch;
+    t.tm = first_m + (in_grp - tn * rows_in_group);
+    t.tn = tn;
+    return t;
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_fn();
+
+// The output as a rank-5 tensor [m1, m2, n1, n2, batch] for TMA stores of {32 rows, box_cols columns}
+// boxes.  `m` / `n` / `batch` are the output's M, N and batch modes in the order the kernel
+// linearises rows and columns (the operands' order), with the output's element strides in slot 2;
+// `scale` = 2 views a complex output as floats (the unit-stride row mode then holds interleaved
+// real and imaginary rows).  run_m, run_n: extent of the inner mode that the kernel's tiles never leave (0: they
+// follow the linear index).  Fails (returns false) for layouts a tensor store cannot express; the
+// kernel then keeps its per-element stores.
+bool make_output_map(void* base, const std::vector<Mode>& m, const std::vector<Mode>& n, const std::vector<Mode>& batch,
+                     int scale, int64_t run_m, int64_t run_n, int box_cols, CUtensorMap* map, int* cm_e1);
+
+// One operand of a product on split 16-bit operands, as it lies: element (row, k) of the batch's product b at
+// src[row_tab[row] + k_tab[k] + b_tab[b]].
+struct SplitOperand {
+    enum Kind { Real = 0, Parts = 1, Embedded = 2 };
+    const void* src;
+    const int64_t *row_tab, *k_tab, *b_tab;
+    int64_t rows, K, B;  // of the source (Parts, Embedded: complex elements)
+    int kind;            // Real: floats.  Parts: complex, real and imaginary part next to each other along K.  Embedded: rows 2 r and
+                         // 2 r + 1 are (Re, -Im) and (Im, Re) of alpha * element
+    int kfast, conj;
+    float2 alpha;
+    int64_t row_step, k_step;  // of a group with one mode, which needs no table (0: the table)
+    int64_t b_step;            // what all offsets of the batch are multiples of
+};
+// The step of a group of modes in tensor t, 0 where it takes a table.
+inline int64_t common_step(const std::vector<Mode>& g, int t) {
+    int64_t of = 0;
+    for (const Mode& m : g) of = std::gcd(of, m.s[t]);
+    return of;
+}
+inline int64_t one_step(const std::vector<Mode>& g, int t) { return g.size() == 1 ? g[0].s[t] : 0; }
+// C (M x N, real) = alpha * A B + beta * C through offset tables.
+struct SplitProduct {
+    SplitOperand a, b;
+    int64_t M, N, K, B;  // of the real product
+    void* c;
+    const int64_t *c_b, *c_m, *c_n;
+    // the tables above are still to be written, from these of a complex output (null: they exist): row 2 r + i at 2 c_m[r] + i
+    const int64_t *complex_b, *complex_m, *complex_n;
+    bool complex_rows;   // the doubled index is the rows' (else the columns')
+    int cn_e1;
+    int64_t cn_s1, cn_s2;
+    float alpha, beta;
+    bool cols_fast;      // the output's unit stride is along the columns
+    const std::vector<Mode> *m_modes, *n_modes;  // of the output, for offsets in closed form
+    int c_scale;         // floats of its elements
+};
+// Whether the product is worth the pass that splits its operands, which moves `extra_bytes` more than the general form's copies.
+bool split_pays(int64_t M, int64_t N, int64_t K, int64_t B, double extra_bytes);
+// Enqueues it.  `mem` holds the gate's word and has to outlive the launches that read it; *done = false: no room, nothing enqueued.
+tfb_status contract_split(tfb_ctx* ctx, const SplitProduct& p, PoolBlock* mem, Gate* gate, bool* done);
+
+}  // namespace tfb

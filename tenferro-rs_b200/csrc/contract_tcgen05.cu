@@ -34,15 +34,59 @@
 // Semantics: PrimDescriptor::{Contract, BatchedGemm}, tenferro-prims/src/lib.rs:156-168, 227-239.
 #include <cuda.h>
 
-#include "contract_common.cuh"
+#include "contract_pair.cuh"
 #include "contract_tables.h"
-#include "ptx_sm100.cuh"
 
 namespace tfb {
 
-namespace {
+EncodeTiledFn encode_fn() {
+    static EncodeTiledFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return (EncodeTiledFn)p;
+    }();
+    return fn;
+}
 
-constexpr int kBM = 128, kBK = 32;  // tile rows, k per stage (32 f32 = one 128-byte swizzle row)
+bool make_output_map(void* base, const std::vector<Mode>& m, const std::vector<Mode>& n, const std::vector<Mode>& batch,
+                     int scale, int64_t run_m, int64_t run_n, int box_cols, CUtensorMap* map, int* cm_e1) {
+    EncodeTiledFn enc = encode_fn();
+    if (!enc || m.empty() || n.empty() || m.size() > 2 || n.size() > 2 || batch.size() > 1) return false;
+    if ((uintptr_t)base % 16 != 0 || m[0].s[2] != 1) return false;
+    const int64_t e1 = scale * m[0].extent, e2 = m.size() == 2 ? m[1].extent : 1;
+    const int64_t s2 = m.size() == 2 ? scale * m[1].s[2] : 4;
+    const int64_t f1 = n[0].extent, f2 = n.size() == 2 ? n[1].extent : 1;
+    const int64_t t1 = scale * n[0].s[2], t2 = n.size() == 2 ? scale * n[1].s[2] : 4;
+    const int64_t B = batch.empty() ? 1 : batch[0].extent, bs = batch.empty() ? 4 : scale * batch[0].s[2];
+    auto aligned = [](int64_t extent, int64_t st) { return extent <= 1 || (st > 0 && st % 4 == 0); };
+    if (!aligned(e2, s2) || !aligned(f1, t1) || !aligned(f2, t2) || !aligned(B, bs)) return false;
+    // A warp's 32 rows (a box's columns) must lie inside one run of the unit-stride row mode (one run
+    // of the inner column mode): either the mode is the only one of its group, or the run length
+    // is a multiple of the box, or the kernel's tiles never cross a run (tiling inside the inner
+    // mode of a two-mode group, the same mode here).
+    const bool rows_ok = m.size() == 1 || e1 % 32 == 0 || (run_m == e1 && scale == 1);
+    const bool cols_ok = n.size() == 1 || f1 % box_cols == 0 || run_n == f1;
+    if (!rows_ok || !cols_ok) return false;
+    if (e1 >= INT32_MAX || f1 >= INT32_MAX) return false;
+    auto stride_or_dummy = [](int64_t extent, int64_t st) -> cuuint64_t { return (cuuint64_t)(extent > 1 ? st : 4) * 4; };
+    cuuint64_t dims[5] = {(cuuint64_t)e1, (cuuint64_t)e2, (cuuint64_t)f1, (cuuint64_t)f2, (cuuint64_t)B};
+    cuuint64_t strides[4] = {stride_or_dummy(e2, s2), stride_or_dummy(f1, t1), stride_or_dummy(f2, t2), stride_or_dummy(B, bs)};
+    cuuint32_t box[5] = {32, 1, (cuuint32_t)box_cols, 1, 1}, estr[5] = {1, 1, 1, 1, 1};
+    for (int i = 0; i < 4; ++i)
+        if (strides[i] % 16 != 0 || strides[i] >= (1ull << 40)) return false;
+    for (int i = 0; i < 5; ++i)
+        if (dims[i] == 0 || dims[i] > 0xffffffffull) return false;
+    if (enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
+    *cm_e1 = (int)e1;
+    return true;
+}
+
+namespace {
 
 // How one operand's tile maps onto its rank-5 tensor map.  A group (M, N or K) may hold up to
 // two non-fusable modes (inner e1, outer e2); tiles either stay inside the inner mode (INNER:
@@ -79,6 +123,7 @@ struct TcArgs {
     int k_split, kb_per_split;    // split-K: CTAs per output tile, k-blocks per CTA
     float* partial;               // split-K: [tile][split][BN cols][128 rows] raw sums
     int* status;
+    Gate gate;                    // CTA-pair kernels: the product may have run on split 16-bit operands already
     // Output through TMA tensor stores (CTA-pair kernel): finished sums are staged in shared memory,
     // 32 rows x 32 columns per warp at a time, and leave as one bulk store each.  cm_e1: extent of
     // the output's unit-stride row mode (rows of one run); row r of the M group has tensor-map
@@ -116,21 +161,6 @@ __device__ __forceinline__ TileRows tile_rows(const TcGeom& g, int64_t t, int ro
     return r;
 }
 
-// Shared-memory matrix descriptor, sm_100 format: start address, leading and stride byte
-// offsets in 16-byte units, version 1 at bit 46, layout type at bits 61-63
-// (2: 128-byte swizzle of 16-byte units; 1: 128-byte swizzle of 32-byte units, the only
-// layout the tensor core accepts for MN-major 32-bit operands).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint32_t layout) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo_bytes >> 4) << 16) | ((uint64_t)(sbo_bytes >> 4) << 32) |
-           (1ull << 46) | ((uint64_t)layout << 61);
-}
-
-
-// Raster of output tiles: m-tiles are visited in groups of `group_m` so that CTAs running
-// together share B panels (and the A panels of the group) through L2.
-struct TileCoord {
-    int64_t batch, tm, tn;
-};
 __device__ __forceinline__ TileCoord decode_tile(int64_t tile, int64_t tiles_m, int64_t tiles_n, int group_m) {
     TileCoord t;
     const int64_t tiles_per_batch = tiles_m * tiles_n;
@@ -268,7 +298,6 @@ __device__ __forceinline__ void convert_stage_bf16(const char* raw, char* out, i
     else convert_stage_bf16<NTHREADS, true, true>(raw, out, t);
 }
 
-constexpr int kChunk = 8;           // k-blocks accumulated inside TMEM before promotion (K = 256)
 constexpr int kSplitThreads = 256;  // warps 2..9
 
 template <int BN>
@@ -664,25 +693,6 @@ struct PairWork {
     TileRows tr_m;      // this CTA's rows
     TileRows tr_n[2];   // the two column halves of the tile
 };
-// decode_tile in 32-bit arithmetic (the host keeps the number of work items below 2^31): a 64-bit
-// division costs several times a 32-bit one, and these run in the threads whose latency the
-// pipeline feels.
-__device__ __forceinline__ TileCoord decode_tile32(uint32_t tile, uint32_t tiles_m, uint32_t tiles_n, uint32_t group_m) {
-    TileCoord t;
-    const uint32_t tiles_per_batch = tiles_m * tiles_n;
-    const uint32_t batch = tile / tiles_per_batch;
-    tile -= batch * tiles_per_batch;
-    const uint32_t group_sz = group_m * tiles_n;
-    const uint32_t grp = tile / group_sz;
-    const uint32_t first_m = grp * group_m;
-    const uint32_t rows_in_group = min(group_m, tiles_m - first_m);
-    const uint32_t in_grp = tile - grp * group_sz;
-    const uint32_t tn = in_grp / rows_in_group;
-    t.batch = batch;
-    t.tm = first_m + (in_grp - tn * rows_in_group);
-    t.tn = tn;
-    return t;
-}
 __device__ __forceinline__ PairWork pair_work(const TcArgs& g, int64_t w, uint32_t rank) {
     PairWork pw;
     const int64_t tiles_mp = (g.tiles_m + 1) / 2, tiles_np = (g.tiles_n + 1) / 2;
@@ -761,6 +771,11 @@ contract_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __g
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
+    if (g.gate.word) {
+        // nothing to set up where the product has run already (the answer is the same in every thread of the launch)
+        grid_dependency_wait();
+        if (g.gate.closed()) return;
+    }
     constexpr int kWarps = kSplitThreads / 32;
     constexpr int kLead = pair_lead_threads(SHORTK), kLeadWarps = kLead / 32;  // threads and warps before the workers
     // warps per CTA that arrive on the "converted" and on the "accumulator drained" barriers
@@ -1312,6 +1327,7 @@ contract_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __g
 // Split-K finish for the pair kernel: one CTA per (pair tile, rank), i.e. per 128 x 256 part.
 __global__ void __launch_bounds__(256) tf32x3_pair_splitk_finish_kernel(TcArgs g) {
     launch_begin();
+    if (g.gate.closed()) return;
     constexpr int BN = PairCfg::BN;
     const int64_t part = blockIdx.x, pair_tile = part >> 1;
     const int rank = (int)(part & 1);
@@ -1358,6 +1374,7 @@ struct RepackArgs {
     int64_t rows, K, Kp, B;
     int src_kfast;
     float* dst;
+    Gate gate;
 };
 constexpr int kRepackTile = 64;
 __device__ __forceinline__ void repack_kmajor(const RepackArgs g, float (&tile)[kRepackTile][kRepackTile + 1]) {
@@ -1399,32 +1416,18 @@ __device__ __forceinline__ void repack_kmajor(const RepackArgs g, float (&tile)[
 __global__ void __launch_bounds__(256) repack_kmajor_kernel(RepackArgs g) {
     __shared__ float tile[kRepackTile][kRepackTile + 1];
     launch_begin();
+    if (g.gate.closed()) return;
     repack_kmajor(g, tile);
 }
 __global__ void __launch_bounds__(256) repack_both_kernel(RepackArgs a, RepackArgs b) {
     __shared__ float tile[kRepackTile][kRepackTile + 1];
     launch_begin();
     const RepackArgs g = blockIdx.y == 0 ? a : b;
+    if (g.gate.closed()) return;
     repack_kmajor(g, tile);
 }
 
 // ------------------------------------------------------------------ host side
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return (EncodeTiledFn)p;
-    }();
-    return fn;
-}
-
 // One operand as TMA sees it: a rank-5 tensor [major1, major2, minor1, minor2, batch] where the
 // "major" group is the one with the unit stride (K for a K-major tile, the free group for an
 // MN-major tile) and every group holds at most two modes.
@@ -1509,47 +1512,6 @@ OperandMap make_operand_map(const ContractProblem& p, const std::vector<Mode>& f
     return out;
 }
 
-// The output as a rank-5 tensor [m1, m2, n1, n2, batch] for TMA stores of {32 rows, kBoxCols columns}
-// boxes.  `m` / `n` / `batch` are the output's M, N and batch modes in the order the kernel
-// linearises rows and columns (the operands' order), with the output's element strides in slot 2;
-// `scale` = 2 views a complex output as floats (the unit-stride row mode then holds interleaved
-// real and imaginary rows).  Fails (returns false) for layouts a tensor store cannot express; the
-// kernel then keeps its per-element stores.
-bool make_output_map(void* base, const std::vector<Mode>& m, const std::vector<Mode>& n, const std::vector<Mode>& batch,
-                     int scale, const TcGeom& ga, const TcGeom& gb, CUtensorMap* map, int* cm_e1) {
-    EncodeTiledFn enc = encode_fn();
-    if (!enc || m.empty() || n.empty() || m.size() > 2 || n.size() > 2 || batch.size() > 1) return false;
-    if ((uintptr_t)base % 16 != 0 || m[0].s[2] != 1) return false;
-    const int64_t e1 = scale * m[0].extent, e2 = m.size() == 2 ? m[1].extent : 1;
-    const int64_t s2 = m.size() == 2 ? scale * m[1].s[2] : 4;
-    const int64_t f1 = n[0].extent, f2 = n.size() == 2 ? n[1].extent : 1;
-    const int64_t t1 = scale * n[0].s[2], t2 = n.size() == 2 ? scale * n[1].s[2] : 4;
-    const int64_t B = batch.empty() ? 1 : batch[0].extent, bs = batch.empty() ? 4 : scale * batch[0].s[2];
-    auto aligned = [](int64_t extent, int64_t st) { return extent <= 1 || (st > 0 && st % 4 == 0); };
-    if (!aligned(e2, s2) || !aligned(f1, t1) || !aligned(f2, t2) || !aligned(B, bs)) return false;
-    // A warp's 32 rows (a box's columns) must lie inside one run of the unit-stride row mode (one run
-    // of the inner column mode): either the mode is the only one of its group, or the run length
-    // is a multiple of the box, or the kernel's tiles never cross a run (tiling inside the inner
-    // mode of a two-mode group, the same mode here).
-    const bool rows_ok = m.size() == 1 || e1 % 32 == 0 || (!ga.pack && ga.e1 == e1 && scale == 1);
-    const bool cols_ok = n.size() == 1 || f1 % kBoxCols == 0 || (!gb.pack && gb.e1 == f1);
-    if (!rows_ok || !cols_ok) return false;
-    if (e1 >= INT32_MAX || f1 >= INT32_MAX) return false;
-    auto stride_or_dummy = [](int64_t extent, int64_t st) -> cuuint64_t { return (cuuint64_t)(extent > 1 ? st : 4) * 4; };
-    cuuint64_t dims[5] = {(cuuint64_t)e1, (cuuint64_t)e2, (cuuint64_t)f1, (cuuint64_t)f2, (cuuint64_t)B};
-    cuuint64_t strides[4] = {stride_or_dummy(e2, s2), stride_or_dummy(f1, t1), stride_or_dummy(f2, t2), stride_or_dummy(B, bs)};
-    cuuint32_t box[5] = {32, 1, kBoxCols, 1, 1}, estr[5] = {1, 1, 1, 1, 1};
-    for (int i = 0; i < 4; ++i)
-        if (strides[i] % 16 != 0 || strides[i] >= (1ull << 40)) return false;
-    for (int i = 0; i < 5; ++i)
-        if (dims[i] == 0 || dims[i] > 0xffffffffull) return false;
-    if (enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
-    *cm_e1 = (int)e1;
-    return true;
-}
-
 // Split K when the tiles alone leave SMs idle: pick the split that minimises
 // (waves of CTAs) x (k-blocks per CTA + a fixed cost for prologue, epilogue and the finishing
 // pass), preferring fewer splits unless more of them save a tenth.  `slots` = tiles that run at once.
@@ -1623,6 +1585,28 @@ tfb_status launch_tc(tfb_ctx* ctx, const OperandMap& a, const OperandMap& b, TcA
     return TFB_OK;
 }
 
+// Tiles, K ranges and the scratch of a product on CTA pairs; nothing is enqueued.
+tfb_status prepare_tc_pair(tfb_ctx* ctx, const OperandMap& a, const OperandMap& b, TcArgs* g, PoolBlock* ws) {
+    g->a = a.geom;
+    g->b = b.geom;
+    auto tiles = [](const TcGeom& o, int64_t total, int rows) -> int64_t {
+        if (o.pack) return (total + rows - 1) / rows;
+        return (total / o.e1) * o.tiles1;
+    };
+    g->tiles_m = tiles(g->a, g->M, kBM);  // 128-row tiles; a pair takes two of each
+    g->tiles_n = tiles(g->b, g->N, g->half_w);
+    g->group_m = env_int("TFB_TC_GROUP_M", 8);
+    const int64_t pair_tiles = ((g->tiles_m + 1) / 2) * ((g->tiles_n + 1) / 2) * g->B;
+    choose_k_split(g, pair_tiles, ctx->sm_count / 2);
+    const int64_t n_work = pair_tiles * g->k_split;
+    if (2 * n_work > 0x7fffffff) return fail(TFB_ERR_INVALID_ARGUMENT, "contraction too large for one launch");
+    if (g->k_split > 1) {
+        TFB_TRY(ws->alloc(ctx, (size_t)(2 * n_work) * PairCfg::BN * kBM * sizeof(float)));
+        g->partial = (float*)ws->ptr;
+    }
+    return TFB_OK;
+}
+
 tfb_status launch_tc_pair(tfb_ctx* ctx, const OperandMap& a, const OperandMap& b, const CUtensorMap* c_map, TcArgs g) {
     using Cfg = PairCfg;
     static std::mutex mu;
@@ -1645,28 +1629,10 @@ tfb_status launch_tc_pair(tfb_ctx* ctx, const OperandMap& a, const OperandMap& b
             configured[ctx->device] = true;
         }
     }
-    g.a = a.geom;
-    g.b = b.geom;
-    auto tiles = [](const TcGeom& o, int64_t total, int rows) -> int64_t {
-        if (o.pack) return (total + rows - 1) / rows;
-        return (total / o.e1) * o.tiles1;
-    };
-    g.tiles_m = tiles(g.a, g.M, kBM);  // 128-row tiles; a pair takes two of each
-    if (g.half_w == 0) g.half_w = 128;
-    g.tiles_n = tiles(g.b, g.N, g.half_w);
-    g.group_m = env_int("TFB_TC_GROUP_M", 8);
-    const int64_t pair_tiles = ((g.tiles_m + 1) / 2) * ((g.tiles_n + 1) / 2) * g.B;
-    choose_k_split(&g, pair_tiles, ctx->sm_count / 2);
-    const int64_t n_work = pair_tiles * g.k_split;
-    if (2 * n_work > 0x7fffffff) return fail(TFB_ERR_INVALID_ARGUMENT, "contraction too large for one launch");
+    const int64_t pair_tiles = ((g.tiles_m + 1) / 2) * ((g.tiles_n + 1) / 2) * g.B, n_work = pair_tiles * g.k_split;
     // one CTA per SM, so at most sm_count / 2 pairs run at once; each walks the work list with that stride
     const int64_t grid = 2 * std::min<int64_t>(n_work, std::max(1, ctx->sm_count / 2));
-    PoolBlock ws;
-    const bool via_partials = g.k_split > 1;
-    if (via_partials) {
-        TFB_TRY(ws.alloc(ctx, (size_t)(2 * n_work) * Cfg::BN * kBM * sizeof(float)));
-        g.partial = (float*)ws.ptr;
-    }
+    const bool via_partials = g.partial != nullptr;
     // Split-K partials leave through the finishing kernel; a fused multiplier through the scalar path.
     if (via_partials || g.mul || !c_map) g.c_tma = 0;
     const CUtensorMap& mc = (g.c_tma && c_map) ? *c_map : a.map;  // unused when c_tma is off
@@ -1832,7 +1798,8 @@ static thread_local bool role_exchanged = false;
 
 tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declined, const int64_t* const* c_tables,
                             const std::vector<Mode>* c_n_modes, int c_scale, const std::vector<Mode>* c_m_modes,
-                            const std::vector<Mode>* c_batch_modes) {
+                            const std::vector<Mode>* c_batch_modes, const SplitProduct* split,
+                            const std::function<tfb_status(const Gate&)>* set_up) {
     const std::vector<Mode>* cn_modes = c_tables ? c_n_modes : &p.n;
     const std::vector<Mode>* cm_modes = c_tables ? c_m_modes : &p.m;
     const std::vector<Mode>* cb_modes = c_tables ? c_batch_modes : &p.batch;
@@ -1855,7 +1822,19 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
         role_exchanged = true;
         // With offset tables from the caller (the Complex32 embedding) the new columns are the caller's
         // rows, which only its table describes: no closed form for them and no tensor-store map.
-        const tfb_status st = c_tables ? contract_tcgen05(ctx, q, declined, swapped, nullptr, c_scale, nullptr, c_batch_modes)
+        SplitProduct other;
+        if (split) {
+            other = *split;
+            std::swap(other.a, other.b);
+            std::swap(other.M, other.N);
+            std::swap(other.c_m, other.c_n);
+            other.complex_rows = !other.complex_rows;
+            other.cols_fast = !other.cols_fast;
+            std::swap(other.m_modes, other.n_modes);
+            other.cn_e1 = 0;
+        }
+        const tfb_status st = c_tables ? contract_tcgen05(ctx, q, declined, swapped, nullptr, c_scale, nullptr, c_batch_modes,
+                                                          split ? &other : nullptr, set_up)
                                        : contract_tcgen05(ctx, q, declined);
         role_exchanged = false;
         return st;
@@ -1879,6 +1858,10 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
     narrow(&b);
     std::shared_ptr<ContractTables> t;
     PoolBlock packed_a, packed_b;
+    RepackArgs job[2];
+    int n_jobs = 0;
+    int64_t tiles[2] = {0, 0};
+    double copied_rows = 0;  // of operands that are copied, split or not
     // Large products only: repack an operand that has no tensor map, or whose tiles would be
     // more than a third padding.
     if (!c_tables && 2.0 * M * N * K >= kTcCopyFlops && p.batch.size() <= 1 && p.k.size() <= 2) {
@@ -1908,9 +1891,7 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
             ContractArgs ca;
             fill_args(p, t.get(), &ca);
             const int64_t Kp = (K + 3) / 4 * 4, Bn = p.B();
-            RepackArgs job[2];
-            int n_jobs = 0;
-            int64_t tiles[2] = {0, 0};
+            copied_rows = (pack_a ? (double)M : 0) + (pack_b ? (double)N : 0);
             auto repack = [&](int tns, PoolBlock* blk, OperandMap* out) -> tfb_status {
                 const int64_t rows = tns == 0 ? M : N;
                 const tfb_status got = blk->alloc(ctx, (size_t)(rows * Kp * Bn) * sizeof(float));
@@ -1921,7 +1902,7 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
                 tiles[n_jobs] = ((rows + kRepackTile - 1) / kRepackTile) * ((Kp + kRepackTile - 1) / kRepackTile) * Bn;
                 job[n_jobs++] =
                     RepackArgs{(const float*)(tns == 0 ? p.a : p.b), tns == 0 ? t->a_m : t->b_n, tns == 0 ? t->a_k : t->b_k,
-                               tns == 0 ? t->a_b : t->b_b, rows, K, Kp, Bn, tns == 0 ? ca.a_kfast : ca.b_kfast, (float*)blk->ptr};
+                               tns == 0 ? t->a_b : t->b_b, rows, K, Kp, Bn, tns == 0 ? ca.a_kfast : ca.b_kfast, (float*)blk->ptr, Gate{}};
                 // the same product with this operand contiguous: one free mode, K split as in the other operand
                 ContractProblem q = p;
                 std::vector<Mode> free_q{Mode{rows, {0, 0, 0}}};
@@ -1936,20 +1917,6 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
             if (pack_b) {
                 TFB_TRY(repack(1, &packed_b, &b));
                 narrow(&b);
-            }
-            // Small copies are bound by latency and run side by side in one launch; larger ones fill the chip one by one, in a
-            // kernel that keeps one operand's parameters (us in one launch, in two: 801 x 805 x 803, 338 tiles, 35.8, 38.2; 4001 x
-            // 4003 x 303, 630, 91.2, 93.7; 1401 x 1405 x 1403, 968, 60.2, 58.8; 4001 x 4003 x 2999, 5922, 456, 447).
-            auto blocks = [&](int64_t t) { return (unsigned)std::min<int64_t>(t, (int64_t)ctx->sm_count * 16); };
-            if (n_jobs == 2 && tiles[0] + tiles[1] <= (int64_t)ctx->sm_count * 5) {
-                LaunchScope ls(ctx, "repack_operand");
-                TFB_CUDA(launch_overlapped(ctx, repack_both_kernel, dim3(blocks(std::max(tiles[0], tiles[1])), 2), dim3(256), 0, 0u, job[0],
-                                           job[1]));
-            } else {
-                for (int j = 0; j < n_jobs; ++j) {
-                    LaunchScope ls(ctx, "repack_operand");
-                    TFB_CUDA(launch_overlapped(ctx, repack_kmajor_kernel, dim3(blocks(tiles[j])), dim3(256), 0, 0u, job[j]));
-                }
             }
         }
     }
@@ -1994,10 +1961,68 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
     if (pair && g.beta == 0.f && !p.mul && g.cn_e1 != 0 && cm_modes && cn_modes && cb_modes &&
         env_int("TFB_TC_TMA_STORE", 1)) {
         int cm_e1 = 0;
-        have_c_map = make_output_map(p.c, *cm_modes, *cn_modes, *cb_modes, c_scale, a.geom, b.geom, &c_map, &cm_e1);
+        have_c_map = make_output_map(p.c, *cm_modes, *cn_modes, *cb_modes, c_scale, a.geom.pack ? 0 : a.geom.e1, b.geom.pack ? 0 : b.geom.e1,
+                                     kBoxCols, &c_map, &cm_e1);
         if (have_c_map) {
             g.c_tma = 1;
             g.cm_e1 = cm_e1;
+        }
+    }
+    PoolBlock ws, halves;
+    if (pair) {
+        TFB_TRY(prepare_tc_pair(ctx, a, b, &g, &ws));
+        // With everything that the general form needs in hand, the product may run on operands split into 16-bit halves; what
+        // follows is then enqueued behind a gate that the splitting pass opens where the operands' range asks for it.
+        SplitProduct own;
+        if (!split && !c_tables && !p.mul && split_pays(M, N, K, g.B, 8.0 * ((double)(M + N) - copied_rows) * (double)K * (double)g.B)) {
+            if (!t) TFB_TRY(get_tables(ctx, p, &t));
+            ContractArgs ca;
+            fill_args(p, t.get(), &ca);
+            own = SplitProduct{};
+            own.a = SplitOperand{p.a, t->a_m, t->a_k, t->a_b, M, K, g.B, SplitOperand::Real, ca.a_kfast, 0, make_float2(1.f, 0.f),
+                                 one_step(p.m, 0), one_step(p.k, 0), common_step(p.batch, 0)};
+            own.b = SplitOperand{p.b, t->b_n, t->b_k, t->b_b, N, K, g.B, SplitOperand::Real, ca.b_kfast, 0, make_float2(1.f, 0.f),
+                                 one_step(p.n, 1), one_step(p.k, 1), common_step(p.batch, 1)};
+            own.M = M;
+            own.N = N;
+            own.K = K;
+            own.B = g.B;
+            own.c = p.c;
+            own.c_b = g.c_b;
+            own.c_m = g.c_m;
+            own.c_n = g.c_n;
+            own.cn_e1 = g.cn_e1;
+            own.cn_s1 = g.cn_s1;
+            own.cn_s2 = g.cn_s2;
+            own.alpha = g.alpha;
+            own.beta = g.beta;
+            own.m_modes = cm_modes;
+            own.n_modes = cn_modes;
+            own.c_scale = 1;
+            own.cols_fast = !p.n.empty() && std::llabs(p.n[0].s[2]) == 1;
+            split = &own;
+        }
+        if (split) {
+            bool done = false;
+            TFB_TRY(contract_split(ctx, *split, &halves, &g.gate, &done));
+        }
+    }
+    if (set_up) TFB_TRY((*set_up)(g.gate));
+    for (int j = 0; j < n_jobs; ++j) job[j].gate = g.gate;
+    // Small copies are bound by latency and run side by side in one launch; larger ones fill the chip one by one, in a
+    // kernel that keeps one operand's parameters (us in one launch, in two: 801 x 805 x 803, 338 tiles, 35.8, 38.2; 4001 x
+    // 4003 x 303, 630, 91.2, 93.7; 1401 x 1405 x 1403, 968, 60.2, 58.8; 4001 x 4003 x 2999, 5922, 456, 447).
+    // Behind a gate they have fewer blocks, which as a rule return at once.
+    const bool gated = g.gate.word != nullptr;
+    auto blocks = [&](int64_t t) { return (unsigned)std::min<int64_t>(t, (int64_t)ctx->sm_count * (gated ? 8 : 16)); };
+    if (n_jobs == 2 && tiles[0] + tiles[1] <= (int64_t)ctx->sm_count * 5) {
+        LaunchScope ls(ctx, "repack_operand");
+        TFB_CUDA(launch_overlapped(ctx, repack_both_kernel, dim3(blocks(std::max(tiles[0], tiles[1])), 2), dim3(256), 0, 0u, job[0],
+                                   job[1]));
+    } else {
+        for (int j = 0; j < n_jobs; ++j) {
+            LaunchScope ls(ctx, "repack_operand");
+            TFB_CUDA(launch_overlapped(ctx, repack_kmajor_kernel, dim3(blocks(tiles[j])), dim3(256), 0, 0u, job[j]));
         }
     }
     if (pair) return launch_tc_pair(ctx, a, b, have_c_map ? &c_map : nullptr, g);

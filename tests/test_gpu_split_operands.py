@@ -1,0 +1,162 @@
+"""Single precision products on operands split into two 16-bit floats (TFB_TC_SPLIT16=2 takes every product of the CTA-pair
+kernels there, 0 none), against float64 and against the TF32 form, over orders, strides, odd sizes and the edges of tiles,
+chunks of K and output runs."""
+import numpy as np
+import pytest
+
+from conftest import Strided, random_array
+
+pytestmark = pytest.mark.gpu
+
+# Rounding of 22-bit operands (2^-22 each, 2.4e-7) and the truncating sums of 256 of K in tensor memory, 48 MMAs at 2^-25 each:
+# 1.4e-6 at most, whatever K is; measured 5e-7 to 9.4e-7.
+BOUND = 1.7e-6
+
+
+def contract(tb, a, b, c, la, lb, lc, alpha, beta, monkeypatch, split):
+    monkeypatch.setenv("TFB_TC_SPLIT16", str(split))
+    shapes = [x.logical.shape if isinstance(x, Strided) else x.shape for x in (a, b, c)]
+    plan = tb.CudaBackend.plan(tb.PrimDescriptor.Contract(la, lb, lc), shapes, c.logical.dtype)
+    out = c.to_device(tb)
+    ctx = tb.Context.get(0)
+    ctx.profile_begin()
+    tb.CudaBackend.execute(plan, alpha, [a.to_device(tb), b.to_device(tb)], beta, out)
+    ctx.synchronize()
+    ran = ctx.profile_read("contract_f16x3")[0]
+    ctx.profile_end()
+    # what TMA cannot describe and is too small to copy runs on the exact kernel in either case
+    assert ran == (1 if split and plan.kernel_name == "tcgen05_tf32x3" else 0)
+    return out.to_numpy(), ran
+
+
+CASES = [
+    # labels and extents: rows i.., columns j.., contracted k.., batch b
+    ("ik,kj->ij", dict(i=129, j=256, k=1024)), ("ik,kj->ij", dict(i=256, j=256, k=2048)), ("ik,kj->ij", dict(i=257, j=511, k=3871)),
+    ("ik,kj->ij", dict(i=640, j=520, k=256)), ("ik,kj->ij", dict(i=1700, j=1640, k=255)), ("ik,kj->ij", dict(i=4001, j=3999, k=33)),
+    ("ik,kj->ij", dict(i=2100, j=40, k=513)), ("ik,kj->ij", dict(i=97, j=4100, k=300)), ("ik,kj->ij", dict(i=300, j=130, k=9000)),
+    ("ki,jk->ij", dict(i=515, j=770, k=320)), ("ki,kj->ji", dict(i=515, j=770, k=321)),
+    ("bik,bkj->bij", dict(b=3, i=300, j=270, k=300)), ("kib,bjk->jbi", dict(b=2, i=261, j=400, k=290)),
+    ("ilk,kjm->ijlm", dict(i=45, l=17, k=310, j=20, m=23)),       # column runs shorter than sixteen apart, rows in two modes
+    ("ilk,kjm->imlj", dict(i=96, l=7, k=192, j=11, m=48)),
+    ("ilkn,nkjm->mjil", dict(i=12, l=25, k=40, n=9, j=24, m=16)),  # two contracted modes, opposite orders
+]
+
+
+@pytest.mark.parametrize("layout", ["col", "row", "random"])
+@pytest.mark.parametrize("case", CASES, ids=lambda c: c[0] + "-" + "x".join(str(v) for v in c[1].values()))
+@pytest.mark.parametrize("dtype", [np.float32, np.complex64])
+def test_split_operands_in_every_order(tb, oracle, dtype, case, layout, monkeypatch):
+    notation, size = case
+    rng = np.random.default_rng(sum(map(ord, notation)) + sum(size.values()))
+    ins, out = notation.split("->")
+    labels = [[ord(x) - 97 for x in t] for t in ins.split(",") + [out]]
+    shapes = [tuple(size[x] for x in t) for t in ins.split(",") + [out]]
+    cplx = dtype == np.complex64
+    a, b = (Strided(random_array(rng, s, dtype), rng, layout, conj=cplx and t == 1) for t, s in enumerate(shapes[:2]))
+    for alpha, beta in ((1.0, 0.0), ((0.5 - 0.25j, 1.5j) if cplx else (-1.5, 0.5))):
+        c = Strided(random_array(rng, shapes[2], dtype), rng, layout if layout != "random" else "col")
+        got, ran = contract(tb, a, b, c, *labels, alpha, beta, monkeypatch, 2)
+        assert ran or not cplx
+        want = oracle.np_contract(labels[0], a.logical, labels[1], b.logical, labels[2], alpha, beta, c.logical)
+        general, _ = contract(tb, a, b, c, *labels, alpha, beta, monkeypatch, 0)
+        err, err0 = oracle.rel_frobenius(got, want), oracle.rel_frobenius(general, want)
+        assert err <= BOUND, err
+        assert err <= err0 + 1e-7, (err, err0)  # no further off than the general form
+
+
+def product(tb, a, b, monkeypatch, split, beta=0.0, c0=None):
+    monkeypatch.setenv("TFB_TC_SPLIT16", str(split))
+    out = tb.Tensor.from_numpy(c0.copy()) if c0 is not None else tb.Tensor.zeros((a.shape[0], b.shape[1]), dtype=a.dtype)
+    tb.einsum_into("ik,kj->ij", [tb.Tensor.from_numpy(a), tb.Tensor.from_numpy(b)], 1.0, beta, out)
+    return out.to_numpy()
+
+
+def wide_spread(rng, a, b):
+    a *= np.exp2(rng.integers(-12, 13, a.shape)).astype(a.dtype)
+
+
+def one_row(rng, a, b):  # one row of one operand, in one chunk of K, is enough
+    b[b.shape[0] // 2:b.shape[0] // 2 + 20, -1] *= np.float32(1e9)
+
+
+def infinite(rng, a, b):
+    a[5, 7] = np.inf
+
+
+def nan(rng, a, b):
+    b[3, 9] = np.nan
+
+
+def huge(rng, a, b):
+    a[17] *= np.float32(1e31)
+
+
+@pytest.mark.parametrize("spoil", [wide_spread, one_row, infinite, nan, huge])
+@pytest.mark.parametrize("shape", [(520, 600, 700), (260, 96, 4000), (130, 2048, 256)])
+@pytest.mark.parametrize("dtype", [np.float32, np.complex64])
+def test_wide_ranges_run_in_the_general_form(tb, oracle, dtype, shape, spoil, monkeypatch):
+    """Elements far below the largest of their row and chunk, infinities, NaN and magnitudes near the end of the range: bit for
+    bit what the TF32 form gives, the old output included once."""
+    m, n, k = shape
+    rng = np.random.default_rng(m + n + k)
+    a, b = random_array(rng, (m, k), dtype), random_array(rng, (k, n), dtype)
+    spoil(rng, a, b)
+    c0 = random_array(rng, (m, n), dtype)
+    with np.errstate(all="ignore"):
+        for beta in (0.0, 0.5):
+            got = product(tb, a, b, monkeypatch, 2, beta, c0)
+            want = product(tb, a, b, monkeypatch, 0, beta, c0)
+            assert np.array_equal(got, want, equal_nan=True)
+    # the next product of ordinary operands is not held back by it
+    a, b = random_array(rng, (m, k), dtype), random_array(rng, (k, n), dtype)
+    assert oracle.rel_frobenius(product(tb, a, b, monkeypatch, 2), oracle.np_einsum("ik,kj->ij", [a, b])) <= BOUND
+
+
+@pytest.mark.parametrize("low,high", [(-90, 90), (-140, -60), (20, 60)])
+def test_rows_of_any_magnitude(tb, oracle, low, high, monkeypatch):
+    """Scales are a row's own: rows of the first operand and columns of the second spread over the range, each
+    compared by itself; subnormal rows keep what f32 holds of them."""
+    rng = np.random.default_rng(high - low)
+    m, n, k = 384, 300, 600
+    a, b = random_array(rng, (m, k), np.float32), random_array(rng, (k, n), np.float32)
+    ea, eb = np.linspace(low, high, m).round(), np.linspace(-20, 20, n).round()
+    a = (a * np.exp2(ea)[:, None]).astype(np.float32)
+    b = (b * np.exp2(eb)[None, :]).astype(np.float32)
+    got = product(tb, a, b, monkeypatch, 2).astype(np.float64)
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    keep = np.abs(want).max(axis=1) > 1e-30  # results that are normal numbers in every column
+    err = np.linalg.norm(got - want, axis=1)[keep] / np.linalg.norm(want, axis=1)[keep]
+    assert err.max() <= 2 * BOUND  # (the largest of 384 rows)
+
+
+def test_exact_operands_stay_exact(tb, monkeypatch):
+    """Small integers are halves without a rest, and their sums below 2^24 come out exact, also after many chunks of K."""
+    rng = np.random.default_rng(6)
+    a, b = rng.integers(-8, 9, (400, 5000)).astype(np.float32), rng.integers(-8, 9, (5000, 333)).astype(np.float32)
+    assert np.array_equal(product(tb, a, b, monkeypatch, 2), (a.astype(np.float64) @ b.astype(np.float64)).astype(np.float32))
+
+
+def test_replays_see_new_operands(tb, oracle, monkeypatch):
+    """A captured product of this form: replays read the operands anew, and one of wide range takes the general form."""
+    monkeypatch.setenv("TFB_TC_SPLIT16", "2")
+    rng = np.random.default_rng(8)
+    m, n, k = 300, 280, 520
+    arrays = [(random_array(rng, (m, k), np.float32), random_array(rng, (k, n), np.float32)) for _ in range(3)]
+    wide_spread(rng, *arrays[1])
+    ta, tb_ = (tb.Tensor.from_numpy(x) for x in arrays[0])
+    out = tb.Tensor.zeros((m, n), dtype=np.float32)
+    ctx = tb.Context.get(0)
+    tree = tb.ContractionTree.optimize(tb.Subscripts.parse("ik,kj->ij"), [(m, k), (k, n)])
+    tb.einsum_with_plan_into(tree, [ta, tb_], 1.0, 0.0, out)
+    ctx.synchronize()
+    ctx.capture_begin()
+    tb.einsum_with_plan_into(tree, [ta, tb_], 1.0, 0.0, out)
+    graph = ctx.capture_end()
+    for a, b in arrays:
+        for dst, src in ((ta, a), (tb_, b)):
+            fresh = tb.Tensor.from_numpy(src)
+            tb.einsum_into("ij->ij", [fresh], 1.0, 0.0, dst)
+        ctx.synchronize()
+        graph.launch()
+        ctx.synchronize()
+        assert oracle.rel_frobenius(out.to_numpy(), oracle.np_einsum("ik,kj->ij", [a, b])) <= 2e-6
