@@ -123,6 +123,7 @@ struct TcArgs {
     int k_split, kb_per_split;    // split-K: CTAs per output tile, k-blocks per CTA
     float* partial;               // split-K: [tile][split][BN cols][128 rows] raw sums
     int* status;
+    int cols_fast;                // the output's unit stride is along the columns
     Gate gate;                    // CTA-pair kernels: the product may have run on split 16-bit operands already
     // Output through TMA tensor stores (CTA-pair kernel): finished sums are staged in shared memory,
     // 32 rows x 32 columns per warp at a time, and leave as one bulk store each.  cm_e1: extent of
@@ -1324,8 +1325,12 @@ contract_tf32x3_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     }
 }
 
-// Split-K finish for the pair kernel: one CTA per (pair tile, rank), i.e. per 128 x 256 part.
+// Split-K finish for the pair kernel: 32 x 32 elements of a 128 x 256 part of a tile a block.  The sums lie with rows next to each
+// other; where the output's unit stride runs along the columns (a narrow product whose operands exchanged roles) the patch is turned in shared
+// memory, or every store would be a sector (9216 x 192 of complex parts, two ranges: 20.5 us stored by rows, 14.3 so).  Four columns a
+// thread in flight (two columns of eight a pass before: 1024^3, 33.6 us a call then, 29.4 so).
 __global__ void __launch_bounds__(256) tf32x3_pair_splitk_finish_kernel(TcArgs g) {
+    __shared__ float patch[32][33];
     launch_begin();
     if (g.gate.closed()) return;
     constexpr int BN = PairCfg::BN;
@@ -1333,31 +1338,48 @@ __global__ void __launch_bounds__(256) tf32x3_pair_splitk_finish_kernel(TcArgs g
     const int rank = (int)(part & 1);
     const int64_t tiles_mp = (g.tiles_m + 1) / 2, tiles_np = (g.tiles_n + 1) / 2;
     const TileCoord tc = decode_tile(pair_tile, tiles_mp, tiles_np, g.group_m);
-    if (2 * tc.tm + rank >= g.tiles_m) return;
-    const TileRows tr_m = tile_rows(g.a, 2 * tc.tm + rank, kBM, g.M);
-    const int row = threadIdx.x & (kBM - 1);
-    if (row >= tr_m.valid) return;
-    float* C = reinterpret_cast<float*>(g.c) + g.c_b[tc.batch];
-    const int64_t cm = g.c_m[tr_m.base + row];
+    const int c0 = (int)(blockIdx.y >> 2) * 32, r0 = (int)(blockIdx.y & 3) * 32, h = c0 / 128, j0 = c0 % 128;
+    if (2 * tc.tm + rank >= g.tiles_m || 2 * tc.tn + h >= g.tiles_n) return;
+    const TileRows tr_m = tile_rows(g.a, 2 * tc.tm + rank, kBM, g.M), tr_n = tile_rows(g.b, 2 * tc.tn + h, g.half_w, g.N);
+    const int rows = min(32, tr_m.valid - r0), cols = min(32, tr_n.valid - j0);
+    if (rows <= 0 || cols <= 0) return;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const float* P = g.partial + ((size_t)part * g.k_split * BN + c0) * kBM + r0 + tx;
+    float sum[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[i] = 0.f;
+#pragma unroll 2
+    for (int s = 0; s < g.k_split; ++s)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (tx < rows && ty + 8 * i < cols) sum[i] += P[((size_t)s * BN + ty + 8 * i) * kBM];
+    if (g.cols_fast) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) patch[ty + 8 * i][tx] = sum[i];
+        __syncthreads();
+    }
     const bool read_c = g.beta != 0.f;
-    const float* P = g.partial + (size_t)part * g.k_split * BN * kBM + row;
-    const float* D = g.mul ? g.mul + g.d_b[tc.batch] + g.d_m[tr_m.base + row] : nullptr;
-    // blockIdx.y takes kFinishCols columns of one of the two 128-column halves
-    {
-        const int h = (int)(blockIdx.y * kFinishCols) / 128, j0 = (int)(blockIdx.y * kFinishCols) % 128;
-        if (2 * tc.tn + h >= g.tiles_n) return;
-        const TileRows trn = tile_rows(g.b, 2 * tc.tn + h, g.half_w, g.N);
-        const int j_end = min(trn.valid, j0 + kFinishCols);
-        for (int j = j0 + threadIdx.x / kBM; j < j_end; j += 256 / kBM) {
-            float sum = 0.f;
-#pragma unroll 8
-            for (int s = 0; s < g.k_split; ++s) sum += P[((size_t)s * BN + h * 128 + j) * kBM];
-            float* p = C + cm + g.c_n[trn.base + j];
-            float v = g.alpha * sum;
-            if (D) v *= D[g.d_n[trn.base + j]];
-            if (read_c) v += g.beta * *p;
-            *p = v;
-        }
+    float* C = reinterpret_cast<float*>(g.c) + g.c_b[tc.batch];
+    const float* D = g.mul ? g.mul + g.d_b[tc.batch] : nullptr;
+    float* at[4];
+    float old[4], mul[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = g.cols_fast ? ty + 8 * i : tx, c = g.cols_fast ? tx : ty + 8 * i;
+        const bool live = r < rows && c < cols;
+        const int64_t m = tr_m.base + r0 + r, n = tr_n.base + j0 + c;
+        at[i] = live ? C + g.c_m[m] + g.c_n[n] : nullptr;
+        if (g.cols_fast) sum[i] = patch[c][r];
+        mul[i] = D && live ? D[g.d_m[m] + g.d_n[n]] : 1.f;
+        old[i] = read_c && live ? *at[i] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (!at[i]) continue;
+        float v = g.alpha * sum[i];
+        if (D) v *= mul[i];
+        if (read_c) v += g.beta * old[i];
+        *at[i] = v;
     }
 }
 
@@ -1662,7 +1684,7 @@ tfb_status launch_tc_pair(tfb_ctx* ctx, const OperandMap& a, const OperandMap& b
     }
     if (via_partials) {
         LaunchScope ls(ctx, "contract_tf32x3_finish");
-        TFB_CUDA(launch_overlapped(ctx, tf32x3_pair_splitk_finish_kernel, dim3((unsigned)(2 * pair_tiles), Cfg::BN / kFinishCols),
+        TFB_CUDA(launch_overlapped(ctx, tf32x3_pair_splitk_finish_kernel, dim3((unsigned)(2 * pair_tiles), Cfg::BN / 32 * 4),
                                    dim3(256), 0, 0u, g));
     }
     return TFB_OK;
@@ -1949,6 +1971,8 @@ tfb_status contract_tcgen05(tfb_ctx* ctx, const ContractProblem& p, bool* declin
     g.half_w = half_w ? half_w : 128;
     g.alpha = (float)p.alpha.re;
     g.beta = (float)p.beta.re;
+    // (columns that only the caller's tables describe are parts of complex numbers)
+    g.cols_fast = c_tables ? cn_modes == nullptr : !p.n.empty() && std::llabs(p.n[0].s[2]) == 1;
     // Both operands walk K in the same blocks: 32 at a time inside the inner K mode.
     g.k_e1 = (int)p.k[0].extent;
     g.k_blocks1 = (g.k_e1 + kBK - 1) / kBK;
