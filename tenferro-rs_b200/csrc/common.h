@@ -88,6 +88,17 @@ struct tfb_ctx {
         cudaEvent_t start, stop;
     };
     std::vector<ProfRec> prof;
+    // Pool memory given up a moment ago, for the next allocation of its size: a call's intermediates and scratch come and go with every
+    // call, and the driver takes about a microsecond for each.  This queue is in order, so whoever is handed a block enqueues behind
+    // the work that used it.  Bounded; given back when an allocation fails and with the context.
+    struct Kept {
+        void* ptr;
+        size_t bytes;
+    };
+    static constexpr size_t kKeptBlocks = 16, kKeptBytes = (size_t)64 << 20;
+    std::vector<Kept> kept;
+    size_t kept_bytes = 0;
+    std::mutex kept_mu;
     bool capturing = false;  // between tfb_ctx_capture_begin and _end: launches are recorded, not run
     std::vector<void*> capture_keeps;  // pool memory that the recorded launches read: the graph's from capture_end on
     std::vector<void*> free_later;     // pool memory given up while capturing: freed by capture_end
@@ -104,6 +115,7 @@ struct tfb_graph {
 struct tfb_event {
     cudaEvent_t ev = nullptr;
     int device = 0;
+    bool recorded = false;  // (not while its context was capturing)
 };
 
 namespace tfb {
@@ -228,6 +240,7 @@ tfb_status contract_c32_embedded(tfb_ctx* ctx, const ContractProblem& p, bool* d
 struct PoolBlock {
     tfb_ctx* ctx = nullptr;
     void* ptr = nullptr;
+    size_t bytes = 0;       // 0: not for the context to keep
     bool in_graph = false;  // allocated by a node of the graph being captured
     ~PoolBlock();
     tfb_status alloc(tfb_ctx* c, size_t bytes);

@@ -5,6 +5,7 @@
 // 660-713 (CompletionEvent, to_memory_space_async, wait, is_ready).
 #include "common.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 
@@ -47,6 +48,52 @@ Scalar load_scalar(int dtype, const void* p) {
     return s;
 }
 
+// Events that nobody holds any more, for the next one recorded on their device: every call records one, and creating and destroying it
+// takes as long as the record.  A wait that has been enqueued for one keeps its meaning when the event is recorded anew.  Only events that
+// were recorded come here (one that was not reads as complete until it is), 64 a device, given back with a context of it.
+struct IdleEvents {
+    std::mutex mu;
+    std::map<int, std::vector<cudaEvent_t>> of;
+};
+static IdleEvents& idle_events() {
+    static IdleEvents* e = new IdleEvents;  // outlives whoever destroys an event at exit
+    return *e;
+}
+static cudaError_t take_event(int device, cudaEvent_t* ev) {
+    {
+        IdleEvents& e = idle_events();
+        std::lock_guard<std::mutex> lock(e.mu);
+        auto& v = e.of[device];
+        if (!v.empty()) {
+            *ev = v.back();
+            v.pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaEventCreate(ev);
+}
+static void give_event(int device, cudaEvent_t ev, bool recorded) {
+    if (recorded) {
+        IdleEvents& e = idle_events();
+        std::lock_guard<std::mutex> lock(e.mu);
+        auto& v = e.of[device];
+        if (v.size() < 64) {
+            v.push_back(ev);
+            return;
+        }
+    }
+    cudaEventDestroy(ev);
+}
+static void drop_idle_events(int device) {
+    std::vector<cudaEvent_t> all;
+    {
+        IdleEvents& e = idle_events();
+        std::lock_guard<std::mutex> lock(e.mu);
+        all.swap(e.of[device]);
+    }
+    for (cudaEvent_t ev : all) cudaEventDestroy(ev);
+}
+
 static std::atomic<unsigned long long> g_launches{0};
 void count_launch(int n) { g_launches += (unsigned long long)n; }
 unsigned long long launch_count() { return g_launches.load(); }
@@ -77,9 +124,30 @@ static void pool_free(tfb_ctx* c, void* ptr, bool in_graph) {
     DeviceGuard g(c->device);
     cudaFreeAsync(ptr, c->stream);
 }
+// Gives back what the context keeps; true if that was anything.
+static bool drop_kept(tfb_ctx* c) {
+    std::vector<tfb_ctx::Kept> all;
+    {
+        std::lock_guard<std::mutex> lock(c->kept_mu);
+        all.swap(c->kept);
+        c->kept_bytes = 0;
+    }
+    for (const auto& k : all) cudaFreeAsync(k.ptr, c->stream);
+    return !all.empty();
+}
+// Whether memory may pass from one call to the next without the driver: one stream in order, and nothing being recorded from it.
+static bool may_keep(const tfb_ctx* c) { return c->stream != cudaStreamPerThread && !is_recorded(c); }
+static cudaError_t pool_malloc(tfb_ctx* c, size_t bytes, cudaStream_t stream, void** ptr) {
+    cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, c->pool, stream);
+    if (e != cudaSuccess && !c->capturing && drop_kept(c)) {
+        cudaGetLastError();
+        e = cudaMallocFromPoolAsync(ptr, bytes, c->pool, stream);
+    }
+    return e;
+}
 static tfb_status pool_alloc(tfb_ctx* c, size_t bytes, cudaStream_t stream, void** ptr) {
     if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, c->pool, stream);
+    cudaError_t e = pool_malloc(c, bytes, stream, ptr);
     if (e != cudaSuccess) {
         cudaGetLastError();
         *ptr = nullptr;
@@ -88,12 +156,50 @@ static tfb_status pool_alloc(tfb_ctx* c, size_t bytes, cudaStream_t stream, void
     return TFB_OK;
 }
 PoolBlock::~PoolBlock() {
-    if (ptr && ctx) pool_free(ctx, ptr, in_graph);
+    if (!ptr || !ctx) return;
+    if (bytes != 0 && bytes <= tfb_ctx::kKeptBytes / 4 && may_keep(ctx)) {
+        void* out[tfb_ctx::kKeptBlocks + 1];  // what has to make room for it, oldest first
+        size_t n = 0;
+        {
+            std::lock_guard<std::mutex> lock(ctx->kept_mu);
+            auto& kept = ctx->kept;
+            while (kept.size() >= tfb_ctx::kKeptBlocks || ctx->kept_bytes + bytes > tfb_ctx::kKeptBytes) {
+                out[n++] = kept.front().ptr;
+                ctx->kept_bytes -= kept.front().bytes;
+                kept.erase(kept.begin());
+            }
+            kept.push_back({ptr, bytes});
+            ctx->kept_bytes += bytes;
+        }
+        for (size_t i = 0; i < n; ++i) pool_free(ctx, out[i], false);
+        return;
+    }
+    pool_free(ctx, ptr, in_graph);
 }
-tfb_status PoolBlock::alloc(tfb_ctx* c, size_t bytes) {
+tfb_status PoolBlock::alloc(tfb_ctx* c, size_t want) {
     ctx = c;
     in_graph = c->capturing;
-    return pool_alloc(c, bytes, c->stream, &ptr);
+    bytes = 0;
+    if (want == 0) want = 16;
+    want = (want + 511) & ~(size_t)511;  // the pool's own granularity
+    if (want <= tfb_ctx::kKeptBytes / 4 && may_keep(c)) {
+        bytes = want;
+        std::lock_guard<std::mutex> lock(c->kept_mu);
+        auto& kept = c->kept;
+        size_t best = kept.size();
+        for (size_t i = 0; i < kept.size(); ++i)
+            if (kept[i].bytes >= want && kept[i].bytes <= 2 * want && (best == kept.size() || kept[i].bytes < kept[best].bytes)) best = i;
+        if (best < kept.size()) {
+            ptr = kept[best].ptr;
+            bytes = kept[best].bytes;
+            c->kept_bytes -= bytes;
+            kept.erase(kept.begin() + best);
+            return TFB_OK;
+        }
+    }
+    const tfb_status st = pool_alloc(c, want, c->stream, &ptr);
+    if (st != TFB_OK) bytes = 0;
+    return st;
 }
 tfb_status PoolBlock::upload(tfb_ctx* c, const void* host, size_t bytes) {
     ctx = c;
@@ -120,6 +226,7 @@ tfb_status PoolBlock::upload(tfb_ctx* c, const void* host, size_t bytes) {
 void PoolBlock::keep_for_graph() {
     if (!ptr || !ctx->capturing) return;
     ctx->capture_keeps.push_back(ptr);
+    bytes = 0;
     ptr = nullptr;
 }
 
@@ -272,7 +379,9 @@ tfb_status tfb_ctx_profile_end(tfb_ctx* ctx) {
 tfb_status tfb_ctx_destroy(tfb_ctx* ctx) {
     if (!ctx) return TFB_OK;
     DeviceGuard g(ctx->device);
+    drop_kept(ctx);
     cudaStreamSynchronize(ctx->stream);
+    drop_idle_events(ctx->device);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     if (ctx->dev_status) cudaFree(ctx->dev_status);
     if (ctx->sk_partial) cudaFree(ctx->sk_partial);
@@ -414,7 +523,7 @@ tfb_status tfb_alloc(tfb_ctx* ctx, size_t bytes, void** out) {
     *out = nullptr;
     DeviceGuard g(ctx->device);
     if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMallocFromPoolAsync(out, bytes, ctx->pool, ctx->stream);
+    cudaError_t e = pool_malloc(ctx, bytes, ctx->stream, out);
     if (e != cudaSuccess) {
         *out = nullptr;
         cudaGetLastError();
@@ -438,7 +547,10 @@ tfb_status tfb_pool_stats(tfb_ctx* ctx, size_t* reserved, size_t* used) {
     TFB_CUDA(cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &r));
     TFB_CUDA(cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &u));
     if (reserved) *reserved = (size_t)r;
-    if (used) *used = (size_t)u;
+    if (used) {  // what the context keeps for its next call is nobody's
+        std::lock_guard<std::mutex> lock(ctx->kept_mu);
+        *used = (size_t)u - std::min((size_t)u, ctx->kept_bytes);
+    }
     return TFB_OK;
 }
 
@@ -515,7 +627,7 @@ tfb_status tfb_event_record(tfb_ctx* ctx, tfb_event** out) {
     DeviceGuard g(ctx->device);
     std::unique_ptr<tfb_event> ev(new tfb_event);
     ev->device = ctx->device;
-    TFB_CUDA(cudaEventCreate(&ev->ev));
+    TFB_CUDA(take_event(ctx->device, &ev->ev));
     // While the context is capturing nothing is enqueued, so there is nothing to mark: the event stays
     // unrecorded, which reads as complete (an event recorded into the capture could be neither
     // queried nor waited for from outside it).
@@ -524,6 +636,7 @@ tfb_status tfb_event_record(tfb_ctx* ctx, tfb_event** out) {
         cudaEventDestroy(ev->ev);
         return fail(TFB_ERR_DEVICE, "cudaEventRecord failed: %s", cudaGetErrorString(e));
     }
+    ev->recorded = !ctx->capturing;
     *out = ev.release();
     return TFB_OK;
 }
@@ -566,7 +679,7 @@ tfb_status tfb_event_elapsed_ms(tfb_event* start, tfb_event* stop, float* ms) {
 
 tfb_status tfb_event_destroy(tfb_event* ev) {
     if (!ev) return TFB_OK;
-    cudaEventDestroy(ev->ev);
+    give_event(ev->device, ev->ev, ev->recorded);
     delete ev;
     return TFB_OK;
 }

@@ -17,11 +17,8 @@
 // contraction.  Without a profiler attached the calls return at once; TFB_NVTX=0 removes them.
 struct NodeRange {
     bool on;
-    NodeRange(bool enabled, size_t step, size_t lhs, size_t rhs, bool fused) : on(enabled) {
-        if (!on) return;
-        char name[96];
-        snprintf(name, sizeof name, "tfb einsum node %zu: (%zu, %zu)%s", step, lhs, rhs, fused ? " + fused multiply" : "");
-        nvtxRangePushA(name);
+    NodeRange(bool enabled, const std::string& name) : on(enabled) {
+        if (on) nvtxRangePushA(name.c_str());
     }
     ~NodeRange() {
         if (on) nvtxRangePop();
@@ -44,6 +41,7 @@ struct tfb_subscripts {
 struct TreeStep {
     size_t lhs, rhs;                // operand ids; intermediates count from n_inputs
     std::vector<uint32_t> labels;   // labels of the result, in storage order
+    std::string name[2];            // of its range in a timeline, without and with a fused multiply
 };
 
 struct tfb_tree {
@@ -233,6 +231,9 @@ struct Builder {
         live.erase(y);
         size_t id = next_id++;
         live[id] = st.labels;
+        for (int fused = 0; fused < 2; ++fused)
+            st.name[fused] = "tfb einsum node " + std::to_string(tree->steps.size()) + ": (" + std::to_string(st.lhs) + ", " +
+                             std::to_string(st.rhs) + (fused ? ") + fused multiply" : ")");
         tree->steps.push_back(st);
         return id;
     }
@@ -462,10 +463,9 @@ tfb_status tfb_einsum_with_plan_into(tfb_ctx* ctx, const tfb_tree* tree, int32_t
     };
     std::map<size_t, Live> live;
     for (size_t i = 0; i < n; ++i) {
-        Live l;
+        Live& l = live[i];
         TFB_TRY(to_hview(operands[i], dtype, &l.view, "operand"));
         l.labels = tree->subs.inputs[i];
-        live[i] = l;
     }
     const char* used = nullptr;
     if (n == 1) {
@@ -498,17 +498,16 @@ tfb_status tfb_einsum_with_plan_into(tfb_ctx* ctx, const tfb_tree* tree, int32_t
     // operand instead of widening the contraction.
     auto presum = [&](size_t id, size_t partner) -> tfb_status {
         Live& l = live[id];
-        std::vector<uint32_t> keep;
-        bool drop = false;
-        for (auto lab : unique_of(l.labels)) {
-            bool needed = has(out_labels, lab);
+        auto needed = [&](uint32_t lab) {
+            if (has(live[partner].labels, lab) || has(out_labels, lab)) return true;
             for (auto& kv : live)
-                if (kv.first != id && has(unique_of(kv.second.labels), lab)) needed = true;
-            (void)partner;
-            if (needed) keep.push_back(lab);
-            else drop = true;
-        }
-        if (!drop) return TFB_OK;
+                if (kv.first != id && has(kv.second.labels, lab)) return true;
+            return false;
+        };
+        if (std::all_of(l.labels.begin(), l.labels.end(), needed)) return TFB_OK;
+        std::vector<uint32_t> keep;
+        for (auto lab : unique_of(l.labels))
+            if (needed(lab)) keep.push_back(lab);
         Live t;
         TFB_TRY(make_temp(keep, 0, &t));
         TFB_TRY(run_unary(ctx, dtype, l.labels, l.view, t.labels, t.view, one, zero, TFB_REDUCE_SUM, &used));
@@ -602,7 +601,7 @@ tfb_status tfb_einsum_with_plan_into(tfb_ctx* ctx, const tfb_tree* tree, int32_t
         Live& x = live[st.lhs];
         Live& y = live[st.rhs];
         const size_t c = last ? 0 : fusable_consumer(s, x, y);
-        NodeRange range(nvtx, s, st.lhs, st.rhs, c != 0);
+        NodeRange range(nvtx, st.name[c != 0]);
         if (last) {
             TFB_TRY(run_binary(ctx, dtype, x.labels, x.view, y.labels, y.view, out_labels, vout, a, b, 0, &used));
         } else if (c != 0) {

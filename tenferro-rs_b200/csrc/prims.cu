@@ -17,11 +17,11 @@ namespace tfb {
 
 // ------------------------------------------------------------------ mode lists
 void fuse_in_order(std::vector<Mode>& modes, int n_tensors) {
-    std::vector<Mode> out;
-    for (auto& m : modes) {
+    size_t n = 0;
+    for (const Mode m : modes) {
         if (m.extent == 1) continue;
-        if (!out.empty()) {
-            Mode& p = out.back();
+        if (n != 0) {
+            Mode& p = modes[n - 1];
             bool ok = true;
             for (int t = 0; t < n_tensors; ++t)
                 if (m.s[t] != p.s[t] * p.extent) ok = false;
@@ -30,19 +30,25 @@ void fuse_in_order(std::vector<Mode>& modes, int n_tensors) {
                 continue;
             }
         }
-        out.push_back(m);
+        modes[n++] = m;
     }
-    modes.swap(out);
+    modes.resize(n);
 }
-
 void sort_and_fuse(std::vector<Mode>& modes, int key, int n_tensors) {
     auto mag = [](int64_t v) { return v < 0 ? -v : v; };
-    std::stable_sort(modes.begin(), modes.end(), [&](const Mode& x, const Mode& y) {
+    // by insertion, which is stable and takes no memory: a handful of modes
+    auto before = [&](const Mode& x, const Mode& y) {
         // Stride 0 (broadcast) sorts last: it says nothing about locality.
         int64_t a = mag(x.s[key]), b = mag(y.s[key]);
         if ((a == 0) != (b == 0)) return b == 0;
         return a < b;
-    });
+    };
+    for (size_t i = 1; i < modes.size(); ++i) {
+        const Mode m = modes[i];
+        size_t j = i;
+        for (; j > 0 && before(m, modes[j - 1]); --j) modes[j] = modes[j - 1];
+        modes[j] = m;
+    }
     fuse_in_order(modes, n_tensors);
 }
 
@@ -212,9 +218,11 @@ tfb_status run_binary(tfb_ctx* ctx, int dtype, const std::vector<uint32_t>& labe
         p.mul = d->ptr;
         p.conj_mul = d->conj;
     }
-    std::set<uint32_t> seen;
+    std::vector<uint32_t> seen;
+    seen.reserve(la.labels.size() + lb.labels.size() + lc.labels.size());
     auto classify = [&](uint32_t l) -> tfb_status {
-        if (!seen.insert(l).second) return TFB_OK;
+        if (std::find(seen.begin(), seen.end(), l) != seen.end()) return TFB_OK;
+        seen.push_back(l);
         int ia = la.find(l), ib = lb.find(l), ic = lc.find(l), id = d ? ld.find(l) : -1;
         int64_t e = ia >= 0 ? la.extent[ia] : ib >= 0 ? lb.extent[ib] : lc.extent[ic];
         if (id >= 0 && ld.extent[id] != e)

@@ -145,6 +145,12 @@ class ContractionTree:
 
 
 @functools.lru_cache(maxsize=64)
+def view_array(n: int):
+    """The C array type of n operand views."""
+    return _lib.TfbView * max(n, 1)
+
+
+@functools.lru_cache(maxsize=64)
 def _computes_on_its_own(space_id: int) -> bool:
     devices = [d for d in preferred_compute_devices(LogicalMemorySpace.GpuMemory(space_id), OpKind.Contract) if d.kind == "cuda"]
     return bool(devices) and devices[0].device_id == space_id
@@ -180,16 +186,26 @@ def _select_context(operands: Sequence[Tensor], output: Optional[Tensor] = None)
 
 def einsum_with_plan_into(tree: ContractionTree, operands: Sequence[Tensor], alpha, beta, output: Tensor) -> None:
     """tenferro-einsum/src/lib.rs:584-621: output = alpha * einsum(operands) + beta * output."""
-    ctx = _select_context(operands, output)
-    dtype = output.dtype
+    dtype, space, keep = output.dtype, output._space, []
+    # One pass over the operands where all are of one space object and none is pinned, as nearly always.
+    plain, views = output._preferred is None, []
     for t in operands:
-        if t.dtype is not dtype and t.dtype != dtype:
-            raise InvalidArgument(f"operand dtype {t.dtype} differs from the output's {dtype}")
-    keep: list = []
-    views = (_lib.TfbView * max(len(operands), 1))(*[t.as_operand_view(keep) for t in operands])
-    out_view = output.as_operand_view(keep)
-    check(lib.tfb_einsum_with_plan_into(ctx.handle, tree.handle, dtype_code(dtype), len(operands), views,
-                                        scalar_arg(alpha, dtype), scalar_arg(beta, dtype), C.byref(out_view)))
+        if t._space is not space or t._preferred is not None or t.dtype is not dtype:
+            plain = False
+            break
+        views.append(t._view or t.as_operand_view(keep))
+    if plain and space.space_id is not None and _computes_on_its_own(space.space_id):
+        ctx = Context.get(space.space_id)
+    else:
+        ctx = _select_context(operands, output)
+        for t in operands:
+            if t.dtype is not dtype and t.dtype != dtype:
+                raise InvalidArgument(f"operand dtype {t.dtype} differs from the output's {dtype}")
+        views = [t.as_operand_view(keep) for t in operands]
+    n = len(views)
+    check(lib.tfb_einsum_with_plan_into(ctx.handle, tree.handle, dtype_code(dtype), n, view_array(n)(*views),
+                                        scalar_arg(alpha, dtype), scalar_arg(beta, dtype),
+                                        C.byref(output._view or output.as_operand_view(keep))))
     output.event = ctx.record_event()
 
 

@@ -35,6 +35,9 @@ DTYPES = {np.dtype("float32"): 0, np.dtype("float64"): 1, np.dtype("complex64"):
 
 
 def dtype_code(dt) -> int:
+    code = DTYPES.get(dt)
+    if code is not None:
+        return code
     dt = np.dtype(dt)
     if dt not in DTYPES:
         raise InvalidArgument(f"unsupported scalar type {dt}; Standard algebra covers f32, f64, Complex32, Complex64")
