@@ -11,16 +11,19 @@
 //   * a unit of work is one output tile (64 x 64 real, 32 x 32 complex); the host deals
 //     them out when the table is prepared, longest first, each to the CTA with the least work so
 //     far, so nothing is uploaded, sorted or drawn from a ticket per call;
-//   * a CTA walks its list in 16-deep k stages through a ring of cp.async stages that runs across
+//   * a CTA walks its list in 32-deep k stages through a ring of cp.async stages that runs across
 //     units: while one unit is computed and stored the next ones' operands are on their way;
 //   * f64 and Complex64 run on the FP64 tensor pipe (m16n8k8; four real products per complex one, so
 //     that Re and Im each keep their own accuracy), f32 and Complex32 as FMAs (exact products);
 //   * the four warps tile a unit as 2 x 2, 4 x 1 or 1 x 4 fragment blocks, whichever leaves the
 //     least padding, and dead blocks are not issued.
 // Measured against one thread-per-output tile drawn from an atomic ticket, the table uploaded per call:
-// 1024 f64 blocks with sides 4 .. 160 (41 MB, 128 MFLOP, floor 6 us of HBM) 159 -> 30 us a run, 3000 of
-// them 440 -> 88 us, f32 with such sides 183 -> 64 us; one-shot calls 122 -> 119 us (1024), 67 -> 58 us
-// (64).  What is left is latency: a third of the CTAs' time waits for the longest blocks' stages.
+// 1024 f64 blocks with sides 4 .. 160 (41 MB, 128 MFLOP, floor 6 us of HBM) 159 -> 25.6 us a run, 4096 of
+// them 82 us, f32 with such sides 183 -> 25 us.  What a table runs out of is issue slots and, while it is small, the longest
+// block's chain of stages: 32-deep stages, two of them, instead of 16-deep ones, three (64 blocks 16.5 -> 14.4 us, 1024 26.7 -> 25.6,
+// f32 28.4 -> 24.7), fetches worked out once a unit (64: 18.5 -> 16.5; 1024 with sides 16 .. 128 34.4 -> 31.2) and
+// one addition per stored element (1024: 30.9 -> 26.2, 4096: 101 -> 84).  Eight warps a CTA double the units' fixed instructions
+// (1024: 55.6 us).
 #include "common.h"
 #include "contract_common.cuh"
 #include "grouped_layout.h"
@@ -58,49 +61,88 @@ __device__ __forceinline__ void cp_async_one(uint32_t dst, const void* src, int 
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
 }
 
-// One operand's part of a stage: `rows` rows (row stride rs), k from `src` on (stride ks), `kv` <= 16 of
-// them live.  What lies past a live k is filled with zeros up to the next multiple of 8, which is
+// How this thread fetches its part of one operand's stages, worked out once per unit: what is left per stage is the copies and
+// the additions between them.  (Worked out for every stage, the strides read anew, it was most of a stage's 480 instructions a warp
+// where units are small, and issue slots are what such a table runs out of: ncu, 1024 f64 blocks, 37 % of them in use at 2.8 warps a
+// scheduler, 10 % of DRAM.)
+// A stage is up to 32 of K; what lies past a live k is filled with zeros up to the next multiple of 8, which is
 // as far as the arithmetic reads; rows past the live ones may hold anything, nothing stored
 // depends on them (V > 1: a chunk's dead part is zero-filled).
-template <typename T, int V>
-__device__ __forceinline__ void load_operand(uint32_t dst, const T* src, int64_t rs, int64_t ks, int rows, int kv, bool kfast,
-                                             int tid) {
+template <typename T>
+struct OperandFeed {
     using Cfg = GroupCfg<T>;
-    constexpr int ES = (int)sizeof(T);
-    const int kr = (kv + 7) & ~7;
-    if (kfast) {
-        constexpr int KC = kGroupK / V;
-        const int k = (tid % KC) * V;
-        if (k >= kr) return;
-        const int live = min(max(kv - k, 0), V) * ES;
-        const T* p = src + (live ? (int64_t)k * ks : 0) + (int64_t)(tid / KC) * rs;
-        uint32_t d = dst + ((tid / KC) * Cfg::PK + k) * ES;
-        for (int r = tid / KC; r < rows; r += kGroupThreads / KC) {
-            if constexpr (V == 1) cp_async_one<ES>(d, p, live);
-            else cp_async_part(d, p, live);
-            p += (kGroupThreads / KC) * rs;
-            d += (kGroupThreads / KC) * Cfg::PK * ES;
+    static constexpr int ES = (int)sizeof(T), VEC = 16 / ES;
+    const T* p;        // this thread's first element of the next stage
+    const T* corner;   // a valid address for copies of nothing
+    int64_t step, adv; // elements from one of its copies to the next, from a stage to the next
+    uint32_t off;      // of the first one inside the operand's part of a stage
+    int dstep;         // bytes between them
+    int n;             // k fast: copies of a stage.  Row fast: 0 or 1, whether it has any
+    int k, kstep;      // k of the first copy, from one to the next (row fast)
+    int live;          // bytes of a copy (row fast)
+    bool kfast, vec;
+
+    // `rows` rows with row stride rs, k with stride ks.
+    __device__ __forceinline__ void set(const T* src, int64_t rs, int64_t ks, int rows, bool is_kfast, bool is_vec, int tid) {
+        const int V = VEC > 1 && is_vec ? VEC : 1;
+        corner = src;
+        kfast = is_kfast;
+        vec = is_vec;
+        adv = kGroupK * ks;
+        int r;
+        if (kfast) {
+            const int kc = kGroupK / V, per = kGroupThreads / kc;
+            r = tid / kc;
+            k = (tid - r * kc) * V;
+            n = r < rows ? (rows - r + per - 1) / per : 0;
+            step = per * rs;
+            off = (uint32_t)((r * Cfg::PK + k) * ES);
+            dstep = per * Cfg::PK * ES;
+        } else {
+            // a power-of-two group of threads along the rows
+            const int chunks = (rows + V - 1) / V;
+            int lg = 2;
+            while ((1 << lg) < chunks) ++lg;
+            const int x = tid & ((1 << lg) - 1);
+            r = x * V;
+            k = tid >> lg;
+            kstep = kGroupThreads >> lg;
+            n = x < chunks;
+            live = min(rows - r, V) * ES;
+            step = kstep * ks;
+            off = (uint32_t)((k * Cfg::PM + r) * ES);
+            dstep = kstep * Cfg::PM * ES;
         }
-    } else {
-        // a power-of-two group of threads along the rows
-        const int chunks = (rows + V - 1) / V;
-        int lg = 2;
-        while ((1 << lg) < chunks) ++lg;
-        const int x = tid & ((1 << lg) - 1), step = kGroupThreads >> lg;
-        if (x >= chunks) return;
-        const int live = min(rows - x * V, V) * ES;
-        int k = tid >> lg;
-        const T* p = src + (int64_t)x * V * rs + (int64_t)k * ks;
-        uint32_t d = dst + (k * Cfg::PM + x * V) * ES;
-        for (; k < kr; k += step) {
-            const bool ok = k < kv;
-            if constexpr (V == 1) cp_async_one<ES>(d, ok ? p : src, ok ? live : 0);
-            else cp_async_part(d, ok ? p : src, ok ? live : 0);
-            p += step * ks;
-            d += step * Cfg::PM * ES;
+        p = src + r * rs + k * ks;
+    }
+    template <int V>
+    __device__ __forceinline__ void copies(uint32_t d, int kv) {
+        const int kr = (kv + 7) & ~7;
+        auto copy = [&](const T* q, int bytes) {
+            if constexpr (V == 1) cp_async_one<ES>(d, q, bytes);
+            else cp_async_part(d, q, bytes);
+            d += dstep;
+        };
+        if (kfast) {
+            if (k >= kr) return;
+            const int bytes = min(max(kv - k, 0), V) * ES;
+            const T* q = bytes ? p : corner;
+            const int64_t s = bytes ? step : 0;
+#pragma unroll 4
+            for (int i = 0; i < n; ++i, q += s) copy(q, bytes);
+        } else if (n) {
+            const T* q = p;
+#pragma unroll 4
+            for (int kk = k; kk < kr; kk += kstep, q += step) copy(kk < kv ? q : corner, kk < kv ? live : 0);
         }
     }
-}
+    // The next stage, `kv` <= 32 of K live.
+    __device__ __forceinline__ void stage(uint32_t dst, int kv) {
+        if (VEC > 1 && vec) copies<VEC>(dst + off, kv);
+        else copies<1>(dst + off, kv);
+        p += adv;
+    }
+};
 
 __device__ __forceinline__ void group_dmma(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
     asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
@@ -188,25 +230,33 @@ struct TensorPath {
     }
     __device__ __forceinline__ void store(const GroupUnit& u, T alpha, T beta, bool read_c, int tid) {
         const int g = (tid & 31) >> 2, t = tid & 3;
-        T* C = reinterpret_cast<T*>(u.c);
+        // a thread's rows are eight apart, its columns two neighbours of every eight: one addition an element
+        const int m0 = wm + g, n0 = wn + 2 * t, rows = ((int)u.mt - m0 + 7) >> 3;
+        const int64_t row8 = 8 * u.c_rs, cs = u.c_cs;
+        T* col = reinterpret_cast<T*>(u.c) + m0 * u.c_rs + n0 * cs;
 #pragma unroll
-        for (int i = 0; i < Cfg::NI; ++i)
+        for (int j = 0; j < Cfg::NJ; ++j) {
+            if (j < nj) {
 #pragma unroll
-            for (int j = 0; j < Cfg::NJ; ++j) {
-                if (i >= ni || j >= nj) continue;
+                for (int e = 0; e < 2; ++e) {
+                    if (n0 + 8 * j + e < u.nt) {
+                        T* p = col + e * cs;
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int m = wm + 16 * i + 8 * (e >> 1) + g, n = wn + 8 * j + 2 * t + (e & 1);
-                    if (m >= u.mt || n >= u.nt) continue;
-                    T* p = C + m * u.c_rs + n * u.c_cs;
-                    T x;
-                    if constexpr (CPLX) x = make_double2(acc[i][j][0][e], acc[i][j][1][e]);
-                    else x = acc[i][j][0][e];
-                    T v = Ops<T>::mul(alpha, x);
-                    if (read_c) v = Ops<T>::add(v, Ops<T>::mul(beta, *p));
-                    *p = v;
+                        for (int r = 0; r < 2 * Cfg::NI; ++r, p += row8) {
+                            if (r < 2 * ni && r < rows) {
+                                T x;
+                                if constexpr (CPLX) x = make_double2(acc[r >> 1][j][0][2 * (r & 1) + e], acc[r >> 1][j][1][2 * (r & 1) + e]);
+                                else x = acc[r >> 1][j][0][2 * (r & 1) + e];
+                                T v = Ops<T>::mul(alpha, x);
+                                if (read_c) v = Ops<T>::add(v, Ops<T>::mul(beta, *p));
+                                *p = v;
+                            }
+                        }
+                    }
                 }
+                col += 8 * cs;
             }
+        }
     }
 };
 
@@ -252,20 +302,21 @@ struct FmaPath {
 #undef TFB_CALL
     }
     __device__ __forceinline__ void store(const GroupUnit& u, T alpha, T beta, bool read_c, int tid) {
-        T* C = reinterpret_cast<T*>(u.c);
-        const int tx = tid & 15, ty = tid >> 4;
+        const int tx = tid & 15, ty = tid >> 4, rows = ((int)u.mt - tx + 15) >> 4;
+        const int64_t row16 = 16 * u.c_rs, col8 = 8 * u.c_cs;
+        T* col = reinterpret_cast<T*>(u.c) + tx * u.c_rs + ty * u.c_cs;
 #pragma unroll
-        for (int j = 0; j < Cfg::NJ; ++j) {
-            const int n = ty + 8 * j;
-            if (n >= u.nt) continue;
+        for (int j = 0; j < Cfg::NJ; ++j, col += col8) {
+            if (ty + 8 * j < u.nt) {
+                T* p = col;
 #pragma unroll
-            for (int i = 0; i < Cfg::NI; ++i) {
-                const int m = tx + 16 * i;
-                if (m >= u.mt) continue;
-                T* p = C + m * u.c_rs + n * u.c_cs;
-                T v = Ops<T>::mul(alpha, acc[i][j]);
-                if (read_c) v = Ops<T>::add(v, Ops<T>::mul(beta, *p));
-                *p = v;
+                for (int i = 0; i < Cfg::NI; ++i, p += row16) {
+                    if (i < rows) {
+                        T v = Ops<T>::mul(alpha, acc[i][j]);
+                        if (read_c) v = Ops<T>::add(v, Ops<T>::mul(beta, *p));
+                        *p = v;
+                    }
+                }
             }
         }
     }
@@ -290,24 +341,26 @@ __global__ void __launch_bounds__(kGroupThreads, GroupCfg<T>::CTAS) grouped_unit
     cp_async_wait<0>();
     __syncthreads();
 
-    // The next stage to request: unit pu, from k = pk on.  At most S - 1 units ahead of the unit being
+    // The next stage to request: unit pu, `left` of its K.  At most S - 1 units ahead of the unit being
     // computed, so its record is in the shared window of kGroupRecs.
-    int pu = 0;
-    int64_t pk = 0;
+    int pu = 0, pk = 0;  // (pk: whether it has begun)
+    int64_t left = 0;
+    OperandFeed<T> feed_a, feed_b;
     auto request = [&](int slot) {
         if (pu < n_units) {
-            const GroupUnit& u = recs[pu % kGroupRecs];
-            const int kv = (int)min((int64_t)kGroupK, u.k - pk);
+            if (pk == 0) {
+                const GroupUnit& u = recs[pu % kGroupRecs];
+                left = u.k;
+                feed_a.set(reinterpret_cast<const T*>(u.a), u.a_rs, u.a_cs, u.mt, u.shape & kAFast, u.shape & kAVec, tid);
+                feed_b.set(reinterpret_cast<const T*>(u.b), u.b_cs, u.b_rs, u.nt, u.shape & kBFast, u.shape & kBVec, tid);
+            }
+            const int kv = (int)min((int64_t)kGroupK, left);
             const uint32_t da = ring_addr + slot * Sm::STAGE, db = da + Sm::ELEMS * (int)sizeof(T);
-            const T* a = reinterpret_cast<const T*>(u.a) + pk * u.a_cs;
-            const T* b = reinterpret_cast<const T*>(u.b) + pk * u.b_rs;
-            constexpr int V = 16 / (int)sizeof(T);
-            if (V > 1 && (u.shape & kAVec)) load_operand<T, V>(da, a, u.a_rs, u.a_cs, u.mt, kv, u.shape & kAFast, tid);
-            else load_operand<T, 1>(da, a, u.a_rs, u.a_cs, u.mt, kv, u.shape & kAFast, tid);
-            if (V > 1 && (u.shape & kBVec)) load_operand<T, V>(db, b, u.b_cs, u.b_rs, u.nt, kv, u.shape & kBFast, tid);
-            else load_operand<T, 1>(db, b, u.b_cs, u.b_rs, u.nt, kv, u.shape & kBFast, tid);
-            pk += kGroupK;
-            if (pk >= u.k) {
+            feed_a.stage(da, kv);
+            feed_b.stage(db, kv);
+            pk = 1;
+            left -= kGroupK;
+            if (left <= 0) {
                 pk = 0;
                 ++pu;
             }

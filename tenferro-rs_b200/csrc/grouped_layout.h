@@ -8,7 +8,7 @@
 
 namespace tfb {
 
-constexpr int kGroupK = 16;     // depth of a stage
+constexpr int kGroupK = 32;     // depth of a stage
 constexpr int kGroupRecs = 16;  // unit records a CTA holds in shared memory
 
 // One output tile of one problem: pointers already moved to the tile's corner.
@@ -32,10 +32,10 @@ static_assert(sizeof(GroupUnit) % 16 == 0, "records travel as 16-byte chunks");
 // banks.  CTAS x STAGES x tile fill an SM's shared memory.
 template <typename T>
 struct GroupCfg;
-template <> struct GroupCfg<double>  { static constexpr int TILE = 64, PK = 20, PM = 68, STAGES = 3, CTAS = 3, NI = 2, NJ = 4; };
-template <> struct GroupCfg<double2> { static constexpr int TILE = 32, PK = 20, PM = 34, STAGES = 3, CTAS = 3, NI = 2, NJ = 2; };
-template <> struct GroupCfg<float>   { static constexpr int TILE = 64, PK = 20, PM = 68, STAGES = 4, CTAS = 4, NI = 4, NJ = 8; };
-template <> struct GroupCfg<float2>  { static constexpr int TILE = 32, PK = 20, PM = 36, STAGES = 4, CTAS = 4, NI = 2, NJ = 4; };
+template <> struct GroupCfg<double>  { static constexpr int TILE = 64, PK = 36, PM = 68, STAGES = 2, CTAS = 3, NI = 2, NJ = 4; };
+template <> struct GroupCfg<double2> { static constexpr int TILE = 32, PK = 36, PM = 34, STAGES = 2, CTAS = 3, NI = 2, NJ = 2; };
+template <> struct GroupCfg<float>   { static constexpr int TILE = 64, PK = 36, PM = 68, STAGES = 3, CTAS = 4, NI = 4, NJ = 8; };
+template <> struct GroupCfg<float2>  { static constexpr int TILE = 32, PK = 36, PM = 36, STAGES = 3, CTAS = 4, NI = 2, NJ = 4; };
 
 // Host buffers of the layout below, kept per thread: a one-shot call would spend as long faulting fresh
 // pages in as on the layout itself.  Given back above kKeep bytes.

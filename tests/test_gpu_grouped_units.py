@@ -1,6 +1,6 @@
 """The grouped product's general kernel (double precision, complex, and every f32 table the two
 tensor-core kernels decline): sizes around the edges of its output tiles (64 real, 32 complex),
-stage depth (16) and MMA steps (8), stored column- or row-major, back to back or aligned, against
+stage depth (32) and MMA steps (8), stored column- or row-major, back to back or aligned, against
 the host product in double precision.
 
 The bound is the standard one of a dot product, component by component: K + 4 roundings of
@@ -115,3 +115,12 @@ def test_strides(tb, oracle, dtype, beta):
         rest = np.ones(out.size, bool)
         rest[ic] = False
         assert np.array_equal(out[rest], fc[rest])
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.complex64, np.complex128])
+@pytest.mark.parametrize("layout", ["CCF", "FFC"])
+def test_edges_of_deeper_stages(tb, oracle, dtype, layout, monkeypatch):
+    """K around one, two and three stages of 32, with sides that leave warps and lanes without a part."""
+    sizes = [(20, 20, 31), (20, 21, 33), (64, 64, 63), (65, 30, 64), (33, 65, 65), (16, 16, 95), (9, 70, 96), (70, 9, 97), (1, 64, 32), (64, 1, 34)]
+    monkeypatch.setitem(globals(), "SIZES", sizes)
+    test_grouped_units(tb, oracle, dtype, layout, 3, 0.5)
