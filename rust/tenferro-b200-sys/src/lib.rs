@@ -192,6 +192,7 @@ extern "C" {
     pub fn tfb_graph_launch(graph: *mut tfb_graph) -> tfb_status;
     pub fn tfb_graph_destroy(graph: *mut tfb_graph);
     pub fn tfb_event_record(ctx: *mut tfb_ctx, out: *mut *mut tfb_event) -> tfb_status;
+    pub fn tfb_event_record_completion(ctx: *mut tfb_ctx, out: *mut *mut tfb_event) -> tfb_status;
     pub fn tfb_event_wait(ctx: *mut tfb_ctx, ev: *mut tfb_event) -> tfb_status;
     pub fn tfb_event_synchronize(ev: *mut tfb_event) -> tfb_status;
     pub fn tfb_event_query(ev: *mut tfb_event, ready: *mut c_int) -> tfb_status;

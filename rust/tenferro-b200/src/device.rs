@@ -82,7 +82,7 @@ impl Context {
     pub fn record_event(&self) -> Result<CompletionEvent> {
         let mut ev = core::ptr::null_mut();
         // SAFETY: valid context and out-pointer.
-        check(unsafe { sys::tfb_event_record(self.raw, &mut ev) })?;
+        check(unsafe { sys::tfb_event_record_completion(self.raw, &mut ev) })?;
         Ok(CompletionEvent { raw: ev })
     }
 

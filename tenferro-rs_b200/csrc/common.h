@@ -116,6 +116,7 @@ struct tfb_event {
     cudaEvent_t ev = nullptr;
     int device = 0;
     bool recorded = false;  // (not while its context was capturing)
+    bool timed = true;
 };
 
 namespace tfb {

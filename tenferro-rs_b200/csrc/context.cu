@@ -50,33 +50,33 @@ Scalar load_scalar(int dtype, const void* p) {
 
 // Events that nobody holds any more, for the next one recorded on their device: every call records one, and creating and destroying it
 // takes as long as the record.  A wait that has been enqueued for one keeps its meaning when the event is recorded anew.  Only events that
-// were recorded come here (one that was not reads as complete until it is), 64 a device, given back with a context of it.
+// were recorded come here (one that was not reads as complete until it is), 64 a device and kind, given back with a context of it.
 struct IdleEvents {
     std::mutex mu;
-    std::map<int, std::vector<cudaEvent_t>> of;
+    std::map<int, std::vector<cudaEvent_t>> of;  // 2 * device + whether they take the time
 };
 static IdleEvents& idle_events() {
     static IdleEvents* e = new IdleEvents;  // outlives whoever destroys an event at exit
     return *e;
 }
-static cudaError_t take_event(int device, cudaEvent_t* ev) {
+static cudaError_t take_event(int device, bool timed, cudaEvent_t* ev) {
     {
         IdleEvents& e = idle_events();
         std::lock_guard<std::mutex> lock(e.mu);
-        auto& v = e.of[device];
+        auto& v = e.of[2 * device + timed];
         if (!v.empty()) {
             *ev = v.back();
             v.pop_back();
             return cudaSuccess;
         }
     }
-    return cudaEventCreate(ev);
+    return cudaEventCreateWithFlags(ev, timed ? cudaEventDefault : cudaEventDisableTiming);
 }
-static void give_event(int device, cudaEvent_t ev, bool recorded) {
+static void give_event(int device, bool timed, cudaEvent_t ev, bool recorded) {
     if (recorded) {
         IdleEvents& e = idle_events();
         std::lock_guard<std::mutex> lock(e.mu);
-        auto& v = e.of[device];
+        auto& v = e.of[2 * device + timed];
         if (v.size() < 64) {
             v.push_back(ev);
             return;
@@ -89,7 +89,10 @@ static void drop_idle_events(int device) {
     {
         IdleEvents& e = idle_events();
         std::lock_guard<std::mutex> lock(e.mu);
-        all.swap(e.of[device]);
+        all.swap(e.of[2 * device]);
+        auto& timed = e.of[2 * device + 1];
+        all.insert(all.end(), timed.begin(), timed.end());
+        timed.clear();
     }
     for (cudaEvent_t ev : all) cudaEventDestroy(ev);
 }
@@ -622,12 +625,13 @@ tfb_status tfb_host_free(void* ptr) {
     return TFB_OK;
 }
 
-tfb_status tfb_event_record(tfb_ctx* ctx, tfb_event** out) {
+static tfb_status record_event(tfb_ctx* ctx, bool timed, tfb_event** out) {
     if (!ctx || !out) return fail(TFB_ERR_INVALID_ARGUMENT, "tfb_event_record: NULL argument");
     DeviceGuard g(ctx->device);
     std::unique_ptr<tfb_event> ev(new tfb_event);
     ev->device = ctx->device;
-    TFB_CUDA(take_event(ctx->device, &ev->ev));
+    ev->timed = timed;
+    TFB_CUDA(take_event(ctx->device, timed, &ev->ev));
     // While the context is capturing nothing is enqueued, so there is nothing to mark: the event stays
     // unrecorded, which reads as complete (an event recorded into the capture could be neither
     // queried nor waited for from outside it).
@@ -640,6 +644,9 @@ tfb_status tfb_event_record(tfb_ctx* ctx, tfb_event** out) {
     *out = ev.release();
     return TFB_OK;
 }
+
+tfb_status tfb_event_record(tfb_ctx* ctx, tfb_event** out) { return record_event(ctx, true, out); }
+tfb_status tfb_event_record_completion(tfb_ctx* ctx, tfb_event** out) { return record_event(ctx, false, out); }
 
 tfb_status tfb_event_wait(tfb_ctx* ctx, tfb_event* ev) {
     if (!ctx || !ev) return fail(TFB_ERR_INVALID_ARGUMENT, "tfb_event_wait: NULL argument");
@@ -673,13 +680,15 @@ tfb_status tfb_event_query(tfb_event* ev, int* ready) {
 
 tfb_status tfb_event_elapsed_ms(tfb_event* start, tfb_event* stop, float* ms) {
     if (!start || !stop || !ms) return fail(TFB_ERR_INVALID_ARGUMENT, "tfb_event_elapsed_ms: NULL argument");
+    if (!start->timed || !stop->timed)
+        return fail(TFB_ERR_INVALID_ARGUMENT, "tfb_event_elapsed_ms: a call's completion event carries no time; record one with tfb_event_record");
     TFB_CUDA(cudaEventElapsedTime(ms, start->ev, stop->ev));
     return TFB_OK;
 }
 
 tfb_status tfb_event_destroy(tfb_event* ev) {
     if (!ev) return TFB_OK;
-    give_event(ev->device, ev->ev, ev->recorded);
+    give_event(ev->device, ev->timed, ev->ev, ev->recorded);
     delete ev;
     return TFB_OK;
 }

@@ -102,6 +102,7 @@ PROTOTYPES = {
     "tfb_graph_destroy": (None, [_VP]),
     "tfb_probe_mma_issue_cycles": (C.c_int, [_VP, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "tfb_event_record": (C.c_int, [_VP, _VPP]),
+    "tfb_event_record_completion": (C.c_int, [_VP, _VPP]),
     "tfb_event_wait": (C.c_int, [_VP, _VP]),
     "tfb_event_synchronize": (C.c_int, [_VP]),
     "tfb_event_query": (C.c_int, [_VP, C.POINTER(C.c_int)]),

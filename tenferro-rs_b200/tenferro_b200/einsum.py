@@ -206,7 +206,7 @@ def einsum_with_plan_into(tree: ContractionTree, operands: Sequence[Tensor], alp
     check(lib.tfb_einsum_with_plan_into(ctx.handle, tree.handle, dtype_code(dtype), n, view_array(n)(*views),
                                         scalar_arg(alpha, dtype), scalar_arg(beta, dtype),
                                         C.byref(output._view or output.as_operand_view(keep))))
-    output.event = ctx.record_event()
+    output.event = ctx.completion()
 
 
 class PreparedEinsum:

@@ -233,7 +233,7 @@ class CudaBackend:
         a = scalar_arg(alpha, plan.dtype)
         b = scalar_arg(beta, plan.dtype)
         check(lib.tfb_execute(plan.handle, a, len(inputs), views, b, C.byref(out_view)))
-        output.event = ctx.record_event()
+        output.event = ctx.completion()
 
     @staticmethod
     def has_extension_for(dtype, ext: Extension, algebra: Algebra = Algebra.Standard) -> bool:
@@ -307,4 +307,4 @@ def reduce_static(modes_a, a: Tensor, modes_c, c: Tensor, op: ReduceOp = ReduceO
     mc = (C.c_uint32 * max(len(modes_c), 1))(*[int(m) for m in modes_c])
     check(lib.tfb_reduce_static(ctx.handle, dtype_code(c.dtype), int(op), ma, len(modes_a), C.byref(va), mc,
                                 len(modes_c), C.byref(vc), scalar_arg(alpha, c.dtype), scalar_arg(beta, c.dtype)))
-    c.event = ctx.record_event()
+    c.event = ctx.completion()

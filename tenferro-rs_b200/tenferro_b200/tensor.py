@@ -175,7 +175,7 @@ class Tensor:
             t._block.array(np.uint8)[:] = 0
             return t
         t._block.ctx.memset(t._block.ptr, 0, t._block.nbytes)
-        t.event = t._block.ctx.record_event()
+        t.event = t._block.ctx.completion()
         return t
 
     @classmethod
@@ -408,7 +408,7 @@ class Tensor:
             dctx = dst.ctx
             if self.len():
                 dctx.h2d(dst._block.ptr, C.c_void_p(self._block.ptr), self.len() * self.dtype.itemsize)
-            dst.event = dctx.record_event()
+            dst.event = dctx.completion()
             self._block.event = dst.event  # the staging buffer is busy until the copy has read it
             dst._conj = self._conj
             dst._keepalive = self
@@ -424,18 +424,18 @@ class Tensor:
             if nbytes:
                 sctx.d2h(C.c_void_p(block.ptr), src_ptr, nbytes)
             dst = Tensor(block, src._dims, contiguous_strides(src._dims, order), 0, src.dtype, target, conj=src._conj)
-            dst.event = sctx.record_event()
+            dst.event = sctx.completion()
             dst._keepalive = src
             return dst
         dst = Tensor.empty(src._dims, src.dtype, target, order)
         dctx = dst.ctx
         # the copy runs on the destination's stream: it must come after the latest write to the
         # source buffer, whichever view of it that write went through
-        ev = src.event if src.event is not None else src.ctx.record_event()
+        ev = src.event if src.event is not None else src.ctx.completion()
         dctx.wait_event(ev)
         check(lib.tfb_memcpy_p2p_async(dctx.handle, C.c_void_p(dst._block.ptr), target.space_id,
                                        C.c_void_p(src_ptr), src._space.space_id, nbytes))
-        dst.event = dctx.record_event()
+        dst.event = dctx.completion()
         dst._conj = src._conj
         dst._keepalive = src  # the source block must outlive the copy
         return dst
