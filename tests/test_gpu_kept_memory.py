@@ -1,0 +1,73 @@
+"""What a context keeps from one call to the next: working memory and completion events."""
+import os
+
+import numpy as np
+import pytest
+
+from conftest import random_array
+
+pytestmark = pytest.mark.gpu
+
+
+def call(tb, a, b, c, ctx):
+    plan = tb.CudaBackend.plan(tb.PrimDescriptor.Contract([0, 1], [1, 2], [0, 2]), [a.dims(), b.dims(), c.dims()], np.float64, ctx=ctx)
+    tb.CudaBackend.execute(plan, 1.0, [a, b], 0.0, c)
+
+
+@pytest.mark.parametrize("cap", [None, 64 << 20])
+def test_kept_memory_is_free_and_gives_way(tb, oracle, cap):
+    """Products of several sizes with their working memory, which the statistics count as free; a capped pool
+    then still hands out nearly all that it may hold."""
+    if cap:
+        os.environ["TFB_POOL_BYTES"] = str(cap)
+    try:
+        ctx = tb.Context(0)
+    finally:
+        os.environ.pop("TFB_POOL_BYTES", None)
+    rng = np.random.default_rng(91)
+    for n, k in [(64, 4096), (128, 5000), (63, 8191), (64, 4096), (200, 3000)]:
+        a, b = random_array(rng, (n, k), np.float64), random_array(rng, (k, n), np.float64)
+        ta, tb_, c = tb.Tensor.from_numpy(a), tb.Tensor.from_numpy(b), tb.Tensor.zeros((n, n))
+        tb.Context.get(0).synchronize()
+        for _ in range(3):
+            call(tb, ta, tb_, c, ctx)
+        ctx.synchronize()
+        assert oracle.rel_frobenius(c.to_numpy(), a @ b) <= 1e-12
+        assert ctx.pool_stats()[1] == 0
+    if cap:
+        most = ctx.alloc(cap - (2 << 20))  # past what is left unless the kept blocks go back
+        ctx.free(most)
+        ctx.synchronize()
+
+
+def test_blocks_of_two_contexts_stay_apart(tb, oracle):
+    """Calls of two contexts in turn, nothing waited for between them: neither is given memory that the other still uses."""
+    rng = np.random.default_rng(92)
+    ctxs = [tb.Context(0), tb.Context(0)]
+    ab = [(random_array(rng, (64, 6000), np.float64), random_array(rng, (6000, 64), np.float64)) for _ in range(2)]
+    dev = [(tb.Tensor.from_numpy(a), tb.Tensor.from_numpy(b), tb.Tensor.zeros((64, 64))) for a, b in ab]
+    tb.Context.get(0).synchronize()
+    for _ in range(20):
+        for ctx, (a, b, c) in zip(ctxs, dev):
+            call(tb, a, b, c, ctx)
+    for ctx, (a, b), (_, _, c) in zip(ctxs, ab, dev):
+        ctx.synchronize()
+        assert oracle.rel_frobenius(c.to_numpy(), a @ b) <= 1e-12
+
+
+def test_events_of_calls_and_timed_events(tb):
+    """A call's event says when it is ready and is reused without carrying a time; recorded events still do."""
+    ctx = tb.Context.get(0)
+    a = tb.Tensor.from_numpy(np.ones((256, 256)))
+    start = ctx.record_event()
+    outs = [tb.einsum("ij,jk->ik", [a, a]) for _ in range(40)]
+    stop = ctx.record_event()
+    ctx.synchronize()
+    assert all(o.is_ready() for o in outs)
+    assert start.elapsed_ms(stop) > 0
+    with pytest.raises(tb.InvalidArgument):
+        outs[0].event.elapsed_ms(outs[1].event)
+    del outs  # their events go back; the next ones are not ready before their work is
+    again = tb.einsum("ij,jk->ik", [a, a])
+    again.wait()
+    assert again.is_ready() and np.array_equal(again.to_numpy(), np.full((256, 256), 256.0))
